@@ -144,11 +144,11 @@ int hm_debug_fail_allocations_after(long long n);
  * 1 = its higher-id neighbours, read straight from the id-sorted rows (what
  * pooled server stores use). Counts are the same either way; tests run both. */
 int hm_debug_touch_orientation(hm_graph* g, int by_id);
-/* Walk of the static count on graph g: 1 (the default) walks oriented rows
- * grouped by the member each neighbour shares with the row owner, and counts
- * the triangles of a pair sharing one member u through the neighbours that
- * share only u by the group's size counts instead of visiting them; 0 visits
- * every oriented entry. Counts are the same either way; tests run both. */
+/* Method of the static count on graph g: 1 (the default) counts the triangles
+ * of pairs sharing one member in closed form and enumerates only those with two
+ * or three pairs sharing more, where that is the cheaper way, else walks
+ * oriented rows grouped by the member each neighbour shares with the row owner;
+ * 0 visits every oriented entry. Counts are the same every way; tests run them. */
 int hm_debug_static_groups(hm_graph* g, int on);
 
 /* ---- the device store ------------------------------------------------- */
@@ -390,8 +390,8 @@ int hm_graph_autotune(hm_graph* g, uint32_t sample_stride, hm_tune_report* repor
 /* Device times of the last count / update call on this graph (CUDA events
  * on the context stream). */
 typedef struct hm_timings_t {
-  float open_ms;     /* open-pair phase of the static count */
-  float closed_ms;   /* closed-triangle phase of the static count */
+  float open_ms;     /* open-pair phase of the static count (0 when both phases run side by side) */
+  float closed_ms;   /* closed-triangle phase of the static count, or both phases */
   float count_ms;    /* whole static count */
   float update_ms;   /* last batch update */
   float temporal_ms; /* last temporal count */

@@ -98,7 +98,8 @@ extern "C" int hm_graph_info(const hm_graph* g, hm_graph_info_t* info) {
   info->n_nodes = g->n_nodes;
   info->n_members = g->h2v_nnz;
   info->n_adjacent = g->h2h_nnz;
-  info->n_oriented = g->plus_valid ? g->plus_nnz : 0;
+  // every adjacent pair is oriented one way, whichever count has looked at them
+  info->n_oriented = g->plus_valid ? g->plus_nnz : g->decomp.decided ? g->h2h_nnz / 2 : 0;
   info->device_bytes = g->ctx->used.load();
   info->temporal = g->temporal ? 1 : 0;
   return HM_OK;

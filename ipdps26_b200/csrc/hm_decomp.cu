@@ -1,0 +1,1832 @@
+// The static count by decomposition: light pairs are counted, not visited.
+//
+// Call a pair of adjacent hyperedges heavy when it shares two or more members
+// and light when it shares one. On the named workloads 85 to 99.9 % of the
+// adjacent pairs are light, and a light pair is fully described by its one
+// shared node, so triangles with at most one heavy pair have closed forms:
+//
+//   three light pairs   the three share one node u (a star: choose 3 of u's
+//                       hyperedges), or the pairs use three distinct nodes
+//                       x, y, z (choose one hyperedge per node pair: triangles
+//                       of the node graph weighted by W(x, y), the number of
+//                       hyperedges holding both x and y);
+//   heavy pair (a, b)   with S = a & b: the third hyperedge meets a | b in one
+//                       node of S (the hyperedges of that node), or in one
+//                       node of a \ S and one of b \ S (the sum of W over
+//                       those node pairs).
+//
+// Each form counts hyperedge triples with multiplicity, and every surplus
+// comes from a triple with two or three heavy pairs (or from one hyperedge
+// used twice), so those are the only triangles enumerated: a triangle with
+// overlaps C and triple overlap g has
+//   R = C_ab C_bc C_ca - g (C_ab + C_bc + C_ca) + 2 g
+// ways to pick three distinct nodes, one per pair, and each heavy pair (x, y)
+// of it with third hyperedge z is met (C_xz - g)(C_yz - g) times by the second
+// heavy form and g times by the first. All sums are exact in uint64 modulo
+// 2^64. The classes follow MoCHy's (MoCHy-master/motif_id.cpp:5-34) because
+// every form fixes which of the seven regions are empty from the sizes alone.
+//
+// What is enumerated: for centre a (the lower-ranked end, by (degree, id), of
+// the pair {a, c}), every heavy neighbour b of a and every heavy neighbour c
+// of b ranked above a, tested against a's row. That is sum_b h(b)^2 / 2 tests,
+// h the heavy degree, against sum_{(a, b)} d+(b) oriented entries in the
+// enumeration of all triangles (hm_static.cu).
+#include <cub/cub.cuh>
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "hm_classes.h"
+#include "hm_device.h"
+#include "hm_pairs.cuh"
+
+namespace hm {
+namespace {
+
+constexpr unsigned kWarp = 32;
+constexpr unsigned kBlock = 256;
+constexpr unsigned kWarps = kBlock / kWarp;
+constexpr uint32_t kEmpty = 0xffffffffu;
+
+__device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
+__device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
+__device__ __forceinline__ uint64_t gtid() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ uint64_t gstride() { return (uint64_t)gridDim.x * blockDim.x; }
+__device__ __forceinline__ uint64_t global_warp() { return gtid() >> 5; }
+__device__ __forceinline__ uint64_t n_warps() { return gstride() >> 5; }
+
+__device__ __forceinline__ uint64_t warp_sum(uint64_t v) {
+  for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
+// Size category: 0 for |x| = 1, 1 for |x| = 2, 2 for |x| >= 3.
+__device__ __forceinline__ uint32_t size_cat(uint32_t s) { return s >= 3 ? 2u : s - 1u; }
+
+// ---- raw sums of one count (u64 each) ---------------------------------------------
+// Stars by the sorted size categories of the three (10), triangles without a
+// common node by how many of the three have a member of their own (4), the
+// one-heavy-pair triangles through a shared node by (members of a beyond the
+// pair, of b, category of c) (27), the enumerated triangles by class (30) and
+// by the open-pair classes they remove (6), the open pairs (6), work queues.
+constexpr unsigned kRawStar = 0, kRawDist = 10, kRawPair = 14, kRawClass = 41, kRawRem = 71, kRawOpen = 77,
+                   kRawQueue = 83, kRawSize = 96;
+
+__device__ __forceinline__ uint32_t star_index(uint32_t x, uint32_t y, uint32_t z) {  // any order
+  const uint32_t lo = min(x, min(y, z)), hi = max(x, max(y, z)), mid = x + y + z - lo - hi;
+  // 000 001 002 011 012 022 | 111 112 122 222
+  return lo == 0 ? (mid == 0 ? hi : mid == 1 ? 2 + hi : 5u) : lo == 1 ? (mid == 1 ? 5 + hi : 8u) : 9u;
+}
+__device__ __forceinline__ uint32_t pair_index(uint32_t ua, uint32_t ub, uint32_t cat) {
+  return (min(ua, 2u) * 3 + min(ub, 2u)) * 3 + cat;
+}
+
+// ---- preparation: ranks, heavy rows -------------------------------------------------
+
+// Per slot: degree (sort key), heavy neighbours; sums: [0] h^2, [1] d^2,
+// [2] node pairs of all hyperedges, [3] heavy entries.
+__global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint8_t* ovl, const uint8_t* esize,
+                              uint32_t n, uint32_t* heavy, uint32_t* ids, unsigned long long* sums) {
+  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0;
+  for (uint64_t a = global_warp(); a < n; a += n_warps()) {
+    const uint64_t s = off[a];
+    const uint32_t l = len[a];
+    uint32_t c = 0;
+    for (uint32_t i = lane_id(); i < l; i += kWarp) c += ovl[s + i] >= 2;
+    for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
+    if (lane_id() == 0) {
+      heavy[a] = c;
+      ids[a] = (uint32_t)a;
+      const unsigned long long z = esize[a];
+      h2 += (unsigned long long)c * c;
+      d2 += (unsigned long long)l * l;
+      np += z * (z - (z > 0)) / 2;
+      hs += c;
+    }
+  }
+  if (lane_id() == 0) {
+    if (h2) atomicAdd(&sums[0], h2);
+    if (d2) atomicAdd(&sums[1], d2);
+    if (np) atomicAdd(&sums[2], np);
+    if (hs) atomicAdd(&sums[3], hs);
+  }
+}
+
+__global__ void k_rank_scatter(const uint32_t* slot, uint32_t n, const uint32_t* heavy, uint32_t* rank,
+                               uint32_t* hcnt) {
+  for (uint64_t r = gtid(); r < n; r += gstride()) {
+    const uint32_t s = slot[r];
+    rank[s] = (uint32_t)r;
+    hcnt[r] = heavy[s];
+  }
+}
+
+// Heavy entries of every row, keyed (owner rank, neighbour rank), with their
+// position in the owner's H2H row.
+__global__ void k_heavy_emit(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint64_t* off,
+                             const uint32_t* len, const uint32_t* nbr, const uint8_t* ovl, const uint64_t* hoff,
+                             unsigned bits, uint64_t* key, uint32_t* pos) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    uint64_t w = hoff[r];
+    if (hoff[r + 1] == w) continue;
+    const uint32_t a = slot[r];
+    const uint64_t s = off[a];
+    const uint32_t l = len[a];
+    for (uint32_t i0 = 0; i0 < l; i0 += kWarp) {
+      const uint32_t i = i0 + lane_id();
+      const bool hv = i < l && ovl[s + i] >= 2;
+      const unsigned m = __ballot_sync(0xffffffffu, hv);
+      if (hv) {
+        const uint64_t d = w + __popc(m & lanemask_lt());
+        key[d] = (r << bits) | rank[nbr[s + i]];
+        pos[d] = i;
+      }
+      w += __popc(m);
+    }
+  }
+}
+
+// The sorted entries' fields; next = the first position of the neighbour's
+// row that ranks above the owner (the owner is in that row: adjacency is
+// symmetric).
+__global__ void k_heavy_rows(const uint64_t* key, const uint32_t* pos, uint64_t nh, unsigned bits,
+                             const uint32_t* slot, const uint64_t* off, const uint8_t* ovl, const uint8_t* esize,
+                             const uint64_t* hoff, uint32_t* hnbr, uint32_t* hown, uint16_t* hos, uint32_t* hpos,
+                             uint32_t* hnext) {
+  const uint64_t low = (1ull << bits) - 1;
+  for (uint64_t i = gtid(); i < nh; i += gstride()) {
+    const uint64_t k = key[i];
+    const uint32_t r = (uint32_t)(k >> bits), q = (uint32_t)(k & low);
+    const uint32_t p = pos[i];
+    hnbr[i] = q;
+    hown[i] = r;
+    hos[i] = (uint16_t)(((uint32_t)esize[slot[q]] << 8) | ovl[off[slot[r]] + p]);
+    hpos[i] = p;
+    const uint64_t back = ((uint64_t)q << bits) | r;
+    uint64_t lo = hoff[q], hi = hoff[q + 1];
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (key[mid] <= back) lo = mid + 1;
+      else hi = mid;
+    }
+    hnext[i] = (uint32_t)lo;
+  }
+}
+
+// ---- preparation: node graph --------------------------------------------------------
+
+// Hyperedges of each node by size category (3 per node).
+__global__ void k_node_cats(const uint64_t* voff, const uint32_t* vlen, const uint32_t* vedge, const uint8_t* esize,
+                            uint32_t n_nodes, uint32_t* ncat) {
+  for (uint64_t v = global_warp(); v < n_nodes; v += n_warps()) {
+    const uint64_t s = voff[v];
+    const uint32_t l = vlen[v];
+    uint32_t c[3] = {0, 0, 0};
+    for (uint32_t i = lane_id(); i < l; i += kWarp) {
+      const uint32_t z = esize[vedge[s + i]];
+      c[0] += z == 1;
+      c[1] += z == 2;
+      c[2] += z >= 3;
+    }
+    for (int k = 0; k < 3; ++k) {
+      for (int d = 16; d; d >>= 1) c[k] += __shfl_xor_sync(0xffffffffu, c[k], d);
+      if (lane_id() == 0) ncat[3 * v + k] = c[k];
+    }
+  }
+}
+
+// Node-pair table: open addressing over 16-byte entries {x, y, W2, W3},
+// x < y, W2 / W3 the hyperedges of two / more members holding both; an entry
+// of key 0 is empty (y > x >= 0). At most half full.
+__device__ __forceinline__ uint32_t pair_hash(uint32_t x, uint32_t y) {
+  uint32_t h = x * 2654435761u ^ (y * 2246822519u + 0x9E3779B9u);
+  h ^= h >> 15;
+  h *= 2246822519u;
+  return h ^ (h >> 13);
+}
+
+__device__ __forceinline__ uint2 pair_weight(const uint4* tab, uint32_t mask, uint32_t x, uint32_t y) {
+  const uint32_t a = min(x, y), b = max(x, y);
+  for (uint32_t h = pair_hash(a, b) & mask;; h = (h + 1) & mask) {
+    const uint4 e = __ldg(tab + h);
+    if (e.x == a && e.y == b) return make_uint2(e.z, e.w);
+    if (e.y == 0) return make_uint2(0, 0);
+  }
+}
+
+// One warp per hyperedge, lanes over its node pairs.
+__global__ void k_pair_insert(const uint64_t* off, const uint32_t* mem, const uint8_t* esize, uint32_t n, uint4* tab,
+                              uint32_t mask) {
+  for (uint64_t e = global_warp(); e < n; e += n_warps()) {
+    const uint32_t s = esize[e];
+    if (s < 2) continue;
+    const uint32_t* m = mem + off[e];
+    const uint32_t np = s * (s - 1) / 2;
+    for (uint32_t t = lane_id(); t < np; t += kWarp) {
+      // t-th pair (i < j): j the largest with j (j - 1) / 2 <= t
+      uint32_t j = (uint32_t)((1.0f + sqrtf(8.0f * (float)t + 1.0f)) * 0.5f);
+      while (j * (j - 1) / 2 > t) --j;
+      while ((j + 1) * j / 2 <= t) ++j;
+      const uint32_t x = m[t - j * (j - 1) / 2], y = m[j];
+      const unsigned long long key = ((unsigned long long)y << 32) | x;  // memory order {x, y}
+      uint32_t h = pair_hash(x, y) & mask;
+      for (;; h = (h + 1) & mask) {
+        const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long*>(tab + h), 0ull, key);
+        if (old == 0ull || old == key) break;
+      }
+      atomicAdd(s == 2 ? &tab[h].z : &tab[h].w, 1u);
+    }
+  }
+}
+
+__global__ void k_pair_degrees(const uint4* tab, uint64_t slots, uint32_t* deg) {
+  for (uint64_t i = gtid(); i < slots; i += gstride()) {
+    const uint4 e = tab[i];
+    if (!e.y) continue;
+    atomicAdd(&deg[e.x], 1u);
+    atomicAdd(&deg[e.y], 1u);
+  }
+}
+
+__device__ __forceinline__ bool owns(uint32_t x, uint32_t y, const uint32_t* deg) {  // x below y by (degree, id)
+  const uint32_t dx = deg[x], dy = deg[y];
+  return dx < dy || (dx == dy && x < y);
+}
+
+__global__ void k_pair_plus_count(const uint4* tab, uint64_t slots, const uint32_t* deg, uint32_t* plen) {
+  for (uint64_t i = gtid(); i < slots; i += gstride()) {
+    const uint4 e = tab[i];
+    if (e.y) atomicAdd(&plen[owns(e.x, e.y, deg) ? e.x : e.y], 1u);
+  }
+}
+
+__global__ void k_pair_plus_fill(const uint4* tab, uint64_t slots, const uint32_t* deg, const uint64_t* poff,
+                                 uint32_t* cursor, uint32_t* nbr, uint2* w) {
+  for (uint64_t i = gtid(); i < slots; i += gstride()) {
+    const uint4 e = tab[i];
+    if (!e.y) continue;
+    const bool lo = owns(e.x, e.y, deg);
+    const uint32_t u = lo ? e.x : e.y, v = lo ? e.y : e.x;
+    const uint64_t d = poff[u] + atomicAdd(&cursor[u], 1u);
+    nbr[d] = v;
+    w[d] = make_uint2(e.z, e.w);
+  }
+}
+
+// ---- work lists -----------------------------------------------------------------------
+// Items are put in (launch shape, log2 of their work) buckets, heaviest first
+// within a shape; bucket codes are shape * 32 + 31 - log2(work), 255 for none.
+constexpr unsigned kBuckets = 128;
+
+__device__ __forceinline__ uint8_t bucket_code(unsigned shape, uint64_t work) {
+  const unsigned lg = min(31u, (unsigned)(63 - __clzll((long long)work)));
+  return (uint8_t)(shape * 32 + 31 - lg);
+}
+
+__global__ void k_bucket_starts(uint32_t* hist, uint32_t* starts, uint32_t* shape_end) {  // one block of kBuckets
+  __shared__ uint32_t s[kBuckets];
+  const unsigned t = threadIdx.x;
+  s[t] = hist[t];
+  __syncthreads();
+  if (t == 0) {
+    uint32_t run = 0;
+    for (unsigned k = 0; k < kBuckets; ++k) {
+      const uint32_t c = s[k];
+      s[k] = run;
+      run += c;
+      if (k % 32 == 31) shape_end[k / 32] = run;
+    }
+  }
+  __syncthreads();
+  starts[t] = s[t];
+}
+
+__global__ void k_bucket_scatter(const uint8_t* code, uint32_t n, uint32_t* starts, uint32_t* list) {
+  for (uint64_t i = gtid(); i < n; i += gstride()) {
+    const uint8_t c = code[i];
+    if (c < kBuckets) list[atomicAdd(&starts[c], 1u)] = (uint32_t)i;
+  }
+}
+
+// Launch shapes of the enumeration: 0 a warp searching a's row (few tests,
+// less than an eighth of the row, or a row no table holds), 1 and 2 the
+// histogram kernel with 32-bit and 64-bit masks (up to 3072 entries ranked
+// above a), 3 the large tables (up to 12288, and centres of more than 64
+// members).
+constexpr uint32_t kHHSmall = 3072, kHHLarge = 12288;
+constexpr uint32_t kDenseSlots = 14336;  // up to this many hyperedges the tables are indexed by rank
+__global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint8_t* esize,
+                           const uint64_t* off, const uint32_t* len, const uint32_t* nbr, const uint64_t* hoff,
+                           const uint32_t* hnbr, const uint32_t* hnext, uint8_t* code, uint32_t* hist) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    uint64_t work = 0;
+    for (uint64_t e = hoff[r] + lane_id(); e < hoff[r + 1]; e += kWarp) work += hoff[hnbr[e] + 1] - hnext[e];
+    work = warp_sum(work);
+    uint8_t c = 255;
+    if (work) {
+      const uint32_t a = slot[r], l = len[a];
+      unsigned shape = 0;
+      if (work * 8 >= l) {
+        const bool narrow = esize[a] <= 32;
+        uint32_t up = 0;
+        if (!(narrow && n <= kDenseSlots)) {
+          const uint64_t s = off[a];
+          for (uint32_t i = lane_id(); i < l; i += kWarp) up += rank[nbr[s + i]] > r;
+          for (int d = 16; d; d >>= 1) up += __shfl_xor_sync(0xffffffffu, up, d);
+        }
+        shape = up <= kHHSmall && esize[a] <= 64 ? (narrow ? 1u : 2u) : up <= kHHLarge ? 3u : 0u;
+      }
+      c = bucket_code(shape, work);
+    }
+    if (lane_id() == 0) {
+      code[r] = c;
+      if (c != 255) atomicAdd(&hist[c], 1u);
+    }
+  }
+}
+
+// Node rows: one warp (up to 128 neighbours), one block with a 4096-slot or a
+// 16384-slot table, or the global pair table for the longest.
+constexpr uint32_t kNodeWarpRow = 128, kNodeSmall = 3072, kNodeLarge = 12288;
+__global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const uint32_t* nbr, uint32_t n,
+                             uint8_t* code, uint32_t* hist) {
+  for (uint64_t u = global_warp(); u < n; u += n_warps()) {
+    const uint32_t d = plen[u];
+    uint8_t c = 255;
+    if (d >= 2) {
+      uint64_t work = 0;
+      for (uint32_t i = lane_id(); i < d; i += kWarp) work += plen[nbr[poff[u] + i]];
+      work = warp_sum(work);
+      if (work) c = bucket_code(d <= kNodeWarpRow ? 0u : d <= kNodeSmall ? 1u : d <= kNodeLarge ? 2u : 3u, work);
+    }
+    if (lane_id() == 0) {
+      code[u] = c;
+      if (c != 255) atomicAdd(&hist[c], 1u);
+    }
+  }
+}
+
+// ---- counting: nodes, open pairs ------------------------------------------------------
+
+__device__ __forceinline__ uint64_t choose2(uint64_t n) { return n * (n - (n > 0)) / 2; }
+__device__ __forceinline__ uint64_t choose3(uint64_t n) {
+  if (n < 3) return 0;
+  const uint64_t p = choose2(n);
+  return (n - 2) % 3 == 0 ? p * ((n - 2) / 3) : p / 3 * (n - 2);  // the division first: the product may pass 2^64
+}
+
+// All hyperedge triples through one node, by size categories.
+__device__ void part_stars(unsigned vb, unsigned nb, const uint32_t* ncat, uint32_t n_nodes, unsigned long long* raw) {
+  uint64_t s[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (uint64_t v = (uint64_t)vb * kBlock + threadIdx.x; v < n_nodes; v += (uint64_t)nb * kBlock) {
+    const uint64_t a = ncat[3 * v], b = ncat[3 * v + 1], c = ncat[3 * v + 2];
+    s[0] += choose3(a);
+    s[1] += choose2(a) * b;
+    s[2] += choose2(a) * c;
+    s[3] += a * choose2(b);
+    s[4] += a * b * c;
+    s[5] += a * choose2(c);
+    s[6] += choose3(b);
+    s[7] += choose2(b) * c;
+    s[8] += b * choose2(c);
+    s[9] += choose3(c);
+  }
+#pragma unroll
+  for (int k = 0; k < 10; ++k) {
+    const uint64_t t = warp_sum(s[k]);
+    if (lane_id() == 0 && t) atomicAdd(&raw[kRawStar + k], (unsigned long long)t);
+  }
+}
+
+// Open pairs of every centre (see k_open_pairs in hm_static.cu), from the
+// heavy neighbours and the node counts: the light neighbours of a are the
+// (node, other hyperedge) incidences of its members minus the overlaps of its
+// heavy neighbours. Also takes back the node triangles a hyperedge forms
+// alone, C(|a|, 3).
+using OpenHist = uint32_t[kWarps][2][256];
+__device__ void part_open(unsigned vb, unsigned nb, OpenHist& hist, const uint32_t* slot, uint32_t n,
+                          const uint64_t* h2v_off, const uint32_t* h2v_mem, const uint8_t* esize,
+                          const uint32_t* h2h_len, const uint32_t* ncat, const uint64_t* hoff, const uint16_t* hos,
+                          unsigned long long* raw) {
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  uint64_t acc[6] = {0, 0, 0, 0, 0, 0};
+  uint64_t alone = 0;
+  for (uint64_t r = (uint64_t)vb * kWarps + w; r < n; r += (uint64_t)nb * kWarps) {
+    const uint32_t a = slot[r];
+    const uint32_t s = esize[a];
+    if (lane == 0) alone += choose3(s);
+    if (h2h_len[a] < 2) continue;
+    for (uint32_t i = lane; i <= s; i += kWarp) {
+      hist[w][0][i] = 0;
+      hist[w][1][i] = 0;
+    }
+    uint32_t one[2] = {0, 0};
+    const uint32_t* m = h2v_mem + h2v_off[a];
+    for (uint32_t i = lane; i < s; i += kWarp) {
+      const uint32_t* c = ncat + 3 * (uint64_t)m[i];
+      one[0] += c[0];
+      one[1] += c[1] + c[2];
+      one[s > 1] -= 1;  // a itself
+    }
+    __syncwarp();
+    for (uint64_t e = hoff[r] + lane; e < hoff[r + 1]; e += kWarp) {
+      const uint32_t os = hos[e], c = os & 0xffu;
+      one[1] -= c;  // a heavy neighbour has two members or more
+      atomicAdd(&hist[w][c < (os >> 8)][c], 1u);
+    }
+    for (int d = 16; d; d >>= 1) {
+      one[0] += __shfl_xor_sync(0xffffffffu, one[0], d);
+      one[1] += __shfl_xor_sync(0xffffffffu, one[1], d);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      uint32_t* h0 = hist[w][0];
+      uint32_t* h1 = hist[w][1];
+      h0[1] += one[0];
+      h1[1] += one[1];
+      for (uint32_t k = 1; k <= s; ++k) {
+        h0[k] += h0[k - 1];
+        h1[k] += h1[k - 1];
+      }
+      open_pair_counts(h0, h1, s, acc, false);
+    }
+    __syncwarp();
+  }
+  if (lane == 0) {
+    for (int k = 0; k < 6; ++k)
+      if (acc[k]) atomicAdd(&raw[kRawOpen + k], (unsigned long long)acc[k]);
+    if (alone) atomicAdd(&raw[kRawDist + 3], 0ull - (unsigned long long)alone);
+  }
+}
+
+// ---- counting: node triangles ----------------------------------------------------------
+
+struct NodeArgs {
+  const uint64_t* poff;
+  const uint32_t* plen;
+  const uint32_t* nbr;
+  const uint2* w;
+  const uint4* tab;  // the global pair table
+  uint32_t tmask;
+  const uint32_t* work;
+  uint32_t n_work;
+  unsigned int* queue;
+  unsigned long long* raw;
+};
+
+__device__ __forceinline__ uint32_t node_hash(uint32_t key, uint32_t shift) { return (key * 2654435761u) >> shift; }
+
+__device__ __forceinline__ void node_insert(uint32_t* keys, uint2* val, uint32_t shift, uint32_t mask, uint32_t key,
+                                            uint2 v) {
+  uint32_t h = node_hash(key, shift);
+  while (atomicCAS(&keys[h], kEmpty, key) != kEmpty) h = (h + 1) & mask;
+  val[h] = v;
+}
+
+// One entry x of v's row (its weights at w) against u's table: if u, v, x is a
+// node triangle, adds it to T[k] by how many of the pairs (u, x) and (v, x)
+// take a hyperedge of three members or more. The weights are loaded on a hit
+// only: most entries miss.
+__device__ __forceinline__ bool node_probe(const uint32_t* keys, const uint2* val, uint32_t shift, uint32_t mask,
+                                           uint32_t x, const uint2* w, uint64_t T[3]) {
+  uint32_t h = node_hash(x, shift);
+  for (;;) {
+    const uint32_t k = keys[h];
+    if (k == x) {
+      const uint2 p = val[h], q = __ldg(w);
+      T[0] += (uint64_t)p.x * q.x;
+      T[1] += (uint64_t)p.x * q.y + (uint64_t)p.y * q.x;
+      T[2] += (uint64_t)p.y * q.y;
+      return true;
+    }
+    if (k == kEmpty) return false;
+    h = (h + 1) & mask;
+  }
+}
+
+// Adds p, the weights of (u, v), times T to the sums by number of hyperedges
+// of three members or more.
+__device__ __forceinline__ void node_fold(uint2 p, uint64_t T[3], uint64_t F[4]) {
+  F[0] += p.x * T[0];
+  F[1] += p.y * T[0] + p.x * T[1];
+  F[2] += p.y * T[1] + p.x * T[2];
+  F[3] += p.y * T[2];
+  T[0] = T[1] = T[2] = 0;
+}
+
+__device__ __forceinline__ void node_flush(const uint64_t F[4], unsigned long long* raw) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint64_t t = warp_sum(F[k]);
+    if (lane_id() == 0 && t) atomicAdd(&raw[kRawDist + k], (unsigned long long)t);
+  }
+}
+
+// One warp per node with a short row: its table of 256 slots (load <= 1/2),
+// then the rows of its neighbours one after the other; the row bounds of 32
+// neighbours are loaded at once and the first 32 entries of a row while the
+// row before is probed.
+constexpr uint32_t kNodeWarpSlots = 2 * kNodeWarpRow;
+struct NodeWarp {
+  uint2 val[kNodeWarpSlots];
+  uint32_t keys[kNodeWarpSlots];
+};
+__device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
+  const unsigned lane = lane_id();
+  uint32_t* keys = S->keys;
+  uint2* val = S->val;
+  uint64_t F[4] = {0, 0, 0, 0};
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(A.queue, 1u);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= A.n_work) break;
+    const uint32_t u = A.work[it];
+    const uint64_t uo = A.poff[u];
+    const uint32_t d = A.plen[u];
+    uint32_t slots = 64;
+    while (slots < 2 * d && slots < kNodeWarpSlots) slots <<= 1;
+    const uint32_t shift = 32u - (31u - (uint32_t)__clz(slots)), mask = slots - 1;
+    for (uint32_t i = lane; i < slots; i += kWarp) keys[i] = kEmpty;
+    __syncwarp();
+    for (uint32_t i = lane; i < d; i += kWarp) node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
+    __syncwarp();
+    for (uint32_t i0 = 0; i0 < d; i0 += kWarp) {
+      uint64_t vo = 0;
+      uint32_t vl = 0;
+      if (i0 + lane < d) {
+        const uint32_t v = A.nbr[uo + i0 + lane];
+        vo = A.poff[v];
+        vl = A.plen[v];
+      }
+      const uint32_t m = min(kWarp, d - i0);
+      uint64_t o = __shfl_sync(0xffffffffu, vo, 0);
+      uint32_t l = __shfl_sync(0xffffffffu, vl, 0);
+      uint32_t x = lane < l ? __ldg(A.nbr + o + lane) : kEmpty;
+      for (uint32_t t = 0; t < m; ++t) {
+        const uint64_t on = __shfl_sync(0xffffffffu, vo, (t + 1) & 31u);
+        const uint32_t ln = __shfl_sync(0xffffffffu, vl, (t + 1) & 31u);
+        const uint32_t xn = t + 1 < m && lane < ln ? __ldg(A.nbr + on + lane) : kEmpty;
+        uint64_t T[3] = {0, 0, 0};
+        bool hit = x != kEmpty && node_probe(keys, val, shift, mask, x, A.w + o + lane, T);
+        for (uint32_t j = kWarp + lane; j < l; j += kWarp)
+          hit |= node_probe(keys, val, shift, mask, __ldg(A.nbr + o + j), A.w + o + j, T);
+        if (__any_sync(0xffffffffu, hit)) node_fold(A.w[uo + i0 + t], T, F);
+        o = on;
+        l = ln;
+        x = xn;
+      }
+    }
+    __syncwarp();
+  }
+  node_flush(F, A.raw);
+}
+
+// One block per node, kTab slots in shared memory (load <= 3/4); kTab = 0:
+// probes the global pair table instead.
+template <unsigned kTab, unsigned kThreads, unsigned kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
+  extern __shared__ uint64_t smem64[];
+  uint2* val = reinterpret_cast<uint2*>(smem64);
+  uint32_t* keys = reinterpret_cast<uint32_t*>(val + kTab);
+  __shared__ uint32_t s_item;
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  uint64_t F[4] = {0, 0, 0, 0};
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= A.n_work) break;
+    const uint32_t u = A.work[it];
+    const uint64_t uo = A.poff[u];
+    const uint32_t d = A.plen[u];
+    uint32_t slots = 64, shift = 26, mask = 63;
+    if (kTab) {
+      while (slots < 2 * d && slots < kTab) slots <<= 1;
+      shift = 32u - (31u - (uint32_t)__clz(slots));
+      mask = slots - 1;
+      for (uint32_t i = threadIdx.x; i < slots; i += kThreads) keys[i] = kEmpty;
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < d; i += kThreads) node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
+    }
+    __syncthreads();
+    for (uint32_t i = w; i < d; i += kThreads / kWarp) {
+      const uint32_t v = A.nbr[uo + i];
+      const uint64_t o = A.poff[v];
+      const uint32_t l = A.plen[v];
+      uint64_t T[3] = {0, 0, 0};
+      for (uint32_t j = lane; j < l; j += kWarp) {
+        const uint32_t x = __ldg(A.nbr + o + j);
+        if (kTab) {
+          node_probe(keys, val, shift, mask, x, A.w + o + j, T);
+        } else {
+          const uint2 p = pair_weight(A.tab, A.tmask, u, x), q = __ldg(A.w + o + j);
+          T[0] += (uint64_t)p.x * q.x;
+          T[1] += (uint64_t)p.x * q.y + (uint64_t)p.y * q.x;
+          T[2] += (uint64_t)p.y * q.y;
+        }
+      }
+      node_fold(A.w[uo + i], T, F);
+    }
+    __syncthreads();
+  }
+  node_flush(F, A.raw);
+}
+
+// ---- counting: heavy pairs --------------------------------------------------------------
+// A heavy pair (a, b) is owned by its larger member (the lower rank at equal
+// size). q(a, b), the sum of W over (a \ S) x (b \ S), is summed entry by entry
+// for most pairs. A large owner with many partners first spreads
+// y(w) = sum over v in a of W(v, w) over a node vector of its block, and then
+//   q = sum_{w in b \ S} y(w) - sum_{v in S} self_b(v) + sum_{v != w in S} W(v, w),
+// self_b(v) = sum_{w in b} W(v, w) kept per H2V entry: about |b| reads per pair.
+
+struct PairArgs {
+  const uint32_t* hown;
+  const uint32_t* hnbr;
+  const uint16_t* hos;
+  const uint32_t* hpos;
+  const uint32_t* hnext;
+  const uint64_t* hoff;
+  uint64_t nh;
+  const uint32_t* slot;
+  const uint64_t* off;   // H2H
+  const uint64_t* mask;
+  const uint64_t* voff;  // H2V
+  const uint32_t* vmem;
+  const uint8_t* esize;
+  const uint32_t* ncat;
+  const uint4* tab;
+  uint32_t tmask;
+  const uint64_t* foff;  // the node graph's rows, both directions (for spreading)
+  const uint32_t* fnbr;
+  const uint2* fw;
+  const uint8_t* spread;  // per rank: its owned pairs go through y
+  const uint32_t* list;   // the ranks with spread set
+  uint32_t n_list;
+  uint2* self;            // per H2V entry {W2, W3}
+  uint2* y;               // per block of k_spread_pairs: n_nodes entries (rounded up to even), zero between items
+  uint32_t n_nodes;
+  uint32_t per_warp, wide;  // entries a warp takes at once; combinations from which it takes a pair as a whole
+  unsigned int* queue;
+  unsigned long long* raw;
+};
+
+__device__ __forceinline__ bool owns_pair(uint32_t ra, uint32_t sa, uint32_t rb, uint32_t sb) {
+  return sa > sb || (sa == sb && ra < rb);
+}
+
+// The sums of one pair into the block's counters: q (third hyperedge of two /
+// more members) and r (hyperedges of S's nodes by category, a and b included).
+__device__ __forceinline__ void add_pair(unsigned long long* cnt, uint32_t sa, uint32_t sb, uint32_t C, uint64_t q2,
+                                         uint64_t q3, uint64_t r0, uint64_t r1, uint64_t r2) {
+  const uint32_t ca = size_cat(sa), cb = size_cat(sb);
+  const uint32_t n_ex = (sa > C + 1) + (sb > C + 1), n_big = (ca == 2) + (cb == 2);
+  uint64_t r[3] = {r0, r1 - C * (uint64_t)((ca == 1) + (cb == 1)), r2 - C * (uint64_t)((ca == 2) + (cb == 2))};
+  if (q2) {
+    atomicAdd(&cnt[kRawDist + n_ex], (unsigned long long)q2);
+    atomicAdd(&cnt[kRawDist + n_big], 0ull - (unsigned long long)q2 * C);
+  }
+  if (q3) {
+    atomicAdd(&cnt[kRawDist + n_ex + 1], (unsigned long long)q3);
+    atomicAdd(&cnt[kRawDist + n_big + 1], 0ull - (unsigned long long)q3 * C);
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < 3; ++k)
+    if (r[k]) {
+      atomicAdd(&cnt[kRawPair + pair_index(sa - C, sb - C, k)], (unsigned long long)r[k]);
+      atomicAdd(&cnt[kRawStar + star_index(ca, cb, k)], 0ull - (unsigned long long)r[k]);
+    }
+  // one hyperedge of the pair standing for two node pairs of a triangle
+  const unsigned long long c2 = (unsigned long long)C * (C - 1) / 2;
+  if (sa >= 3) atomicAdd(&cnt[kRawDist + 2 + (sb >= 3)], 0ull - c2 * (sa - 2));
+  if (sb >= 3) atomicAdd(&cnt[kRawDist + 2 + (sa >= 3)], 0ull - c2 * (sb - 2));
+}
+
+__device__ __forceinline__ bool in_list(const uint32_t* list, uint32_t n, uint32_t key) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(list + mid) < key) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo < n && __ldg(list + lo) == key;
+}
+
+// Four entries per warp, eight lanes each over the |a| x |b| combinations, the
+// positions in S read off the two entries' masks (members past 64: a search
+// of the other list). Pairs of more than kPairWide combinations are taken by
+// the whole warp, one after the other; with too few entries to fill the GPU
+// that way (kPairFew) all are, one entry per warp.
+constexpr uint32_t kPairWide = 384, kPairFew = 1u << 16;
+using PairCounts = unsigned long long[kRawClass];
+__device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const PairArgs& A) {
+  const unsigned lane = lane_id(), grp = lane >> 3, sub = lane & 7u;
+  for (unsigned k = threadIdx.x; k < kRawClass; k += kBlock) cnt[k] = 0;
+  __syncthreads();
+  for (uint64_t e0 = ((uint64_t)vb * kWarps + threadIdx.x / kWarp) * A.per_warp; e0 < A.nh;
+       e0 += (uint64_t)nb * kWarps * A.per_warp) {
+    const uint64_t e = e0 + grp;
+    uint32_t sa = 0, sb = 0, C = 0;
+    const uint32_t *pa = nullptr, *pb = nullptr;
+    uint64_t ma = 0, mb = 0;
+    if (grp < A.per_warp && e < A.nh) {
+      const uint32_t ra = A.hown[e], rb = A.hnbr[e], os = A.hos[e];
+      const uint32_t a = A.slot[ra];
+      const uint32_t za = A.esize[a], zb = os >> 8;
+      if (owns_pair(ra, za, rb, zb) && !A.spread[ra]) {
+        const uint32_t b = A.slot[rb];
+        sa = za;
+        sb = zb;
+        C = os & 0xffu;
+        pa = A.vmem + A.voff[a];
+        pb = A.vmem + A.voff[b];
+        ma = A.mask[A.off[a] + A.hpos[e]];
+        mb = A.mask[A.off[b] + A.hpos[A.hnext[e] - 1]];  // (b -> a) precedes b's entries above a
+      }
+    }
+    uint64_t q2 = 0, q3 = 0, r0 = 0, r1 = 0, r2 = 0;
+    // lanes first, first + step, ... of the |a| x |b| combinations; the
+    // combinations of b's first member stand for a's member alone
+    auto run = [&](uint32_t first, uint32_t step, uint32_t na, uint32_t nb, const uint32_t* xa, const uint32_t* xb,
+                   uint64_t sma, uint64_t smb) {
+      const uint32_t all = na * nb;
+      for (uint32_t t = first; t < all; t += step) {
+        const uint32_t i = t / nb, j = t - i * nb;
+        const uint32_t v = __ldg(xa + i);
+        if (i < 64 ? (sma >> i) & 1ull : in_list(xb, nb, v)) {
+          if (j) continue;
+          const uint32_t* c = A.ncat + 3 * (uint64_t)v;
+          r0 += c[0];
+          r1 += c[1];
+          r2 += c[2];
+          continue;
+        }
+        const uint32_t w = __ldg(xb + j);
+        if (j < 64 ? (smb >> j) & 1ull : in_list(xa, na, w)) continue;
+        const uint2 p = pair_weight(A.tab, A.tmask, v, w);
+        q2 += p.x;
+        q3 += p.y;
+      }
+    };
+    const bool wide = sa * sb > A.wide;
+    if (!wide) run(sub, 8, sa, sb, pa, pb, ma, mb);
+    unsigned todo = __ballot_sync(0xffffffffu, wide && sub == 0);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint64_t k2 = q2, k3 = q3, s0 = r0, s1 = r1, s2 = r2;  // this lane's own pair, set aside
+      q2 = q3 = r0 = r1 = r2 = 0;
+      run(lane, 32, __shfl_sync(0xffffffffu, sa, src), __shfl_sync(0xffffffffu, sb, src),
+          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pa, src)),
+          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pb, src)),
+          __shfl_sync(0xffffffffu, (unsigned long long)ma, src), __shfl_sync(0xffffffffu, (unsigned long long)mb, src));
+      __syncwarp();
+      const uint64_t t2 = warp_sum(q2), t3 = warp_sum(q3), u0 = warp_sum(r0), u1 = warp_sum(r1), u2 = warp_sum(r2);
+      if ((int)lane == src) add_pair(cnt, sa, sb, C, t2, t3, u0, u1, u2);
+      q2 = k2;
+      q3 = k3;
+      r0 = s0;
+      r1 = s1;
+      r2 = s2;
+      __syncwarp();
+    }
+    uint64_t t[5] = {q2, q3, r0, r1, r2};
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+      for (int d = 4; d; d >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], d);
+    if (sa && !wide && sub == 0) add_pair(cnt, sa, sb, C, t[0], t[1], t[2], t[3], t[4]);
+  }
+  __syncthreads();
+  for (unsigned k = threadIdx.x; k < kRawClass; k += kBlock)
+    if (cnt[k]) atomicAdd(&A.raw[k], cnt[k]);
+}
+
+// Which owners spread: those whose entry-by-entry sums are longer than building
+// and reading the vector (an increment and a clear per neighbour of a member),
+// and long enough that one block's pass over it is not the slower one.
+constexpr uint64_t kSpreadMin = 1u << 17;
+__global__ void k_spread_flags(const uint32_t* slot, uint32_t n, const uint64_t* hoff, const uint32_t* hnbr,
+                               const uint16_t* hos, const uint64_t* voff, const uint32_t* vmem, const uint8_t* esize,
+                               const uint32_t* ndeg, uint8_t* spread, uint32_t* list, uint32_t* n_list) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    const uint32_t a = slot[r], s = esize[a];
+    uint64_t direct = 0, reads = 0;
+    for (uint64_t e = hoff[r] + lane_id(); e < hoff[r + 1]; e += kWarp) {
+      const uint32_t os = hos[e], z = os >> 8, C = os & 0xffu;
+      if (!owns_pair((uint32_t)r, s, hnbr[e], z)) continue;
+      direct += (uint64_t)(s - C) * (z - C);
+      reads += z;
+    }
+    direct = warp_sum(direct);
+    reads = warp_sum(reads);
+    bool on = direct >= kSpreadMin && direct > reads;
+    if (on) {
+      uint64_t build = 0;
+      for (uint32_t i = lane_id(); i < s; i += kWarp) build += ndeg[vmem[voff[a] + i]];
+      on = direct > reads + 2 * warp_sum(build);
+    }
+    if (lane_id() == 0) {
+      spread[r] = on;
+      if (on) list[atomicAdd(n_list, 1u)] = (uint32_t)r;
+    }
+  }
+}
+
+__global__ void k_pair_rows_fill(const uint4* tab, uint64_t slots, const uint64_t* off, uint32_t* cursor, uint32_t* nbr,
+                                 uint2* w) {
+  for (uint64_t i = gtid(); i < slots; i += gstride()) {
+    const uint4 e = tab[i];
+    if (!e.y) continue;
+    uint64_t d = off[e.x] + atomicAdd(&cursor[e.x], 1u);
+    nbr[d] = e.y;
+    w[d] = make_uint2(e.z, e.w);
+    d = off[e.y] + atomicAdd(&cursor[e.y], 1u);
+    nbr[d] = e.x;
+    w[d] = make_uint2(e.z, e.w);
+  }
+}
+
+// self_b(v) for every member v of every hyperedge with heavy neighbours.
+__global__ void k_self_weights(PairArgs A, uint32_t n) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    if (A.hoff[r + 1] == A.hoff[r]) continue;
+    const uint32_t a = A.slot[r], s = A.esize[a];
+    const uint64_t o = A.voff[a];
+    for (uint32_t i = lane_id(); i < s; i += kWarp) {
+      const uint32_t v = A.vmem[o + i];
+      uint2 t = make_uint2(0, 0);
+      for (uint32_t j = 0; j < s; ++j) {
+        if (j == i) continue;
+        const uint2 p = pair_weight(A.tab, A.tmask, v, __ldg(A.vmem + o + j));
+        t.x += p.x;
+        t.y += p.y;
+      }
+      A.self[o + i] = t;
+    }
+  }
+}
+
+// One block per spreading owner a. In the vector a's own members hold
+// {~0, ~0}, which tells S from b \ S.
+constexpr unsigned kSpreadThreads = 1024;
+__global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
+  __shared__ unsigned long long cnt[kRawClass];
+  __shared__ uint32_t s_item;
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  constexpr unsigned kW = kSpreadThreads / kWarp;
+  uint2* y = A.y + (uint64_t)blockIdx.x * ((A.n_nodes + 1) & ~1u);
+  for (unsigned k = threadIdx.x; k < kRawClass; k += kSpreadThreads) cnt[k] = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
+    __syncthreads();
+    if (s_item >= A.n_list) break;
+    const uint32_t ra = A.list[s_item], a = A.slot[ra], sa = A.esize[a];
+    const uint32_t* pa = A.vmem + A.voff[a];
+    // a warp takes the rows of one member after another
+    uint64_t cells = 0;
+    for (uint32_t i = w; i < sa; i += kW) {
+      const uint32_t v = __ldg(pa + i);
+      const uint64_t o = A.foff[v];
+      const uint32_t l = (uint32_t)(A.foff[v + 1] - o);
+      for (uint32_t k = lane; k < l; k += kWarp) {
+        const uint32_t x = __ldg(A.fnbr + o + k);
+        const uint2 q = __ldg(A.fw + o + k);
+        if (q.x) atomicAdd(&y[x].x, q.x);
+        if (q.y) atomicAdd(&y[x].y, q.y);
+      }
+    }
+    for (uint32_t i = 0; i < sa; ++i) cells += A.foff[pa[i] + 1] - A.foff[pa[i]];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < sa; i += kSpreadThreads) y[pa[i]] = make_uint2(~0u, ~0u);
+    __syncthreads();
+    const uint64_t he = A.hoff[ra + 1];
+    for (uint64_t e = A.hoff[ra] + w; e < he; e += kW) {
+      const uint32_t rb = A.hnbr[e], os = A.hos[e], sb = os >> 8, C = os & 0xffu;
+      if (!owns_pair(ra, sa, rb, sb)) continue;
+      const uint32_t b = A.slot[rb];
+      const uint64_t bo = A.voff[b];
+      uint64_t q2 = 0, q3 = 0, r0 = 0, r1 = 0, r2 = 0;
+      for (uint32_t j = lane; j < sb; j += kWarp) {
+        const uint32_t v = __ldg(A.vmem + bo + j);
+        const uint2 t = y[v];
+        if (t.x != ~0u || t.y != ~0u) {
+          q2 += t.x;
+          q3 += t.y;
+          continue;
+        }
+        const uint32_t* c = A.ncat + 3 * (uint64_t)v;
+        r0 += c[0];
+        r1 += c[1];
+        r2 += c[2];
+        const uint2 z = A.self[bo + j];
+        q2 -= z.x;
+        q3 -= z.y;
+        for (uint32_t k = 0; k < sb; ++k) {  // the other members of S
+          if (k == j) continue;
+          const uint32_t x = __ldg(A.vmem + bo + k);
+          const uint2 u = y[x];
+          if (u.x != ~0u || u.y != ~0u) continue;
+          const uint2 p = pair_weight(A.tab, A.tmask, v, x);
+          q2 += p.x;
+          q3 += p.y;
+        }
+      }
+      q2 = warp_sum(q2);
+      q3 = warp_sum(q3);
+      r0 = warp_sum(r0);
+      r1 = warp_sum(r1);
+      r2 = warp_sum(r2);
+      if (lane == 0) add_pair(cnt, sa, sb, C, q2, q3, r0, r1, r2);
+    }
+    __syncthreads();
+    if (A.n_nodes <= 4 * cells) {  // clear it all, two entries at a time (the vectors start at even entries)
+      for (uint32_t i = threadIdx.x; i < (A.n_nodes + 1) / 2; i += kSpreadThreads)
+        reinterpret_cast<uint4*>(y)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+      for (uint32_t i = w; i < sa; i += kW) {
+        const uint32_t v = __ldg(pa + i);
+        if (lane == 0) y[v] = make_uint2(0, 0);
+        for (uint64_t k = A.foff[v] + lane; k < A.foff[v + 1]; k += kWarp) y[__ldg(A.fnbr + k)] = make_uint2(0, 0);
+      }
+    }
+  }
+  for (unsigned k = threadIdx.x; k < kRawClass; k += kSpreadThreads)
+    if (cnt[k]) atomicAdd(&A.raw[k], cnt[k]);
+}
+
+// ---- counting: triangles with two or three heavy pairs ------------------------------------
+
+struct HHArgs {
+  const uint32_t* slot;
+  const uint32_t* rank;
+  const uint64_t* hoff;   // heavy rows by rank
+  const uint32_t* hnbr;
+  const uint16_t* hos;
+  const uint32_t* hpos;
+  const uint32_t* hnext;
+  const uint64_t* off;    // H2H
+  const uint32_t* len;
+  const uint32_t* nbr;
+  const uint8_t* ovl;
+  const uint64_t* mask;
+  const uint64_t* voff;   // H2V
+  const uint32_t* vmem;
+  const uint8_t* esize;
+  const uint32_t* work;   // ranks of the centres
+  uint32_t n_work;
+  unsigned int* queue;
+  unsigned long long* raw;
+};
+
+// |a & b & c| by a three-way merge (centres of more than 64 members).
+__device__ uint32_t merge3(const HHArgs& A, uint32_t a, uint32_t b, uint32_t c) {
+  const uint32_t* x = A.vmem + A.voff[a];
+  const uint32_t* y = A.vmem + A.voff[b];
+  const uint32_t* z = A.vmem + A.voff[c];
+  const uint32_t nx = A.esize[a], ny = A.esize[b], nz = A.esize[c];
+  uint32_t i = 0, j = 0, k = 0, g = 0;
+  while (i < nx && j < ny && k < nz) {
+    const uint32_t u = x[i], v = y[j], t = z[k];
+    const uint32_t m = max(u, max(v, t));
+    if (u == m && v == m && t == m) {
+      ++g; ++i; ++j; ++k;
+    } else {
+      i += (u < m);
+      j += (v < m);
+      k += (t < m);
+    }
+  }
+  return g;
+}
+
+// Counters a triangle adds to, 32-bit, one of kCol columns per lane (lanes of
+// a warp often meet the same counter): 30 classes, 6 removals, 4 stars by the
+// number of hyperedges with three members or more, 18 pair entries (ua, ub,
+// c of three or more).
+constexpr unsigned kSmClass = 0, kSmRem = 30, kSmStar = 36, kSmPair = 40, kSmRows = 58;
+// A test adds at most 3 x 255 to one 32-bit counter: flushed every 2^22 tests,
+// none can wrap.
+constexpr uint32_t kFlushTests = 1u << 22;
+
+template <unsigned kCol>
+struct WarpCounts {
+  unsigned long long dist[4][kWarp];  // per lane: no conflicts, no atomics
+  uint32_t c[kSmRows][kCol];
+};
+
+template <unsigned kCol>
+__device__ __forceinline__ void clear_counts(WarpCounts<kCol>* W) {
+  for (unsigned k = 0; k < 4; ++k) W->dist[k][lane_id()] = 0;
+  for (unsigned k = lane_id(); k < kSmRows * kCol; k += kWarp) (&W->c[0][0])[k] = 0;
+  __syncwarp();
+}
+
+template <unsigned kCol>
+__device__ __forceinline__ void flush_counts(WarpCounts<kCol>* W, unsigned long long* raw) {
+  __syncwarp();
+  for (unsigned k = 0; k < 4; ++k) {
+    const uint64_t t = warp_sum(W->dist[k][lane_id()]);
+    if (lane_id() == 0 && t) atomicAdd(&raw[kRawDist + k], (unsigned long long)t);
+  }
+  for (unsigned k = lane_id(); k < kSmRows; k += kWarp) {
+    unsigned long long t = 0;
+    for (unsigned j = 0; j < kCol; ++j) t += W->c[k][j];
+    if (!t) continue;
+    if (k < kSmRem) atomicAdd(&raw[kRawClass + k], t);
+    else if (k < kSmStar) atomicAdd(&raw[kRawRem + (k - kSmRem)], t);
+    else if (k < kSmPair) atomicAdd(&raw[kRawStar + 6 + (k - kSmStar)], t);  // sorted categories 111 112 122 222
+    else {
+      const uint32_t q = k - kSmPair;  // (ua, ub) * 2 + big, taken back
+      atomicAdd(&raw[kRawPair + (q >> 1) * 3 + 1 + (q & 1u)], 0ull - t);
+    }
+  }
+  __syncwarp();
+  clear_counts(W);
+}
+
+// One triangle with overlaps cab, cbc, cac (two of them heavy or all) and
+// triple overlap g: its class and removals, and what the closed forms counted
+// it for (see the head of this file).
+template <unsigned kCol>
+__device__ __forceinline__ void add_triangle(WarpCounts<kCol>* W, const int8_t* cls, uint32_t sa, uint32_t sb,
+                                             uint32_t sc, uint32_t cab, uint32_t cbc, uint32_t cac, uint32_t g,
+                                             uint32_t n = 1) {
+  const unsigned lane = lane_id(), col = lane & (kCol - 1);
+  const int k = cls[region_pattern((int)sa, (int)sb, (int)sc, (int)cab, (int)cbc, (int)cac, (int)g)];
+  atomicAdd(&W->c[kSmClass + k][col], n);
+  const uint32_t oa = (cab + cac < sa) + 2 * ((cab < sb) + (cac < sc));
+  const uint32_t ob = (cab + cbc < sb) + 2 * ((cab < sa) + (cbc < sc));
+  const uint32_t oc = (cac + cbc < sc) + 2 * ((cac < sa) + (cbc < sb));
+  atomicAdd(&W->c[kSmRem + oa][col], n);
+  atomicAdd(&W->c[kSmRem + ob][col], n);
+  atomicAdd(&W->c[kSmRem + oc][col], n);
+  const uint32_t ba = sa >= 3, bb = sb >= 3, bc = sc >= 3;
+  const uint32_t xab = cab - g, xbc = cbc - g, xac = cac - g;
+  // below 2^26 in absolute value: sizes are at most 255
+  int dk = (int)(g * (cab + cbc + cac)) - 2 * (int)g - (int)(cab * cbc * cac);  // -R
+  const uint32_t eab = cab >= 2 ? xac * xbc : 0u, ebc = cbc >= 2 ? xab * xac : 0u, eac = cac >= 2 ? xab * xbc : 0u;
+  dk += (int)(cab * eab + cbc * ebc + cac * eac);
+  W->dist[ba + bb + bc][lane] += (unsigned long long)((long long)dk * n);
+  if (eab) W->dist[(sa > cab + 1) + (sb > cab + 1) + bc][lane] -= (unsigned long long)eab * n;
+  if (ebc) W->dist[(sb > cbc + 1) + (sc > cbc + 1) + ba][lane] -= (unsigned long long)ebc * n;
+  if (eac) W->dist[(sa > cac + 1) + (sc > cac + 1) + bb][lane] -= (unsigned long long)eac * n;
+  if (g) {
+    const uint32_t gn = g * n;
+    atomicAdd(&W->c[kSmStar + ba + bb + bc][col], gn * ((cab >= 2) + (cbc >= 2) + (cac >= 2) - 1));
+    auto pair = [&](uint32_t ux, uint32_t uy, uint32_t big) {
+      atomicAdd(&W->c[kSmPair + (min(ux, 2u) * 3 + min(uy, 2u)) * 2 + big][col], gn);
+    };
+    if (cab >= 2) pair(sa - cab, sb - cab, bc);
+    if (cbc >= 2) pair(sb - cbc, sc - cbc, ba);
+    if (cac >= 2) pair(sa - cac, sc - cac, bb);
+  }
+}
+
+// A record packs |b|, |c|, C_ab, C_bc, C_ac and g, 8 bits each, and how many
+// triangles it stands for, 16 bits.
+__device__ __forceinline__ uint64_t pack6(uint32_t sb, uint32_t sc, uint32_t cab, uint32_t cbc, uint32_t cac,
+                                          uint32_t g, uint32_t n = 1) {
+  return (uint64_t)(sb | (sc << 8) | (cab << 16) | (cbc << 24)) | ((uint64_t)(cac | (g << 8) | (n << 16)) << 32);
+}
+template <unsigned kCol>
+__device__ __forceinline__ void add_record(WarpCounts<kCol>* W, const int8_t* cls, uint32_t sa, uint64_t r) {
+  const uint32_t lo = (uint32_t)r, hi = (uint32_t)(r >> 32);
+  add_triangle(W, cls, sa, lo & 0xffu, (lo >> 8) & 0xffu, (lo >> 16) & 0xffu, lo >> 24, hi & 0xffu, (hi >> 8) & 0xffu,
+               hi >> 16);
+}
+
+// Whole warp: appends the lanes' records to the warp's queue (64 places) and
+// classifies 32 at a time.
+template <unsigned kCol>
+__device__ __forceinline__ void queue_records(WarpCounts<kCol>* W, const int8_t* cls, uint32_t sa, bool push,
+                                              uint64_t rec, uint64_t* q, uint32_t& qn) {
+  const unsigned bal = __ballot_sync(0xffffffffu, push);
+  if (!bal) return;
+  if (push) q[qn + __popc(bal & lanemask_lt())] = rec;
+  qn += (uint32_t)__popc(bal);
+  __syncwarp();
+  if (qn >= kWarp) {
+    add_record(W, cls, sa, q[lane_id()]);
+    __syncwarp();
+    if (lane_id() < qn - kWarp) q[lane_id()] = q[kWarp + lane_id()];
+    __syncwarp();
+    qn -= kWarp;
+  }
+}
+
+__device__ __forceinline__ void fill_classes(int8_t* cls) {
+  for (unsigned p = threadIdx.x; p < 128; p += blockDim.x) {
+    const int k = static_class_of_pattern((int)p);
+    cls[p] = (int8_t)(k < 0 ? 0 : k);  // a closed triangle always has a class
+  }
+}
+
+// One warp per centre with few tests: each c is searched in a's id-sorted row.
+constexpr unsigned kSearchCol = 4;
+struct SearchShared {
+  WarpCounts<kSearchCol> wc[kWarps];
+  int8_t cls[128];
+};
+__device__ void part_search(const HHArgs& A, SearchShared& S) {
+  const unsigned lane = lane_id();
+  WarpCounts<kSearchCol>* W = &S.wc[threadIdx.x / kWarp];
+  int8_t* cls = S.cls;
+  fill_classes(cls);
+  clear_counts(W);
+  __syncthreads();
+  uint32_t tests = 0;
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(A.queue, 1u);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= A.n_work) break;
+    const uint32_t ra = A.work[it], a = A.slot[ra];
+    const uint64_t ao = A.off[a];
+    const uint32_t al = A.len[a];
+    const uint32_t sa = A.esize[a];
+    const uint64_t he = A.hoff[ra + 1];
+    for (uint64_t e = A.hoff[ra]; e < he; ++e) {
+      const uint32_t rb = A.hnbr[e], osb = A.hos[e];
+      const uint64_t mab = A.mask[ao + A.hpos[e]];
+      const uint64_t end = A.hoff[rb + 1];
+      for (uint64_t j0 = A.hnext[e]; j0 < end; j0 += kWarp) {
+        const uint64_t j = j0 + lane;
+        if (j < end) {
+          const uint32_t rc = A.hnbr[j], osc = A.hos[j], c = A.slot[rc];
+          uint32_t lo = 0, hi = al;
+          while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(A.nbr + ao + mid) < c) lo = mid + 1;
+            else hi = mid;
+          }
+          if (lo < al && A.nbr[ao + lo] == c) {
+            const uint32_t cac = A.ovl[ao + lo];
+            if (cac < 2 || rb > rc) {  // three heavy pairs: once, b ranked highest
+              const uint32_t g = sa <= 64 ? (uint32_t)__popcll(mab & A.mask[ao + lo]) : merge3(A, a, A.slot[rb], c);
+              add_triangle(W, cls, sa, osb >> 8, osc >> 8, osb & 0xffu, osc & 0xffu, cac, g);
+            }
+          }
+        }
+        __syncwarp();
+        if ((tests += kWarp) >= kFlushTests) {
+          flush_counts(W, A.raw);
+          tests = 0;
+        }
+      }
+    }
+  }
+  flush_counts(W, A.raw);
+}
+
+// One block per centre a: the entries of a's row ranked above a in a shared
+// table keyed by rank (4 keys per 16-byte bucket, load <= 3/4), each with its
+// place in a's row. Warps take b among a's heavy neighbours, lanes walk b's
+// heavy row past a. For the longest rows and centres of more than 64 members.
+constexpr unsigned kHHSlots = 16384, kHHThreads = 1024, kHHCol = 4;
+constexpr size_t kHHSmem = kHHSlots * 2 * sizeof(uint32_t) +
+                           kHHThreads / kWarp * (sizeof(WarpCounts<kHHCol>) + 2 * kWarp * sizeof(uint64_t));
+static_assert(kHHSmem <= 226 * 1024 && kHHLarge <= kHHSlots * 3 / 4, "one block per SM, table load");
+__global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
+  constexpr unsigned kSlots = kHHSlots, kThreads = kHHThreads, kCol = kHHCol, kW = kThreads / kWarp;
+  extern __shared__ uint64_t smem64[];
+  uint32_t* val = reinterpret_cast<uint32_t*>(smem64);
+  uint32_t* keys = val + kSlots;
+  WarpCounts<kCol>* W = reinterpret_cast<WarpCounts<kCol>*>(keys + kSlots) + threadIdx.x / kWarp;
+  uint64_t* q = reinterpret_cast<uint64_t*>(reinterpret_cast<WarpCounts<kCol>*>(keys + kSlots) + kW) +
+                (threadIdx.x / kWarp) * 2 * kWarp;
+  __shared__ int8_t cls[128];
+  __shared__ uint32_t s_item;
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  fill_classes(cls);
+  clear_counts(W);
+  uint32_t qn = 0, tests = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= A.n_work) break;
+    const uint32_t ra = A.work[it], a = A.slot[ra];
+    const uint64_t ao = A.off[a];
+    const uint32_t al = A.len[a];
+    const uint32_t sa = A.esize[a];
+    const bool exact = sa <= 64;
+    uint32_t slots = 64;
+    while (slots < 2 * al && slots < kSlots) slots <<= 1;
+    const uint32_t shift = 32u - (31u - (uint32_t)__clz(slots / 4)), bmask = slots / 4 - 1;
+    for (uint32_t i = threadIdx.x; i < slots; i += kThreads) keys[i] = kEmpty;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < al; i += kThreads) {
+      const uint32_t key = __ldg(A.rank + __ldg(A.nbr + ao + i));
+      if (key <= ra) continue;
+      uint32_t bk = (key * 2654435761u) >> shift, h = 0;
+      for (bool done = false; !done; bk = (bk + 1) & bmask)
+        for (uint32_t t = 0; t < 4; ++t)
+          if (atomicCAS(&keys[4 * bk + t], kEmpty, key) == kEmpty) {
+            h = 4 * bk + t;
+            done = true;
+            break;
+          }
+      val[h] = i;
+    }
+    __syncthreads();
+    const uint64_t he = A.hoff[ra + 1];
+    for (uint64_t e = A.hoff[ra] + w; e < he; e += kW) {
+      const uint32_t rb = A.hnbr[e], osb = A.hos[e];
+      // the masks of the triple overlap: over a's members, or over b's when a
+      // has more than 64 (b's entry of a precedes its entries above a)
+      const bool by_b = !exact && (osb >> 8) <= 64;
+      const uint64_t bo = A.off[A.slot[rb]];
+      const uint64_t mab = exact ? A.mask[ao + A.hpos[e]] : by_b ? A.mask[bo + A.hpos[A.hnext[e] - 1]] : 0;
+      const uint64_t end = A.hoff[rb + 1];
+      uint64_t j = (uint64_t)A.hnext[e] + lane;
+      uint32_t rc = kEmpty, osc = 0;
+      if (j < end) {
+        rc = __ldg(A.hnbr + j);
+        osc = __ldg(A.hos + j);
+      }
+      for (uint64_t j0 = A.hnext[e]; j0 < end; j0 += kWarp) {
+        j += kWarp;  // the next round's entries are loaded before this round's tests
+        uint32_t rn = kEmpty, on = 0;
+        if (j < end) {
+          rn = __ldg(A.hnbr + j);
+          on = __ldg(A.hos + j);
+        }
+        bool push = false;
+        uint64_t rec = 0;
+        if (rc != kEmpty) {
+          uint32_t bk = (rc * 2654435761u) >> shift;
+          int t;
+          for (;;) {
+            const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
+            t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
+            if (t >= 0 || k4.w == kEmpty) break;
+            bk = (bk + 1) & bmask;
+          }
+          if (t >= 0) {
+            const uint64_t at = ao + val[4 * bk + (uint32_t)t];
+            const uint64_t v = exact ? __ldg(A.mask + at) : (uint64_t)__ldg(A.ovl + at);
+            const uint32_t cac = exact ? (uint32_t)__popcll(v) : (uint32_t)v;
+            if (cac < 2 || rb > rc) {  // three heavy pairs: once, b ranked highest
+              const uint32_t g = exact  ? (uint32_t)__popcll(mab & v)
+                                 : by_b ? (uint32_t)__popcll(mab & __ldg(A.mask + bo + A.hpos[j - kWarp]))
+                                        : merge3(A, a, A.slot[rb], A.slot[rc]);
+              push = true;
+              rec = pack6(osb >> 8, osc >> 8, osb & 0xffu, osc & 0xffu, cac, g);
+            }
+          }
+        }
+        queue_records(W, cls, sa, push, rec, q, qn);
+        if ((tests += kWarp) >= kFlushTests) {
+          flush_counts(W, A.raw);
+          tests = 0;
+        }
+        rc = rn;
+        osc = on;
+      }
+    }
+    __syncwarp();
+    if (lane < qn) add_record(W, cls, sa, q[lane]);  // the centre's last triangles (they depend on |a|)
+    qn = 0;
+    __syncthreads();
+  }
+  flush_counts(W, A.raw);
+}
+
+// The same for centres of at most 32 members (32-bit masks, the bulk) or 64,
+// with most triangles counted in a histogram instead of queued. For one (a, b) a
+// triangle's contributions depend on C_bc, C_ac, g and |c| (only up to
+// C_bc + C_ac + 1), and most overlaps are 1 to 3: those go to 192 bins per
+// warp, which become weighted records when the walk of b's row ends. Rows
+// shorter than kHistMin queue every triangle. The enumeration is issue-bound
+// (87 % of the issue slots with one record per triangle), so instructions per
+// test are what counts. Graphs of up to kDenseSlots hyperedges index their
+// table by rank and need no hash.
+constexpr uint32_t kHistMin = 96, kHistMax = 1u << 21, kHistBins = 192;
+constexpr unsigned kFastThreads = 512, kFastWarps = kFastThreads / kWarp, kFastCol = 4, kFastSlots = 4096;
+struct FastWarp {
+  WarpCounts<kFastCol> counts;
+  uint64_t q[2 * kWarp];
+  uint32_t hist[kHistBins];
+};
+template <class Mask>
+constexpr size_t fast_smem() { return kFastWarps * sizeof(FastWarp) + kFastSlots * (sizeof(uint32_t) + sizeof(Mask)); }
+constexpr size_t kDenseSmem = kFastWarps * sizeof(FastWarp) + kDenseSlots * sizeof(uint32_t);
+static_assert(fast_smem<uint64_t>() <= 113 * 1024 && kDenseSmem <= 113 * 1024, "two blocks per SM");
+
+template <bool kDense, class Mask>
+__global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t n_ranks) {
+  extern __shared__ uint64_t smem64[];
+  FastWarp* F = reinterpret_cast<FastWarp*>(smem64) + threadIdx.x / kWarp;
+  WarpCounts<kFastCol>* W = &F->counts;
+  Mask* val = reinterpret_cast<Mask*>(reinterpret_cast<FastWarp*>(smem64) + kFastWarps);
+  uint32_t* keys = reinterpret_cast<uint32_t*>(val + kFastSlots);  // hash only
+  auto bits = [](Mask m) { return (uint32_t)(sizeof(Mask) == 8 ? __popcll(m) : __popc((uint32_t)m)); };
+  __shared__ int8_t cls[128];
+  __shared__ uint32_t s_item;
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  fill_classes(cls);
+  clear_counts(W);
+  for (unsigned k = lane; k < kHistBins; k += kWarp) F->hist[k] = 0;
+  uint32_t qn = 0, tests = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= A.n_work) break;
+    const uint32_t ra = A.work[it], a = A.slot[ra];
+    const uint64_t ao = A.off[a];
+    const uint32_t al = A.len[a];
+    const uint32_t sa = A.esize[a];
+    uint32_t shift = 0, bmask = 0;
+    if (kDense) {
+      const uint32_t quads = (n_ranks - ra + 3) / 4;  // places ra + 1 .. n_ranks - 1, at rank - ra
+      for (uint32_t i = threadIdx.x; i < quads; i += kFastThreads)
+        reinterpret_cast<uint4*>(val)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+      uint32_t slots = 64;
+      while (slots < 2 * al && slots < kFastSlots) slots <<= 1;
+      shift = 32u - (31u - (uint32_t)__clz(slots / 4));
+      bmask = slots / 4 - 1;
+      for (uint32_t i = threadIdx.x; i < slots; i += kFastThreads) keys[i] = kEmpty;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < al; i += kFastThreads) {
+      const uint32_t key = __ldg(A.rank + __ldg(A.nbr + ao + i));
+      if (key <= ra) continue;
+      const Mask m = (Mask)__ldg(A.mask + ao + i);
+      if (kDense) {
+        val[key - ra] = m;
+      } else {
+        uint32_t bk = (key * 2654435761u) >> shift, h = 0;
+        for (bool done = false; !done; bk = (bk + 1) & bmask)
+          for (uint32_t t = 0; t < 4; ++t)
+            if (atomicCAS(&keys[4 * bk + t], kEmpty, key) == kEmpty) {
+              h = 4 * bk + t;
+              done = true;
+              break;
+            }
+        val[h] = m;
+      }
+    }
+    __syncthreads();
+    const uint64_t he = A.hoff[ra + 1];
+    for (uint64_t e = A.hoff[ra] + w; e < he; e += kFastWarps) {
+      const uint32_t rb = A.hnbr[e], osb = A.hos[e];
+      const Mask mab = (Mask)A.mask[ao + A.hpos[e]];
+      const uint32_t first = A.hnext[e], n = (uint32_t)(A.hoff[rb + 1] - first);
+      const bool bins = n >= kHistMin && n <= kHistMax;
+      const uint32_t* hn = A.hnbr + first;
+      const uint16_t* ho = A.hos + first;
+      uint32_t rc = kEmpty, osc = 0;
+      if (lane < n) {
+        rc = __ldg(hn + lane);
+        osc = __ldg(ho + lane);
+      }
+      for (uint32_t j0 = 0; j0 < n; j0 += kWarp) {
+        const uint32_t jn = j0 + kWarp + lane;  // the next round's entries are loaded before this round's tests
+        uint32_t rn = kEmpty, on = 0;
+        if (jn < n) {
+          rn = __ldg(hn + jn);
+          on = __ldg(ho + jn);
+        }
+        Mask v = 0;
+        if (rc != kEmpty) {
+          if (kDense) {
+            v = val[rc - ra];
+          } else {
+            uint32_t bk = (rc * 2654435761u) >> shift;
+            int t;
+            for (;;) {
+              const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
+              t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
+              if (t >= 0 || k4.w == kEmpty) break;
+              bk = (bk + 1) & bmask;
+            }
+            if (t >= 0) v = val[4 * bk + (uint32_t)t];
+          }
+        }
+        const uint32_t cac = bits(v);
+        bool push = false;
+        uint64_t rec = 0;
+        if (v && (cac < 2 || rb > rc)) {  // three heavy pairs: once, b ranked highest
+          const uint32_t g = bits(v & mab), cbc = osc & 0xffu, sc = osc >> 8;
+          if (bins && cbc <= 3 && cac <= 3) {
+            atomicAdd(&F->hist[cac * 64 + cbc * 32 + g * 8 + min(sc, 7u) - 128], 1u);
+          } else {
+            push = true;
+            rec = pack6(osb >> 8, sc, osb & 0xffu, cbc, cac, g);
+          }
+        }
+        queue_records(W, cls, sa, push, rec, F->q, qn);
+        if (n > kHistMax && (j0 & (kHistMax - 1)) == kHistMax - kWarp) flush_counts(W, A.raw);
+        rc = rn;
+        osc = on;
+      }
+      if ((tests += min(n, kHistMax)) >= kFlushTests - kHistMax) {
+        flush_counts(W, A.raw);
+        tests = 0;
+      }
+      if (bins) {
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < kHistBins; k0 += kWarp) {
+          const uint32_t k = k0 + lane + 128;
+          uint32_t c = F->hist[k - 128];
+          if (c) F->hist[k - 128] = 0;
+          while (__any_sync(0xffffffffu, c != 0)) {
+            const uint32_t m = min(c, 0xffffu);
+            c -= m;
+            // bits: |c| (7 standing for 7 or more) 0-2, g 3-4, C_bc - 2 5, C_ac from 6 (biased by 2)
+            queue_records(W, cls, sa, m != 0, pack6(osb >> 8, k & 7u, osb & 0xffu, 2 + ((k >> 5) & 1u), (k >> 6) - 1, (k >> 3) & 3u, m),
+                          F->q, qn);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (lane < qn) add_record(W, cls, sa, F->q[lane]);  // the centre's last triangles (they depend on |a|)
+    qn = 0;
+    __syncthreads();
+  }
+  flush_counts(W, A.raw);
+}
+
+static_assert(kHHSmall <= kFastSlots * 3 / 4, "table load");
+constexpr size_t node_smem(unsigned slots) { return slots * (sizeof(uint2) + sizeof(uint32_t)); }
+constexpr unsigned kNodeSlots = 4096, kNodeBigSlots = 16384;
+static_assert(kNodeSmall <= kNodeSlots * 3 / 4 && kNodeLarge <= kNodeBigSlots * 3 / 4, "table load");
+
+// The parts of a count that run in small blocks, side by side in one launch:
+// blocks [0, end[0]) search, [end[0], end[1]) sum the heavy pairs, then node
+// triangles of the short rows, open pairs, stars. At small sizes each part is
+// one wave of latency, so one launch takes as long as its slowest part.
+struct PartArgs {
+  HHArgs search;
+  PairArgs pairs;
+  NodeArgs nodes;
+  const uint32_t* h2h_len;
+  uint32_t n;         // slots
+  unsigned end[5];
+};
+union PartShared {
+  SearchShared search;
+  PairCounts pairs;
+  NodeWarp nodes[kWarps];
+  OpenHist open;
+};
+__global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ PartArgs A) {
+  __shared__ __align__(16) unsigned char mem[sizeof(PartShared)];
+  PartShared& S = *reinterpret_cast<PartShared*>(mem);
+  const unsigned b = blockIdx.x;
+  if (b < A.end[0]) {
+    part_search(A.search, S.search);
+  } else if (b < A.end[1]) {
+    part_pairs(b - A.end[0], A.end[1] - A.end[0], S.pairs, A.pairs);
+  } else if (b < A.end[2]) {
+    part_nodes(A.nodes, &S.nodes[threadIdx.x / kWarp]);
+  } else if (b < A.end[3]) {
+    part_open(b - A.end[2], A.end[3] - A.end[2], S.open, A.search.slot, A.n, A.search.voff, A.search.vmem,
+              A.search.esize, A.h2h_len, A.pairs.ncat, A.search.hoff, A.search.hos, A.search.raw);
+  } else {
+    part_stars(b - A.end[3], A.end[4] - A.end[3], A.pairs.ncat, A.pairs.n_nodes, A.search.raw);
+  }
+}
+
+// The counter block of the static count (hm_static.cu: 30 closed classes, 6
+// removals, 6 open-pair counts) from the raw sums.
+__global__ void k_decomp_finish(const unsigned long long* raw, unsigned long long* out) {
+  __shared__ unsigned long long s[kRawSize], o[42];
+  const unsigned t = threadIdx.x;
+  for (unsigned k = t; k < kRawSize; k += blockDim.x) s[k] = raw[k];
+  __syncthreads();
+  for (unsigned k = t; k < 42; k += blockDim.x)
+    o[k] = k < 30 ? s[kRawClass + k] : k < 36 ? s[kRawRem + k - 30] : s[kRawOpen + k - 36];
+  __syncthreads();
+  if (t == 0) {
+    for (unsigned k = 0; k < 4; ++k) {
+      const unsigned long long n = s[kRawDist + k];
+      o[26 + k] += n;
+      o[35] += k * n;
+      o[34] += (3 - k) * n;
+    }
+    unsigned i = 0;
+    for (unsigned x = 0; x < 3; ++x)
+      for (unsigned y = x; y < 3; ++y)
+        for (unsigned z = y; z < 3; ++z, ++i) {
+          const unsigned long long n = s[kRawStar + i];
+          const unsigned ex = x > 0, ey = y > 0, ez = z > 0;
+          o[ex + ey + ez] += n;
+          o[30 + (x == 2) + 2 * (ey + ez)] += n;
+          o[30 + (y == 2) + 2 * (ex + ez)] += n;
+          o[30 + (z == 2) + 2 * (ex + ey)] += n;
+        }
+    for (unsigned ua = 0; ua < 3; ++ua)
+      for (unsigned ub = 0; ub < 3; ++ub)
+        for (unsigned c = 0; c < 3; ++c) {
+          const unsigned long long n = s[kRawPair + (ua * 3 + ub) * 3 + c];
+          const unsigned ea = ua > 0, eb = ub > 0, l = c > 0;
+          // regions: a's and b's own, the pair's, the common node, c's own if it has a second member
+          const int pat = (int)(ea | (eb << 1) | (l << 2) | (1u << 3) | (1u << 6));
+          o[static_class_of_pattern(pat)] += n;
+          o[30 + (ua > 1) + 2 * (eb + l)] += n;
+          o[30 + (ub > 1) + 2 * (ea + l)] += n;
+          o[30 + (c == 2) + 4] += n;
+        }
+  }
+  __syncthreads();
+  for (unsigned k = t; k < 42; k += blockDim.x) out[k] = o[k];
+}
+
+unsigned bits_for(uint64_t n) {  // bits of the values 0 .. n - 1
+  unsigned b = 1;
+  while ((1ull << b) < n) ++b;
+  return b;
+}
+
+}  // namespace
+
+static int decomp_attrs() {
+  HM_CUDA(cudaFuncSetAttribute(k_hh_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHHSmem));
+  HM_CUDA(cudaFuncSetAttribute(k_hh_fast<true, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kDenseSmem));
+  HM_CUDA(cudaFuncSetAttribute(k_hh_fast<false, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)fast_smem<uint32_t>()));
+  HM_CUDA(cudaFuncSetAttribute(k_hh_fast<false, uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)fast_smem<uint64_t>()));
+  HM_CUDA(cudaFuncSetAttribute(k_node_tri<kNodeSlots, 512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)node_smem(kNodeSlots)));
+  HM_CUDA(cudaFuncSetAttribute(k_node_tri<kNodeBigSlots, 1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)node_smem(kNodeBigSlots)));
+  return HM_OK;
+}
+
+// Whether the decomposition is the cheaper count, and its structures if so.
+// It enumerates sum h^2 / 2 tests; the oriented rows hold about a quarter of
+// sum d^2 / 2 entries to probe (measured 0.24 to 0.30 on the named laws), and
+// a test costs about as much as a probe, so the line is sum h^2 = sum d^2 / 4.
+static int build_decomp(hm_graph* g) {
+  hm_ctx* ctx = g->ctx;
+  cudaStream_t st = ctx->stream;
+  const uint32_t E = g->n_slots, V = g->n_nodes;
+  Decomp& P = g->decomp;
+  P.release();
+  P.decided = true;
+  if (!E || !V) return HM_OK;
+  DArr<uint32_t> heavy, ids, deg, hcnt;
+  DArr<unsigned long long> sums;
+  HM_TRY(heavy.alloc(ctx, E));
+  HM_TRY(ids.alloc(ctx, E));
+  HM_TRY(deg.alloc(ctx, E));
+  HM_TRY(hcnt.alloc(ctx, E));
+  HM_TRY(sums.alloc(ctx, 4));
+  HM_TRY(P.rank.alloc(ctx, E));
+  HM_TRY(P.slot.alloc(ctx, E));
+  HM_TRY(P.hoff.alloc(ctx, (size_t)E + 1));
+  HM_CUDA(cudaMemsetAsync(sums.p, 0, 4 * sizeof(unsigned long long), st));
+  k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_ovl.p,
+                                                                      g->esize.p, E, heavy.p, ids.p, sums.p);
+  HM_LAUNCH_CHECK();
+  const unsigned bits = bits_for(E);
+  {
+    size_t tb = 0;
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, g->h2h_len.p, deg.p, ids.p, P.slot.p, (int64_t)E, 0, (int)bits,
+                                            st));
+    DArr<uint8_t> tmp;
+    HM_TRY(tmp.alloc(ctx, tb));
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, g->h2h_len.p, deg.p, ids.p, P.slot.p, (int64_t)E, 0, (int)bits,
+                                            st));
+  }
+  k_rank_scatter<<<grid_for(E, kBlock), kBlock, 0, st>>>(P.slot.p, E, heavy.p, P.rank.p, hcnt.p);
+  HM_LAUNCH_CHECK();
+  HM_TRY(exclusive_scan(ctx, hcnt.p, P.hoff.p, E));
+  unsigned long long hs[4];
+  HM_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
+  HM_CUDA(cudaStreamSynchronize(st));
+  const uint64_t h2 = hs[0], d2 = hs[1], pairs = hs[2], nh = hs[3];
+  uint64_t tslots = 1024;
+  while (tslots < 2 * pairs) tslots <<= 1;
+  const size_t need = tslots * sizeof(uint4) + pairs * 36 + nh * (18 + 24);
+  const size_t room = ctx->budget ? ctx->budget - std::min<size_t>(ctx->budget, ctx->used.load()) : SIZE_MAX;
+  if (h2 > d2 / 4 || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
+    P.release();
+    P.decided = true;
+    return HM_OK;
+  }
+  P.nh = nh;
+  HM_TRY(P.hnbr.alloc(ctx, nh));
+  HM_TRY(P.hown.alloc(ctx, nh));
+  HM_TRY(P.hos.alloc(ctx, nh));
+  HM_TRY(P.hpos.alloc(ctx, nh));
+  HM_TRY(P.hnext.alloc(ctx, nh));
+  if (nh) {
+    DArr<uint64_t> key, key_s;
+    DArr<uint32_t> pos, pos_s;
+    HM_TRY(key.alloc(ctx, nh));
+    HM_TRY(key_s.alloc(ctx, nh));
+    HM_TRY(pos.alloc(ctx, nh));
+    HM_TRY(pos_s.alloc(ctx, nh));
+    k_heavy_emit<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.slot.p, P.rank.p, E, g->h2h_off.p,
+                                                                       g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p,
+                                                                       P.hoff.p, bits, key.p, pos.p);
+    HM_LAUNCH_CHECK();
+    size_t tb = 0;
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key_s.p, pos.p, pos_s.p, (int64_t)nh, 0,
+                                            (int)(2 * bits), st));
+    DArr<uint8_t> tmp;
+    HM_TRY(tmp.alloc(ctx, tb));
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key_s.p, pos.p, pos_s.p, (int64_t)nh, 0,
+                                            (int)(2 * bits), st));
+    k_heavy_rows<<<grid_for(nh, kBlock), kBlock, 0, st>>>(key_s.p, pos_s.p, nh, bits, P.slot.p, g->h2h_off.p,
+                                                          g->h2h_ovl.p, g->esize.p, P.hoff.p, P.hnbr.p, P.hown.p,
+                                                          P.hos.p, P.hpos.p, P.hnext.p);
+    HM_LAUNCH_CHECK();
+  }
+  // node graph
+  P.tslots = tslots;
+  HM_TRY(P.ncat.alloc(ctx, 3 * (size_t)V));
+  HM_TRY(P.tab.alloc(ctx, tslots));
+  HM_TRY(P.noff.alloc(ctx, (size_t)V + 1));
+  HM_TRY(P.nlen.alloc(ctx, V));
+  HM_TRY(P.nnbr.alloc(ctx, pairs));
+  HM_TRY(P.nw.alloc(ctx, pairs));
+  HM_TRY(P.hwork.alloc(ctx, E));
+  HM_TRY(P.nwork.alloc(ctx, V));
+  HM_TRY(P.spread.alloc(ctx, E));
+  HM_TRY(P.slist.alloc(ctx, E));
+  DArr<uint32_t> ndeg;     // V degrees, then V write cursors
+  DArr<uint32_t> bk;       // per list: kBuckets counts, kBuckets starts, 4 shape ends
+  DArr<uint8_t> hcode, ncode;
+  constexpr uint32_t kBk = 2 * kBuckets + 4;
+  HM_TRY(ndeg.alloc(ctx, 2 * (size_t)V));
+  HM_TRY(bk.alloc(ctx, 2 * kBk + 1));  // and the number of spreading owners
+  HM_TRY(hcode.alloc(ctx, E));
+  HM_TRY(ncode.alloc(ctx, V));
+  HM_CUDA(cudaMemsetAsync(P.tab.p, 0, sizeof(uint4) * tslots, st));
+  HM_CUDA(cudaMemsetAsync(P.nlen.p, 0, sizeof(uint32_t) * V, st));
+  HM_CUDA(cudaMemsetAsync(ndeg.p, 0, sizeof(uint32_t) * 2 * V, st));
+  HM_CUDA(cudaMemsetAsync(bk.p, 0, sizeof(uint32_t) * (2 * kBk + 1), st));
+  k_node_cats<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p,
+                                                                    g->esize.p, V, P.ncat.p);
+  HM_LAUNCH_CHECK();
+  const uint32_t tmask = (uint32_t)(tslots - 1);
+  k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_mem.p, g->esize.p, E,
+                                                                      P.tab.p, tmask);
+  HM_LAUNCH_CHECK();
+  k_pair_degrees<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p);
+  HM_LAUNCH_CHECK();
+  k_pair_plus_count<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p, P.nlen.p);
+  HM_LAUNCH_CHECK();
+  HM_TRY(exclusive_scan(ctx, P.nlen.p, P.noff.p, V));
+  k_pair_plus_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p, P.noff.p, ndeg.p + V,
+                                                               P.nnbr.p, P.nw.p);
+  HM_LAUNCH_CHECK();
+  k_hh_codes<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.slot.p, P.rank.p, E, g->esize.p, g->h2h_off.p,
+                                                                   g->h2h_len.p, g->h2h_nbr.p, P.hoff.p, P.hnbr.p,
+                                                                   P.hnext.p, hcode.p, bk.p);
+  HM_LAUNCH_CHECK();
+  k_spread_flags<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(
+      P.slot.p, E, P.hoff.p, P.hnbr.p, P.hos.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, ndeg.p, P.spread.p, P.slist.p,
+      bk.p + 2 * kBk);
+  HM_LAUNCH_CHECK();
+  k_node_codes<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(P.noff.p, P.nlen.p, P.nnbr.p, V, ncode.p,
+                                                                     bk.p + kBk);
+  HM_LAUNCH_CHECK();
+  for (int l = 0; l < 2; ++l) {
+    uint32_t* b = bk.p + l * kBk;
+    k_bucket_starts<<<1, kBuckets, 0, st>>>(b, b + kBuckets, b + 2 * kBuckets);
+    HM_LAUNCH_CHECK();
+    const uint32_t n = l ? V : E;
+    k_bucket_scatter<<<grid_for(n, kBlock), kBlock, 0, st>>>(l ? ncode.p : hcode.p, n, b + kBuckets,
+                                                            l ? P.nwork.p : P.hwork.p);
+    HM_LAUNCH_CHECK();
+  }
+  uint32_t ends[2 * kBk + 1];
+  HM_CUDA(cudaMemcpyAsync(ends, bk.p, sizeof(ends), cudaMemcpyDeviceToHost, st));
+  HM_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(P.hend, ends + 2 * kBuckets, sizeof(P.hend));
+  std::memcpy(P.nend, ends + kBk + 2 * kBuckets, sizeof(P.nend));
+  P.n_spread = ends[2 * kBk];
+  if (P.n_spread) {
+    // one node vector per block of k_spread_pairs, a sixteenth of the room at most
+    const size_t vec = ((size_t)V + 1) & ~(size_t)1;
+    P.y_blocks = (uint32_t)std::max<size_t>(
+        1, std::min<size_t>({(size_t)ctx->n_sms, (size_t)P.n_spread, room / 16 / (sizeof(uint2) * vec)}));
+    HM_TRY(P.self.alloc(ctx, g->h2v_tail));
+    HM_TRY(P.y.alloc(ctx, (size_t)P.y_blocks * vec));
+    HM_CUDA(cudaMemsetAsync(P.y.p, 0, sizeof(uint2) * (size_t)P.y_blocks * vec, st));
+    HM_TRY(P.foff.alloc(ctx, (size_t)V + 1));
+    HM_TRY(P.fnbr.alloc(ctx, 2 * pairs));
+    HM_TRY(P.fw.alloc(ctx, 2 * pairs));
+    HM_TRY(exclusive_scan(ctx, ndeg.p, P.foff.p, V));
+    HM_CUDA(cudaMemsetAsync(ndeg.p + V, 0, sizeof(uint32_t) * V, st));
+    k_pair_rows_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, P.foff.p, ndeg.p + V, P.fnbr.p,
+                                                                 P.fw.p);
+    HM_LAUNCH_CHECK();
+  }
+  HM_TRY(P.raw.alloc(ctx, kRawSize));
+  HM_TRY(decomp_attrs());
+  P.usable = true;
+  return HM_OK;
+}
+
+int prepare_decomp(hm_graph* g) {
+  if (g->decomp.decided) return HM_OK;
+  const int s = build_decomp(g);
+  if (s < 0) g->decomp.release();
+  if (s == HM_ERR_NOMEM) {  // no room for it: the enumeration of all triangles needs less
+    g->decomp.decided = true;
+    return HM_OK;
+  }
+  return s;
+}
+
+// One count: the raw sums cleared, the block-per-item launches, the small
+// parts side by side, and the counter block from the sums.
+int launch_decomp(hm_graph* g) {
+  hm_ctx* ctx = g->ctx;
+  cudaStream_t st = ctx->stream;
+  Decomp& P = g->decomp;
+  const unsigned sms = (unsigned)ctx->n_sms;
+  const uint32_t E = g->n_slots, V = g->n_nodes;
+  unsigned int* queue = reinterpret_cast<unsigned int*>(P.raw.p + kRawQueue);
+  HM_CUDA(cudaMemsetAsync(P.raw.p, 0, sizeof(unsigned long long) * kRawSize, st));
+  PartArgs A;
+  A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, g->h2h_off.p, g->h2h_len.p,
+                    g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, nullptr, 0,
+                    nullptr, P.raw.p};
+  A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
+                     g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
+                     (uint32_t)(P.tslots - 1), P.foff.p, P.fnbr.p, P.fw.p, P.spread.p, P.slist.p, P.n_spread, P.self.p, P.y.p,
+                     V, P.nh < kPairFew ? 1u : 4u, P.nh < kPairFew ? 0u : kPairWide, queue + 8, P.raw.p};
+  A.nodes = NodeArgs{P.noff.p, P.nlen.p, P.nnbr.p, P.nw.p, P.tab.p, (uint32_t)(P.tslots - 1), nullptr, 0, nullptr,
+                     P.raw.p};
+  A.h2h_len = g->h2h_len.p;
+  A.n = E;
+  auto hh_part = [&](int k) {
+    const uint32_t b = k ? P.hend[k - 1] : 0;
+    A.search.work = P.hwork.p + b;
+    A.search.n_work = P.hend[k] - b;
+    A.search.queue = queue + k;
+    return A.search.n_work;
+  };
+  auto node_part = [&](int k) {
+    const uint32_t b = k ? P.nend[k - 1] : 0;
+    A.nodes.work = P.nwork.p + b;
+    A.nodes.n_work = P.nend[k] - b;
+    A.nodes.queue = queue + 4 + k;
+    return A.nodes.n_work;
+  };
+  if (const uint32_t n = hh_part(3)) {
+    k_hh_large<<<std::min(sms, n), kHHThreads, kHHSmem, st>>>(A.search);
+    HM_LAUNCH_CHECK();
+  }
+  if (const uint32_t n = hh_part(2)) {
+    k_hh_fast<false, uint64_t><<<std::min(sms * 2, n), kFastThreads, fast_smem<uint64_t>(), st>>>(A.search, E);
+    HM_LAUNCH_CHECK();
+  }
+  if (const uint32_t n = hh_part(1)) {
+    if (E <= kDenseSlots)
+      k_hh_fast<true, uint32_t><<<std::min(sms * 2, n), kFastThreads, kDenseSmem, st>>>(A.search, E);
+    else
+      k_hh_fast<false, uint32_t><<<std::min(sms * 2, n), kFastThreads, fast_smem<uint32_t>(), st>>>(A.search, E);
+    HM_LAUNCH_CHECK();
+  }
+  if (P.n_spread) {
+    k_self_weights<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(A.pairs, E);
+    HM_LAUNCH_CHECK();
+    k_spread_pairs<<<P.y_blocks, kSpreadThreads, 0, st>>>(A.pairs);
+    HM_LAUNCH_CHECK();
+  }
+  if (const uint32_t n = node_part(3)) {
+    k_node_tri<0, 1024, 1><<<std::min(sms * 2, n), 1024, 0, st>>>(A.nodes);
+    HM_LAUNCH_CHECK();
+  }
+  if (const uint32_t n = node_part(2)) {
+    k_node_tri<kNodeBigSlots, 1024, 1><<<std::min(sms, n), 1024, node_smem(kNodeBigSlots), st>>>(A.nodes);
+    HM_LAUNCH_CHECK();
+  }
+  if (const uint32_t n = node_part(1)) {
+    k_node_tri<kNodeSlots, 512, 2><<<std::min(sms * 4, n), 512, node_smem(kNodeSlots), st>>>(A.nodes);
+    HM_LAUNCH_CHECK();
+  }
+  const uint32_t n_search = hh_part(0), n_nodes = node_part(0);
+  auto blocks = [&](uint64_t warps, unsigned most) {
+    return (unsigned)std::min<uint64_t>(sms * most, (warps + kWarps - 1) / kWarps);
+  };
+  unsigned end = 0;
+  A.end[0] = end += blocks(n_search, 4);
+  A.end[1] = end += blocks((P.nh + A.pairs.per_warp - 1) / A.pairs.per_warp, 8);
+  A.end[2] = end += blocks(n_nodes, 8);
+  A.end[3] = end += blocks(E, 8);
+  A.end[4] = end += std::min<unsigned>(sms * 2, (V + kBlock - 1) / kBlock);
+  k_parts<<<end, kBlock, 0, st>>>(A);
+  HM_LAUNCH_CHECK();
+  k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, g->counters.p);
+  HM_LAUNCH_CHECK();
+  return HM_OK;
+}
+
+}  // namespace hm

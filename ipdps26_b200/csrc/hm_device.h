@@ -183,6 +183,57 @@ struct CountCapture {
   }
 };
 
+// What the static count by decomposition (hm_decomp.cu) keeps of a graph:
+// the slots by (degree, id) rank; the heavy rows (neighbours sharing two or
+// more members), by rank and sorted by rank; the node graph (node pairs held
+// by a common hyperedge) as a hash table and as oriented rows; work lists.
+struct Decomp {
+  bool decided = false;  // whether the graph suits it has been looked at
+  bool usable = false;   // it does, and everything below is built
+  DArr<uint32_t> rank, slot;  // slot -> rank, rank -> slot
+  DArr<uint64_t> hoff;        // rank -> its heavy entries
+  DArr<uint32_t> hnbr, hown;  // neighbour's rank, owner's rank
+  DArr<uint16_t> hos;         // (neighbour size << 8) | overlap
+  DArr<uint32_t> hpos;        // place in the owner's H2H row
+  DArr<uint32_t> hnext;       // first entry of the neighbour's row ranked above the owner
+  uint64_t nh = 0;
+  DArr<uint32_t> ncat;        // per node: hyperedges of one, two, more members
+  DArr<uint4> tab;            // node pairs {x, y, W2, W3}
+  uint64_t tslots = 0;
+  DArr<uint64_t> noff;        // oriented node rows
+  DArr<uint32_t> nlen, nnbr;
+  DArr<uint2> nw;             // {W2, W3}
+  DArr<uint32_t> hwork, nwork;  // centres and nodes by launch shape
+  uint32_t hend[4] = {}, nend[4] = {};
+  DArr<uint8_t> spread;         // per rank: its pairs go through a node vector
+  DArr<uint32_t> slist;         // those ranks
+  uint32_t n_spread = 0, y_blocks = 0;
+  DArr<uint2> self, y, fw;
+  DArr<uint64_t> foff;          // node rows in both directions, for those ranks
+  DArr<uint32_t> fnbr;
+  DArr<unsigned long long> raw;
+  CountCapture capture;
+  void release() {
+    capture.reset();
+    decided = usable = false;
+    nh = tslots = 0;
+    for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist}) a->release();
+    n_spread = y_blocks = 0;
+    spread.release();
+    self.release();
+    y.release();
+    foff.release();
+    fnbr.release();
+    fw.release();
+    hoff.release();
+    hos.release();
+    tab.release();
+    noff.release();
+    nw.release();
+    raw.release();
+  }
+};
+
 }  // namespace hm
 
 // The device-resident hypergraph. Three segment tables share one layout:
@@ -268,6 +319,7 @@ struct hm_graph {
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   bool ev_ready = false;
   hm::CountCapture capture;
+  hm::Decomp decomp;
 
   // temporal (optional): timestamps per slot and the time-ordered index
   hm::DArr<int64_t> ts;
@@ -288,6 +340,7 @@ struct hm_graph {
 
   ~hm_graph() {
     capture.reset();
+    decomp.capture.reset();
     if (ev_ready)
       for (auto& e : ev) cudaEventDestroy(e);
   }
@@ -327,7 +380,11 @@ int exclusive_scan(hm_ctx* ctx, const T* in, uint64_t* out, uint64_t n);
 int count_temporal96_async(hm_graph* g, int64_t delta, uint64_t* d_out96);
 
 // Static count (hm_static.cu).
-int prepare_static(hm_graph* g);
+int prepare_static(hm_graph* g);       // for a full count, by whichever method it takes
+int prepare_enumeration(hm_graph* g);  // oriented rows and work list of the triangle enumeration
+// The count by decomposition (hm_decomp.cu), when g->decomp.usable.
+int prepare_decomp(hm_graph* g);
+int launch_decomp(hm_graph* g);
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags);
 int finish_static(hm_graph* g, uint64_t out30[30]);
 int count_static30(hm_graph* g, uint32_t shard, uint32_t n_shards, uint64_t out30[30]);

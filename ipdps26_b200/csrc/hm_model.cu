@@ -90,7 +90,7 @@ extern "C" int hm_graph_traffic(hm_graph* g, hm_traffic_t* t) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots;
-  HM_TRY(hm::prepare_static(g));
+  HM_TRY(hm::prepare_enumeration(g));
   hm::DArr<uint32_t> dp;
   hm::DArr<unsigned long long> acc;
   hm::DArr<uint8_t> flags;

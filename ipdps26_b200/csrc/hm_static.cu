@@ -27,6 +27,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "hm_classes.h"
@@ -790,9 +791,17 @@ static void with_groups(const hm_graph* g, ClosedArgs& A) {
   A.wopos = g->grp_opos.p;
 }
 
-// Everything the count kernels need that only changes with the graph.
-int prepare_static(hm_graph* g) {
-  hm_ctx* ctx = g->ctx;
+static int prepare_counters(hm_graph* g) {
+  if (!g->counters.p) HM_TRY(g->counters.alloc(g->ctx, 64));
+  if (!g->ev_ready) {
+    for (auto& e : g->ev) HM_CUDA(cudaEventCreate(&e));
+    g->ev_ready = true;
+  }
+  return HM_OK;
+}
+
+// Everything the enumeration kernels need that only changes with the graph.
+int prepare_enumeration(hm_graph* g) {
   if (!g->plus_valid) {
     HM_TRY(build_plus(g));
     g->work_valid = false;
@@ -805,12 +814,21 @@ int prepare_static(hm_graph* g) {
     else HM_TRY(s);
   }
   if (!g->work_valid && g->n_slots) HM_TRY(closed_worklist(g));
-  if (!g->counters.p) HM_TRY(g->counters.alloc(ctx, 64));
-  if (!g->ev_ready) {
-    for (auto& e : g->ev) HM_CUDA(cudaEventCreate(&e));
-    g->ev_ready = true;
-  }
+  HM_TRY(prepare_counters(g));
   return prepare_static_attrs();
+}
+
+// A full count of the graph goes by decomposition where that is the cheaper
+// one (prepare_decomp), else by the enumeration of all triangles. Shards,
+// vertex triads, the traffic diagnostics and hm_debug_static_groups(0) always
+// take the enumeration: a shard's counts are those of its own centres.
+static bool by_decomp(const hm_graph* g) { return g->use_groups && g->decomp.usable; }
+int prepare_static(hm_graph* g) {
+  if (g->use_groups) {
+    HM_TRY(prepare_decomp(g));
+    if (by_decomp(g)) return prepare_counters(g);
+  }
+  return prepare_enumeration(g);
 }
 
 // The closed phase over a work list split at bounds[0..3]: rows longer than
@@ -865,6 +883,27 @@ static int capture_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
   return HM_OK;
 }
 
+// Replays the two phases' captures, capturing them first when the key has
+// changed.
+template <class F0, class F1>
+static int run_captured(hm_graph* g, CountCapture& C, const uint64_t key[CountCapture::kKey], F0&& open_phase,
+                        bool any_open, F1&& closed_phase, bool any_closed) {
+  cudaStream_t st = g->ctx->stream;
+  if (!C.valid || std::memcmp(C.key, key, sizeof(C.key)) != 0) {
+    C.reset();
+    if (any_open) HM_TRY(capture_graph(st, open_phase, &C.exec[0]));
+    if (any_closed) HM_TRY(capture_graph(st, closed_phase, &C.exec[1]));
+    std::memcpy(C.key, key, sizeof(C.key));
+    C.valid = true;
+  }
+  HM_CUDA(cudaEventRecord(g->ev[0], st));
+  if (C.exec[0]) HM_CUDA(cudaGraphLaunch(C.exec[0], st));
+  HM_CUDA(cudaEventRecord(g->ev[1], st));
+  if (C.exec[1]) HM_CUDA(cudaGraphLaunch(C.exec[1], st));
+  HM_CUDA(cudaEventRecord(g->ev[2], st));
+  return HM_OK;
+}
+
 // Launches both phases for one shard of the centres; the counters land in
 // g->counters ([0,30) closed classes, [30,36) open-pair removals, [36,42)
 // open-pair counts, [42..44] work queues). edge_flags is for diagnostics.
@@ -873,6 +912,15 @@ static int capture_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
 // the shard) is unchanged; the diagnostic form launches directly.
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags) {
   hm_ctx* ctx = g->ctx;
+  if (n_shards == 1 && !edge_flags && by_decomp(g)) {
+    const uint64_t key[CountCapture::kKey] = {
+        (uint64_t)g->h2h_off.p, (uint64_t)g->h2h_len.p, (uint64_t)g->h2h_nbr.p, (uint64_t)g->h2h_ovl.p,
+        (uint64_t)g->h2h_mask.p, (uint64_t)g->h2v_off.p, (uint64_t)g->h2v_mem.p, (uint64_t)g->esize.p,
+        (uint64_t)g->counters.p};
+    // one graph: its parts run side by side, so the open pairs have no time of their own
+    auto count = [&]() { return launch_decomp(g); };
+    return run_captured(g, g->decomp.capture, key, count, false, count, true);
+  }
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots;
   unsigned long long* dev = g->counters.p;
@@ -911,24 +959,9 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
       g->n_work_big,           g->n_work_mid,            shard,                   n_shards,
       (uint64_t)args.wnbr,     (uint64_t)args.wos,       (uint64_t)args.wbase,    (uint64_t)args.wtab,
       (uint64_t)args.wopos,    (uint64_t)g->h2h_mask.p,  0};
-  CountCapture& C = g->capture;
-  bool same = C.valid;
-  for (unsigned k = 0; k < CountCapture::kKey && same; ++k) same = C.key[k] == key[k];
-  if (!same) {
-    C.reset();
-    HM_TRY(capture_graph(st, open_phase, &C.exec[0]));
-    bool any_closed = false;
-    for (int part = 0; part < 3; ++part) any_closed = any_closed || bounds[part + 1] - bounds[part] > shard;
-    if (any_closed) HM_TRY(capture_graph(st, closed_phase, &C.exec[1]));
-    for (unsigned k = 0; k < CountCapture::kKey; ++k) C.key[k] = key[k];
-    C.valid = true;
-  }
-  HM_CUDA(cudaEventRecord(g->ev[0], st));
-  HM_CUDA(cudaGraphLaunch(C.exec[0], st));
-  HM_CUDA(cudaEventRecord(g->ev[1], st));
-  if (C.exec[1]) HM_CUDA(cudaGraphLaunch(C.exec[1], st));
-  HM_CUDA(cudaEventRecord(g->ev[2], st));
-  return HM_OK;
+  bool any_closed = false;
+  for (int part = 0; part < 3; ++part) any_closed = any_closed || bounds[part + 1] - bounds[part] > shard;
+  return run_captured(g, g->capture, key, open_phase, true, closed_phase, any_closed);
 }
 
 namespace {
@@ -1130,7 +1163,7 @@ __global__ void k_triads12(const uint64_t* off, const uint32_t* len, const uint3
 int count_vertex_triads(hm_graph* g, uint64_t out3[3]) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
-  HM_TRY(prepare_static(g));
+  HM_TRY(prepare_enumeration(g));
   DArr<unsigned long long> cnt;
   HM_TRY(cnt.alloc(ctx, 8));  // [0] type 3, [1..3] queues, [4] type 1, [5] type 2
   HM_CUDA(cudaMemsetAsync(cnt.p, 0, 8 * sizeof(unsigned long long), st));
@@ -1156,7 +1189,7 @@ int count_vertex_triads(hm_graph* g, uint64_t out3[3]) {
 
 int count_static30(hm_graph* g, uint32_t shard, uint32_t n_shards, uint64_t out30[30]) {
   if (n_shards == 0 || shard >= n_shards) return set_error(HM_ERR_INVALID, "static count: shard %u of %u", shard, n_shards);
-  HM_TRY(prepare_static(g));
+  HM_TRY(n_shards == 1 ? prepare_static(g) : prepare_enumeration(g));
   HM_TRY(launch_static(g, shard, n_shards, nullptr));
   return finish_static(g, out30);
 }
@@ -1216,7 +1249,7 @@ static_assert(kTuneCount <= HM_TUNE_MAX_CANDIDATES, "report holds every candidat
 int autotune_closed(hm_graph* g, uint32_t stride, hm_tune_report& R) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
-  HM_TRY(prepare_static(g));
+  HM_TRY(prepare_enumeration(g));
   R.n_candidates = kTuneCount;
   for (unsigned c = 0; c < kTuneCount; ++c) {
     R.rows[c][0] = kTuneCandidates[c].warp_row;

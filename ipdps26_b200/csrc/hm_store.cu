@@ -438,7 +438,9 @@ void release_plus(hm_graph* g) {
   release_plus_groups(g);
 }
 
+// The static count's own structures: the grouped rows and the decomposition.
 void release_plus_groups(hm_graph* g) {
+  g->decomp.release();
   g->grp_nbr.release();
   g->grp_os.release();
   g->grp_base.release();

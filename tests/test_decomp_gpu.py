@@ -1,0 +1,90 @@
+"""The static count by decomposition (light pairs in closed form, triangles with
+two or three heavy pairs enumerated) at the sizes where its kernels change:
+position masks of 32 and 64 members, centres above 64, tables indexed by rank
+and hashed, short and long heavy rows, spread owners, and graphs it leaves to
+the enumeration of all triangles. Exact integers, so equality."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from tests.helpers import csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(rng, n, n_nodes, sizes, hubs=0, n_hubs=6):
+    """n hyperedges with the given sizes; `hubs` of each one's members come
+    from n_hubs shared nodes (overlaps of two or more)."""
+    out = []
+    for _ in range(n):
+        k = int(rng.choice(sizes))
+        h = min(k, hubs)
+        r = set(rng.choice(n_hubs, size=min(h, n_hubs), replace=False).tolist())
+        while len(r) < k:
+            r.add(int(rng.integers(0, n_nodes)))
+        out.append(sorted(r))
+    return out
+
+
+CASES = {
+    # sizes, hub members per hyperedge, hubs, hyperedges, nodes
+    "sizes-1-to-4": ([1, 2, 3, 4], 1, 40, 900, 300),
+    "masks-31-32-33": ([2, 3, 31, 32, 33], 2, 12, 260, 220),
+    "masks-63-64-65": ([2, 4, 63, 64, 65], 2, 20, 220, 400),
+    "centres-above-64": ([66, 90, 130, 255], 3, 30, 120, 900),
+    "overlaps-past-3": ([6, 7, 8, 9, 10], 5, 9, 300, 60),
+    "rows-of-95-96-97": ([3, 4], 2, 8, 420, 4000),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("seed", range(3))
+def test_decomposition_matches_oracle(ctx, name, seed):
+    from ipdps26_b200 import engine
+
+    sizes, hubs, n_hubs, n, n_nodes = CASES[name]
+    rng = np.random.default_rng(1000 + seed)
+    rows = _rows(rng, n, n_nodes, sizes, hubs, n_hubs) + [[0], [0, 1], [1, 2], [0, 1, 2]]
+    off, mem = csr(rows)
+    want = oracle.static30(off, mem, n_nodes)
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        assert g.count_static30().tolist() == want.tolist()
+        g.set_static_groups(False)
+        assert g.count_static30().tolist() == want.tolist()
+        g.set_static_groups(True)
+        assert g.count_static30().tolist() == want.tolist()
+
+
+@pytest.mark.parametrize("n,law", [(14_335, "small"), (14_336, "small"), (14_337, "small"), (20_000, "wide"),
+                                   (14_000, "wide")])
+def test_decomposition_equals_enumeration(ctx, n, law):
+    """Graphs on both sides of the rank-indexed table's limit, one of them with
+    owners that spread their pairs over a node vector; and after an update."""
+    from ipdps26_b200 import engine, gen
+
+    p = (gen.params(n, n // 2, n, 2, 25, 2.5, 1.2, 60.0) if law == "small"
+         else gen.config2(seed=n, n_nodes=n // 2, n_edges=n, q=10.0))
+    h = gen.static(p)
+    with engine.Graph.from_hypergraph(ctx, h) as g:
+        for _ in range(2):
+            got = g.count_static30()
+            g.set_static_groups(False)
+            assert got.tolist() == g.count_static30().tolist()
+            g.set_static_groups(True)
+            dels, ins = gen.batch(p, 5, g.live_ids(), 200)
+            _, delta = g.apply_batch(dels, ins.offsets, ins.members)
+            after = g.count_static30()
+            assert (got.astype(np.int64) + delta).tolist() == after.astype(np.int64).tolist()
+
+
+def test_all_pairs_heavy_is_enumerated(ctx):
+    """Every pair shares two nodes: the decomposition would enumerate more than
+    the enumeration does, and is not taken."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(3)
+    rows = [[0, 1] + sorted(rng.choice(np.arange(2, 200), size=int(rng.integers(0, 4)), replace=False).tolist())
+            for _ in range(400)]
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, 200) as g:
+        assert g.count_static30().tolist() == oracle.static30(off, mem, 200).tolist()
