@@ -346,9 +346,11 @@ __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t 
   }
 }
 
-// Node rows: one warp (up to 128 neighbours), one block with a 4096-slot or a
-// 16384-slot table, or the global pair table for the longest.
-constexpr uint32_t kNodeWarpRow = 128, kNodeSmall = 3072, kNodeLarge = 12288;
+// Launch shapes of the node triangles: 0 one warp (short rows with little to
+// probe: an item of 128 rows of 100 entries takes one warp 0.2 ms, longer than
+// the rest of a 100K-hyperedge count), 1 and 2 blocks with 1024-slot and
+// 4096-slot tables, 3 the largest table, or the global pair table past it.
+constexpr uint32_t kNodeWarpRow = 128, kNodeWarpWork = 2048, kNodeSmall = 768, kNodeMid = 3072, kNodeLarge = 12288;
 __global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const uint32_t* nbr, uint32_t n,
                              uint8_t* code, uint32_t* hist) {
   for (uint64_t u = global_warp(); u < n; u += n_warps()) {
@@ -358,7 +360,9 @@ __global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const u
       uint64_t work = 0;
       for (uint32_t i = lane_id(); i < d; i += kWarp) work += plen[nbr[poff[u] + i]];
       work = warp_sum(work);
-      if (work) c = bucket_code(d <= kNodeWarpRow ? 0u : d <= kNodeSmall ? 1u : d <= kNodeLarge ? 2u : 3u, work);
+      if (work)
+        c = bucket_code(d <= kNodeWarpRow && work <= kNodeWarpWork ? 0u : d <= kNodeSmall ? 1u : d <= kNodeMid ? 2u : 3u,
+                        work);
     }
     if (lane_id() == 0) {
       code[u] = c;
@@ -417,10 +421,12 @@ __device__ void part_open(unsigned vb, unsigned nb, OpenHist& hist, const uint32
     const uint32_t s = esize[a];
     if (lane == 0) alone += choose3(s);
     if (h2h_len[a] < 2) continue;
-    for (uint32_t i = lane; i <= s; i += kWarp) {
-      hist[w][0][i] = 0;
-      hist[w][1][i] = 0;
-    }
+    const bool heavy = hoff[r + 1] > hoff[r];
+    if (heavy)
+      for (uint32_t i = lane; i <= s; i += kWarp) {
+        hist[w][0][i] = 0;
+        hist[w][1][i] = 0;
+      }
     uint32_t one[2] = {0, 0};
     const uint32_t* m = h2v_mem + h2v_off[a];
     for (uint32_t i = lane; i < s; i += kWarp) {
@@ -440,7 +446,13 @@ __device__ void part_open(unsigned vb, unsigned nb, OpenHist& hist, const uint32
       one[1] += __shfl_xor_sync(0xffffffffu, one[1], d);
     }
     __syncwarp();
-    if (lane == 0) {
+    if (lane == 0 && !heavy) {
+      // every overlap is 1: all pairs agree on [2 < |a|], the class is the ends' alone
+      const uint32_t x = s > 2;
+      acc[x] += choose2(one[0]);
+      acc[2 + x] += (uint64_t)one[0] * one[1];
+      acc[4 + x] += choose2(one[1]);
+    } else if (lane == 0) {
       uint32_t* h0 = hist[w][0];
       uint32_t* h1 = hist[w][1];
       h0[1] += one[0];
@@ -484,35 +496,83 @@ __device__ __forceinline__ void node_insert(uint32_t* keys, uint2* val, uint32_t
   val[h] = v;
 }
 
-// One entry x of v's row (its weights at w) against u's table: if u, v, x is a
-// node triangle, adds it to T[k] by how many of the pairs (u, x) and (v, x)
-// take a hyperedge of three members or more. The weights are loaded on a hit
-// only: most entries miss.
-__device__ __forceinline__ bool node_probe(const uint32_t* keys, const uint2* val, uint32_t shift, uint32_t mask,
-                                           uint32_t x, const uint2* w, uint64_t T[3]) {
-  uint32_t h = node_hash(x, shift);
-  for (;;) {
-    const uint32_t k = keys[h];
-    if (k == x) {
-      const uint2 p = val[h], q = __ldg(w);
-      T[0] += (uint64_t)p.x * q.x;
-      T[1] += (uint64_t)p.x * q.y + (uint64_t)p.y * q.x;
-      T[2] += (uint64_t)p.y * q.y;
-      return true;
-    }
-    if (k == kEmpty) return false;
-    h = (h + 1) & mask;
-  }
+// The node triangles a warp has found and not yet summed: per record the place
+// of u's entry for v in u's row, the slot of the third node in u's table and
+// the place of its entry in v's row. Most looked-up entries miss; a hit's three
+// weights are loaded 32 hits at a time, instead of stalling the walk on each.
+__device__ __forceinline__ uint64_t node_record(uint32_t i, uint32_t slot, uint64_t at) {
+  return ((uint64_t)i << 48) | ((uint64_t)slot << 32) | at;  // i, slot < 2^14, at < 2^31
+}
+__device__ __forceinline__ void node_sum(uint64_t r, const uint2* wu, const uint2* val, const uint2* w, uint64_t F[4]) {
+  const uint2 a = __ldg(wu + (r >> 48)), p = val[(r >> 32) & 0xffffu], q = __ldg(w + (uint32_t)r);
+  const uint64_t t0 = (uint64_t)p.x * q.x, t1 = (uint64_t)p.x * q.y + (uint64_t)p.y * q.x, t2 = (uint64_t)p.y * q.y;
+  F[0] += a.x * t0;
+  F[1] += a.y * t0 + a.x * t1;
+  F[2] += a.y * t1 + a.x * t2;
+  F[3] += a.y * t2;
 }
 
-// Adds p, the weights of (u, v), times T to the sums by number of hyperedges
-// of three members or more.
-__device__ __forceinline__ void node_fold(uint2 p, uint64_t T[3], uint64_t F[4]) {
-  F[0] += p.x * T[0];
-  F[1] += p.y * T[0] + p.x * T[1];
-  F[2] += p.y * T[1] + p.x * T[2];
-  F[3] += p.y * T[2];
-  T[0] = T[1] = T[2] = 0;
+// Whole warp: the rows of u's neighbours i0, i0 + stride, ... (32 of them at
+// most) against u's table. Their bounds are loaded at once, and each chunk of
+// 32 entries while the one before is looked up. With filter (one bit per hash
+// value in 1024, a word per lane) most misses are told by a shuffle.
+template <bool kFilter>
+__device__ __forceinline__ void node_walk(const uint64_t* poff, const uint32_t* plen, const uint32_t* nbr,
+                                          const uint2* w, const uint32_t* keys, const uint2* val, uint32_t shift,
+                                          uint32_t mask, uint32_t filter, uint64_t uo, uint32_t d, uint32_t i0,
+                                          uint32_t stride, uint64_t* q, uint32_t& qn, uint64_t F[4]) {
+  const unsigned lane = lane_id();
+  const uint32_t mine = i0 + lane * stride;
+  uint64_t vo = 0;
+  uint32_t vl = 0;
+  if (mine < d) {
+    const uint32_t v = __ldg(nbr + uo + mine);
+    vo = __ldg(poff + v);
+    vl = __ldg(plen + v);
+  }
+  const uint32_t m = min(kWarp, (d - i0 + stride - 1) / stride);
+  uint64_t o = __shfl_sync(0xffffffffu, vo, 0);
+  uint32_t l = __shfl_sync(0xffffffffu, vl, 0), t = 0, j = lane;
+  uint32_t x = j < l ? __ldg(nbr + o + j) : kEmpty;
+  while (t < m) {
+    const bool last = j - lane + kWarp >= l;  // the row's last chunk
+    const uint32_t tn = t + last;
+    const uint64_t on = __shfl_sync(0xffffffffu, vo, tn & 31u);
+    const uint32_t ln = __shfl_sync(0xffffffffu, vl, tn & 31u), jn = last ? lane : j + kWarp;
+    const uint32_t xn = tn < m && jn < ln ? __ldg(nbr + on + jn) : kEmpty;
+    bool look = x != kEmpty;
+    if (kFilter) {
+      const uint32_t b = node_hash(x, 22);
+      const uint32_t word = __shfl_sync(0xffffffffu, filter, b >> 5);
+      look = look && ((word >> (b & 31u)) & 1u);
+    }
+    bool hit = false;
+    uint32_t h = 0;
+    if (look)
+      for (h = node_hash(x, shift);; h = (h + 1) & mask) {
+        const uint32_t k = keys[h];
+        hit = k == x;
+        if (hit || k == kEmpty) break;
+      }
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    if (bal) {
+      if (hit) q[qn + __popc(bal & lanemask_lt())] = node_record(i0 + t * stride, h, o + j);
+      qn += (uint32_t)__popc(bal);
+      __syncwarp();
+      if (qn >= kWarp) {
+        node_sum(q[lane], w + uo, val, w, F);
+        __syncwarp();
+        if (lane < qn - kWarp) q[lane] = q[kWarp + lane];
+        __syncwarp();
+        qn -= kWarp;
+      }
+    }
+    t = tn;
+    o = on;
+    l = ln;
+    j = jn;
+    x = xn;
+  }
 }
 
 __device__ __forceinline__ void node_flush(const uint64_t F[4], unsigned long long* raw) {
@@ -523,14 +583,14 @@ __device__ __forceinline__ void node_flush(const uint64_t F[4], unsigned long lo
   }
 }
 
-// One warp per node with a short row: its table of 256 slots (load <= 1/2),
-// then the rows of its neighbours one after the other; the row bounds of 32
-// neighbours are loaded at once and the first 32 entries of a row while the
-// row before is probed.
+// One warp per node with a short row: a table of up to 256 slots (load <= 1/2).
+constexpr uint32_t kNodesAlone = 8192;  // items from which they get a launch of their own
 constexpr uint32_t kNodeWarpSlots = 2 * kNodeWarpRow;
 struct NodeWarp {
   uint2 val[kNodeWarpSlots];
+  uint64_t q[2 * kWarp];
   uint32_t keys[kNodeWarpSlots];
+  uint32_t filter[kWarp];
 };
 __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
   const unsigned lane = lane_id();
@@ -545,51 +605,36 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
     const uint32_t u = A.work[it];
     const uint64_t uo = A.poff[u];
     const uint32_t d = A.plen[u];
-    uint32_t slots = 64;
+    uint32_t slots = 64, qn = 0;
     while (slots < 2 * d && slots < kNodeWarpSlots) slots <<= 1;
     const uint32_t shift = 32u - (31u - (uint32_t)__clz(slots)), mask = slots - 1;
     for (uint32_t i = lane; i < slots; i += kWarp) keys[i] = kEmpty;
+    S->filter[lane] = 0;
     __syncwarp();
-    for (uint32_t i = lane; i < d; i += kWarp) node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
-    __syncwarp();
-    for (uint32_t i0 = 0; i0 < d; i0 += kWarp) {
-      uint64_t vo = 0;
-      uint32_t vl = 0;
-      if (i0 + lane < d) {
-        const uint32_t v = A.nbr[uo + i0 + lane];
-        vo = A.poff[v];
-        vl = A.plen[v];
-      }
-      const uint32_t m = min(kWarp, d - i0);
-      uint64_t o = __shfl_sync(0xffffffffu, vo, 0);
-      uint32_t l = __shfl_sync(0xffffffffu, vl, 0);
-      uint32_t x = lane < l ? __ldg(A.nbr + o + lane) : kEmpty;
-      for (uint32_t t = 0; t < m; ++t) {
-        const uint64_t on = __shfl_sync(0xffffffffu, vo, (t + 1) & 31u);
-        const uint32_t ln = __shfl_sync(0xffffffffu, vl, (t + 1) & 31u);
-        const uint32_t xn = t + 1 < m && lane < ln ? __ldg(A.nbr + on + lane) : kEmpty;
-        uint64_t T[3] = {0, 0, 0};
-        bool hit = x != kEmpty && node_probe(keys, val, shift, mask, x, A.w + o + lane, T);
-        for (uint32_t j = kWarp + lane; j < l; j += kWarp)
-          hit |= node_probe(keys, val, shift, mask, __ldg(A.nbr + o + j), A.w + o + j, T);
-        if (__any_sync(0xffffffffu, hit)) node_fold(A.w[uo + i0 + t], T, F);
-        o = on;
-        l = ln;
-        x = xn;
-      }
+    for (uint32_t i = lane; i < d; i += kWarp) {
+      const uint32_t v = A.nbr[uo + i], b = node_hash(v, 22);
+      node_insert(keys, val, shift, mask, v, A.w[uo + i]);
+      atomicOr(&S->filter[b >> 5], 1u << (b & 31u));
     }
+    __syncwarp();
+    const uint32_t filter = S->filter[lane];
+    for (uint32_t i0 = 0; i0 < d; i0 += kWarp)
+      node_walk<true>(A.poff, A.plen, A.nbr, A.w, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
+    if (lane < qn) node_sum(S->q[lane], A.w + uo, val, A.w, F);  // the records name this node's table
     __syncwarp();
   }
   node_flush(F, A.raw);
 }
 
-// One block per node, kTab slots in shared memory (load <= 3/4); kTab = 0:
+// One block per node, kTab slots in shared memory (load <= 3/4); a longer row
 // probes the global pair table instead.
 template <unsigned kTab, unsigned kThreads, unsigned kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
+  constexpr unsigned kW = kThreads / kWarp;
   extern __shared__ uint64_t smem64[];
   uint2* val = reinterpret_cast<uint2*>(smem64);
   uint32_t* keys = reinterpret_cast<uint32_t*>(val + kTab);
+  __shared__ uint64_t queues[kW][2 * kWarp];
   __shared__ uint32_t s_item;
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   uint64_t F[4] = {0, 0, 0, 0};
@@ -601,33 +646,34 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
     const uint32_t u = A.work[it];
     const uint64_t uo = A.poff[u];
     const uint32_t d = A.plen[u];
-    uint32_t slots = 64, shift = 26, mask = 63;
-    if (kTab) {
+    if (d <= kTab / 4 * 3) {
+      uint32_t slots = 64, qn = 0;
       while (slots < 2 * d && slots < kTab) slots <<= 1;
-      shift = 32u - (31u - (uint32_t)__clz(slots));
-      mask = slots - 1;
+      const uint32_t shift = 32u - (31u - (uint32_t)__clz(slots)), mask = slots - 1;
       for (uint32_t i = threadIdx.x; i < slots; i += kThreads) keys[i] = kEmpty;
       __syncthreads();
-      for (uint32_t i = threadIdx.x; i < d; i += kThreads) node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
-    }
-    __syncthreads();
-    for (uint32_t i = w; i < d; i += kThreads / kWarp) {
-      const uint32_t v = A.nbr[uo + i];
-      const uint64_t o = A.poff[v];
-      const uint32_t l = A.plen[v];
-      uint64_t T[3] = {0, 0, 0};
-      for (uint32_t j = lane; j < l; j += kWarp) {
-        const uint32_t x = __ldg(A.nbr + o + j);
-        if (kTab) {
-          node_probe(keys, val, shift, mask, x, A.w + o + j, T);
-        } else {
-          const uint2 p = pair_weight(A.tab, A.tmask, u, x), q = __ldg(A.w + o + j);
-          T[0] += (uint64_t)p.x * q.x;
-          T[1] += (uint64_t)p.x * q.y + (uint64_t)p.y * q.x;
-          T[2] += (uint64_t)p.y * q.y;
+      for (uint32_t i = threadIdx.x; i < d; i += kThreads)
+        node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
+      __syncthreads();
+      for (uint32_t i0 = w; i0 < d; i0 += kW * kWarp)
+        node_walk<false>(A.poff, A.plen, A.nbr, A.w, keys, val, shift, mask, 0, uo, d, i0, kW, queues[w], qn, F);
+      __syncwarp();
+      if (lane < qn) node_sum(queues[w][lane], A.w + uo, val, A.w, F);
+    } else {
+      for (uint32_t i = w; i < d; i += kW) {
+        const uint32_t v = A.nbr[uo + i];
+        const uint2 a = A.w[uo + i];
+        const uint64_t o = A.poff[v];
+        for (uint32_t j = lane; j < A.plen[v]; j += kWarp) {
+          const uint2 p = pair_weight(A.tab, A.tmask, u, __ldg(A.nbr + o + j)), q = __ldg(A.w + o + j);
+          const uint64_t t0 = (uint64_t)p.x * q.x, t1 = (uint64_t)p.x * q.y + (uint64_t)p.y * q.x,
+                         t2 = (uint64_t)p.y * q.y;
+          F[0] += a.x * t0;
+          F[1] += a.y * t0 + a.x * t1;
+          F[2] += a.y * t1 + a.x * t2;
+          F[3] += a.y * t2;
         }
       }
-      node_fold(A.w[uo + i], T, F);
     }
     __syncthreads();
   }
@@ -1456,8 +1502,14 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
 
 static_assert(kHHSmall <= kFastSlots * 3 / 4, "table load");
 constexpr size_t node_smem(unsigned slots) { return slots * (sizeof(uint2) + sizeof(uint32_t)); }
-constexpr unsigned kNodeSlots = 4096, kNodeBigSlots = 16384;
-static_assert(kNodeSmall <= kNodeSlots * 3 / 4 && kNodeLarge <= kNodeBigSlots * 3 / 4, "table load");
+static_assert(kNodeSmall == 1024 / 4 * 3 && kNodeMid == 4096 / 4 * 3 && kNodeLarge == 16384 / 4 * 3, "table load");
+
+// The short node rows alone (k_parts takes them too when they are few): at the
+// registers of its own it keeps 6 blocks per SM, k_parts 4.
+__global__ void __launch_bounds__(kBlock, 6) k_node_tri_warp(NodeArgs A) {
+  __shared__ NodeWarp S[kWarps];
+  part_nodes(A, &S[threadIdx.x / kWarp]);
+}
 
 // The parts of a count that run in small blocks, side by side in one launch:
 // blocks [0, end[0]) search, [end[0], end[1]) sum the heavy pairs, then node
@@ -1556,10 +1608,10 @@ static int decomp_attrs() {
                                (int)fast_smem<uint32_t>()));
   HM_CUDA(cudaFuncSetAttribute(k_hh_fast<false, uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)fast_smem<uint64_t>()));
-  HM_CUDA(cudaFuncSetAttribute(k_node_tri<kNodeSlots, 512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)node_smem(kNodeSlots)));
-  HM_CUDA(cudaFuncSetAttribute(k_node_tri<kNodeBigSlots, 1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)node_smem(kNodeBigSlots)));
+  HM_CUDA(cudaFuncSetAttribute(k_node_tri<4096, 512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)node_smem(4096)));
+  HM_CUDA(cudaFuncSetAttribute(k_node_tri<16384, 1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)node_smem(16384)));
   return HM_OK;
 }
 
@@ -1801,18 +1853,24 @@ int launch_decomp(hm_graph* g) {
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(3)) {
-    k_node_tri<0, 1024, 1><<<std::min(sms * 2, n), 1024, 0, st>>>(A.nodes);
+    k_node_tri<16384, 1024, 1><<<std::min(sms, n), 1024, node_smem(16384), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(2)) {
-    k_node_tri<kNodeBigSlots, 1024, 1><<<std::min(sms, n), 1024, node_smem(kNodeBigSlots), st>>>(A.nodes);
+    k_node_tri<4096, 512, 2><<<std::min(sms * 4, n), 512, node_smem(4096), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(1)) {
-    k_node_tri<kNodeSlots, 512, 2><<<std::min(sms * 4, n), 512, node_smem(kNodeSlots), st>>>(A.nodes);
+    k_node_tri<1024, 256, 6><<<std::min(sms * 6, n), 256, node_smem(1024), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
-  const uint32_t n_search = hh_part(0), n_nodes = node_part(0);
+  const uint32_t n_search = hh_part(0);
+  uint32_t n_nodes = node_part(0);
+  if (n_nodes > kNodesAlone) {
+    k_node_tri_warp<<<std::min(sms * 12, (n_nodes + kWarps - 1) / kWarps), kBlock, 0, st>>>(A.nodes);
+    HM_LAUNCH_CHECK();
+    n_nodes = 0;
+  }
   auto blocks = [&](uint64_t warps, unsigned most) {
     return (unsigned)std::min<uint64_t>(sms * most, (warps + kWarps - 1) / kWarps);
   };
