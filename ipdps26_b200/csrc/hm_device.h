@@ -335,6 +335,11 @@ struct hm_graph {
   hm::DArr<uint64_t> t_voff;    // node -> positions of the events containing it
   hm::DArr<uint32_t> t_vlen;
   hm::DArr<uint32_t> t_vpos;
+  hm::DArr<uint8_t> t_top;      // node -> its signature bit (the 64 in most events), 0xff for the others
+  hm::DArr<uint64_t> t_exact;   // position -> bits of the event's top nodes
+  hm::DArr<uint64_t> t_other;   // position -> hash word of its other members
+  hm::DArr<uint32_t> t_size;    // position -> members
+  hm::DArr<uint32_t> t_rank;    // position -> rank of its time among the distinct times
 
   hm::PhaseTimes times;
 

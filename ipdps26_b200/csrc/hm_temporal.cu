@@ -16,7 +16,9 @@
 // node-set) and the previous position of that static id; node -> positions
 // of the events containing it; static id -> positions of its occurrences.
 //
-// Kernel: one block per event a (position p), over the window [lo, p):
+// Windows of up to 2048 events go to k_temporal_pairs, which looks at every pair
+// of the window's events (see there). The others go to k_temporal, one block per
+// event a (position p), over the window [lo, p):
 //   1. neighbours b of a: walk the window occurrences of a's nodes, keep the
 //      first occurrence of each static id, and accumulate the overlap C_ab and
 //      the positions of a's members it contains (mask) in a shared hash;
@@ -58,10 +60,6 @@ __device__ __forceinline__ uint64_t n_warps() { return ((uint64_t)gridDim.x * bl
 __device__ __forceinline__ uint64_t gtid() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t gstride() { return (uint64_t)gridDim.x * blockDim.x; }
 
-__device__ __forceinline__ int tclass(int s1, int s2, int s3, int c12, int c23, int c31, int g) {
-  return c_temporal[region_pattern(s1, s2, s3, c12, c23, c31, g)];
-}
-
 // ---- index construction --------------------------------------------------------
 
 __global__ void k_row_hash(const uint64_t* off, const uint32_t* len, const uint32_t* mem, uint32_t n, uint64_t* h) {
@@ -101,6 +99,10 @@ __global__ void k_static_ids(const uint64_t* hs, const uint32_t* ev, uint32_t n,
       }
     sid[ev[i]] = rep;
   }
+}
+
+__global__ void k_iota(uint32_t* x, uint32_t n) {
+  for (uint64_t i = gtid(); i < n; i += gstride()) x[i] = (uint32_t)i;
 }
 
 __global__ void k_time_keys(const int64_t* t, uint32_t n, uint64_t* key, uint32_t* idx) {
@@ -150,18 +152,83 @@ __global__ void k_gather_len(const uint32_t* order, uint32_t n, const uint32_t* 
   for (uint64_t p = gtid(); p < n; p += gstride()) out[p] = len[order[p]];
 }
 
-__global__ void k_window_lo(const int64_t* t, uint32_t n, int64_t delta, uint32_t* lo) {
-  for (uint64_t p = gtid(); p < n; p += gstride()) {
-    const int64_t tp = t[p];
-    // first q with t[q] + delta >= t[p]
-    uint32_t l = 0, h = (uint32_t)p;
-    while (l < h) {
-      const uint32_t mid = (l + h) >> 1;
-      if (t[mid] + delta < tp) l = mid + 1;
-      else h = mid;
+// Launch shapes of the count, by the events in the window: 0 a warp per event,
+// 1 and 2 a block per event (all three in k_temporal_pairs), 3 k_temporal. An
+// event of no members or more than kPairMembers always goes to k_temporal.
+constexpr uint32_t kPairCap0 = 64, kPairCap1 = 512, kPairCap2 = 2048;
+// Streams of fewer events than the GPU holds warps give all but the smallest
+// windows a block: the time is then that of the few events one place takes in
+// turn (2,000 events, windows of about 50: 46 us by warps).
+constexpr uint32_t kFewEvents = 6000, kFewCap0 = 8;
+constexpr uint32_t kPairMembers = 32;
+
+// Window start of every position, and the positions of each shape (list k at
+// lists + k n, its length in counts[k]); an empty window has nothing to count.
+// cap0: windows up to it take a warp.
+__global__ void k_window_lo(const int64_t* t, const uint32_t* size, uint32_t n, int64_t delta, uint32_t cap0,
+                            uint32_t* lo, uint32_t* lists, unsigned int* counts) {
+  for (uint64_t p0 = gtid() & ~31ull; p0 < n; p0 += gstride()) {
+    const uint64_t p = p0 + lane_id();
+    int shape = -1;
+    if (p < n) {
+      const int64_t tp = t[p];
+      // first q with t[q] + delta >= t[p]
+      uint32_t l = 0, h = (uint32_t)p;
+      while (l < h) {
+        const uint32_t mid = (l + h) >> 1;
+        if (t[mid] + delta < tp) l = mid + 1;
+        else h = mid;
+      }
+      lo[p] = l;
+      const uint32_t w = (uint32_t)p - l;
+      if (w)
+        shape = size[p] - 1u >= kPairMembers || w > kPairCap2 ? 3 : w > kPairCap1 ? 2 : w > cap0 ? 1 : 0;
     }
-    lo[p] = l;
+    for (int k = 0; k < 4; ++k) {
+      const unsigned m = __ballot_sync(0xffffffffu, shape == k);
+      if (!m) continue;
+      uint32_t base = 0;
+      if (lane_id() == 0) base = atomicAdd(&counts[k], (unsigned)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (shape == k) lists[(uint64_t)k * n + base + __popc(m & ((1u << lane_id()) - 1u))] = (uint32_t)p;
+    }
   }
+}
+
+// Two signature words per event: a bit each for the 64 nodes in most events,
+// and a 64-bit hash of the other members.
+__global__ void k_set_top(const uint32_t* node, uint32_t n, uint8_t* top) {
+  if (threadIdx.x < n) top[node[threadIdx.x]] = (uint8_t)threadIdx.x;
+}
+
+__device__ __forceinline__ uint64_t other_bit(uint32_t v) { return 1ull << ((v * 2654435761u) >> 26); }
+
+__global__ void k_signatures(const uint32_t* order, uint32_t n, const uint64_t* off, const uint32_t* len,
+                             const uint32_t* mem, const uint8_t* top, uint64_t* exact, uint64_t* other,
+                             uint32_t* size) {
+  for (uint64_t p = gtid(); p < n; p += gstride()) {
+    const uint32_t e = order[p], l = len[e];
+    const uint32_t* m = mem + off[e];
+    uint64_t x = 0, o = 0;
+    for (uint32_t i = 0; i < l; ++i) {
+      const uint32_t v = m[i], t = top[v];
+      if (t < 64) x |= 1ull << t;
+      else o |= other_bit(v);
+    }
+    exact[p] = x;
+    other[p] = o;
+    size[p] = l;
+  }
+}
+
+__global__ void k_time_steps(const int64_t* t, uint32_t n, uint32_t* step) {
+  for (uint64_t p = gtid(); p < n; p += gstride()) step[p] = p > 0 && t[p] != t[p - 1];
+}
+
+// Rank of each position's time among the distinct times, from the inclusive
+// sums of the steps (sums[p + 1] = steps up to p).
+__global__ void k_time_ranks(const uint64_t* sums, uint32_t n, uint32_t* rank) {
+  for (uint64_t p = gtid(); p < n; p += gstride()) rank[p] = (uint32_t)sums[p + 1];
 }
 
 // ---- counting --------------------------------------------------------------------
@@ -189,6 +256,8 @@ struct TArgs {
   // each event in its window, [1] adjacent pairs among them, [2] pairs
   // (b, c) with c adjacent to a neighbour b but not to the event
   unsigned long long* stats;
+  const uint32_t* list;      // the first launch's events
+  const unsigned int* n_list;
   unsigned int* queue2;      // the deferred launch's queue
   unsigned int* n_deferred;  // events set aside by the first launch
   uint32_t* deferred;
@@ -260,7 +329,7 @@ constexpr size_t temporal_smem() {
 }
 
 // Block per event; kS hash slots hold up to kM window neighbours. The first
-// launch (kFirst) takes every event and sets aside those with more
+// launch (kFirst) takes the events of shape 3 and sets aside those with more
 // neighbours in a deferred list; the second takes that list with a larger
 // table, and reports an event that overflows it too.
 template <uint32_t kS, uint32_t kM, bool kFirst>
@@ -299,8 +368,8 @@ __global__ void __launch_bounds__(kBlock) k_temporal(TArgs A) {
     }
     __syncthreads();
     const uint32_t item = s_item;
-    if (kFirst ? item >= A.n : item >= *A.n_deferred) break;
-    const uint32_t p = kFirst ? item : A.deferred[item];
+    if (item >= (kFirst ? *A.n_list : *A.n_deferred)) break;
+    const uint32_t p = kFirst ? A.list[item] : A.deferred[item];
     const uint32_t lo = A.lo[p];
     const uint32_t ea = A.order[p];
     const uint32_t sa = A.sp[p];
@@ -530,6 +599,266 @@ __global__ void __launch_bounds__(kBlock) k_temporal(TArgs A) {
   }
 }
 
+// ---- counting: every pair of the window's events ------------------------------------
+//
+// For event a the window's events split into N (sharing a member with a, a's
+// own earlier occurrences included) and O. An instance with its occurrence
+// pair is a pair of window events {i, j} with i in N and j in N, or j in O
+// sharing a member with i; taking events one by one gives each pair of
+// occurrences its own term, so repeated node-sets need no lists, and the
+// motifs 87-96 (copies of one node-set) follow from the same region pattern as
+// the rest. The events of a pair are ordered by time; at equal times j of O
+// comes before i, in N the larger static id first and a's own occurrences last.
+//
+// |i & j| is the popcount of the common bits of the 64 most frequent nodes,
+// exact, plus members outside those, which a 64-bit hash word excludes for
+// nearly all pairs (they hold a quarter of the memberships under Zipf(1.2));
+// the pairs it does not exclude are queued and their member lists merged 32
+// at a time. |a & i & j| comes from the same bits and a mask of a's other
+// members. Counts go to per-warp histograms by region pattern. What a pair
+// costs is instructions (about 60), all its data being in shared memory.
+// Against one block per event that merged member lists for every pair: 200K
+// events, delta 1e3: 19.9 -> 0.81 ms; 30K events, delta 1e5: 85 -> 9.0 ms.
+struct PairArgs {
+  const uint32_t* list;        // positions of the events
+  const unsigned int* n_list;
+  unsigned int* queue;
+  const uint32_t* lo;
+  const uint32_t* sp;
+  const uint32_t* prev;
+  const uint32_t* rank;        // position -> time rank
+  const uint64_t* exact;       // position -> bits of the top nodes, hash of the others
+  const uint64_t* other;
+  const uint32_t* size;
+  const uint32_t* order;
+  const uint64_t* hoff;
+  const uint32_t* hmem;
+  const uint8_t* top;
+  unsigned long long* out;     // 96
+  unsigned long long* stats;
+};
+
+constexpr unsigned kPatterns = 128, kPatternCols = 4;
+
+// One event's window in shared memory: N from the front, O from the back.
+template <uint32_t kCap>
+struct PairWindow {
+  uint64_t exact[kCap], other[kCap];
+  uint64_t when[kCap];   // (time rank << 32) | ~(static id + 1), 0 for a's own id: ascending order
+  uint32_t rest[kCap];   // a's members outside the top nodes that the event holds, by position in a
+  uint32_t meta[kCap];   // size | |a & i| << 8 | first occurrence << 16 | place in the window << 17
+  uint32_t n, o;
+};
+struct PairWarp {
+  uint32_t hist[kPatterns][kPatternCols];
+  uint32_t queue[2 * kWarp];
+};
+template <uint32_t kGroupWarps, uint32_t kCap, unsigned kThreads>
+constexpr size_t pair_smem() {
+  return kThreads / kWarp / kGroupWarps * sizeof(PairWindow<kCap>) + kThreads / kWarp * sizeof(PairWarp);
+}
+
+// kGroupWarps warps (one, or the whole block) per event.
+template <uint32_t kGroupWarps, uint32_t kCap, unsigned kThreads, unsigned kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_temporal_pairs(PairArgs A) {
+  constexpr unsigned kW = kThreads / kWarp, kGroups = kW / kGroupWarps, kGroupThreads = kGroupWarps * kWarp;
+  static_assert(kGroupWarps == 1 || kGroupWarps == kW, "a warp or the block");
+  static_assert(kCap <= 2048, "places take 11 bits");
+  extern __shared__ unsigned long long tsm[];
+  __shared__ int8_t tab[kPatterns];
+  __shared__ uint32_t s_item;
+  const unsigned w = threadIdx.x / kWarp, lane = lane_id();
+  const unsigned gw = kGroupWarps == 1 ? 0 : w, gt = kGroupWarps == 1 ? lane : threadIdx.x;
+  PairWindow<kCap>& S = reinterpret_cast<PairWindow<kCap>*>(tsm)[kGroupWarps == 1 ? w : 0];
+  PairWarp& Q = reinterpret_cast<PairWarp*>(reinterpret_cast<PairWindow<kCap>*>(tsm) + kGroups)[w];
+  auto sync = [&] {
+    if (kGroupWarps == 1) __syncwarp();
+    else __syncthreads();
+  };
+  for (unsigned k = threadIdx.x; k < kPatterns; k += kThreads) tab[k] = c_temporal[k];
+  for (unsigned k = lane; k < kPatterns * kPatternCols; k += kWarp) (&Q.hist[0][0])[k] = 0;
+  __syncthreads();
+  unsigned long long n_nbrs = 0, n_closed = 0, n_open = 0;
+  auto flush = [&] {
+    __syncwarp();
+    for (unsigned k = lane; k < kPatterns; k += kWarp) {
+      unsigned long long t = 0;
+      for (unsigned c = 0; c < kPatternCols; ++c) {
+        t += Q.hist[k][c];
+        Q.hist[k][c] = 0;
+      }
+      if (t && tab[k] >= 0) atomicAdd(&A.out[tab[k]], t);
+    }
+    __syncwarp();
+  };
+  uint32_t counted = 0;  // pairs since the last flush: a bin stays below 2^32
+  const uint32_t n_list = *A.n_list;
+  for (;;) {
+    uint32_t item = 0;
+    if (kGroupWarps == 1) {
+      if (lane == 0) item = atomicAdd(A.queue, 1u);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (lane == 0) S.n = S.o = 0;
+    } else {
+      if (threadIdx.x == 0) {
+        s_item = atomicAdd(A.queue, 1u);
+        S.n = S.o = 0;
+      }
+      __syncthreads();
+      item = s_item;
+    }
+    if (item >= n_list) break;
+    sync();
+    const uint32_t p = A.list[item], lo = A.lo[p];
+    const uint32_t sa = A.sp[p], asz = A.size[p];
+    const uint64_t ea = A.exact[p], ha = A.other[p];
+    const uint32_t* am = A.hmem + A.hoff[A.order[p]];
+    for (uint32_t q0 = lo; q0 < p; q0 += kGroupThreads) {
+      const uint32_t q = q0 + gt;
+      bool in_n = false, in_o = false;
+      uint64_t e = 0, h = 0, when = 0;
+      uint32_t rest = 0, meta = 0;
+      if (q < p) {
+        e = A.exact[q];
+        h = A.other[q];
+        const uint32_t x = A.sp[q], sz = A.size[q], pr = A.prev[q];
+        if (h & ha) {  // a's members outside the top nodes, looked up in the event's list
+          const uint32_t* m = A.hmem + A.hoff[A.order[q]];
+          for (uint32_t i = 0, j = 0; i < asz && j < sz;) {
+            const uint32_t u = am[i], v = m[j];
+            if (u == v && A.top[u] >= 64) rest |= 1u << i;
+            i += u <= v;
+            j += v <= u;
+          }
+        }
+        const uint32_t c = (uint32_t)(__popcll(e & ea) + __popc(rest));
+        const bool first = x != sa && (pr == kNone || pr < lo);
+        when = ((uint64_t)A.rank[q] << 32) | ~(x == sa ? 0u : x + 1u);
+        meta = sz | (c << 8) | ((uint32_t)first << 16) | ((q - lo) << 17);
+        in_n = c != 0;
+        in_o = !in_n;
+        n_nbrs += in_n && first;
+      }
+      const unsigned bn = __ballot_sync(0xffffffffu, in_n), bo = __ballot_sync(0xffffffffu, in_o);
+      uint32_t at_n = 0, at_o = 0;
+      if (lane == 0) {
+        at_n = atomicAdd(&S.n, (uint32_t)__popc(bn));
+        at_o = atomicAdd(&S.o, (uint32_t)__popc(bo));
+      }
+      at_n = __shfl_sync(0xffffffffu, at_n, 0);
+      at_o = __shfl_sync(0xffffffffu, at_o, 0);
+      const unsigned below = (1u << lane) - 1u;
+      if (in_n || in_o) {
+        const uint32_t d = in_n ? at_n + __popc(bn & below) : kCap - 1 - at_o - __popc(bo & below);
+        S.exact[d] = e;
+        S.other[d] = h;
+        S.when[d] = when;
+        S.rest[d] = rest;
+        S.meta[d] = meta;
+      }
+    }
+    sync();
+    const uint32_t n = S.n, o0 = kCap - S.o;  // N is [0, n), O is [o0, kCap)
+    // both in N, |i & j| = c: the region pattern of (earlier, later, a)
+    auto both = [&](uint64_t wi, uint32_t mi, uint64_t wj, uint32_t mj, uint32_t c, uint32_t g) {
+      const int si = mi & 0xffu, sj = mj & 0xffu, ci = (mi >> 8) & 0xffu, cj = (mj >> 8) & 0xffu;
+      const bool ij = wi < wj;
+      const uint32_t xi = si - ci - (int)c + (int)g > 0, xj = sj - cj - (int)c + (int)g > 0;
+      const uint32_t pi = ci > (int)g, pj = cj > (int)g;
+      const uint32_t pat = ((ij ? xi : xj) | ((ij ? xj : xi) << 1)) | ((uint32_t)((int)asz - ci - cj + (int)g > 0) << 2) |
+                           ((uint32_t)(c > g) << 3) | ((ij ? pj : pi) << 4) | ((ij ? pi : pj) << 5) |
+                           ((uint32_t)(g > 0) << 6);
+      atomicAdd(&Q.hist[pat][lane & (kPatternCols - 1)], 1u);
+      n_closed += c != 0 && ((mi & mj) >> 16 & 1u);
+    };
+    // j in O, c > 0: open at i
+    auto open = [&](uint64_t wi, uint32_t mi, uint64_t wj, uint32_t mj, uint32_t c) {
+      const int si = mi & 0xffu, sj = mj & 0xffu, ci = (mi >> 8) & 0xffu;
+      const bool ij = (uint32_t)(wi >> 32) < (uint32_t)(wj >> 32);  // equal times: j first
+      const uint32_t xi = si - ci - (int)c > 0, xj = sj - (int)c > 0;
+      const uint32_t pat = ((ij ? xi : xj) | ((ij ? xj : xi) << 1)) | ((uint32_t)((int)asz > ci) << 2) | (1u << 3) |
+                           (ij ? 1u << 5 : 1u << 4);
+      atomicAdd(&Q.hist[pat][lane & (kPatternCols - 1)], 1u);
+      n_open += (mi & mj) >> 16 & 1u;
+    };
+    // a queued pair (i, j): the member lists merged
+    auto merged = [&](uint32_t r) {
+      const uint32_t i = r & 0xfffu, j = r >> 12;
+      const uint32_t mi = S.meta[i], mj = S.meta[j];
+      const uint32_t* x = A.hmem + A.hoff[A.order[lo + (mi >> 17)]];
+      const uint32_t* y = A.hmem + A.hoff[A.order[lo + (mj >> 17)]];
+      uint32_t first;
+      const uint32_t c = overlap(x, mi & 0xffu, y, mj & 0xffu, first);
+      if (j < n)
+        both(S.when[i], mi, S.when[j], mj, c,
+             (uint32_t)(__popcll(S.exact[i] & S.exact[j] & ea) + __popc(S.rest[i] & S.rest[j])));
+      else if (c)
+        open(S.when[i], mi, S.when[j], mj, c);
+    };
+    uint32_t qn = 0;
+    auto defer = [&](bool push, uint32_t i, uint32_t j) {  // whole warp
+      const unsigned bal = __ballot_sync(0xffffffffu, push);
+      if (!bal) return;
+      if (push) Q.queue[qn + __popc(bal & ((1u << lane) - 1u))] = i | (j << 12);
+      qn += (uint32_t)__popc(bal);
+      __syncwarp();
+      if (qn >= kWarp) {
+        merged(Q.queue[lane]);
+        __syncwarp();
+        if (lane < qn - kWarp) Q.queue[lane] = Q.queue[kWarp + lane];
+        __syncwarp();
+        qn -= kWarp;
+      }
+    };
+    for (uint32_t i = gw; i < n; i += kGroupWarps) {
+      const uint64_t ei = S.exact[i], hi = S.other[i], wi = S.when[i];
+      const uint32_t ri = S.rest[i], mi = S.meta[i];
+      for (uint32_t j0 = i + 1; j0 < n; j0 += kWarp) {
+        const uint32_t j = j0 + lane;
+        bool push = false;
+        if (j < n) {
+          push = (hi & S.other[j]) != 0;
+          if (!push) {
+            const uint64_t e = ei & S.exact[j];
+            both(wi, mi, S.when[j], S.meta[j], (uint32_t)__popcll(e),
+                 (uint32_t)(__popcll(e & ea) + __popc(ri & S.rest[j])));
+          }
+        }
+        defer(push, i, j);
+      }
+      for (uint32_t j0 = o0; j0 < kCap; j0 += kWarp) {
+        const uint32_t j = j0 + lane;
+        bool push = false;
+        if (j < kCap) {
+          push = (hi & S.other[j]) != 0;
+          const uint64_t e = ei & S.exact[j];
+          if (!push && e) open(wi, mi, S.when[j], S.meta[j], (uint32_t)__popcll(e));
+        }
+        defer(push, i, j);
+      }
+    }
+    __syncwarp();
+    if (lane < qn) merged(Q.queue[lane]);
+    counted += kCap * kCap / 2;
+    if (counted >= (1u << 31)) {
+      flush();
+      counted = 0;
+    }
+    sync();
+  }
+  flush();
+  for (int d = 16; d; d >>= 1) {
+    n_nbrs += __shfl_xor_sync(0xffffffffu, n_nbrs, d);
+    n_closed += __shfl_xor_sync(0xffffffffu, n_closed, d);
+    n_open += __shfl_xor_sync(0xffffffffu, n_open, d);
+  }
+  if (lane == 0) {
+    if (n_nbrs) atomicAdd(&A.stats[0], n_nbrs);
+    if (n_closed) atomicAdd(&A.stats[1], n_closed);
+    if (n_open) atomicAdd(&A.stats[2], n_open);
+  }
+}
+
 // Table shapes: the first launch's (4 blocks per SM) and the deferred one's.
 constexpr uint32_t kSlotsSmall = 2048, kNbrsSmall = 1024;
 constexpr uint32_t kSlotsLarge = 8192, kNbrsLarge = 4096;
@@ -570,12 +899,8 @@ static int build_temporal_index(hm_graph* g) {
   HM_TRY(sid.alloc(ctx, n));
   k_row_hash<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p, n, hs.p);
   HM_LAUNCH_CHECK();
-  {
-    std::vector<uint32_t> iota(n);
-    for (uint32_t i = 0; i < n; ++i) iota[i] = i;
-    HM_CUDA(cudaMemcpyAsync(ev.p, iota.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-  }
+  k_iota<<<grid_for(n, kBlock), kBlock, 0, st>>>(ev.p, n);
+  HM_LAUNCH_CHECK();
   HM_TRY(sort_pairs(ctx, hs.p, hs_sorted.p, ev.p, ev_sorted.p, n, 64));
   k_static_ids<<<grid_for(n, kBlock), kBlock, 0, st>>>(hs_sorted.p, ev_sorted.p, n, g->h2v_off.p, g->h2v_len.p,
                                                         g->h2v_mem.p, sid.p);
@@ -638,6 +963,38 @@ static int build_temporal_index(hm_graph* g) {
   if (nnz) HM_TRY(sort_pairs(ctx, nk.p, nk_s.p, nv.p, g->t_vpos.p, nnz, vb));
   HM_TRY(g->t_voff.alloc(ctx, (size_t)V + 1));
   HM_TRY(exclusive_scan(ctx, g->t_vlen.p, g->t_voff.p, V));
+  // signatures: the 64 nodes in most events have a bit of their own
+  DArr<uint32_t> vid, vid_s, vlen_s;
+  HM_TRY(vid.alloc(ctx, V));
+  HM_TRY(vid_s.alloc(ctx, V));
+  HM_TRY(vlen_s.alloc(ctx, V));
+  HM_TRY(g->t_top.alloc(ctx, V));
+  HM_CUDA(cudaMemsetAsync(g->t_top.p, 0xff, V, st));
+  if (V) {
+    k_iota<<<grid_for(V, kBlock), kBlock, 0, st>>>(vid.p, V);
+    HM_LAUNCH_CHECK();
+    size_t tb = 0;
+    HM_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, g->t_vlen.p, vlen_s.p, vid.p, vid_s.p, (int64_t)V, 0,
+                                                      eb, st));
+    DArr<uint8_t> tmp;
+    HM_TRY(tmp.alloc(ctx, tb));
+    HM_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.p, tb, g->t_vlen.p, vlen_s.p, vid.p, vid_s.p, (int64_t)V, 0,
+                                                      eb, st));
+    k_set_top<<<1, 64, 0, st>>>(vid_s.p, std::min<uint32_t>(V, 64), g->t_top.p);
+    HM_LAUNCH_CHECK();
+  }
+  HM_TRY(g->t_exact.alloc(ctx, n));
+  HM_TRY(g->t_other.alloc(ctx, n));
+  HM_TRY(g->t_size.alloc(ctx, n));
+  HM_TRY(g->t_rank.alloc(ctx, n));
+  k_signatures<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_order.p, n, g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p,
+                                                        g->t_top.p, g->t_exact.p, g->t_other.p, g->t_size.p);
+  HM_LAUNCH_CHECK();
+  k_time_steps<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, n, plen.p);
+  HM_LAUNCH_CHECK();
+  HM_TRY(exclusive_scan(ctx, plen.p, poff.p, n));
+  k_time_ranks<<<grid_for(n, kBlock), kBlock, 0, st>>>(poff.p, n, g->t_rank.p);
+  HM_LAUNCH_CHECK();
   HM_CUDA(cudaStreamSynchronize(st));
   g->t_ready = true;
   return HM_OK;
@@ -653,22 +1010,52 @@ __global__ void k_temporal_finish(const unsigned long long* acc, uint64_t* out96
 }  // namespace
 
 // Queues the window starts and the counting kernels on the context stream:
-// acc receives the 96 counts, [96] the work queue, [97] the overflow flag,
-// [98..100] the window-projection sizes, [101] the deferred launch's queue,
-// [102] the number of deferred events; lo holds the window starts and then
-// the deferred events. Events e0/e1 bracket the kernels.
+// acc receives the 96 counts, [96] unused, [97] the overflow flag, [98..100]
+// the window-projection sizes, [101] the deferred launch's queue, [102] the
+// number of deferred events, [103..106] queues and [107..110] lengths of the
+// four shapes' lists; lo holds the window starts, the lists and the deferred
+// events. Events e0/e1 bracket the kernels.
+constexpr size_t kAccSize = 111;
+template <uint32_t kGroupWarps, uint32_t kCap, unsigned kThreads, unsigned kMinBlocks>
+static int launch_pairs(hm_ctx* ctx, const PairArgs& A, uint32_t n) {
+  constexpr size_t smem = pair_smem<kGroupWarps, kCap, kThreads>();
+  static_assert(smem * kMinBlocks <= 226 * 1024, "blocks per SM");
+  HM_CUDA(cudaFuncSetAttribute(k_temporal_pairs<kGroupWarps, kCap, kThreads, kMinBlocks>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr uint32_t per_block = kThreads / kWarp / kGroupWarps;
+  const unsigned grid = std::min<unsigned>((unsigned)ctx->n_sms * kMinBlocks, (n + per_block - 1) / per_block);
+  k_temporal_pairs<kGroupWarps, kCap, kThreads, kMinBlocks><<<grid, kThreads, smem, ctx->stream>>>(A);
+  HM_LAUNCH_CHECK();
+  return HM_OK;
+}
+
 static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<unsigned long long>& acc,
                            cudaEvent_t e0, cudaEvent_t e1) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
   const uint32_t n = g->n_slots;
   if (!g->t_ready) HM_TRY(build_temporal_index(g));
-  HM_TRY(lo.alloc(ctx, 2 * (size_t)n));
-  HM_TRY(acc.alloc(ctx, 103));
-  HM_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(unsigned long long) * 103, st));
+  HM_TRY(lo.alloc(ctx, 6 * (size_t)n));
+  HM_TRY(acc.alloc(ctx, kAccSize));
+  HM_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(unsigned long long) * kAccSize, st));
   if (e0) HM_CUDA(cudaEventRecord(e0, st));
-  k_window_lo<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, n, delta, lo.p);
+  uint32_t* lists = lo.p + n;
+  auto u32 = [&](size_t k) { return reinterpret_cast<unsigned int*>(acc.p + k); };
+  unsigned int* counts = u32(107);  // four consecutive counts
+  k_window_lo<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, g->t_size.p, n, delta,
+                                                      n < kFewEvents ? kFewCap0 : kPairCap0, lo.p, lists, counts);
   HM_LAUNCH_CHECK();
+  PairArgs P{nullptr, nullptr, nullptr, lo.p, g->t_static.p, g->t_prev.p, g->t_rank.p, g->t_exact.p, g->t_other.p,
+             g->t_size.p, g->t_order.p, g->h2v_off.p, g->h2v_mem.p, g->t_top.p, acc.p, acc.p + 98};
+  auto shape = [&](int k) {
+    P.list = lists + (size_t)k * n;
+    P.n_list = counts + k;
+    P.queue = u32(103 + k);
+    return P;
+  };
+  HM_TRY((launch_pairs<16, kPairCap2, 512, 2>(ctx, shape(2), n)));
+  HM_TRY((launch_pairs<8, kPairCap1, 256, 5>(ctx, shape(1), n)));
+  HM_TRY((launch_pairs<1, kPairCap0, 256, 5>(ctx, shape(0), n)));
   TArgs A{n,
           g->t_order.p,
           g->t_static.p,
@@ -684,23 +1071,21 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
           g->t_olen.p,
           g->t_opos.p,
           g->t_time.p,
-          reinterpret_cast<unsigned int*>(acc.p + 96),
+          u32(106),
           acc.p,
           reinterpret_cast<int*>(acc.p + 97),
           acc.p + 98,
-          reinterpret_cast<unsigned int*>(acc.p + 101),
-          reinterpret_cast<unsigned int*>(acc.p + 102),
-          lo.p + n};
+          lists + 3 * (size_t)n,
+          counts + 3,
+          u32(101),
+          u32(102),
+          lo.p + 5 * (size_t)n};
   constexpr size_t kSmemSmall = temporal_smem<kSlotsSmall, kNbrsSmall>();
   constexpr size_t kSmemLarge = temporal_smem<kSlotsLarge, kNbrsLarge>();
-  static bool attr = false;
-  if (!attr) {
-    HM_CUDA(cudaFuncSetAttribute(k_temporal<kSlotsSmall, kNbrsSmall, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSmall));
-    HM_CUDA(cudaFuncSetAttribute(k_temporal<kSlotsLarge, kNbrsLarge, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLarge));
-    attr = true;
-  }
+  HM_CUDA(cudaFuncSetAttribute(k_temporal<kSlotsSmall, kNbrsSmall, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kSmemSmall));
+  HM_CUDA(cudaFuncSetAttribute(k_temporal<kSlotsLarge, kNbrsLarge, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kSmemLarge));
   k_temporal<kSlotsSmall, kNbrsSmall, true>
       <<<std::min<unsigned>((unsigned)ctx->n_sms * 4, n), kBlock, kSmemSmall, st>>>(A);
   HM_LAUNCH_CHECK();
@@ -729,7 +1114,7 @@ int count_temporal96(hm_graph* g, int64_t delta, uint64_t out96[96]) {
   HM_CUDA(cudaEventCreate(&e0));
   HM_CUDA(cudaEventCreate(&e1));
   const int rc = launch_temporal(g, delta, lo, acc, e0, e1);
-  unsigned long long h[103];
+  unsigned long long h[103];  // up to the projection sizes
   cudaError_t ce = rc < 0 ? cudaSuccess : cudaMemcpyAsync(h, acc.p, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (rc >= 0 && ce == cudaSuccess) ce = cudaStreamSynchronize(st);
   float ms = 0;

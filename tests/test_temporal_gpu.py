@@ -153,3 +153,33 @@ def test_temporal_window_limit_is_an_error(ctx):
             g.count_temporal(1_000_000)
         assert e.value.status == HM_ERR_LIMIT
         assert g.count_temporal(10).tolist() == oracle.temporal96(off, mem, times, 10).tolist()
+
+
+@pytest.mark.parametrize("ties", [1, 3])
+@pytest.mark.parametrize("window", [31, 63, 64, 65, 511, 512, 513, 2047, 2048, 2049])
+def test_temporal_at_the_window_shapes_edges(ctx, window, ties):
+    """Windows of exactly `window` events (and of one more where times tie),
+    around the sizes where the count changes its launch shape, with events of
+    0, 31, 32, 33 and 40 members (the pair kernel takes 1 to 32), repeated
+    node-sets, and nodes in and outside the 64 with a signature bit of their
+    own. Against the oracle."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(window * 10 + ties)
+    n_nodes = 30 if window < 64 else 5 * window
+    rows = []
+    for i in range(window + 40):
+        if i % 7 == 3 and rows:
+            rows.append(list(rows[int(rng.integers(0, len(rows)))]))
+            continue
+        k = int(rng.choice([1, 2, 3, 4, 5], p=[0.1, 0.4, 0.3, 0.15, 0.05]))
+        if i % 29 == 5 and n_nodes > 100:
+            k = int(rng.choice([0, 31, 32, 33, 40]))
+        rows.append(rng.choice(n_nodes, size=min(k, n_nodes), replace=False).tolist())
+    off, mem = csr(rows)
+    times = (np.arange(len(rows)) // ties * ties).astype(np.int64)
+    want = oracle.temporal96(off, mem, times, window)
+    with engine.Graph(ctx, off, mem, n_nodes, times) as g:
+        assert g.count_temporal(window).tolist() == want.tolist()
+        t = g.temporal_traffic()
+        assert t.events == len(rows) and t.window_neighbours > 0
