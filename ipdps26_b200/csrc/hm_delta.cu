@@ -152,8 +152,9 @@ __device__ uint32_t triple_overlap3(const uint64_t* hoff, const uint32_t* hmem, 
 struct TouchArgs {
   const uint32_t* ids;      // items [0, n_long): slices of rows in global tables
   uint32_t n_long;
-  const uint32_t* short_ids;  // items [n_long, n): whole rows, heaviest first
+  const uint32_t* short_ids;  // items [n_long, n): slices of whole rows, heaviest first
   uint32_t n;
+  uint32_t slices;          // per row of short_ids: item n_long + k is slice k % slices of row k / slices
   const uint8_t* mark;
   const uint64_t* off;
   const uint32_t* len;
@@ -474,7 +475,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_touch_closed(TouchArgs
     const uint32_t item = s_item;
     if (item >= A.n) break;
     const bool long_row = item < A.n_long;
-    const uint32_t m = long_row ? A.ids[item] : A.short_ids[item - A.n_long];
+    const uint32_t rest = item - A.n_long, slice = rest % A.slices;
+    const uint32_t m = long_row ? A.ids[item] : A.short_ids[rest / A.slices];
     const uint32_t row = row_of(A, m);
     if (row != cur_row) {
       if (cur_row != kNoRow) flush_touch(wc, A.out + (size_t)cur_row * kRowStride);
@@ -496,8 +498,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_touch_closed(TouchArgs
     }
     __syncthreads();
     const uint32_t cat_m = size_cat(sm);
-    const uint32_t b_begin = long_row ? A.brange[2 * item] : 0u;
-    const uint32_t b_end = long_row ? A.brange[2 * item + 1] : md;
+    const uint32_t b_begin = long_row ? A.brange[2 * item] : (uint32_t)((uint64_t)md * slice / A.slices);
+    const uint32_t b_end = long_row ? A.brange[2 * item + 1] : (uint32_t)((uint64_t)md * (slice + 1) / A.slices);
     for (uint32_t bi = b_begin + w; bi < b_end; bi += kW) {
       touch_pairs_of_b(A, m, mo, sm, cat_m, bi, T, wc, q, qn);
       __syncwarp();
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_touch_warp(TouchArgs A) {
     if (lane == 0) it = atomicAdd(A.queue, 1u);
     it = __shfl_sync(0xffffffffu, it, 0);
     if (it >= A.n) break;
-    const uint32_t m = A.short_ids[it];
+    const uint32_t m = A.short_ids[it / A.slices], slice = it % A.slices;
     const uint32_t row = row_of(A, m);
     if (row != cur_row) {
       if (cur_row != kNoRow) flush_touch(wc, A.out + (size_t)cur_row * kRowStride);
@@ -551,7 +553,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_touch_warp(TouchArgs A) {
     fill_mark_table(A, mo, md, sm <= 64, keys, sval, T.shift, T.bmask, lane, kWarp);
     __syncwarp();
     const uint32_t cat_m = size_cat(sm);
-    for (uint32_t bi = 0; bi < md; ++bi) {
+    const uint32_t b_end = md * (slice + 1) / A.slices;  // md <= kWarpRow
+    for (uint32_t bi = md * slice / A.slices; bi < b_end; ++bi) {
       touch_pairs_of_b(A, m, mo, sm, cat_m, bi, T, wc, q, qn);
       __syncwarp();
     }
@@ -697,7 +700,15 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
     }
   }
   const uint32_t n_items_long = (uint32_t)oid.size();
-  const uint32_t n_items = n_items_long + (n_large - n_long);  // the large-table launch
+  const unsigned sms = (unsigned)ctx->n_sms;
+  // Launches with fewer rows than places on the GPU split each row's
+  // neighbours into slices (every slice builds the row's table again): a small
+  // batch's time is that of its longest row, walked neighbour by neighbour.
+  auto slices_for = [](uint32_t rows, uint32_t places, uint32_t most) {
+    return rows ? std::min(most, std::max(1u, places / rows)) : 1u;
+  };
+  const uint32_t s_large = slices_for(n_large - n_long, sms, 16);
+  const uint32_t n_items = n_items_long + (n_large - n_long) * s_large;  // the large-table launch
   DArr<uint32_t> d_oid, d_oslots, d_orange;
   DArr<uint64_t> d_ooff;
   DArr<uint4> gtab;
@@ -732,13 +743,12 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
       HM_TRY(s);
     }
   }
-  TouchArgs A{d_oid.p, n_items_long, sids.p + n_long, n_items, mark.p, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
+  TouchArgs A{d_oid.p, n_items_long, sids.p + n_long, n_items, s_large, mark.p, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
               g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, g->plus_off.p, g->plus_len.p,
               g->plus_nbr.p, g->plus_os.p, d_ooff.p, d_oslots.p, d_orange.p, gtab.p,
               rows.gos, rows.rog, by_id, queues, cnt.p};
   if (trace) cudaStreamSynchronize(st);
   auto t_cl0 = std::chrono::steady_clock::now();
-  const unsigned sms = (unsigned)ctx->n_sms;
   cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};
   if (trace)
     for (auto& e : tev) cudaEventCreate(&e);
@@ -752,9 +762,10 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
     TouchArgs B = A;
     B.n_long = 0;
     B.short_ids = sids.p + n_large;
-    B.n = n_mid;
+    B.slices = slices_for(n_mid, sms * 4, 32);
+    B.n = n_mid * B.slices;
     B.queue = queues + 1;
-    k_touch_closed<kMidSlots, kBlock, 4><<<std::min<unsigned>(sms * 4, n_mid), kBlock, touch_smem(kMidSlots), st>>>(B);
+    k_touch_closed<kMidSlots, kBlock, 4><<<std::min<unsigned>(sms * 4, B.n), kBlock, touch_smem(kMidSlots), st>>>(B);
     HM_LAUNCH_CHECK();
   }
   if (trace) cudaEventRecord(tev[2], st);
@@ -763,9 +774,10 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
     TouchArgs C = A;
     C.n_long = 0;
     C.short_ids = sids.p + n_large + n_mid;
-    C.n = n_short;
+    C.slices = slices_for(n_short, sms * 4 * kWarps, 16);
+    C.n = n_short * C.slices;
     C.queue = queues + 2;
-    k_touch_warp<<<std::min<unsigned>(sms * 4, (n_short + kWarps - 1) / kWarps), kBlock, 0, st>>>(C);
+    k_touch_warp<<<std::min<unsigned>(sms * 4, (C.n + kWarps - 1) / kWarps), kBlock, 0, st>>>(C);
     HM_LAUNCH_CHECK();
   }
   if (trace) {
