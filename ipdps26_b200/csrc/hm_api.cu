@@ -85,7 +85,7 @@ extern "C" int hm_graph_destroy(hm_graph* g) {
     CtxLock lock(ctx);
     cudaStreamSynchronize(ctx->stream);
     delete g;
-    hm::trim_pool(ctx);
+    hm::trim_pool(ctx, hm::pool_keep(ctx));
   }
   return HM_OK;
 }

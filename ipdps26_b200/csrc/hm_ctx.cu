@@ -1,5 +1,6 @@
 // Context: device binding, stream, and the device-memory budget every
 // allocation of the engine is charged against.
+#include <algorithm>
 #include <cstdio>
 
 #include "hm_device.h"
@@ -57,10 +58,12 @@ void dev_free(hm_ctx* ctx, void* p, size_t bytes) {
   ctx->used.fetch_sub(bytes);
 }
 
-void trim_pool(hm_ctx* ctx) {
+void trim_pool(hm_ctx* ctx, size_t keep) {
   cudaStreamSynchronize(ctx->stream);
-  cudaMemPoolTrimTo(ctx->pool, 0);
+  cudaMemPoolTrimTo(ctx->pool, keep);
 }
+
+size_t pool_keep(const hm_ctx* ctx) { return std::min(kPoolKeep, ctx->budget / 32); }
 
 }  // namespace hm
 

@@ -42,7 +42,11 @@ namespace hm {
 
 int dev_alloc(hm_ctx* ctx, void** p, size_t bytes);
 void dev_free(hm_ctx* ctx, void* p, size_t bytes);
-void trim_pool(hm_ctx* ctx);  // returns the pool's cached free blocks to the device
+void trim_pool(hm_ctx* ctx, size_t keep = 0);  // returns the pool's cached free blocks past `keep` bytes to the device
+// What the pool keeps cached when a graph or server goes, so that the next one
+// of a context finds its memory mapped: at most kPoolKeep, a 32nd of the budget.
+constexpr size_t kPoolKeep = size_t(256) << 20;
+size_t pool_keep(const hm_ctx* ctx);
 
 // Owning device array; the context's budget is charged for its bytes.
 template <class T>
@@ -89,10 +93,11 @@ bool vmm_available();  // the driver's virtual memory management calls were foun
 // space is reserved ahead and physical chunks are mapped at its end as it
 // grows (CUDA virtual memory management). When the reservation is full a
 // larger one is reserved and the chunks already held are mapped into it, so
-// growth never copies data and never holds two copies at once. Without VMM
-// support on the device it falls back to allocate-copy-free. Each grow and
-// release synchronises the device (chunks are unmapped only when no kernel
-// can use them). Budget-charged like DArr.
+// growth never copies data and never holds two copies at once. Each grow that
+// moves and each release synchronises the device (chunks are unmapped only
+// when no kernel can use them). A small first allocation comes from the
+// context's pool and moves to chunks when it grows; without VMM support all
+// growth is allocate-copy-free. Budget-charged like DArr.
 struct GrowSpace {
   hm_ctx* ctx = nullptr;
   char* base = nullptr;
@@ -102,6 +107,8 @@ struct GrowSpace {
   std::vector<unsigned long long> handles;
   std::vector<size_t> sizes;
   int grow(hm_ctx* c, size_t bytes);  // mapped >= bytes afterwards, contents kept
+  int grow_mapped(size_t bytes);      // the same, in mapped chunks
+  int move_to_chunks(size_t bytes);   // from the pool to mapped chunks
   void shrink(size_t bytes);          // gives back whole chunks past bytes (VMM only)
   void release();
   GrowSpace() = default;

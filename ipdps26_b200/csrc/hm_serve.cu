@@ -713,7 +713,7 @@ extern "C" int hm_serve_destroy(hm_server* s) {
   for (hm_graph* g : s->graphs) delete g;
   delete s->pool;
   s->gos.release();
-  hm::trim_pool(s->ctx);
+  hm::trim_pool(s->ctx, hm::pool_keep(s->ctx));
   delete s;
   return HM_OK;
 }

@@ -613,11 +613,18 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     HM_LAUNCH_CHECK();
   }
   HM_TRY(exclusive_scan(ctx, wedges.p, woff.p, n_rows));
-  std::vector<uint64_t> hw((size_t)n_rows + 1);
-  HM_CUDA(cudaMemcpyAsync(hw.data(), woff.p, sizeof(uint64_t) * ((size_t)n_rows + 1), cudaMemcpyDeviceToHost, st));
+  uint64_t W = 0;
+  HM_CUDA(cudaMemcpyAsync(&W, woff.p + n_rows, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
   wedges.release();
-  const uint64_t W = hw[n_rows];
+  // the rows' offsets are needed on the host only to cut the stream into chunks
+  constexpr uint64_t kChunkCap = 1ull << 28;
+  std::vector<uint64_t> hw;
+  if (W > kChunkCap) {
+    hw.resize((size_t)n_rows + 1);
+    HM_CUDA(cudaMemcpyAsync(hw.data(), woff.p, sizeof(uint64_t) * ((size_t)n_rows + 1), cudaMemcpyDeviceToHost, st));
+    HM_CUDA(cudaStreamSynchronize(st));
+  }
   uint64_t base = 0;
   HM_TRY(reserve(W, &base));
   if (n_rows == 0) return HM_OK;
@@ -640,9 +647,9 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     HM_LAUNCH_CHECK();
     return HM_OK;
   }
-  uint64_t chunk_cap = std::min<uint64_t>(W, 1ull << 28);
+  uint64_t chunk_cap = std::min<uint64_t>(W, kChunkCap);
   uint64_t max_row = 0;
-  for (uint32_t r = 0; r < n_rows; ++r) max_row = std::max(max_row, hw[r + 1] - hw[r]);
+  for (size_t r = 0; r + 1 < hw.size(); ++r) max_row = std::max(max_row, hw[r + 1] - hw[r]);
   if (max_row >= (1ull << 31)) return set_error(HM_ERR_LIMIT, "H2H: one row has %llu wedges", (unsigned long long)max_row);
   chunk_cap = std::max(chunk_cap, max_row);
   DArr<uint32_t> kin, kout, starts, cnt;
@@ -660,11 +667,11 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
   uint64_t out = 0;
   uint32_t r0 = 0;
   while (r0 < n_rows) {
-    uint32_t r1 = r0;
+    uint32_t r1 = hw.empty() ? n_rows : r0;
     while (r1 < n_rows && hw[r1 + 1] - hw[r0] <= chunk_cap) ++r1;
     const uint32_t nrows = r1 - r0;
-    const uint64_t cbase = hw[r0];
-    const uint64_t nk = hw[r1] - cbase;
+    const uint64_t cbase = hw.empty() ? 0 : hw[r0];
+    const uint64_t nk = hw.empty() ? W : hw[r1] - cbase;
     k_expand<<<grid_for((uint64_t)nrows * 32, kBlock), kBlock, 0, st>>>(
         g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p, g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p, woff.p, d_rows, cbase,
         r0, r1, kin.p);
