@@ -176,22 +176,29 @@ __global__ void k_heavy_rows(const uint64_t* key, const uint32_t* pos, uint64_t 
 
 // ---- preparation: node graph --------------------------------------------------------
 
-// Hyperedges of each node by size category (3 per node).
+// Hyperedges of each node by size category (3 per node); with marks, the
+// marked ones alone into ncat_m too.
 __global__ void k_node_cats(const uint64_t* voff, const uint32_t* vlen, const uint32_t* vedge, const uint8_t* esize,
-                            uint32_t n_nodes, uint32_t* ncat) {
+                            const uint8_t* mark, uint32_t n_nodes, uint32_t* ncat, uint32_t* ncat_m) {
   for (uint64_t v = global_warp(); v < n_nodes; v += n_warps()) {
     const uint64_t s = voff[v];
     const uint32_t l = vlen[v];
-    uint32_t c[3] = {0, 0, 0};
+    uint32_t c[6] = {0, 0, 0, 0, 0, 0};
     for (uint32_t i = lane_id(); i < l; i += kWarp) {
-      const uint32_t z = esize[vedge[s + i]];
+      const uint32_t e = vedge[s + i], z = esize[e];
+      const bool m = mark && mark[e];
       c[0] += z == 1;
       c[1] += z == 2;
       c[2] += z >= 3;
+      c[3] += m && z == 1;
+      c[4] += m && z == 2;
+      c[5] += m && z >= 3;
     }
-    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
       for (int d = 16; d; d >>= 1) c[k] += __shfl_xor_sync(0xffffffffu, c[k], d);
-      if (lane_id() == 0) ncat[3 * v + k] = c[k];
+      if (lane_id() == 0 && k < 3) ncat[3 * v + k] = c[k];
+      if (lane_id() == 0 && k >= 3 && mark) ncat_m[3 * v + k - 3] = c[k];
     }
   }
 }
@@ -206,18 +213,20 @@ __device__ __forceinline__ uint32_t pair_hash(uint32_t x, uint32_t y) {
   return h ^ (h >> 13);
 }
 
-__device__ __forceinline__ uint2 pair_weight(const uint4* tab, uint32_t mask, uint32_t x, uint32_t y) {
+// With wm (the marked hyperedges' weights, per table entry) those are returned.
+__device__ __forceinline__ uint2 pair_weight(const uint4* tab, uint32_t mask, uint32_t x, uint32_t y,
+                                             const uint2* wm = nullptr) {
   const uint32_t a = min(x, y), b = max(x, y);
   for (uint32_t h = pair_hash(a, b) & mask;; h = (h + 1) & mask) {
     const uint4 e = __ldg(tab + h);
-    if (e.x == a && e.y == b) return make_uint2(e.z, e.w);
+    if (e.x == a && e.y == b) return wm ? __ldg(wm + h) : make_uint2(e.z, e.w);
     if (e.y == 0) return make_uint2(0, 0);
   }
 }
 
 // One warp per hyperedge, lanes over its node pairs.
-__global__ void k_pair_insert(const uint64_t* off, const uint32_t* mem, const uint8_t* esize, uint32_t n, uint4* tab,
-                              uint32_t mask) {
+__global__ void k_pair_insert(const uint64_t* off, const uint32_t* mem, const uint8_t* esize, const uint8_t* mark,
+                              uint32_t n, uint4* tab, uint2* wm, uint32_t mask) {
   for (uint64_t e = global_warp(); e < n; e += n_warps()) {
     const uint32_t s = esize[e];
     if (s < 2) continue;
@@ -236,6 +245,7 @@ __global__ void k_pair_insert(const uint64_t* off, const uint32_t* mem, const ui
         if (old == 0ull || old == key) break;
       }
       atomicAdd(s == 2 ? &tab[h].z : &tab[h].w, 1u);
+      if (mark && mark[e]) atomicAdd(s == 2 ? &wm[h].x : &wm[h].y, 1u);
     }
   }
 }
@@ -261,8 +271,8 @@ __global__ void k_pair_plus_count(const uint4* tab, uint64_t slots, const uint32
   }
 }
 
-__global__ void k_pair_plus_fill(const uint4* tab, uint64_t slots, const uint32_t* deg, const uint64_t* poff,
-                                 uint32_t* cursor, uint32_t* nbr, uint2* w) {
+__global__ void k_pair_plus_fill(const uint4* tab, const uint2* wm, uint64_t slots, const uint32_t* deg,
+                                 const uint64_t* poff, uint32_t* cursor, uint32_t* nbr, uint2* w, uint2* w_m) {
   for (uint64_t i = gtid(); i < slots; i += gstride()) {
     const uint4 e = tab[i];
     if (!e.y) continue;
@@ -271,6 +281,61 @@ __global__ void k_pair_plus_fill(const uint4* tab, uint64_t slots, const uint32_
     const uint64_t d = poff[u] + atomicAdd(&cursor[u], 1u);
     nbr[d] = v;
     w[d] = make_uint2(e.z, e.w);
+    if (wm) w_m[d] = wm[i];
+  }
+}
+
+// ---- preparation: marked hyperedges ----------------------------------------------------
+// Counting only the triples with a marked hyperedge (see count_touching_decomp):
+// the marks by rank, each heavy row's marked neighbours as a row of their own,
+// and per heavy entry where that row passes the entry's owner.
+
+__global__ void k_rank_marks(const uint32_t* slot, uint32_t n, const uint8_t* mark, uint8_t* rmark) {
+  for (uint64_t r = gtid(); r < n; r += gstride()) rmark[r] = mark[slot[r]];
+}
+
+__global__ void k_marked_count(const uint64_t* hoff, const uint32_t* hnbr, const uint8_t* rmark, uint32_t n,
+                               uint32_t* cnt) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    uint32_t c = 0;
+    for (uint64_t e = hoff[r] + lane_id(); e < hoff[r + 1]; e += kWarp) c += rmark[hnbr[e]];
+    for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
+    if (lane_id() == 0) cnt[r] = c;
+  }
+}
+
+__global__ void k_marked_fill(const uint64_t* hoff, const uint32_t* hnbr, const uint16_t* hos, const uint32_t* hpos,
+                              const uint8_t* rmark, uint32_t n, const uint64_t* moff, uint32_t* mnbr, uint16_t* mos,
+                              uint32_t* mpos) {
+  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
+    uint64_t w = moff[r];
+    if (moff[r + 1] == w) continue;
+    for (uint64_t e0 = hoff[r]; e0 < hoff[r + 1]; e0 += kWarp) {
+      const uint64_t e = e0 + lane_id();
+      const bool keep = e < hoff[r + 1] && rmark[hnbr[e]];
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const uint64_t d = w + __popc(m & lanemask_lt());
+        mnbr[d] = hnbr[e];
+        mos[d] = hos[e];
+        mpos[d] = hpos[e];
+      }
+      w += __popc(m);
+    }
+  }
+}
+
+__global__ void k_marked_next(const uint32_t* hown, const uint32_t* hnbr, uint64_t nh, const uint64_t* moff,
+                              const uint32_t* mnbr, uint32_t* mnext) {
+  for (uint64_t e = gtid(); e < nh; e += gstride()) {
+    const uint32_t r = hown[e];
+    uint64_t lo = moff[hnbr[e]], hi = moff[hnbr[e] + 1];
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (mnbr[mid] <= r) lo = mid + 1;
+      else hi = mid;
+    }
+    mnext[e] = (uint32_t)lo;
   }
 }
 
@@ -318,10 +383,14 @@ constexpr uint32_t kHHSmall = 3072, kHHLarge = 12288;
 constexpr uint32_t kDenseSlots = 14336;  // up to this many hyperedges the tables are indexed by rank
 __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint8_t* esize,
                            const uint64_t* off, const uint32_t* len, const uint32_t* nbr, const uint64_t* hoff,
-                           const uint32_t* hnbr, const uint32_t* hnext, uint8_t* code, uint32_t* hist) {
+                           const uint32_t* hnbr, const uint32_t* hnext, const uint8_t* rmark, const uint64_t* moff,
+                           const uint32_t* mnext, uint8_t* code, uint32_t* hist) {
   for (uint64_t r = global_warp(); r < n; r += n_warps()) {
     uint64_t work = 0;
-    for (uint64_t e = hoff[r] + lane_id(); e < hoff[r + 1]; e += kWarp) work += hoff[hnbr[e] + 1] - hnext[e];
+    for (uint64_t e = hoff[r] + lane_id(); e < hoff[r + 1]; e += kWarp) {
+      const uint32_t q = hnbr[e];
+      work += !rmark || rmark[r] || rmark[q] ? hoff[q + 1] - hnext[e] : moff[q + 1] - mnext[e];
+    }
     work = warp_sum(work);
     uint8_t c = 255;
     if (work) {
@@ -381,20 +450,25 @@ __device__ __forceinline__ uint64_t choose3(uint64_t n) {
 }
 
 // All hyperedge triples through one node, by size categories.
-__device__ void part_stars(unsigned vb, unsigned nb, const uint32_t* ncat, uint32_t n_nodes, unsigned long long* raw) {
+__device__ void part_stars(unsigned vb, unsigned nb, const uint32_t* ncat, const uint32_t* ncat_m, uint32_t n_nodes,
+                           unsigned long long* raw) {
   uint64_t s[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  auto add = [&](uint64_t a, uint64_t b, uint64_t c, uint64_t f) {  // f: 1 or -1
+    s[0] += f * choose3(a);
+    s[1] += f * choose2(a) * b;
+    s[2] += f * choose2(a) * c;
+    s[3] += f * a * choose2(b);
+    s[4] += f * a * b * c;
+    s[5] += f * a * choose2(c);
+    s[6] += f * choose3(b);
+    s[7] += f * choose2(b) * c;
+    s[8] += f * b * choose2(c);
+    s[9] += f * choose3(c);
+  };
   for (uint64_t v = (uint64_t)vb * kBlock + threadIdx.x; v < n_nodes; v += (uint64_t)nb * kBlock) {
     const uint64_t a = ncat[3 * v], b = ncat[3 * v + 1], c = ncat[3 * v + 2];
-    s[0] += choose3(a);
-    s[1] += choose2(a) * b;
-    s[2] += choose2(a) * c;
-    s[3] += a * choose2(b);
-    s[4] += a * b * c;
-    s[5] += a * choose2(c);
-    s[6] += choose3(b);
-    s[7] += choose2(b) * c;
-    s[8] += b * choose2(c);
-    s[9] += choose3(c);
+    add(a, b, c, 1);
+    if (ncat_m) add(a - ncat_m[3 * v], b - ncat_m[3 * v + 1], c - ncat_m[3 * v + 2], ~0ull);  // those without a mark
   }
 #pragma unroll
   for (int k = 0; k < 10; ++k) {
@@ -408,67 +482,90 @@ __device__ void part_stars(unsigned vb, unsigned nb, const uint32_t* ncat, uint3
 // (node, other hyperedge) incidences of its members minus the overlaps of its
 // heavy neighbours. Also takes back the node triangles a hyperedge forms
 // alone, C(|a|, 3).
+// With marks, the pairs with a marked hyperedge: of an unmarked centre, all
+// pairs (pass 0) minus those of its unmarked neighbours (pass 1).
 using OpenHist = uint32_t[kWarps][2][256];
-__device__ void part_open(unsigned vb, unsigned nb, OpenHist& hist, const uint32_t* slot, uint32_t n,
-                          const uint64_t* h2v_off, const uint32_t* h2v_mem, const uint8_t* esize,
-                          const uint32_t* h2h_len, const uint32_t* ncat, const uint64_t* hoff, const uint16_t* hos,
-                          unsigned long long* raw) {
+struct OpenArgs {
+  const uint32_t* slot;
+  uint32_t n;
+  const uint64_t* voff;
+  const uint32_t* vmem;
+  const uint8_t* esize;
+  const uint32_t* h2h_len;
+  const uint32_t* ncat;
+  const uint32_t* ncat_m;
+  const uint64_t* hoff;
+  const uint32_t* hnbr;
+  const uint16_t* hos;
+  const uint8_t* rmark;
+  unsigned long long* raw;
+};
+__device__ void part_open(unsigned vb, unsigned nb, OpenHist& hist, const OpenArgs& A) {
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   uint64_t acc[6] = {0, 0, 0, 0, 0, 0};
   uint64_t alone = 0;
-  for (uint64_t r = (uint64_t)vb * kWarps + w; r < n; r += (uint64_t)nb * kWarps) {
-    const uint32_t a = slot[r];
-    const uint32_t s = esize[a];
-    if (lane == 0) alone += choose3(s);
-    if (h2h_len[a] < 2) continue;
-    const bool heavy = hoff[r + 1] > hoff[r];
-    if (heavy)
-      for (uint32_t i = lane; i <= s; i += kWarp) {
-        hist[w][0][i] = 0;
-        hist[w][1][i] = 0;
+  for (uint64_t r = (uint64_t)vb * kWarps + w; r < A.n; r += (uint64_t)nb * kWarps) {
+    const uint32_t a = A.slot[r];
+    const uint32_t s = A.esize[a];
+    const bool whole = !A.rmark || A.rmark[r];
+    if (lane == 0 && whole) alone += choose3(s);
+    if (A.h2h_len[a] < 2) continue;
+    const bool heavy = A.hoff[r + 1] > A.hoff[r];
+    const uint32_t* m = A.vmem + A.voff[a];
+    for (int pass = 0; pass < (whole ? 1 : 2); ++pass) {
+      if (heavy)
+        for (uint32_t i = lane; i <= s; i += kWarp) {
+          hist[w][0][i] = 0;
+          hist[w][1][i] = 0;
+        }
+      uint32_t one[2] = {0, 0};
+      for (uint32_t i = lane; i < s; i += kWarp) {
+        const uint64_t v = 3 * (uint64_t)m[i];
+        one[0] += A.ncat[v];
+        one[1] += A.ncat[v + 1] + A.ncat[v + 2];
+        if (pass) {
+          one[0] -= A.ncat_m[v];
+          one[1] -= A.ncat_m[v + 1] + A.ncat_m[v + 2];
+        }
+        one[s > 1] -= 1;  // a itself
       }
-    uint32_t one[2] = {0, 0};
-    const uint32_t* m = h2v_mem + h2v_off[a];
-    for (uint32_t i = lane; i < s; i += kWarp) {
-      const uint32_t* c = ncat + 3 * (uint64_t)m[i];
-      one[0] += c[0];
-      one[1] += c[1] + c[2];
-      one[s > 1] -= 1;  // a itself
-    }
-    __syncwarp();
-    for (uint64_t e = hoff[r] + lane; e < hoff[r + 1]; e += kWarp) {
-      const uint32_t os = hos[e], c = os & 0xffu;
-      one[1] -= c;  // a heavy neighbour has two members or more
-      atomicAdd(&hist[w][c < (os >> 8)][c], 1u);
-    }
-    for (int d = 16; d; d >>= 1) {
-      one[0] += __shfl_xor_sync(0xffffffffu, one[0], d);
-      one[1] += __shfl_xor_sync(0xffffffffu, one[1], d);
-    }
-    __syncwarp();
-    if (lane == 0 && !heavy) {
-      // every overlap is 1: all pairs agree on [2 < |a|], the class is the ends' alone
-      const uint32_t x = s > 2;
-      acc[x] += choose2(one[0]);
-      acc[2 + x] += (uint64_t)one[0] * one[1];
-      acc[4 + x] += choose2(one[1]);
-    } else if (lane == 0) {
-      uint32_t* h0 = hist[w][0];
-      uint32_t* h1 = hist[w][1];
-      h0[1] += one[0];
-      h1[1] += one[1];
-      for (uint32_t k = 1; k <= s; ++k) {
-        h0[k] += h0[k - 1];
-        h1[k] += h1[k - 1];
+      __syncwarp();
+      for (uint64_t e = A.hoff[r] + lane; e < A.hoff[r + 1]; e += kWarp) {
+        if (pass && A.rmark[A.hnbr[e]]) continue;
+        const uint32_t os = A.hos[e], c = os & 0xffu;
+        one[1] -= c;  // a heavy neighbour has two members or more
+        atomicAdd(&hist[w][c < (os >> 8)][c], 1u);
       }
-      open_pair_counts(h0, h1, s, acc, false);
+      for (int d = 16; d; d >>= 1) {
+        one[0] += __shfl_xor_sync(0xffffffffu, one[0], d);
+        one[1] += __shfl_xor_sync(0xffffffffu, one[1], d);
+      }
+      __syncwarp();
+      if (lane == 0 && !heavy) {
+        // every overlap is 1: all pairs agree on [2 < |a|], the class is the ends' alone
+        const uint32_t x = s > 2;
+        const uint64_t f = pass ? ~0ull : 1ull;
+        acc[x] += f * choose2(one[0]);
+        acc[2 + x] += f * one[0] * one[1];
+        acc[4 + x] += f * choose2(one[1]);
+      } else if (lane == 0) {
+        uint32_t* h0 = hist[w][0];
+        uint32_t* h1 = hist[w][1];
+        h0[1] += one[0];
+        h1[1] += one[1];
+        for (uint32_t k = 1; k <= s; ++k) {
+          h0[k] += h0[k - 1];
+          h1[k] += h1[k - 1];
+        }
+        open_pair_counts(h0, h1, s, acc, pass != 0);
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
   if (lane == 0) {
     for (int k = 0; k < 6; ++k)
-      if (acc[k]) atomicAdd(&raw[kRawOpen + k], (unsigned long long)acc[k]);
-    if (alone) atomicAdd(&raw[kRawDist + 3], 0ull - (unsigned long long)alone);
+      if (acc[k]) atomicAdd(&A.raw[kRawOpen + k], (unsigned long long)acc[k]);
+    if (alone) atomicAdd(&A.raw[kRawDist + 3], 0ull - (unsigned long long)alone);
   }
 }
 
@@ -481,6 +578,8 @@ struct NodeArgs {
   const uint2* w;
   const uint4* tab;  // the global pair table
   uint32_t tmask;
+  const uint2* w_m;  // marked hyperedges' weights, per entry of nbr and per table entry (null: no marks)
+  const uint2* tab_m;
   const uint32_t* work;
   uint32_t n_work;
   unsigned int* queue;
@@ -503,13 +602,30 @@ __device__ __forceinline__ void node_insert(uint32_t* keys, uint2* val, uint32_t
 __device__ __forceinline__ uint64_t node_record(uint32_t i, uint32_t slot, uint64_t at) {
   return ((uint64_t)i << 48) | ((uint64_t)slot << 32) | at;  // i, slot < 2^14, at < 2^31
 }
-__device__ __forceinline__ void node_sum(uint64_t r, const uint2* wu, const uint2* val, const uint2* w, uint64_t F[4]) {
-  const uint2 a = __ldg(wu + (r >> 48)), p = val[(r >> 32) & 0xffffu], q = __ldg(w + (uint32_t)r);
-  const uint64_t t0 = (uint64_t)p.x * q.x, t1 = (uint64_t)p.x * q.y + (uint64_t)p.y * q.x, t2 = (uint64_t)p.y * q.y;
+__device__ __forceinline__ void node_add(uint2 a, uint2 p, uint2 q, uint64_t f, uint64_t F[4]) {  // f: 1 or -1
+  const uint64_t t0 = f * p.x * q.x, t1 = f * ((uint64_t)p.x * q.y + (uint64_t)p.y * q.x), t2 = f * p.y * q.y;
   F[0] += a.x * t0;
   F[1] += a.y * t0 + a.x * t1;
   F[2] += a.y * t1 + a.x * t2;
   F[3] += a.y * t2;
+}
+__device__ __forceinline__ uint2 less(uint2 a, uint2 b) { return make_uint2(a.x - b.x, a.y - b.y); }
+// With marks the table's value is the place in u's row, and what the unmarked
+// hyperedges give is taken off.
+__device__ __forceinline__ void node_sum(uint64_t r, const uint2* val, const NodeArgs& A, uint64_t uo, uint64_t F[4]) {
+  const uint32_t i = (uint32_t)(r >> 48), at = (uint32_t)r;
+  const uint2 a = __ldg(A.w + uo + i), q = __ldg(A.w + at);
+  uint2 p = val[(r >> 32) & 0xffffu];
+  if (!A.w_m) {
+    node_add(a, p, q, 1, F);
+    return;
+  }
+  const uint64_t ux = uo + p.x;
+  p = __ldg(A.w + ux);
+  const uint2 am = __ldg(A.w_m + uo + i), pm = __ldg(A.w_m + ux), qm = __ldg(A.w_m + at);
+  if (!(am.x | am.y | pm.x | pm.y | qm.x | qm.y)) return;
+  node_add(a, p, q, 1, F);
+  node_add(less(a, am), less(p, pm), less(q, qm), ~0ull, F);
 }
 
 // Whole warp: the rows of u's neighbours i0, i0 + stride, ... (32 of them at
@@ -517,18 +633,18 @@ __device__ __forceinline__ void node_sum(uint64_t r, const uint2* wu, const uint
 // 32 entries while the one before is looked up. With filter (one bit per hash
 // value in 1024, a word per lane) most misses are told by a shuffle.
 template <bool kFilter>
-__device__ __forceinline__ void node_walk(const uint64_t* poff, const uint32_t* plen, const uint32_t* nbr,
-                                          const uint2* w, const uint32_t* keys, const uint2* val, uint32_t shift,
+__device__ __forceinline__ void node_walk(const NodeArgs& A, const uint32_t* keys, const uint2* val, uint32_t shift,
                                           uint32_t mask, uint32_t filter, uint64_t uo, uint32_t d, uint32_t i0,
                                           uint32_t stride, uint64_t* q, uint32_t& qn, uint64_t F[4]) {
+  const uint32_t* nbr = A.nbr;
   const unsigned lane = lane_id();
   const uint32_t mine = i0 + lane * stride;
   uint64_t vo = 0;
   uint32_t vl = 0;
   if (mine < d) {
     const uint32_t v = __ldg(nbr + uo + mine);
-    vo = __ldg(poff + v);
-    vl = __ldg(plen + v);
+    vo = __ldg(A.poff + v);
+    vl = __ldg(A.plen + v);
   }
   const uint32_t m = min(kWarp, (d - i0 + stride - 1) / stride);
   uint64_t o = __shfl_sync(0xffffffffu, vo, 0);
@@ -560,7 +676,7 @@ __device__ __forceinline__ void node_walk(const uint64_t* poff, const uint32_t* 
       qn += (uint32_t)__popc(bal);
       __syncwarp();
       if (qn >= kWarp) {
-        node_sum(q[lane], w + uo, val, w, F);
+        node_sum(q[lane], val, A, uo, F);
         __syncwarp();
         if (lane < qn - kWarp) q[lane] = q[kWarp + lane];
         __syncwarp();
@@ -613,14 +729,14 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
     __syncwarp();
     for (uint32_t i = lane; i < d; i += kWarp) {
       const uint32_t v = A.nbr[uo + i], b = node_hash(v, 22);
-      node_insert(keys, val, shift, mask, v, A.w[uo + i]);
+      node_insert(keys, val, shift, mask, v, A.w_m ? make_uint2(i, 0) : A.w[uo + i]);
       atomicOr(&S->filter[b >> 5], 1u << (b & 31u));
     }
     __syncwarp();
     const uint32_t filter = S->filter[lane];
     for (uint32_t i0 = 0; i0 < d; i0 += kWarp)
-      node_walk<true>(A.poff, A.plen, A.nbr, A.w, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
-    if (lane < qn) node_sum(S->q[lane], A.w + uo, val, A.w, F);  // the records name this node's table
+      node_walk<true>(A, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
+    if (lane < qn) node_sum(S->q[lane], val, A, uo, F);  // the records name this node's table
     __syncwarp();
   }
   node_flush(F, A.raw);
@@ -653,25 +769,24 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
       for (uint32_t i = threadIdx.x; i < slots; i += kThreads) keys[i] = kEmpty;
       __syncthreads();
       for (uint32_t i = threadIdx.x; i < d; i += kThreads)
-        node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w[uo + i]);
+        node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w_m ? make_uint2(i, 0) : A.w[uo + i]);
       __syncthreads();
       for (uint32_t i0 = w; i0 < d; i0 += kW * kWarp)
-        node_walk<false>(A.poff, A.plen, A.nbr, A.w, keys, val, shift, mask, 0, uo, d, i0, kW, queues[w], qn, F);
+        node_walk<false>(A, keys, val, shift, mask, 0, uo, d, i0, kW, queues[w], qn, F);
       __syncwarp();
-      if (lane < qn) node_sum(queues[w][lane], A.w + uo, val, A.w, F);
+      if (lane < qn) node_sum(queues[w][lane], val, A, uo, F);
     } else {
       for (uint32_t i = w; i < d; i += kW) {
         const uint32_t v = A.nbr[uo + i];
         const uint2 a = A.w[uo + i];
         const uint64_t o = A.poff[v];
         for (uint32_t j = lane; j < A.plen[v]; j += kWarp) {
-          const uint2 p = pair_weight(A.tab, A.tmask, u, __ldg(A.nbr + o + j)), q = __ldg(A.w + o + j);
-          const uint64_t t0 = (uint64_t)p.x * q.x, t1 = (uint64_t)p.x * q.y + (uint64_t)p.y * q.x,
-                         t2 = (uint64_t)p.y * q.y;
-          F[0] += a.x * t0;
-          F[1] += a.y * t0 + a.x * t1;
-          F[2] += a.y * t1 + a.x * t2;
-          F[3] += a.y * t2;
+          const uint32_t x = __ldg(A.nbr + o + j);
+          const uint2 p = pair_weight(A.tab, A.tmask, u, x), q = __ldg(A.w + o + j);
+          node_add(a, p, q, 1, F);
+          if (A.w_m)
+            node_add(less(a, A.w_m[uo + i]), less(p, pair_weight(A.tab, A.tmask, u, x, A.tab_m)),
+                     less(q, __ldg(A.w_m + o + j)), ~0ull, F);
         }
       }
     }
@@ -705,6 +820,13 @@ struct PairArgs {
   const uint32_t* ncat;
   const uint4* tab;
   uint32_t tmask;
+  // with marks (else null): pairs of two unmarked hyperedges count their marked
+  // third ones only, from the marked hyperedges' sums
+  const uint8_t* rmark;
+  const uint32_t* ncat_m;
+  const uint2* tab_m;
+  const uint2* fw_m;
+  uint2* self_m;
   const uint64_t* foff;  // the node graph's rows, both directions (for spreading)
   const uint32_t* fnbr;
   const uint2* fw;
@@ -726,10 +848,12 @@ __device__ __forceinline__ bool owns_pair(uint32_t ra, uint32_t sa, uint32_t rb,
 // The sums of one pair into the block's counters: q (third hyperedge of two /
 // more members) and r (hyperedges of S's nodes by category, a and b included).
 __device__ __forceinline__ void add_pair(unsigned long long* cnt, uint32_t sa, uint32_t sb, uint32_t C, uint64_t q2,
-                                         uint64_t q3, uint64_t r0, uint64_t r1, uint64_t r2) {
+                                         uint64_t q3, uint64_t r0, uint64_t r1, uint64_t r2, bool unmarked) {
   const uint32_t ca = size_cat(sa), cb = size_cat(sb);
   const uint32_t n_ex = (sa > C + 1) + (sb > C + 1), n_big = (ca == 2) + (cb == 2);
-  uint64_t r[3] = {r0, r1 - C * (uint64_t)((ca == 1) + (cb == 1)), r2 - C * (uint64_t)((ca == 2) + (cb == 2))};
+  // a and b themselves are not third hyperedges (and not among the marked if unmarked)
+  const uint64_t own = unmarked ? 0 : C;
+  uint64_t r[3] = {r0, r1 - own * ((ca == 1) + (cb == 1)), r2 - own * ((ca == 2) + (cb == 2))};
   if (q2) {
     atomicAdd(&cnt[kRawDist + n_ex], (unsigned long long)q2);
     atomicAdd(&cnt[kRawDist + n_big], 0ull - (unsigned long long)q2 * C);
@@ -744,6 +868,7 @@ __device__ __forceinline__ void add_pair(unsigned long long* cnt, uint32_t sa, u
       atomicAdd(&cnt[kRawPair + pair_index(sa - C, sb - C, k)], (unsigned long long)r[k]);
       atomicAdd(&cnt[kRawStar + star_index(ca, cb, k)], 0ull - (unsigned long long)r[k]);
     }
+  if (unmarked) return;
   // one hyperedge of the pair standing for two node pairs of a triangle
   const unsigned long long c2 = (unsigned long long)C * (C - 1) / 2;
   if (sa >= 3) atomicAdd(&cnt[kRawDist + 2 + (sb >= 3)], 0ull - c2 * (sa - 2));
@@ -775,6 +900,7 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
        e0 += (uint64_t)nb * kWarps * A.per_warp) {
     const uint64_t e = e0 + grp;
     uint32_t sa = 0, sb = 0, C = 0;
+    bool un = false;
     const uint32_t *pa = nullptr, *pb = nullptr;
     uint64_t ma = 0, mb = 0;
     if (grp < A.per_warp && e < A.nh) {
@@ -783,6 +909,7 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
       const uint32_t za = A.esize[a], zb = os >> 8;
       if (owns_pair(ra, za, rb, zb) && !A.spread[ra]) {
         const uint32_t b = A.slot[rb];
+        un = A.rmark && !A.rmark[ra] && !A.rmark[rb];
         sa = za;
         sb = zb;
         C = os & 0xffu;
@@ -796,14 +923,16 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
     // lanes first, first + step, ... of the |a| x |b| combinations; the
     // combinations of b's first member stand for a's member alone
     auto run = [&](uint32_t first, uint32_t step, uint32_t na, uint32_t nb, const uint32_t* xa, const uint32_t* xb,
-                   uint64_t sma, uint64_t smb) {
+                   uint64_t sma, uint64_t smb, bool unmarked) {
+      const uint32_t* ncat = unmarked ? A.ncat_m : A.ncat;
+      const uint2* wm = unmarked ? A.tab_m : nullptr;
       const uint32_t all = na * nb;
       for (uint32_t t = first; t < all; t += step) {
         const uint32_t i = t / nb, j = t - i * nb;
         const uint32_t v = __ldg(xa + i);
         if (i < 64 ? (sma >> i) & 1ull : in_list(xb, nb, v)) {
           if (j) continue;
-          const uint32_t* c = A.ncat + 3 * (uint64_t)v;
+          const uint32_t* c = ncat + 3 * (uint64_t)v;
           r0 += c[0];
           r1 += c[1];
           r2 += c[2];
@@ -811,13 +940,13 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
         }
         const uint32_t w = __ldg(xb + j);
         if (j < 64 ? (smb >> j) & 1ull : in_list(xa, na, w)) continue;
-        const uint2 p = pair_weight(A.tab, A.tmask, v, w);
+        const uint2 p = pair_weight(A.tab, A.tmask, v, w, wm);
         q2 += p.x;
         q3 += p.y;
       }
     };
     const bool wide = sa * sb > A.wide;
-    if (!wide) run(sub, 8, sa, sb, pa, pb, ma, mb);
+    if (!wide) run(sub, 8, sa, sb, pa, pb, ma, mb, un);
     unsigned todo = __ballot_sync(0xffffffffu, wide && sub == 0);
     while (todo) {
       const int src = __ffs(todo) - 1;
@@ -827,10 +956,11 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
       run(lane, 32, __shfl_sync(0xffffffffu, sa, src), __shfl_sync(0xffffffffu, sb, src),
           reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pa, src)),
           reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pb, src)),
-          __shfl_sync(0xffffffffu, (unsigned long long)ma, src), __shfl_sync(0xffffffffu, (unsigned long long)mb, src));
+          __shfl_sync(0xffffffffu, (unsigned long long)ma, src), __shfl_sync(0xffffffffu, (unsigned long long)mb, src),
+          __shfl_sync(0xffffffffu, (int)un, src) != 0);
       __syncwarp();
       const uint64_t t2 = warp_sum(q2), t3 = warp_sum(q3), u0 = warp_sum(r0), u1 = warp_sum(r1), u2 = warp_sum(r2);
-      if ((int)lane == src) add_pair(cnt, sa, sb, C, t2, t3, u0, u1, u2);
+      if ((int)lane == src) add_pair(cnt, sa, sb, C, t2, t3, u0, u1, u2, un);
       q2 = k2;
       q3 = k3;
       r0 = s0;
@@ -842,7 +972,7 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
 #pragma unroll
     for (int k = 0; k < 5; ++k)
       for (int d = 4; d; d >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], d);
-    if (sa && !wide && sub == 0) add_pair(cnt, sa, sb, C, t[0], t[1], t[2], t[3], t[4]);
+    if (sa && !wide && sub == 0) add_pair(cnt, sa, sb, C, t[0], t[1], t[2], t[3], t[4], un);
   }
   __syncthreads();
   for (unsigned k = threadIdx.x; k < kRawClass; k += kBlock)
@@ -880,17 +1010,19 @@ __global__ void k_spread_flags(const uint32_t* slot, uint32_t n, const uint64_t*
   }
 }
 
-__global__ void k_pair_rows_fill(const uint4* tab, uint64_t slots, const uint64_t* off, uint32_t* cursor, uint32_t* nbr,
-                                 uint2* w) {
+__global__ void k_pair_rows_fill(const uint4* tab, const uint2* wm, uint64_t slots, const uint64_t* off,
+                                 uint32_t* cursor, uint32_t* nbr, uint2* w, uint2* w_m) {
   for (uint64_t i = gtid(); i < slots; i += gstride()) {
     const uint4 e = tab[i];
     if (!e.y) continue;
     uint64_t d = off[e.x] + atomicAdd(&cursor[e.x], 1u);
     nbr[d] = e.y;
     w[d] = make_uint2(e.z, e.w);
+    if (wm) w_m[d] = wm[i];
     d = off[e.y] + atomicAdd(&cursor[e.y], 1u);
     nbr[d] = e.x;
     w[d] = make_uint2(e.z, e.w);
+    if (wm) w_m[d] = wm[i];
   }
 }
 
@@ -902,14 +1034,16 @@ __global__ void k_self_weights(PairArgs A, uint32_t n) {
     const uint64_t o = A.voff[a];
     for (uint32_t i = lane_id(); i < s; i += kWarp) {
       const uint32_t v = A.vmem[o + i];
-      uint2 t = make_uint2(0, 0);
-      for (uint32_t j = 0; j < s; ++j) {
-        if (j == i) continue;
-        const uint2 p = pair_weight(A.tab, A.tmask, v, __ldg(A.vmem + o + j));
-        t.x += p.x;
-        t.y += p.y;
+      for (int k = 0; k < (A.rmark ? 2 : 1); ++k) {
+        uint2 t = make_uint2(0, 0);
+        for (uint32_t j = 0; j < s; ++j) {
+          if (j == i) continue;
+          const uint2 p = pair_weight(A.tab, A.tmask, v, __ldg(A.vmem + o + j), k ? A.tab_m : nullptr);
+          t.x += p.x;
+          t.y += p.y;
+        }
+        (k ? A.self_m : A.self)[o + i] = t;
       }
-      A.self[o + i] = t;
     }
   }
 }
@@ -922,7 +1056,10 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
   __shared__ uint32_t s_item;
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   constexpr unsigned kW = kSpreadThreads / kWarp;
-  uint2* y = A.y + (uint64_t)blockIdx.x * ((A.n_nodes + 1) & ~1u);
+  // y of all hyperedges and, for an unmarked owner, of the marked ones
+  const uint32_t vec = (A.n_nodes + 1) & ~1u;
+  uint2* y = A.y + (uint64_t)blockIdx.x * vec * (A.rmark ? 2 : 1);
+  uint2* ym = y + vec;
   for (unsigned k = threadIdx.x; k < kRawClass; k += kSpreadThreads) cnt[k] = 0;
   for (;;) {
     __syncthreads();
@@ -931,6 +1068,7 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
     if (s_item >= A.n_list) break;
     const uint32_t ra = A.list[s_item], a = A.slot[ra], sa = A.esize[a];
     const uint32_t* pa = A.vmem + A.voff[a];
+    const bool both = A.rmark && !A.rmark[ra];
     // a warp takes the rows of one member after another
     uint64_t cells = 0;
     for (uint32_t i = w; i < sa; i += kW) {
@@ -942,6 +1080,11 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
         const uint2 q = __ldg(A.fw + o + k);
         if (q.x) atomicAdd(&y[x].x, q.x);
         if (q.y) atomicAdd(&y[x].y, q.y);
+        if (both) {
+          const uint2 m = __ldg(A.fw_m + o + k);
+          if (m.x) atomicAdd(&ym[x].x, m.x);
+          if (m.y) atomicAdd(&ym[x].y, m.y);
+        }
       }
     }
     for (uint32_t i = 0; i < sa; ++i) cells += A.foff[pa[i] + 1] - A.foff[pa[i]];
@@ -954,20 +1097,24 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
       if (!owns_pair(ra, sa, rb, sb)) continue;
       const uint32_t b = A.slot[rb];
       const uint64_t bo = A.voff[b];
+      const bool un = both && !A.rmark[rb];
+      const uint32_t* ncat = un ? A.ncat_m : A.ncat;
+      const uint2* self = un ? A.self_m : A.self;
       uint64_t q2 = 0, q3 = 0, r0 = 0, r1 = 0, r2 = 0;
       for (uint32_t j = lane; j < sb; j += kWarp) {
         const uint32_t v = __ldg(A.vmem + bo + j);
-        const uint2 t = y[v];
+        uint2 t = y[v];
         if (t.x != ~0u || t.y != ~0u) {
+          if (un) t = ym[v];
           q2 += t.x;
           q3 += t.y;
           continue;
         }
-        const uint32_t* c = A.ncat + 3 * (uint64_t)v;
+        const uint32_t* c = ncat + 3 * (uint64_t)v;
         r0 += c[0];
         r1 += c[1];
         r2 += c[2];
-        const uint2 z = A.self[bo + j];
+        const uint2 z = self[bo + j];
         q2 -= z.x;
         q3 -= z.y;
         for (uint32_t k = 0; k < sb; ++k) {  // the other members of S
@@ -975,7 +1122,7 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
           const uint32_t x = __ldg(A.vmem + bo + k);
           const uint2 u = y[x];
           if (u.x != ~0u || u.y != ~0u) continue;
-          const uint2 p = pair_weight(A.tab, A.tmask, v, x);
+          const uint2 p = pair_weight(A.tab, A.tmask, v, x, un ? A.tab_m : nullptr);
           q2 += p.x;
           q3 += p.y;
         }
@@ -985,17 +1132,21 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
       r0 = warp_sum(r0);
       r1 = warp_sum(r1);
       r2 = warp_sum(r2);
-      if (lane == 0) add_pair(cnt, sa, sb, C, q2, q3, r0, r1, r2);
+      if (lane == 0) add_pair(cnt, sa, sb, C, q2, q3, r0, r1, r2, un);
     }
     __syncthreads();
     if (A.n_nodes <= 4 * cells) {  // clear it all, two entries at a time (the vectors start at even entries)
-      for (uint32_t i = threadIdx.x; i < (A.n_nodes + 1) / 2; i += kSpreadThreads)
+      for (uint32_t i = threadIdx.x; i < (both ? vec : vec / 2); i += kSpreadThreads)
         reinterpret_cast<uint4*>(y)[i] = make_uint4(0, 0, 0, 0);
     } else {
       for (uint32_t i = w; i < sa; i += kW) {
         const uint32_t v = __ldg(pa + i);
         if (lane == 0) y[v] = make_uint2(0, 0);
-        for (uint64_t k = A.foff[v] + lane; k < A.foff[v + 1]; k += kWarp) y[__ldg(A.fnbr + k)] = make_uint2(0, 0);
+        for (uint64_t k = A.foff[v] + lane; k < A.foff[v + 1]; k += kWarp) {
+          const uint32_t x = __ldg(A.fnbr + k);
+          y[x] = make_uint2(0, 0);
+          if (both) ym[x] = make_uint2(0, 0);
+        }
       }
     }
   }
@@ -1021,11 +1172,30 @@ struct HHArgs {
   const uint64_t* voff;   // H2V
   const uint32_t* vmem;
   const uint8_t* esize;
+  // with marks (else null): b's marked neighbours alone, walked when neither a nor b is marked
+  const uint8_t* rmark;
+  const uint64_t* moff;
+  const uint32_t* mnbr;
+  const uint16_t* mos;
+  const uint32_t* mpos;
+  const uint32_t* mnext;
   const uint32_t* work;   // ranks of the centres
   uint32_t n_work;
   unsigned int* queue;
   unsigned long long* raw;
 };
+
+// The part of b's heavy row past a that is walked for (a, b), entry e.
+struct Walk {
+  const uint32_t* nbr;
+  const uint16_t* os;
+  const uint32_t* pos;
+  uint64_t first, end;
+};
+__device__ __forceinline__ Walk walk_of(const HHArgs& A, uint32_t ra, uint32_t rb, uint64_t e) {
+  if (!A.rmark || A.rmark[ra] || A.rmark[rb]) return Walk{A.hnbr, A.hos, A.hpos, A.hnext[e], A.hoff[rb + 1]};
+  return Walk{A.mnbr, A.mos, A.mpos, A.mnext[e], A.moff[rb + 1]};
+}
 
 // |a & b & c| by a three-way merge (centres of more than 64 members).
 __device__ uint32_t merge3(const HHArgs& A, uint32_t a, uint32_t b, uint32_t c) {
@@ -1197,11 +1367,11 @@ __device__ void part_search(const HHArgs& A, SearchShared& S) {
     for (uint64_t e = A.hoff[ra]; e < he; ++e) {
       const uint32_t rb = A.hnbr[e], osb = A.hos[e];
       const uint64_t mab = A.mask[ao + A.hpos[e]];
-      const uint64_t end = A.hoff[rb + 1];
-      for (uint64_t j0 = A.hnext[e]; j0 < end; j0 += kWarp) {
+      const Walk B = walk_of(A, ra, rb, e);
+      for (uint64_t j0 = B.first; j0 < B.end; j0 += kWarp) {
         const uint64_t j = j0 + lane;
-        if (j < end) {
-          const uint32_t rc = A.hnbr[j], osc = A.hos[j], c = A.slot[rc];
+        if (j < B.end) {
+          const uint32_t rc = B.nbr[j], osc = B.os[j], c = A.slot[rc];
           uint32_t lo = 0, hi = al;
           while (lo < hi) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -1286,19 +1456,19 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
       const bool by_b = !exact && (osb >> 8) <= 64;
       const uint64_t bo = A.off[A.slot[rb]];
       const uint64_t mab = exact ? A.mask[ao + A.hpos[e]] : by_b ? A.mask[bo + A.hpos[A.hnext[e] - 1]] : 0;
-      const uint64_t end = A.hoff[rb + 1];
-      uint64_t j = (uint64_t)A.hnext[e] + lane;
+      const Walk B = walk_of(A, ra, rb, e);
+      uint64_t j = B.first + lane;
       uint32_t rc = kEmpty, osc = 0;
-      if (j < end) {
-        rc = __ldg(A.hnbr + j);
-        osc = __ldg(A.hos + j);
+      if (j < B.end) {
+        rc = __ldg(B.nbr + j);
+        osc = __ldg(B.os + j);
       }
-      for (uint64_t j0 = A.hnext[e]; j0 < end; j0 += kWarp) {
+      for (uint64_t j0 = B.first; j0 < B.end; j0 += kWarp) {
         j += kWarp;  // the next round's entries are loaded before this round's tests
         uint32_t rn = kEmpty, on = 0;
-        if (j < end) {
-          rn = __ldg(A.hnbr + j);
-          on = __ldg(A.hos + j);
+        if (j < B.end) {
+          rn = __ldg(B.nbr + j);
+          on = __ldg(B.os + j);
         }
         bool push = false;
         uint64_t rec = 0;
@@ -1317,7 +1487,7 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
             const uint32_t cac = exact ? (uint32_t)__popcll(v) : (uint32_t)v;
             if (cac < 2 || rb > rc) {  // three heavy pairs: once, b ranked highest
               const uint32_t g = exact  ? (uint32_t)__popcll(mab & v)
-                                 : by_b ? (uint32_t)__popcll(mab & __ldg(A.mask + bo + A.hpos[j - kWarp]))
+                                 : by_b ? (uint32_t)__popcll(mab & __ldg(A.mask + bo + B.pos[j - kWarp]))
                                         : merge3(A, a, A.slot[rb], A.slot[rc]);
               push = true;
               rec = pack6(osb >> 8, osc >> 8, osb & 0xffu, osc & 0xffu, cac, g);
@@ -1422,10 +1592,11 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
     for (uint64_t e = A.hoff[ra] + w; e < he; e += kFastWarps) {
       const uint32_t rb = A.hnbr[e], osb = A.hos[e];
       const Mask mab = (Mask)A.mask[ao + A.hpos[e]];
-      const uint32_t first = A.hnext[e], n = (uint32_t)(A.hoff[rb + 1] - first);
+      const Walk B = walk_of(A, ra, rb, e);
+      const uint32_t n = (uint32_t)(B.end - B.first);
       const bool bins = n >= kHistMin && n <= kHistMax;
-      const uint32_t* hn = A.hnbr + first;
-      const uint16_t* ho = A.hos + first;
+      const uint32_t* hn = B.nbr + B.first;
+      const uint16_t* ho = B.os + B.first;
       uint32_t rc = kEmpty, osc = 0;
       if (lane < n) {
         rc = __ldg(hn + lane);
@@ -1519,8 +1690,7 @@ struct PartArgs {
   HHArgs search;
   PairArgs pairs;
   NodeArgs nodes;
-  const uint32_t* h2h_len;
-  uint32_t n;         // slots
+  OpenArgs open;
   unsigned end[5];
 };
 union PartShared {
@@ -1540,10 +1710,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ Par
   } else if (b < A.end[2]) {
     part_nodes(A.nodes, &S.nodes[threadIdx.x / kWarp]);
   } else if (b < A.end[3]) {
-    part_open(b - A.end[2], A.end[3] - A.end[2], S.open, A.search.slot, A.n, A.search.voff, A.search.vmem,
-              A.search.esize, A.h2h_len, A.pairs.ncat, A.search.hoff, A.search.hos, A.search.raw);
+    part_open(b - A.end[2], A.end[3] - A.end[2], S.open, A.open);
   } else {
-    part_stars(b - A.end[3], A.end[4] - A.end[3], A.pairs.ncat, A.pairs.n_nodes, A.search.raw);
+    part_stars(b - A.end[3], A.end[4] - A.end[3], A.pairs.ncat, A.pairs.ncat_m, A.pairs.n_nodes, A.search.raw);
   }
 }
 
@@ -1619,11 +1788,11 @@ static int decomp_attrs() {
 // It enumerates sum h^2 / 2 tests; the oriented rows hold about a quarter of
 // sum d^2 / 2 entries to probe (measured 0.24 to 0.30 on the named laws), and
 // a test costs about as much as a probe, so the line is sum h^2 = sum d^2 / 4.
-static int build_decomp(hm_graph* g) {
+// With mark (per slot) the structures of a touched-triple count.
+static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots, V = g->n_nodes;
-  Decomp& P = g->decomp;
   P.release();
   P.decided = true;
   if (!E || !V) return HM_OK;
@@ -1660,7 +1829,8 @@ static int build_decomp(hm_graph* g) {
   const uint64_t h2 = hs[0], d2 = hs[1], pairs = hs[2], nh = hs[3];
   uint64_t tslots = 1024;
   while (tslots < 2 * pairs) tslots <<= 1;
-  const size_t need = tslots * sizeof(uint4) + pairs * 36 + nh * (18 + 24);
+  const size_t need = tslots * (sizeof(uint4) + (mark ? sizeof(uint2) : 0)) + pairs * (mark ? 60 : 36) +
+                      nh * (18 + 24 + (mark ? 14 : 0));
   const size_t room = ctx->budget ? ctx->budget - std::min<size_t>(ctx->budget, ctx->used.load()) : SIZE_MAX;
   if (h2 > d2 / 4 || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
     P.release();
@@ -1696,6 +1866,31 @@ static int build_decomp(hm_graph* g) {
                                                           P.hos.p, P.hpos.p, P.hnext.p);
     HM_LAUNCH_CHECK();
   }
+  if (mark) {
+    HM_TRY(P.rmark.alloc(ctx, E));
+    HM_TRY(P.moff.alloc(ctx, (size_t)E + 1));
+    HM_TRY(P.mnbr.alloc(ctx, nh));
+    HM_TRY(P.mos.alloc(ctx, nh));
+    HM_TRY(P.mpos.alloc(ctx, nh));
+    HM_TRY(P.mnext.alloc(ctx, nh));
+    k_rank_marks<<<grid_for(E, kBlock), kBlock, 0, st>>>(P.slot.p, E, mark, P.rmark.p);
+    HM_LAUNCH_CHECK();
+    k_marked_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.hoff.p, P.hnbr.p, P.rmark.p, E, hcnt.p);
+    HM_LAUNCH_CHECK();
+    HM_TRY(exclusive_scan(ctx, hcnt.p, P.moff.p, E));
+    k_marked_fill<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p,
+                                                                        P.rmark.p, E, P.moff.p, P.mnbr.p, P.mos.p,
+                                                                        P.mpos.p);
+    HM_LAUNCH_CHECK();
+    if (nh) {
+      k_marked_next<<<grid_for(nh, kBlock), kBlock, 0, st>>>(P.hown.p, P.hnbr.p, nh, P.moff.p, P.mnbr.p, P.mnext.p);
+      HM_LAUNCH_CHECK();
+    }
+    HM_TRY(P.ncat_m.alloc(ctx, 3 * (size_t)V));
+    HM_TRY(P.tab_m.alloc(ctx, tslots));
+    HM_TRY(P.nw_m.alloc(ctx, pairs));
+    HM_CUDA(cudaMemsetAsync(P.tab_m.p, 0, sizeof(uint2) * tslots, st));
+  }
   // node graph
   P.tslots = tslots;
   HM_TRY(P.ncat.alloc(ctx, 3 * (size_t)V));
@@ -1721,23 +1916,23 @@ static int build_decomp(hm_graph* g) {
   HM_CUDA(cudaMemsetAsync(ndeg.p, 0, sizeof(uint32_t) * 2 * V, st));
   HM_CUDA(cudaMemsetAsync(bk.p, 0, sizeof(uint32_t) * (2 * kBk + 1), st));
   k_node_cats<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p,
-                                                                    g->esize.p, V, P.ncat.p);
+                                                                    g->esize.p, mark, V, P.ncat.p, P.ncat_m.p);
   HM_LAUNCH_CHECK();
   const uint32_t tmask = (uint32_t)(tslots - 1);
-  k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_mem.p, g->esize.p, E,
-                                                                      P.tab.p, tmask);
+  k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_mem.p, g->esize.p, mark,
+                                                                      E, P.tab.p, P.tab_m.p, tmask);
   HM_LAUNCH_CHECK();
   k_pair_degrees<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p);
   HM_LAUNCH_CHECK();
   k_pair_plus_count<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p, P.nlen.p);
   HM_LAUNCH_CHECK();
   HM_TRY(exclusive_scan(ctx, P.nlen.p, P.noff.p, V));
-  k_pair_plus_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p, P.noff.p, ndeg.p + V,
-                                                               P.nnbr.p, P.nw.p);
+  k_pair_plus_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, P.tab_m.p, tslots, ndeg.p, P.noff.p,
+                                                               ndeg.p + V, P.nnbr.p, P.nw.p, P.nw_m.p);
   HM_LAUNCH_CHECK();
   k_hh_codes<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.slot.p, P.rank.p, E, g->esize.p, g->h2h_off.p,
                                                                    g->h2h_len.p, g->h2h_nbr.p, P.hoff.p, P.hnbr.p,
-                                                                   P.hnext.p, hcode.p, bk.p);
+                                                                   P.hnext.p, P.rmark.p, P.moff.p, P.mnext.p, hcode.p, bk.p);
   HM_LAUNCH_CHECK();
   k_spread_flags<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(
       P.slot.p, E, P.hoff.p, P.hnbr.p, P.hos.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, ndeg.p, P.spread.p, P.slist.p,
@@ -1765,17 +1960,20 @@ static int build_decomp(hm_graph* g) {
     // one node vector per block of k_spread_pairs, a sixteenth of the room at most
     const size_t vec = ((size_t)V + 1) & ~(size_t)1;
     P.y_blocks = (uint32_t)std::max<size_t>(
-        1, std::min<size_t>({(size_t)ctx->n_sms, (size_t)P.n_spread, room / 16 / (sizeof(uint2) * vec)}));
+        1, std::min<size_t>({(size_t)ctx->n_sms, (size_t)P.n_spread, room / 16 / (sizeof(uint2) * vec * (mark ? 2 : 1))}));
+    const size_t y_all = (size_t)P.y_blocks * vec * (mark ? 2 : 1);
     HM_TRY(P.self.alloc(ctx, g->h2v_tail));
-    HM_TRY(P.y.alloc(ctx, (size_t)P.y_blocks * vec));
-    HM_CUDA(cudaMemsetAsync(P.y.p, 0, sizeof(uint2) * (size_t)P.y_blocks * vec, st));
+    if (mark) HM_TRY(P.self_m.alloc(ctx, g->h2v_tail));
+    if (mark) HM_TRY(P.fw_m.alloc(ctx, 2 * pairs));
+    HM_TRY(P.y.alloc(ctx, y_all));
+    HM_CUDA(cudaMemsetAsync(P.y.p, 0, sizeof(uint2) * y_all, st));
     HM_TRY(P.foff.alloc(ctx, (size_t)V + 1));
     HM_TRY(P.fnbr.alloc(ctx, 2 * pairs));
     HM_TRY(P.fw.alloc(ctx, 2 * pairs));
     HM_TRY(exclusive_scan(ctx, ndeg.p, P.foff.p, V));
     HM_CUDA(cudaMemsetAsync(ndeg.p + V, 0, sizeof(uint32_t) * V, st));
-    k_pair_rows_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, P.foff.p, ndeg.p + V, P.fnbr.p,
-                                                                 P.fw.p);
+    k_pair_rows_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, P.tab_m.p, tslots, P.foff.p, ndeg.p + V,
+                                                                 P.fnbr.p, P.fw.p, P.fw_m.p);
     HM_LAUNCH_CHECK();
   }
   HM_TRY(P.raw.alloc(ctx, kRawSize));
@@ -1786,7 +1984,7 @@ static int build_decomp(hm_graph* g) {
 
 int prepare_decomp(hm_graph* g) {
   if (g->decomp.decided) return HM_OK;
-  const int s = build_decomp(g);
+  const int s = build_decomp(g, g->decomp, nullptr);
   if (s < 0) g->decomp.release();
   if (s == HM_ERR_NOMEM) {  // no room for it: the enumeration of all triangles needs less
     g->decomp.decided = true;
@@ -1797,26 +1995,26 @@ int prepare_decomp(hm_graph* g) {
 
 // One count: the raw sums cleared, the block-per-item launches, the small
 // parts side by side, and the counter block from the sums.
-int launch_decomp(hm_graph* g) {
+static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
-  Decomp& P = g->decomp;
   const unsigned sms = (unsigned)ctx->n_sms;
   const uint32_t E = g->n_slots, V = g->n_nodes;
   unsigned int* queue = reinterpret_cast<unsigned int*>(P.raw.p + kRawQueue);
   HM_CUDA(cudaMemsetAsync(P.raw.p, 0, sizeof(unsigned long long) * kRawSize, st));
   PartArgs A;
   A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, g->h2h_off.p, g->h2h_len.p,
-                    g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, nullptr, 0,
-                    nullptr, P.raw.p};
+                    g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.rmark.p,
+                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, nullptr, 0, nullptr, P.raw.p};
   A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
                      g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
-                     (uint32_t)(P.tslots - 1), P.foff.p, P.fnbr.p, P.fw.p, P.spread.p, P.slist.p, P.n_spread, P.self.p, P.y.p,
+                     (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_m.p, P.fw_m.p, P.self_m.p, P.foff.p,
+                     P.fnbr.p, P.fw.p, P.spread.p, P.slist.p, P.n_spread, P.self.p, P.y.p,
                      V, P.nh < kPairFew ? 1u : 4u, P.nh < kPairFew ? 0u : kPairWide, queue + 8, P.raw.p};
-  A.nodes = NodeArgs{P.noff.p, P.nlen.p, P.nnbr.p, P.nw.p, P.tab.p, (uint32_t)(P.tslots - 1), nullptr, 0, nullptr,
-                     P.raw.p};
-  A.h2h_len = g->h2h_len.p;
-  A.n = E;
+  A.nodes = NodeArgs{P.noff.p, P.nlen.p, P.nnbr.p, P.nw.p, P.tab.p, (uint32_t)(P.tslots - 1), P.nw_m.p, P.tab_m.p,
+                     nullptr, 0, nullptr, P.raw.p};
+  A.open = OpenArgs{P.slot.p, E, g->h2v_off.p, g->h2v_mem.p, g->esize.p, g->h2h_len.p, P.ncat.p, P.ncat_m.p, P.hoff.p,
+                    P.hnbr.p, P.hos.p, P.rmark.p, P.raw.p};
   auto hh_part = [&](int k) {
     const uint32_t b = k ? P.hend[k - 1] : 0;
     A.search.work = P.hwork.p + b;
@@ -1882,8 +2080,34 @@ int launch_decomp(hm_graph* g) {
   A.end[4] = end += std::min<unsigned>(sms * 2, (V + kBlock - 1) / kBlock);
   k_parts<<<end, kBlock, 0, st>>>(A);
   HM_LAUNCH_CHECK();
-  k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, g->counters.p);
+  k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, counters);
   HM_LAUNCH_CHECK();
+  return HM_OK;
+}
+
+int launch_decomp(hm_graph* g) { return launch_parts(g, g->decomp, g->counters.p); }
+
+// The triples with a marked hyperedge, count(G) - count(G without them), by the
+// same forms: every sum over nodes, node pairs and heavy pairs minus the same
+// sum over the unmarked hyperedges (linear in the marked ones' weights where a
+// pair is unmarked), and only the triangles with two or three heavy pairs that
+// hold a mark enumerated. *done = false (and nothing counted) where the graph
+// does not suit the decomposition or the device has no room for it.
+int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done) {
+  *done = false;
+  Decomp P;
+  DArr<unsigned long long> cnt;
+  int s = build_decomp(g, P, mark);
+  if (s >= 0) s = cnt.alloc(g->ctx, 42);
+  if (s == HM_ERR_NOMEM || (s >= 0 && !P.usable)) return HM_OK;
+  HM_TRY(s);
+  HM_TRY(launch_parts(g, P, cnt.p));
+  unsigned long long h[42];
+  HM_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, g->ctx->stream));
+  HM_CUDA(cudaStreamSynchronize(g->ctx->stream));
+  for (int k = 0; k < 30; ++k) out30[k] = h[k];
+  for (int k = 0; k < 6; ++k) out30[20 + k] += h[36 + k] - h[30 + k];
+  *done = true;
   return HM_OK;
 }
 

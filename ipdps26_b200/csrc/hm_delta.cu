@@ -62,6 +62,19 @@ __global__ void k_flag_touched(const uint32_t* ids, uint32_t n, const uint64_t* 
   }
 }
 
+// Entries in the rows of the marked hyperedges' neighbours: what the walk of
+// every marked row goes through, up to its orientation.
+__global__ void k_touch_cost(const uint32_t* ids, uint32_t n, const uint64_t* off, const uint32_t* len,
+                             const uint32_t* nbr, unsigned long long* cost) {
+  unsigned long long t = 0;
+  for (uint64_t i = global_warp(); i < n; i += n_warps()) {
+    const uint64_t s = off[ids[i]];
+    for (uint32_t k = lane_id(); k < len[ids[i]]; k += kWarp) t += len[nbr[s + k]];
+  }
+  for (int d = 16; d; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+  if (lane_id() == 0 && t) atomicAdd(cost, t);
+}
+
 __global__ void k_list_flagged(const uint32_t* flag, const uint64_t* pos, uint32_t n, uint32_t* out) {
   for (uint64_t i = gtid(); i < n; i += gstride())
     if (flag[i]) out[pos[i]] = (uint32_t)i;
@@ -601,6 +614,8 @@ __global__ void k_count_classes(const uint64_t* key, uint32_t n, unsigned int* c
 
 }  // namespace
 
+constexpr uint64_t kDecompMin = 1ull << 28, kDecompEntries = 32;
+
 int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const TouchRows& rows, uint64_t* out) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
@@ -609,7 +624,7 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   if (!n) return HM_OK;
   const uint32_t E = g->n_slots;
   bool by_id = g->touch_by_id;
-  const size_t n_cnt = (size_t)R * kRowStride + 5;  // + three queues, + class counts (u32 pairs)
+  const size_t n_cnt = (size_t)R * kRowStride + 6;  // + three queues, + class counts (u32 pairs), + cost
   DArr<uint8_t> mark;
   DArr<uint32_t> flag, centres;
   DArr<uint64_t> pos;
@@ -650,11 +665,28 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   }
   k_count_classes<<<grid_for(n, kBlock), kBlock, 0, st>>>(skeys.p, n, classes_d);
   HM_LAUNCH_CHECK();
+  // Whether the decomposition is the cheaper count: the walk goes through about
+  // 1e11 of k_touch_cost's entries per second, the decomposition's preparation
+  // and closed forms take what about kDecompEntries of them per adjacency
+  // entry take.
+  const bool may_decomp = !rows.gos && !by_id;
+  uint64_t cost = 0;
+  if (may_decomp) {
+    k_touch_cost<<<grid_for((uint64_t)n * 32, kBlock), kBlock, 0, st>>>(d_ids, n, g->h2h_off.p, g->h2h_len.p,
+                                                                       g->h2h_nbr.p, cnt.p + n_cnt - 1);
+    HM_LAUNCH_CHECK();
+    HM_CUDA(cudaMemcpyAsync(&cost, cnt.p + n_cnt - 1, sizeof(cost), cudaMemcpyDeviceToHost, st));
+  }
   uint64_t nc = 0;
   unsigned int hcls[3] = {0, 0, 0};
   HM_CUDA(cudaMemcpyAsync(&nc, pos.p + E, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaMemcpyAsync(hcls, classes_d, sizeof(hcls), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
+  if (may_decomp && cost > std::max<uint64_t>(kDecompMin, kDecompEntries * g->h2h_nnz)) {
+    bool done = false;
+    HM_TRY(count_touching_decomp(g, mark.p, out, &done));
+    if (done) return HM_OK;
+  }
   const uint32_t n_long = hcls[0], n_large = hcls[1], n_mid = hcls[2];
   HM_TRY(centres.alloc(ctx, nc));
   k_list_flagged<<<grid_for(E, kBlock), kBlock, 0, st>>>(flag.p, pos.p, E, centres.p);

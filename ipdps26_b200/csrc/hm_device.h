@@ -218,13 +218,27 @@ struct Decomp {
   DArr<uint2> self, y, fw;
   DArr<uint64_t> foff;          // node rows in both directions, for those ranks
   DArr<uint32_t> fnbr;
+  // with marks (touched-triple counts): marks by rank, the heavy rows' marked
+  // neighbours, and the marked hyperedges' node and node-pair sums
+  DArr<uint8_t> rmark;
+  DArr<uint64_t> moff;
+  DArr<uint32_t> mnbr, mpos, mnext, ncat_m;
+  DArr<uint16_t> mos;
+  DArr<uint2> tab_m, nw_m, fw_m, self_m;
   DArr<unsigned long long> raw;
   CountCapture capture;
+  ~Decomp() { capture.reset(); }
   void release() {
     capture.reset();
     decided = usable = false;
     nh = tslots = 0;
-    for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist}) a->release();
+    for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist,
+                    &mnbr, &mpos, &mnext, &ncat_m})
+      a->release();
+    for (auto* a : {&tab_m, &nw_m, &fw_m, &self_m}) a->release();
+    rmark.release();
+    moff.release();
+    mos.release();
     n_spread = y_blocks = 0;
     spread.release();
     self.release();
@@ -352,7 +366,6 @@ struct hm_graph {
 
   ~hm_graph() {
     capture.reset();
-    decomp.capture.reset();
     if (ev_ready)
       for (auto& e : ev) cudaEventDestroy(e);
   }
@@ -397,6 +410,7 @@ int prepare_enumeration(hm_graph* g);  // oriented rows and work list of the tri
 // The count by decomposition (hm_decomp.cu), when g->decomp.usable.
 int prepare_decomp(hm_graph* g);
 int launch_decomp(hm_graph* g);
+int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done);
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags);
 int finish_static(hm_graph* g, uint64_t out30[30]);
 int count_static30(hm_graph* g, uint32_t shard, uint32_t n_shards, uint64_t out30[30]);

@@ -88,3 +88,38 @@ def test_all_pairs_heavy_is_enumerated(ctx):
     off, mem = csr(rows)
     with engine.Graph(ctx, off, mem, 200) as g:
         assert g.count_static30().tolist() == oracle.static30(off, mem, 200).tolist()
+
+
+def _touch_law(name, seed):
+    from ipdps26_b200 import gen
+
+    if name == "hub":
+        return gen.config1(seed=seed, n_nodes=1500, n_edges=3000), 3000
+    if name == "wide":
+        return gen.config2(seed=seed, n_nodes=3000, n_edges=6000, q=3.0), 6000
+    return gen.params(seed, 600, 3000, 20, 110, 1.1, 1.1, 40.0), 3000  # "large": most centres above 32 members
+
+
+@pytest.mark.parametrize("law", ["hub", "wide", "large"])
+@pytest.mark.parametrize("marked", [400, 1500])
+def test_touched_triples_by_decomposition(ctx, law, marked):
+    """Batches whose touched-triple counts are large enough to go by the
+    decomposition: the count of a marked set equals the walk of id-ordered rows
+    (other kernels), marking everything gives the full count, and an update's
+    delta equals the difference of two full counts."""
+    from ipdps26_b200 import engine, gen
+
+    p, n = _touch_law(law, 7 + marked)
+    h = gen.static(p)
+    rng = np.random.default_rng(marked)
+    ids = np.sort(rng.choice(n, size=marked, replace=False)).astype(np.uint32)
+    with engine.Graph.from_hypergraph(ctx, h) as g:
+        got = g.count_touching30(ids)
+        g.set_touch_orientation(True)
+        assert got.tolist() == g.count_touching30(ids).tolist()
+        g.set_touch_orientation(False)
+        full = g.count_static30()
+        assert g.count_touching30(np.arange(n, dtype=np.uint32)).tolist() == full.tolist()
+        dels, ins = gen.batch(p, 3, g.live_ids(), marked)
+        _, delta = g.apply_batch(dels, ins.offsets, ins.members)
+        assert (full.astype(np.int64) + delta).tolist() == g.count_static30().astype(np.int64).tolist()
