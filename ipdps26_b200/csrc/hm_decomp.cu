@@ -610,13 +610,14 @@ __device__ __forceinline__ void node_add(uint2 a, uint2 p, uint2 q, uint64_t f, 
   F[3] += a.y * t2;
 }
 __device__ __forceinline__ uint2 less(uint2 a, uint2 b) { return make_uint2(a.x - b.x, a.y - b.y); }
-// With marks the table's value is the place in u's row, and what the unmarked
-// hyperedges give is taken off.
+// With marks (kTouch) the table's value is the place in u's row, and what the
+// unmarked hyperedges give is taken off.
+template <bool kTouch>
 __device__ __forceinline__ void node_sum(uint64_t r, const uint2* val, const NodeArgs& A, uint64_t uo, uint64_t F[4]) {
   const uint32_t i = (uint32_t)(r >> 48), at = (uint32_t)r;
   const uint2 a = __ldg(A.w + uo + i), q = __ldg(A.w + at);
   uint2 p = val[(r >> 32) & 0xffffu];
-  if (!A.w_m) {
+  if (!kTouch) {
     node_add(a, p, q, 1, F);
     return;
   }
@@ -632,7 +633,7 @@ __device__ __forceinline__ void node_sum(uint64_t r, const uint2* val, const Nod
 // most) against u's table. Their bounds are loaded at once, and each chunk of
 // 32 entries while the one before is looked up. With filter (one bit per hash
 // value in 1024, a word per lane) most misses are told by a shuffle.
-template <bool kFilter>
+template <bool kTouch, bool kFilter>
 __device__ __forceinline__ void node_walk(const NodeArgs& A, const uint32_t* keys, const uint2* val, uint32_t shift,
                                           uint32_t mask, uint32_t filter, uint64_t uo, uint32_t d, uint32_t i0,
                                           uint32_t stride, uint64_t* q, uint32_t& qn, uint64_t F[4]) {
@@ -676,7 +677,7 @@ __device__ __forceinline__ void node_walk(const NodeArgs& A, const uint32_t* key
       qn += (uint32_t)__popc(bal);
       __syncwarp();
       if (qn >= kWarp) {
-        node_sum(q[lane], val, A, uo, F);
+        node_sum<kTouch>(q[lane], val, A, uo, F);
         __syncwarp();
         if (lane < qn - kWarp) q[lane] = q[kWarp + lane];
         __syncwarp();
@@ -708,6 +709,7 @@ struct NodeWarp {
   uint32_t keys[kNodeWarpSlots];
   uint32_t filter[kWarp];
 };
+template <bool kTouch>
 __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
   const unsigned lane = lane_id();
   uint32_t* keys = S->keys;
@@ -729,14 +731,14 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
     __syncwarp();
     for (uint32_t i = lane; i < d; i += kWarp) {
       const uint32_t v = A.nbr[uo + i], b = node_hash(v, 22);
-      node_insert(keys, val, shift, mask, v, A.w_m ? make_uint2(i, 0) : A.w[uo + i]);
+      node_insert(keys, val, shift, mask, v, kTouch ? make_uint2(i, 0) : A.w[uo + i]);
       atomicOr(&S->filter[b >> 5], 1u << (b & 31u));
     }
     __syncwarp();
     const uint32_t filter = S->filter[lane];
     for (uint32_t i0 = 0; i0 < d; i0 += kWarp)
-      node_walk<true>(A, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
-    if (lane < qn) node_sum(S->q[lane], val, A, uo, F);  // the records name this node's table
+      node_walk<kTouch, true>(A, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
+    if (lane < qn) node_sum<kTouch>(S->q[lane], val, A, uo, F);  // the records name this node's table
     __syncwarp();
   }
   node_flush(F, A.raw);
@@ -744,7 +746,7 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
 
 // One block per node, kTab slots in shared memory (load <= 3/4); a longer row
 // probes the global pair table instead.
-template <unsigned kTab, unsigned kThreads, unsigned kMinBlocks>
+template <bool kTouch, unsigned kTab, unsigned kThreads, unsigned kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
   constexpr unsigned kW = kThreads / kWarp;
   extern __shared__ uint64_t smem64[];
@@ -769,12 +771,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
       for (uint32_t i = threadIdx.x; i < slots; i += kThreads) keys[i] = kEmpty;
       __syncthreads();
       for (uint32_t i = threadIdx.x; i < d; i += kThreads)
-        node_insert(keys, val, shift, mask, A.nbr[uo + i], A.w_m ? make_uint2(i, 0) : A.w[uo + i]);
+        node_insert(keys, val, shift, mask, A.nbr[uo + i], kTouch ? make_uint2(i, 0) : A.w[uo + i]);
       __syncthreads();
       for (uint32_t i0 = w; i0 < d; i0 += kW * kWarp)
-        node_walk<false>(A, keys, val, shift, mask, 0, uo, d, i0, kW, queues[w], qn, F);
+        node_walk<kTouch, false>(A, keys, val, shift, mask, 0, uo, d, i0, kW, queues[w], qn, F);
       __syncwarp();
-      if (lane < qn) node_sum(queues[w][lane], val, A, uo, F);
+      if (lane < qn) node_sum<kTouch>(queues[w][lane], val, A, uo, F);
     } else {
       for (uint32_t i = w; i < d; i += kW) {
         const uint32_t v = A.nbr[uo + i];
@@ -784,7 +786,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_node_tri(NodeArgs A) {
           const uint32_t x = __ldg(A.nbr + o + j);
           const uint2 p = pair_weight(A.tab, A.tmask, u, x), q = __ldg(A.w + o + j);
           node_add(a, p, q, 1, F);
-          if (A.w_m)
+          if (kTouch)
             node_add(less(a, A.w_m[uo + i]), less(p, pair_weight(A.tab, A.tmask, u, x, A.tab_m)),
                      less(q, __ldg(A.w_m + o + j)), ~0ull, F);
         }
@@ -1069,13 +1071,15 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
     const uint32_t ra = A.list[s_item], a = A.slot[ra], sa = A.esize[a];
     const uint32_t* pa = A.vmem + A.voff[a];
     const bool both = A.rmark && !A.rmark[ra];
-    // a warp takes the rows of one member after another
+    // the block takes the rows of the members one after another (a node's
+    // row can be hundreds of times another's)
     uint64_t cells = 0;
-    for (uint32_t i = w; i < sa; i += kW) {
+#pragma unroll 4
+    for (uint32_t i = 0; i < sa; ++i) {
       const uint32_t v = __ldg(pa + i);
       const uint64_t o = A.foff[v];
       const uint32_t l = (uint32_t)(A.foff[v + 1] - o);
-      for (uint32_t k = lane; k < l; k += kWarp) {
+      for (uint32_t k = threadIdx.x; k < l; k += kSpreadThreads) {
         const uint32_t x = __ldg(A.fnbr + o + k);
         const uint2 q = __ldg(A.fw + o + k);
         if (q.x) atomicAdd(&y[x].x, q.x);
@@ -1092,47 +1096,56 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
     for (uint32_t i = threadIdx.x; i < sa; i += kSpreadThreads) y[pa[i]] = make_uint2(~0u, ~0u);
     __syncthreads();
     const uint64_t he = A.hoff[ra + 1];
-    for (uint64_t e = A.hoff[ra] + w; e < he; e += kW) {
-      const uint32_t rb = A.hnbr[e], os = A.hos[e], sb = os >> 8, C = os & 0xffu;
-      if (!owns_pair(ra, sa, rb, sb)) continue;
-      const uint32_t b = A.slot[rb];
-      const uint64_t bo = A.voff[b];
-      const bool un = both && !A.rmark[rb];
+    // eight lanes per pair: a pair is a chain of dependent loads, so the more
+    // of them in flight the better
+    for (uint64_t e0 = A.hoff[ra] + w * 4; e0 < he; e0 += kW * 4) {
+      const uint64_t e = e0 + (lane >> 3);
+      uint32_t sb = 0, C = 0;
+      uint64_t bo = 0;
+      bool un = false;
+      if (e < he) {
+        const uint32_t rb = A.hnbr[e], os = A.hos[e];
+        if (owns_pair(ra, sa, rb, os >> 8)) {
+          sb = os >> 8;
+          C = os & 0xffu;
+          bo = A.voff[A.slot[rb]];
+          un = both && !A.rmark[rb];
+        }
+      }
       const uint32_t* ncat = un ? A.ncat_m : A.ncat;
       const uint2* self = un ? A.self_m : A.self;
-      uint64_t q2 = 0, q3 = 0, r0 = 0, r1 = 0, r2 = 0;
-      for (uint32_t j = lane; j < sb; j += kWarp) {
+      uint64_t t[5] = {0, 0, 0, 0, 0};  // q2, q3, r by category
+      for (uint32_t j = lane & 7u; j < sb; j += 8) {
         const uint32_t v = __ldg(A.vmem + bo + j);
-        uint2 t = y[v];
-        if (t.x != ~0u || t.y != ~0u) {
-          if (un) t = ym[v];
-          q2 += t.x;
-          q3 += t.y;
+        uint2 q = y[v];
+        if (q.x != ~0u || q.y != ~0u) {
+          if (un) q = ym[v];
+          t[0] += q.x;
+          t[1] += q.y;
           continue;
         }
         const uint32_t* c = ncat + 3 * (uint64_t)v;
-        r0 += c[0];
-        r1 += c[1];
-        r2 += c[2];
+        t[2] += c[0];
+        t[3] += c[1];
+        t[4] += c[2];
         const uint2 z = self[bo + j];
-        q2 -= z.x;
-        q3 -= z.y;
+        t[0] -= z.x;
+        t[1] -= z.y;
         for (uint32_t k = 0; k < sb; ++k) {  // the other members of S
           if (k == j) continue;
           const uint32_t x = __ldg(A.vmem + bo + k);
           const uint2 u = y[x];
           if (u.x != ~0u || u.y != ~0u) continue;
           const uint2 p = pair_weight(A.tab, A.tmask, v, x, un ? A.tab_m : nullptr);
-          q2 += p.x;
-          q3 += p.y;
+          t[0] += p.x;
+          t[1] += p.y;
         }
       }
-      q2 = warp_sum(q2);
-      q3 = warp_sum(q3);
-      r0 = warp_sum(r0);
-      r1 = warp_sum(r1);
-      r2 = warp_sum(r2);
-      if (lane == 0) add_pair(cnt, sa, sb, C, q2, q3, r0, r1, r2, un);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+        for (int d = 4; d; d >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], d);
+      if (sb && (lane & 7u) == 0) add_pair(cnt, sa, sb, C, t[0], t[1], t[2], t[3], t[4], un);
     }
     __syncthreads();
     if (A.n_nodes <= 4 * cells) {  // clear it all, two entries at a time (the vectors start at even entries)
@@ -1181,6 +1194,7 @@ struct HHArgs {
   const uint32_t* mnext;
   const uint32_t* work;   // ranks of the centres
   uint32_t n_work;
+  uint32_t slices;        // k_hh_large: item k is slice k % slices of centre k / slices
   unsigned int* queue;
   unsigned long long* raw;
 };
@@ -1400,7 +1414,9 @@ __device__ void part_search(const HHArgs& A, SearchShared& S) {
 // One block per centre a: the entries of a's row ranked above a in a shared
 // table keyed by rank (4 keys per 16-byte bucket, load <= 3/4), each with its
 // place in a's row. Warps take b among a's heavy neighbours, lanes walk b's
-// heavy row past a. For the longest rows and centres of more than 64 members.
+// heavy row past a. For the longest rows and centres of more than 64 members,
+// few and long (23,000 neighbours at 60K hyperedges): a centre's b are dealt to
+// several blocks where there are fewer centres than places.
 constexpr unsigned kHHSlots = 16384, kHHThreads = 1024, kHHCol = 4;
 constexpr size_t kHHSmem = kHHSlots * 2 * sizeof(uint32_t) +
                            kHHThreads / kWarp * (sizeof(WarpCounts<kHHCol>) + 2 * kWarp * sizeof(uint64_t));
@@ -1423,8 +1439,8 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
     if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
     __syncthreads();
     const uint32_t it = s_item;
-    if (it >= A.n_work) break;
-    const uint32_t ra = A.work[it], a = A.slot[ra];
+    if (it >= A.n_work * A.slices) break;
+    const uint32_t ra = A.work[it / A.slices], a = A.slot[ra], slice = it % A.slices;
     const uint64_t ao = A.off[a];
     const uint32_t al = A.len[a];
     const uint32_t sa = A.esize[a];
@@ -1449,7 +1465,7 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
     }
     __syncthreads();
     const uint64_t he = A.hoff[ra + 1];
-    for (uint64_t e = A.hoff[ra] + w; e < he; e += kW) {
+    for (uint64_t e = A.hoff[ra] + slice * kW + w; e < he; e += kW * A.slices) {
       const uint32_t rb = A.hnbr[e], osb = A.hos[e];
       // the masks of the triple overlap: over a's members, or over b's when a
       // has more than 64 (b's entry of a precedes its entries above a)
@@ -1677,9 +1693,10 @@ static_assert(kNodeSmall == 1024 / 4 * 3 && kNodeMid == 4096 / 4 * 3 && kNodeLar
 
 // The short node rows alone (k_parts takes them too when they are few): at the
 // registers of its own it keeps 6 blocks per SM, k_parts 4.
+template <bool kTouch>
 __global__ void __launch_bounds__(kBlock, 6) k_node_tri_warp(NodeArgs A) {
   __shared__ NodeWarp S[kWarps];
-  part_nodes(A, &S[threadIdx.x / kWarp]);
+  part_nodes<kTouch>(A, &S[threadIdx.x / kWarp]);
 }
 
 // The parts of a count that run in small blocks, side by side in one launch:
@@ -1699,6 +1716,7 @@ union PartShared {
   NodeWarp nodes[kWarps];
   OpenHist open;
 };
+template <bool kTouch>
 __global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ PartArgs A) {
   __shared__ __align__(16) unsigned char mem[sizeof(PartShared)];
   PartShared& S = *reinterpret_cast<PartShared*>(mem);
@@ -1708,7 +1726,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ Par
   } else if (b < A.end[1]) {
     part_pairs(b - A.end[0], A.end[1] - A.end[0], S.pairs, A.pairs);
   } else if (b < A.end[2]) {
-    part_nodes(A.nodes, &S.nodes[threadIdx.x / kWarp]);
+    part_nodes<kTouch>(A.nodes, &S.nodes[threadIdx.x / kWarp]);
   } else if (b < A.end[3]) {
     part_open(b - A.end[2], A.end[3] - A.end[2], S.open, A.open);
   } else {
@@ -1777,10 +1795,13 @@ static int decomp_attrs() {
                                (int)fast_smem<uint32_t>()));
   HM_CUDA(cudaFuncSetAttribute(k_hh_fast<false, uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)fast_smem<uint64_t>()));
-  HM_CUDA(cudaFuncSetAttribute(k_node_tri<4096, 512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)node_smem(4096)));
-  HM_CUDA(cudaFuncSetAttribute(k_node_tri<16384, 1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)node_smem(16384)));
+  auto node = [](auto* big, auto* mid) -> int {
+    HM_CUDA(cudaFuncSetAttribute(big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)node_smem(16384)));
+    HM_CUDA(cudaFuncSetAttribute(mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)node_smem(4096)));
+    return HM_OK;
+  };
+  HM_TRY(node(k_node_tri<false, 16384, 1024, 1>, k_node_tri<false, 4096, 512, 2>));
+  HM_TRY(node(k_node_tri<true, 16384, 1024, 1>, k_node_tri<true, 4096, 512, 2>));
   return HM_OK;
 }
 
@@ -1995,6 +2016,7 @@ int prepare_decomp(hm_graph* g) {
 
 // One count: the raw sums cleared, the block-per-item launches, the small
 // parts side by side, and the counter block from the sums.
+template <bool kTouch>
 static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
@@ -2005,7 +2027,7 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   PartArgs A;
   A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, g->h2h_off.p, g->h2h_len.p,
                     g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.rmark.p,
-                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, nullptr, 0, nullptr, P.raw.p};
+                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, nullptr, 0, 1, nullptr, P.raw.p};
   A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
                      g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
                      (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_m.p, P.fw_m.p, P.self_m.p, P.foff.p,
@@ -2030,7 +2052,8 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
     return A.nodes.n_work;
   };
   if (const uint32_t n = hh_part(3)) {
-    k_hh_large<<<std::min(sms, n), kHHThreads, kHHSmem, st>>>(A.search);
+    A.search.slices = std::min(16u, std::max(1u, 8 * sms / n));
+    k_hh_large<<<std::min(sms, n * A.search.slices), kHHThreads, kHHSmem, st>>>(A.search);
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = hh_part(2)) {
@@ -2051,21 +2074,21 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(3)) {
-    k_node_tri<16384, 1024, 1><<<std::min(sms, n), 1024, node_smem(16384), st>>>(A.nodes);
+    k_node_tri<kTouch, 16384, 1024, 1><<<std::min(sms, n), 1024, node_smem(16384), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(2)) {
-    k_node_tri<4096, 512, 2><<<std::min(sms * 4, n), 512, node_smem(4096), st>>>(A.nodes);
+    k_node_tri<kTouch, 4096, 512, 2><<<std::min(sms * 4, n), 512, node_smem(4096), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
   if (const uint32_t n = node_part(1)) {
-    k_node_tri<1024, 256, 6><<<std::min(sms * 6, n), 256, node_smem(1024), st>>>(A.nodes);
+    k_node_tri<kTouch, 1024, 256, 6><<<std::min(sms * 6, n), 256, node_smem(1024), st>>>(A.nodes);
     HM_LAUNCH_CHECK();
   }
   const uint32_t n_search = hh_part(0);
   uint32_t n_nodes = node_part(0);
   if (n_nodes > kNodesAlone) {
-    k_node_tri_warp<<<std::min(sms * 12, (n_nodes + kWarps - 1) / kWarps), kBlock, 0, st>>>(A.nodes);
+    k_node_tri_warp<kTouch><<<std::min(sms * 12, (n_nodes + kWarps - 1) / kWarps), kBlock, 0, st>>>(A.nodes);
     HM_LAUNCH_CHECK();
     n_nodes = 0;
   }
@@ -2078,14 +2101,14 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   A.end[2] = end += blocks(n_nodes, 8);
   A.end[3] = end += blocks(E, 8);
   A.end[4] = end += std::min<unsigned>(sms * 2, (V + kBlock - 1) / kBlock);
-  k_parts<<<end, kBlock, 0, st>>>(A);
+  k_parts<kTouch><<<end, kBlock, 0, st>>>(A);
   HM_LAUNCH_CHECK();
   k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, counters);
   HM_LAUNCH_CHECK();
   return HM_OK;
 }
 
-int launch_decomp(hm_graph* g) { return launch_parts(g, g->decomp, g->counters.p); }
+int launch_decomp(hm_graph* g) { return launch_parts<false>(g, g->decomp, g->counters.p); }
 
 // The triples with a marked hyperedge, count(G) - count(G without them), by the
 // same forms: every sum over nodes, node pairs and heavy pairs minus the same
@@ -2101,7 +2124,7 @@ int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], 
   if (s >= 0) s = cnt.alloc(g->ctx, 42);
   if (s == HM_ERR_NOMEM || (s >= 0 && !P.usable)) return HM_OK;
   HM_TRY(s);
-  HM_TRY(launch_parts(g, P, cnt.p));
+  HM_TRY(launch_parts<true>(g, P, cnt.p));
   unsigned long long h[42];
   HM_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, g->ctx->stream));
   HM_CUDA(cudaStreamSynchronize(g->ctx->stream));

@@ -155,50 +155,63 @@ __global__ void k_patch_removals(const uint32_t* dels, uint32_t n, const uint64_
 
 // Additions from the fresh rows of inserted hyperedges to neighbours that
 // were not inserted in this batch; the mask is over the neighbour's members.
-__global__ void k_patch_additions(const uint32_t* ins, uint32_t n, const uint64_t* off, const uint32_t* len,
-                                  const uint32_t* nbr, const uint8_t* ovl, const uint8_t* ins_mark,
-                                  const uint64_t* hoff, const uint32_t* hmem, const uint8_t* esize,
-                                  const uint64_t* out_off, uint64_t* keys, uint32_t* idx, uint8_t* povl,
-                                  uint64_t* pmask) {
-  for (uint64_t i = global_warp(); i < n; i += n_warps()) {
+// Entry t of the rows laid end to end (row i at out_off[i]) is patch t; the
+// entries of neighbours inserted too keep the filler key. A thread per entry:
+// rows differ a thousandfold in length, and a warp per row took as long as its
+// longest (20 ms of a 4K-edit batch, rows of up to 23,000).
+__global__ void k_patch_additions(const uint32_t* ins, uint32_t n, uint64_t total, const uint64_t* off,
+                                  const uint32_t* nbr, const uint8_t* ovl, const uint64_t* amask,
+                                  const uint8_t* ins_mark, const uint64_t* hoff, const uint32_t* hmem,
+                                  const uint8_t* esize, const uint64_t* out_off, uint64_t* keys, uint32_t* idx,
+                                  uint8_t* povl, uint64_t* pmask) {
+  for (uint64_t t = gtid(); t < total; t += gstride()) {
+    uint32_t i = 0, above = n;  // the last row starting at or before t that is not empty
+    while (above - i > 1) {
+      const uint32_t mid = (i + above) >> 1;
+      if (__ldg(out_off + mid) <= t) i = mid;
+      else above = mid;
+    }
     const uint32_t a = ins[i];
-    const uint64_t s = off[a];
-    const uint32_t l = len[a];
-    uint64_t o = out_off[i];
+    const uint64_t at = off[a] + (t - out_off[i]);
+    const uint32_t b = nbr[at];
+    if (ins_mark[b]) continue;
     const uint32_t* ma = hmem + hoff[a];
     const uint32_t sa = esize[a];
-    for (uint32_t k0 = 0; k0 < l; k0 += kWarp) {
-      const uint32_t k = k0 + lane_id();
-      bool keep = false;
-      uint32_t b = 0;
-      if (k < l) {
-        b = nbr[s + k];
-        keep = !ins_mark[b];
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const uint64_t dst = o + __popc(m & lanemask_lt());
-        // positions of b's members that a contains (a merge of the two lists)
-        const uint32_t* mb = hmem + hoff[b];
-        const uint32_t sb = esize[b];
-        uint64_t mask = 0;
-        uint32_t p = 0, q = 0;
-        while (p < sb && q < sa) {
-          if (mb[p] < ma[q]) ++p;
-          else if (mb[p] > ma[q]) ++q;
-          else {
-            if (p < 64) mask |= 1ull << p;
-            ++p;
-            ++q;
-          }
+    // Positions of b's members that a contains: each shared member, known
+    // from a's own mask, searched in b's list (most pairs share one; a
+    // merge of the lists reads them whole), or the merge where a's mask
+    // leaves some out.
+    const uint32_t* mb = hmem + hoff[b];
+    const uint32_t sb = esize[b], shared = ovl[at];
+    uint64_t mask = 0, am = amask[at];
+    if ((uint32_t)__popcll(am) == shared) {
+      uint32_t lo = 0;
+      for (; am; am &= am - 1) {
+        const uint32_t u = __ldg(ma + (__ffsll((long long)am) - 1));
+        uint32_t hi = sb;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (__ldg(mb + mid) < u) lo = mid + 1;
+          else hi = mid;
         }
-        keys[dst] = ((uint64_t)b << 33) | ((uint64_t)a << 1) | 1ull;
-        idx[dst] = (uint32_t)dst;
-        povl[dst] = ovl[s + k];
-        pmask[dst] = mask;
+        if (lo < 64) mask |= 1ull << lo;
       }
-      o += __popc(m);
+    } else {
+      uint32_t p = 0, q = 0;
+      while (p < sb && q < sa) {
+        if (mb[p] < ma[q]) ++p;
+        else if (mb[p] > ma[q]) ++q;
+        else {
+          if (p < 64) mask |= 1ull << p;
+          ++p;
+          ++q;
+        }
+      }
     }
+    keys[t] = ((uint64_t)b << 33) | ((uint64_t)a << 1) | 1ull;
+    idx[t] = (uint32_t)t;
+    povl[t] = (uint8_t)shared;
+    pmask[t] = mask;
   }
 }
 
@@ -263,16 +276,20 @@ __global__ void k_patch_rows(const uint32_t* row, const uint8_t* pop, uint64_t n
   }
 }
 
-// Rewrites one patched row (warp per row) at the arena tail: old entries
+// Rewrites one patched row at the arena tail (a warp per row, or the block
+// where rows are long on average, kGroup threads): old entries
 // minus removals, replaced entries updated, additions merged in id order.
 // remx / addx are exclusive prefix counts of removals / additions over the
 // compacted patch list.
+constexpr uint64_t kLongRows = 512;
+template <unsigned kGroup>
 __global__ void k_patch_apply(const RowPatch* rp, uint32_t n_rows, const uint64_t* dst_off, uint64_t tail,
                               const uint32_t* pid, const uint8_t* pop, const uint32_t* pidx, const uint64_t* remx,
                               const uint64_t* addx, const uint8_t* add_ovl, const uint64_t* add_mask,
                               uint64_t* h2h_off, const uint32_t* h2h_len, uint32_t* nbr, uint8_t* ovl,
                               uint64_t* mask) {
-  for (uint64_t r = global_warp(); r < n_rows; r += n_warps()) {
+  const uint32_t t = threadIdx.x % kGroup;
+  for (uint64_t r = gtid() / kGroup; r < n_rows; r += gstride() / kGroup) {
     const RowPatch P = rp[r];
     const uint64_t so = h2h_off[P.row];
     const uint32_t sl = h2h_len[P.row];
@@ -280,7 +297,7 @@ __global__ void k_patch_apply(const RowPatch* rp, uint32_t n_rows, const uint64_
     const uint32_t np = P.p1 - P.p0;
     const uint64_t rem0 = remx[P.p0], add0 = addx[P.p0];
     // old entries: output rank = i - (removals with id < x) + (additions with id < x)
-    for (uint32_t i = lane_id(); i < sl; i += kWarp) {
+    for (uint32_t i = t; i < sl; i += kGroup) {
       const uint32_t x = nbr[so + i];
       uint32_t lo = 0, hi = np;
       while (lo < hi) {
@@ -303,7 +320,7 @@ __global__ void k_patch_apply(const RowPatch* rp, uint32_t n_rows, const uint64_
       }
     }
     // additions: output rank = (old entries with id < y) - (removals before) + (additions before)
-    for (uint32_t k = lane_id(); k < np; k += kWarp) {
+    for (uint32_t k = t; k < np; k += kGroup) {
       if (pop[P.p0 + k] != 1) continue;
       const uint32_t y = pid[P.p0 + k];
       uint32_t lo = 0, hi = sl;
@@ -318,8 +335,10 @@ __global__ void k_patch_apply(const RowPatch* rp, uint32_t n_rows, const uint64_
       ovl[d] = add_ovl[pidx[P.p0 + k]];
       mask[d] = add_mask[pidx[P.p0 + k]];
     }
-    __syncwarp();
-    if (lane_id() == 0) h2h_off[P.row] = dst;
+    // every thread has read the row's old place
+    if (kGroup == kWarp) __syncwarp();
+    else __syncthreads();
+    if (t == 0) h2h_off[P.row] = dst;
   }
 }
 
@@ -336,21 +355,6 @@ __global__ void k_gather_u32(const uint32_t* ids, uint32_t n, const uint32_t* sr
 
 __global__ void k_set_lens(const RowPatch* rp, uint32_t n_rows, const uint32_t* new_len, uint32_t* h2h_len) {
   for (uint64_t r = gtid(); r < n_rows; r += gstride()) h2h_len[rp[r].row] = new_len[r];
-}
-
-// Arena compaction: every live row copied to its scanned position.
-__global__ void k_compact_rows(const uint64_t* off, const uint32_t* len, uint32_t n, const uint64_t* new_off,
-                               const uint32_t* nbr, const uint8_t* ovl, const uint64_t* mask, uint32_t* nnbr,
-                               uint8_t* novl, uint64_t* nmask) {
-  for (uint64_t r = global_warp(); r < n; r += n_warps()) {
-    const uint64_t s = off[r], d = new_off[r];
-    const uint32_t l = len[r];
-    for (uint32_t k = lane_id(); k < l; k += kWarp) {
-      nnbr[d + k] = nbr[s + k];
-      novl[d + k] = ovl[s + k];
-      nmask[d + k] = mask[s + k];
-    }
-  }
 }
 
 __global__ void k_compact_members(const uint64_t* off, const uint32_t* len, uint32_t n, const uint64_t* new_off,
@@ -861,9 +865,9 @@ int apply_batch_hooks(hm_graph* g, const uint32_t* h_dels, uint32_t n_del, const
       HM_CUDA(cudaMemcpyAsync(idx.p, pidx.p, sizeof(uint32_t) * n_rem, cudaMemcpyDeviceToDevice, st));
     }
     if (n_ins) {
-      k_patch_additions<<<grid_for((uint64_t)n_ins * 32, kBlock), kBlock, 0, st>>>(
-          ids.p, n_ins, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, ins_mark.p, g->h2v_off.p,
-          g->h2v_mem.p, g->esize.p, ioff.p, keys.p + n_rem, idx.p + n_rem, povl.p + n_rem, pmask.p + n_rem);
+      k_patch_additions<<<grid_for(n_add_max, kBlock), kBlock, 0, st>>>(
+          ids.p, n_ins, n_add_max, g->h2h_off.p, g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, ins_mark.p,
+          g->h2v_off.p, g->h2v_mem.p, g->esize.p, ioff.p, keys.p + n_rem, idx.p + n_rem, povl.p + n_rem, pmask.p + n_rem);
       HM_LAUNCH_CHECK();
     }
     // additions index their payload by absolute patch position
@@ -977,9 +981,13 @@ int apply_batch_hooks(hm_graph* g, const uint32_t* h_dels, uint32_t n_del, const
         }
         const uint32_t nr = (uint32_t)(r1 - r0);
         const uint64_t base = g->h2h_tail - hno[r0];  // dst = base + noff[r], modulo 2^64
-        k_patch_apply<<<grid_for((uint64_t)nr * 32, kBlock), kBlock, 0, st>>>(
-            rp.p + r0, nr, noff.p + r0, base, pid.p, pop.p, ppidx.p, remx.p, addx.p, povl.p + n_rem,
-            pmask.p + n_rem, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p);
+        auto apply = [&](auto* kernel, unsigned group) {
+          kernel<<<grid_for((uint64_t)nr * group, kBlock), kBlock, 0, st>>>(
+              rp.p + r0, nr, noff.p + r0, base, pid.p, pop.p, ppidx.p, remx.p, addx.p, povl.p + n_rem, pmask.p + n_rem,
+              g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p);
+        };
+        if ((hno[r1] - hno[r0]) / nr >= kLongRows) apply(k_patch_apply<kBlock>, kBlock);
+        else apply(k_patch_apply<kWarp>, kWarp);
         HM_LAUNCH_CHECK();
         k_set_lens<<<grid_for(nr, kBlock), kBlock, 0, st>>>(rp.p + r0, nr, nlen.p + r0, g->h2h_len.p);
         HM_LAUNCH_CHECK();
