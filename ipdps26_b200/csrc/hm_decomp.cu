@@ -147,13 +147,20 @@ __global__ void k_heavy_emit(const uint32_t* slot, const uint32_t* rank, uint32_
   }
 }
 
+// An entry as the histogram kernel walks it: rank << 8 | (C - 2) * 8 +
+// min(size, 7) for an overlap C of 2 or 3, low byte ~0 for a larger one.
+__device__ __forceinline__ uint32_t walk_code(uint32_t rank, uint32_t os) {
+  const uint32_t c = os & 0xffu;
+  return (rank << 8) | (c <= 3 ? (c - 2) * 8 + min(os >> 8, 7u) : 0xffu);
+}
+
 // The sorted entries' fields; next = the first position of the neighbour's
 // row that ranks above the owner (the owner is in that row: adjacency is
 // symmetric).
 __global__ void k_heavy_rows(const uint64_t* key, const uint32_t* pos, uint64_t nh, unsigned bits,
                              const uint32_t* slot, const uint64_t* off, const uint8_t* ovl, const uint8_t* esize,
                              const uint64_t* hoff, uint32_t* hnbr, uint32_t* hown, uint16_t* hos, uint32_t* hpos,
-                             uint32_t* hnext) {
+                             uint32_t* hnext, uint32_t* hcode) {
   const uint64_t low = (1ull << bits) - 1;
   for (uint64_t i = gtid(); i < nh; i += gstride()) {
     const uint64_t k = key[i];
@@ -161,7 +168,9 @@ __global__ void k_heavy_rows(const uint64_t* key, const uint32_t* pos, uint64_t 
     const uint32_t p = pos[i];
     hnbr[i] = q;
     hown[i] = r;
-    hos[i] = (uint16_t)(((uint32_t)esize[slot[q]] << 8) | ovl[off[slot[r]] + p]);
+    const uint32_t os = ((uint32_t)esize[slot[q]] << 8) | ovl[off[slot[r]] + p];
+    hos[i] = (uint16_t)os;
+    hcode[i] = walk_code(q, os);
     hpos[i] = p;
     const uint64_t back = ((uint64_t)q << bits) | r;
     uint64_t lo = hoff[q], hi = hoff[q + 1];
@@ -306,7 +315,7 @@ __global__ void k_marked_count(const uint64_t* hoff, const uint32_t* hnbr, const
 
 __global__ void k_marked_fill(const uint64_t* hoff, const uint32_t* hnbr, const uint16_t* hos, const uint32_t* hpos,
                               const uint8_t* rmark, uint32_t n, const uint64_t* moff, uint32_t* mnbr, uint16_t* mos,
-                              uint32_t* mpos) {
+                              uint32_t* mpos, uint32_t* mcode) {
   for (uint64_t r = global_warp(); r < n; r += n_warps()) {
     uint64_t w = moff[r];
     if (moff[r + 1] == w) continue;
@@ -318,6 +327,7 @@ __global__ void k_marked_fill(const uint64_t* hoff, const uint32_t* hnbr, const 
         const uint64_t d = w + __popc(m & lanemask_lt());
         mnbr[d] = hnbr[e];
         mos[d] = hos[e];
+        mcode[d] = walk_code(hnbr[e], hos[e]);
         mpos[d] = hpos[e];
       }
       w += __popc(m);
@@ -380,7 +390,7 @@ __global__ void k_bucket_scatter(const uint8_t* code, uint32_t n, uint32_t* star
 // above a), 3 the large tables (up to 12288, and centres of more than 64
 // members).
 constexpr uint32_t kHHSmall = 3072, kHHLarge = 12288;
-constexpr uint32_t kDenseSlots = 14336;  // up to this many hyperedges the tables are indexed by rank
+constexpr uint32_t kDenseSlots = 12288;  // up to this many hyperedges the tables are indexed by rank
 __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint8_t* esize,
                            const uint64_t* off, const uint32_t* len, const uint32_t* nbr, const uint64_t* hoff,
                            const uint32_t* hnbr, const uint32_t* hnext, const uint8_t* rmark, const uint64_t* moff,
@@ -1177,6 +1187,7 @@ struct HHArgs {
   const uint16_t* hos;
   const uint32_t* hpos;
   const uint32_t* hnext;
+  const uint32_t* hcode;  // walk_code of every entry
   const uint64_t* off;    // H2H
   const uint32_t* len;
   const uint32_t* nbr;
@@ -1192,6 +1203,7 @@ struct HHArgs {
   const uint16_t* mos;
   const uint32_t* mpos;
   const uint32_t* mnext;
+  const uint32_t* mcode;
   const uint32_t* work;   // ranks of the centres
   uint32_t n_work;
   uint32_t slices;        // k_hh_large: item k is slice k % slices of centre k / slices
@@ -1204,11 +1216,12 @@ struct Walk {
   const uint32_t* nbr;
   const uint16_t* os;
   const uint32_t* pos;
+  const uint32_t* code;
   uint64_t first, end;
 };
 __device__ __forceinline__ Walk walk_of(const HHArgs& A, uint32_t ra, uint32_t rb, uint64_t e) {
-  if (!A.rmark || A.rmark[ra] || A.rmark[rb]) return Walk{A.hnbr, A.hos, A.hpos, A.hnext[e], A.hoff[rb + 1]};
-  return Walk{A.mnbr, A.mos, A.mpos, A.mnext[e], A.moff[rb + 1]};
+  if (!A.rmark || A.rmark[ra] || A.rmark[rb]) return Walk{A.hnbr, A.hos, A.hpos, A.hcode, A.hnext[e], A.hoff[rb + 1]};
+  return Walk{A.mnbr, A.mos, A.mpos, A.mcode, A.mnext[e], A.moff[rb + 1]};
 }
 
 // |a & b & c| by a three-way merge (centres of more than 64 members).
@@ -1277,6 +1290,24 @@ __device__ __forceinline__ void flush_counts(WarpCounts<kCol>* W, unsigned long 
   clear_counts(W);
 }
 
+// The same for n triangles without a common node: each pair has nodes of its
+// own, so the class (26 to 29) and the removals follow from how many of the
+// three have a member outside the others, as for the closed forms, and R and
+// the products reduce to P = C_ab C_bc C_ac.
+template <unsigned kCol>
+__device__ __forceinline__ void add_triangle0(WarpCounts<kCol>* W, uint32_t sa, uint32_t sb, uint32_t sc, uint32_t cab,
+                                              uint32_t cbc, uint32_t cac, uint32_t n) {
+  const unsigned lane = lane_id();
+  const uint32_t ba = sa >= 3, bb = sb >= 3, bc = sc >= 3;
+  const uint32_t eab = cab >= 2 ? cac * cbc : 0u, ebc = cbc >= 2 ? cab * cac : 0u, eac = cac >= 2 ? cab * cbc : 0u;
+  const uint32_t dk = cab * cbc * cac * ((cab >= 2) + (cbc >= 2) + (cac >= 2) - 1);
+  W->dist[(sa > cab + cac) + (sb > cab + cbc) + (sc > cac + cbc)][lane] += n;
+  W->dist[ba + bb + bc][lane] += (unsigned long long)dk * n;
+  if (eab) W->dist[(sa > cab + 1) + (sb > cab + 1) + bc][lane] -= (unsigned long long)eab * n;
+  if (ebc) W->dist[(sb > cbc + 1) + (sc > cbc + 1) + ba][lane] -= (unsigned long long)ebc * n;
+  if (eac) W->dist[(sa > cac + 1) + (sc > cac + 1) + bb][lane] -= (unsigned long long)eac * n;
+}
+
 // One triangle with overlaps cab, cbc, cac (two of them heavy or all) and
 // triple overlap g: its class and removals, and what the closed forms counted
 // it for (see the head of this file).
@@ -1284,6 +1315,10 @@ template <unsigned kCol>
 __device__ __forceinline__ void add_triangle(WarpCounts<kCol>* W, const int8_t* cls, uint32_t sa, uint32_t sb,
                                              uint32_t sc, uint32_t cab, uint32_t cbc, uint32_t cac, uint32_t g,
                                              uint32_t n = 1) {
+  if (!g) {
+    add_triangle0(W, sa, sb, sc, cab, cbc, cac, n);
+    return;
+  }
   const unsigned lane = lane_id(), col = lane & (kCol - 1);
   const int k = cls[region_pattern((int)sa, (int)sb, (int)sc, (int)cab, (int)cbc, (int)cac, (int)g)];
   atomicAdd(&W->c[kSmClass + k][col], n);
@@ -1303,16 +1338,14 @@ __device__ __forceinline__ void add_triangle(WarpCounts<kCol>* W, const int8_t* 
   if (eab) W->dist[(sa > cab + 1) + (sb > cab + 1) + bc][lane] -= (unsigned long long)eab * n;
   if (ebc) W->dist[(sb > cbc + 1) + (sc > cbc + 1) + ba][lane] -= (unsigned long long)ebc * n;
   if (eac) W->dist[(sa > cac + 1) + (sc > cac + 1) + bb][lane] -= (unsigned long long)eac * n;
-  if (g) {
-    const uint32_t gn = g * n;
-    atomicAdd(&W->c[kSmStar + ba + bb + bc][col], gn * ((cab >= 2) + (cbc >= 2) + (cac >= 2) - 1));
-    auto pair = [&](uint32_t ux, uint32_t uy, uint32_t big) {
-      atomicAdd(&W->c[kSmPair + (min(ux, 2u) * 3 + min(uy, 2u)) * 2 + big][col], gn);
-    };
-    if (cab >= 2) pair(sa - cab, sb - cab, bc);
-    if (cbc >= 2) pair(sb - cbc, sc - cbc, ba);
-    if (cac >= 2) pair(sa - cac, sc - cac, bb);
-  }
+  const uint32_t gn = g * n;
+  atomicAdd(&W->c[kSmStar + ba + bb + bc][col], gn * ((cab >= 2) + (cbc >= 2) + (cac >= 2) - 1));
+  auto pair = [&](uint32_t ux, uint32_t uy, uint32_t big) {
+    atomicAdd(&W->c[kSmPair + (min(ux, 2u) * 3 + min(uy, 2u)) * 2 + big][col], gn);
+  };
+  if (cab >= 2) pair(sa - cab, sb - cab, bc);
+  if (cbc >= 2) pair(sb - cbc, sc - cbc, ba);
+  if (cac >= 2) pair(sa - cac, sc - cac, bb);
 }
 
 // A record packs |b|, |c|, C_ab, C_bc, C_ac and g, 8 bits each, and how many
@@ -1329,17 +1362,16 @@ __device__ __forceinline__ void add_record(WarpCounts<kCol>* W, const int8_t* cl
 }
 
 // Whole warp: appends the lanes' records to the warp's queue (64 places) and
-// classifies 32 at a time.
-template <unsigned kCol>
-__device__ __forceinline__ void queue_records(WarpCounts<kCol>* W, const int8_t* cls, uint32_t sa, bool push,
-                                              uint64_t rec, uint64_t* q, uint32_t& qn) {
+// hands 32 at a time to add.
+template <class Add>
+__device__ __forceinline__ void queue_records(bool push, uint64_t rec, uint64_t* q, uint32_t& qn, Add&& add) {
   const unsigned bal = __ballot_sync(0xffffffffu, push);
   if (!bal) return;
   if (push) q[qn + __popc(bal & lanemask_lt())] = rec;
   qn += (uint32_t)__popc(bal);
   __syncwarp();
   if (qn >= kWarp) {
-    add_record(W, cls, sa, q[lane_id()]);
+    add(q[lane_id()]);
     __syncwarp();
     if (lane_id() < qn - kWarp) q[lane_id()] = q[kWarp + lane_id()];
     __syncwarp();
@@ -1510,7 +1542,7 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
             }
           }
         }
-        queue_records(W, cls, sa, push, rec, q, qn);
+        queue_records(push, rec, q, qn, [&](uint64_t r) { add_record(W, cls, sa, r); });
         if ((tests += kWarp) >= kFlushTests) {
           flush_counts(W, A.raw);
           tests = 0;
@@ -1536,16 +1568,17 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
 // (87 % of the issue slots with one record per triangle), so instructions per
 // test are what counts. Graphs of up to kDenseSlots hyperedges index their
 // table by rank and need no hash.
-constexpr uint32_t kHistMin = 96, kHistMax = 1u << 21, kHistBins = 192;
+constexpr uint32_t kHistMin = 96, kHistMax = 1u << 16, kHistBins = 192;
 constexpr unsigned kFastThreads = 512, kFastWarps = kFastThreads / kWarp, kFastCol = 4, kFastSlots = 4096;
 struct FastWarp {
   WarpCounts<kFastCol> counts;
-  uint64_t q[2 * kWarp];
+  uint64_t q[2 * kWarp];     // weighted records
+  uint64_t late[2 * kWarp];  // triangles outside the bins
   uint32_t hist[kHistBins];
 };
 template <class Mask>
 constexpr size_t fast_smem() { return kFastWarps * sizeof(FastWarp) + kFastSlots * (sizeof(uint32_t) + sizeof(Mask)); }
-constexpr size_t kDenseSmem = kFastWarps * sizeof(FastWarp) + kDenseSlots * sizeof(uint32_t);
+constexpr size_t kDenseSmem = kFastWarps * sizeof(FastWarp) + (kDenseSlots + 4) * sizeof(uint32_t);
 static_assert(fast_smem<uint64_t>() <= 113 * 1024 && kDenseSmem <= 113 * 1024, "two blocks per SM");
 
 template <bool kDense, class Mask>
@@ -1562,7 +1595,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
   fill_classes(cls);
   clear_counts(W);
   for (unsigned k = lane; k < kHistBins; k += kWarp) F->hist[k] = 0;
-  uint32_t qn = 0, tests = 0;
+  uint32_t qn = 0, ln = 0, tests = 0;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1u);
     __syncthreads();
@@ -1574,7 +1607,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
     const uint32_t sa = A.esize[a];
     uint32_t shift = 0, bmask = 0;
     if (kDense) {
-      const uint32_t quads = (n_ranks - ra + 3) / 4;  // places ra + 1 .. n_ranks - 1, at rank - ra
+      const uint32_t quads = (n_ranks - ra) / 4 + 1;  // places ra + 1 .. n_ranks, at rank - ra; the last stays 0
       for (uint32_t i = threadIdx.x; i < quads; i += kFastThreads)
         reinterpret_cast<uint4*>(val)[i] = make_uint4(0, 0, 0, 0);
     } else {
@@ -1605,60 +1638,66 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
     }
     __syncthreads();
     const uint64_t he = A.hoff[ra + 1];
+    // a waiting triangle: the place of c's entry (bit 31: among the marked
+    // rows), C_ac, g, C_ab and |b|
+    auto late = [&](uint64_t r) {
+      const uint32_t at = (uint32_t)r, hi = (uint32_t)(r >> 32);
+      const uint32_t osc = __ldg((at >> 31 ? A.mos : A.hos) + (at & 0x7fffffffu));
+      add_triangle(W, cls, sa, hi >> 24, osc >> 8, (hi >> 16) & 0xffu, osc & 0xffu, hi & 0xffu, (hi >> 8) & 0xffu);
+    };
     for (uint64_t e = A.hoff[ra] + w; e < he; e += kFastWarps) {
       const uint32_t rb = A.hnbr[e], osb = A.hos[e];
       const Mask mab = (Mask)A.mask[ao + A.hpos[e]];
       const Walk B = walk_of(A, ra, rb, e);
       const uint32_t n = (uint32_t)(B.end - B.first);
-      const bool bins = n >= kHistMin && n <= kHistMax;
-      const uint32_t* hn = B.nbr + B.first;
-      const uint16_t* ho = B.os + B.first;
-      uint32_t rc = kEmpty, osc = 0;
-      if (lane < n) {
-        rc = __ldg(hn + lane);
-        osc = __ldg(ho + lane);
-      }
-      for (uint32_t j0 = 0; j0 < n; j0 += kWarp) {
-        const uint32_t jn = j0 + kWarp + lane;  // the next round's entries are loaded before this round's tests
-        uint32_t rn = kEmpty, on = 0;
-        if (jn < n) {
-          rn = __ldg(hn + jn);
-          on = __ldg(ho + jn);
-        }
+      const bool bins = n >= kHistMin && n < kHistMax;  // a bin's count fits a record's 16 bits
+      const uint32_t* hc = B.code + B.first;
+      const uint64_t part = ((uint64_t)osb << 48) | (B.code == A.hcode ? 0u : 0x80000000u);
+      const uint32_t bias = bins ? 0u : 4u;
+      // One round: the entries cur of the lanes, at hc + at. An entry past the
+      // row's end has a rank no table holds.
+      auto round = [&](uint32_t cur, uint32_t at) {
+        const uint32_t rc = cur >> 8, code = cur & 0xffu;
         Mask v = 0;
-        if (rc != kEmpty) {
-          if (kDense) {
-            v = val[rc - ra];
-          } else {
-            uint32_t bk = (rc * 2654435761u) >> shift;
-            int t;
-            for (;;) {
-              const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
-              t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
-              if (t >= 0 || k4.w == kEmpty) break;
-              bk = (bk + 1) & bmask;
-            }
-            if (t >= 0) v = val[4 * bk + (uint32_t)t];
+        if (kDense) {
+          v = val[min(rc - ra, n_ranks - ra)];
+        } else {
+          uint32_t bk = (rc * 2654435761u) >> shift;
+          int t;
+          for (;;) {
+            const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
+            t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
+            if (t >= 0 || k4.w == kEmpty) break;
+            bk = (bk + 1) & bmask;
           }
+          if (t >= 0) v = val[4 * bk + (uint32_t)t];
         }
-        const uint32_t cac = bits(v);
-        bool push = false;
-        uint64_t rec = 0;
-        if (v && (cac < 2 || rb > rc)) {  // three heavy pairs: once, b ranked highest
-          const uint32_t g = bits(v & mab), cbc = osc & 0xffu, sc = osc >> 8;
-          if (bins && cbc <= 3 && cac <= 3) {
-            atomicAdd(&F->hist[cac * 64 + cbc * 32 + g * 8 + min(sc, 7u) - 128], 1u);
-          } else {
-            push = true;
-            rec = pack6(osb >> 8, sc, osb & 0xffu, cbc, cac, g);
-          }
+        const uint32_t cac = bits(v), g = bits(v & mab);
+        const bool take = cac == 1 || (cac > 1 && rb > rc);  // three heavy pairs: once, b ranked highest
+        const bool slow = cac + ((code & 0x80u) >> 5) + bias > 3;
+        if (take && !slow) atomicAdd(&F->hist[g * 48 + cac * 16 + code - 16], 1u);
+        // the others wait as their entry's place and what is known of the
+        // triangle; |c| and C_bc are read when 32 have come together
+        queue_records(take && slow, part | ((uint64_t)(cac | (g << 8)) << 32) | ((uint32_t)B.first + at), F->late, ln,
+                      late);
+      };
+      for (uint32_t c0 = 0; c0 < n; c0 += kHistMax) {
+        const uint32_t c1 = min(n, c0 + kHistMax);
+        // two rounds at a time, their successors' entries loaded before them
+        uint32_t at = c0 + lane;
+        uint32_t x = at < c1 ? __ldg(hc + at) : kEmpty, y = at + kWarp < c1 ? __ldg(hc + at + kWarp) : kEmpty;
+        for (uint32_t j0 = c0; j0 < c1; j0 += 2 * kWarp) {
+          const uint32_t to = at + 2 * kWarp;
+          const uint32_t xn = to < c1 ? __ldg(hc + to) : kEmpty, yn = to + kWarp < c1 ? __ldg(hc + to + kWarp) : kEmpty;
+          round(x, at);
+          if (j0 + kWarp < c1) round(y, at + kWarp);
+          at = to;
+          x = xn;
+          y = yn;
         }
-        queue_records(W, cls, sa, push, rec, F->q, qn);
-        if (n > kHistMax && (j0 & (kHistMax - 1)) == kHistMax - kWarp) flush_counts(W, A.raw);
-        rc = rn;
-        osc = on;
+        if (c1 < n) flush_counts(W, A.raw);
       }
-      if ((tests += min(n, kHistMax)) >= kFlushTests - kHistMax) {
+      if ((tests += min(n, kHistMax)) >= kFlushTests - 2 * kHistMax) {
         flush_counts(W, A.raw);
         tests = 0;
       }
@@ -1666,22 +1705,18 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
         __syncwarp();
 #pragma unroll 1
         for (uint32_t k0 = 0; k0 < kHistBins; k0 += kWarp) {
-          const uint32_t k = k0 + lane + 128;
-          uint32_t c = F->hist[k - 128];
-          if (c) F->hist[k - 128] = 0;
-          while (__any_sync(0xffffffffu, c != 0)) {
-            const uint32_t m = min(c, 0xffffu);
-            c -= m;
-            // bits: |c| (7 standing for 7 or more) 0-2, g 3-4, C_bc - 2 5, C_ac from 6 (biased by 2)
-            queue_records(W, cls, sa, m != 0, pack6(osb >> 8, k & 7u, osb & 0xffu, 2 + ((k >> 5) & 1u), (k >> 6) - 1, (k >> 3) & 3u, m),
-                          F->q, qn);
-          }
+          const uint32_t k = k0 + lane;  // |c| (7 standing for 7 or more) + 8 (C_bc - 2) + 16 (C_ac - 1) + 48 g
+          const uint32_t c = F->hist[k], g = k / 48, m = k - 48 * g;
+          if (c) F->hist[k] = 0;
+          queue_records(c != 0, pack6(osb >> 8, m & 7u, osb & 0xffu, 2 + ((m >> 3) & 1u), (m >> 4) + 1, g, c), F->q, qn,
+                        [&](uint64_t r) { add_record(W, cls, sa, r); });
         }
       }
     }
     __syncwarp();
     if (lane < qn) add_record(W, cls, sa, F->q[lane]);  // the centre's last triangles (they depend on |a|)
-    qn = 0;
+    if (lane < ln) late(F->late[lane]);
+    qn = ln = 0;
     __syncthreads();
   }
   flush_counts(W, A.raw);
@@ -1851,7 +1886,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   uint64_t tslots = 1024;
   while (tslots < 2 * pairs) tslots <<= 1;
   const size_t need = tslots * (sizeof(uint4) + (mark ? sizeof(uint2) : 0)) + pairs * (mark ? 60 : 36) +
-                      nh * (18 + 24 + (mark ? 14 : 0));
+                      nh * (22 + 24 + (mark ? 18 : 0));
   const size_t room = ctx->budget ? ctx->budget - std::min<size_t>(ctx->budget, ctx->used.load()) : SIZE_MAX;
   if (h2 > d2 / 4 || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
     P.release();
@@ -1864,6 +1899,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   HM_TRY(P.hos.alloc(ctx, nh));
   HM_TRY(P.hpos.alloc(ctx, nh));
   HM_TRY(P.hnext.alloc(ctx, nh));
+  HM_TRY(P.hcode.alloc(ctx, nh));
   if (nh) {
     DArr<uint64_t> key, key_s;
     DArr<uint32_t> pos, pos_s;
@@ -1884,7 +1920,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
                                             (int)(2 * bits), st));
     k_heavy_rows<<<grid_for(nh, kBlock), kBlock, 0, st>>>(key_s.p, pos_s.p, nh, bits, P.slot.p, g->h2h_off.p,
                                                           g->h2h_ovl.p, g->esize.p, P.hoff.p, P.hnbr.p, P.hown.p,
-                                                          P.hos.p, P.hpos.p, P.hnext.p);
+                                                          P.hos.p, P.hpos.p, P.hnext.p, P.hcode.p);
     HM_LAUNCH_CHECK();
   }
   if (mark) {
@@ -1894,6 +1930,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
     HM_TRY(P.mos.alloc(ctx, nh));
     HM_TRY(P.mpos.alloc(ctx, nh));
     HM_TRY(P.mnext.alloc(ctx, nh));
+    HM_TRY(P.mcode.alloc(ctx, nh));
     k_rank_marks<<<grid_for(E, kBlock), kBlock, 0, st>>>(P.slot.p, E, mark, P.rmark.p);
     HM_LAUNCH_CHECK();
     k_marked_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.hoff.p, P.hnbr.p, P.rmark.p, E, hcnt.p);
@@ -1901,7 +1938,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
     HM_TRY(exclusive_scan(ctx, hcnt.p, P.moff.p, E));
     k_marked_fill<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p,
                                                                         P.rmark.p, E, P.moff.p, P.mnbr.p, P.mos.p,
-                                                                        P.mpos.p);
+                                                                        P.mpos.p, P.mcode.p);
     HM_LAUNCH_CHECK();
     if (nh) {
       k_marked_next<<<grid_for(nh, kBlock), kBlock, 0, st>>>(P.hown.p, P.hnbr.p, nh, P.moff.p, P.mnbr.p, P.mnext.p);
@@ -2025,9 +2062,9 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   unsigned int* queue = reinterpret_cast<unsigned int*>(P.raw.p + kRawQueue);
   HM_CUDA(cudaMemsetAsync(P.raw.p, 0, sizeof(unsigned long long) * kRawSize, st));
   PartArgs A;
-  A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, g->h2h_off.p, g->h2h_len.p,
+  A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hcode.p, g->h2h_off.p, g->h2h_len.p,
                     g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.rmark.p,
-                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, nullptr, 0, 1, nullptr, P.raw.p};
+                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, P.mcode.p, nullptr, 0, 1, nullptr, P.raw.p};
   A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
                      g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
                      (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_m.p, P.fw_m.p, P.self_m.p, P.foff.p,

@@ -203,6 +203,7 @@ struct Decomp {
   DArr<uint16_t> hos;         // (neighbour size << 8) | overlap
   DArr<uint32_t> hpos;        // place in the owner's H2H row
   DArr<uint32_t> hnext;       // first entry of the neighbour's row ranked above the owner
+  DArr<uint32_t> hcode;       // rank and packed overlap, as the histogram kernel walks it
   uint64_t nh = 0;
   DArr<uint32_t> ncat;        // per node: hyperedges of one, two, more members
   DArr<uint4> tab;            // node pairs {x, y, W2, W3}
@@ -222,7 +223,7 @@ struct Decomp {
   // neighbours, and the marked hyperedges' node and node-pair sums
   DArr<uint8_t> rmark;
   DArr<uint64_t> moff;
-  DArr<uint32_t> mnbr, mpos, mnext, ncat_m;
+  DArr<uint32_t> mnbr, mpos, mnext, mcode, ncat_m;
   DArr<uint16_t> mos;
   DArr<uint2> tab_m, nw_m, fw_m, self_m;
   DArr<unsigned long long> raw;
@@ -233,7 +234,7 @@ struct Decomp {
     decided = usable = false;
     nh = tslots = 0;
     for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist,
-                    &mnbr, &mpos, &mnext, &ncat_m})
+                    &mnbr, &mpos, &mnext, &mcode, &hcode, &ncat_m})
       a->release();
     for (auto* a : {&tab_m, &nw_m, &fw_m, &self_m}) a->release();
     rmark.release();
