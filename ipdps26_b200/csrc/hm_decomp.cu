@@ -148,10 +148,10 @@ __global__ void k_heavy_emit(const uint32_t* slot, const uint32_t* rank, uint32_
 }
 
 // An entry as the histogram kernel walks it: rank << 8 | (C - 2) * 8 +
-// min(size, 7) for an overlap C of 2 or 3, low byte ~0 for a larger one.
+// min(size, 8) - 1 for an overlap C of 2 to 4, low byte ~0 for a larger one.
 __device__ __forceinline__ uint32_t walk_code(uint32_t rank, uint32_t os) {
   const uint32_t c = os & 0xffu;
-  return (rank << 8) | (c <= 3 ? (c - 2) * 8 + min(os >> 8, 7u) : 0xffu);
+  return (rank << 8) | (c <= 4 ? (c - 2) * 8 + min(os >> 8, 8u) - 1 : 0xffu);
 }
 
 // The sorted entries' fields; next = the first position of the neighbour's
@@ -1560,15 +1560,16 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
 }
 
 // The same for centres of at most 32 members (32-bit masks, the bulk) or 64,
-// with most triangles counted in a histogram instead of queued. For one (a, b) a
-// triangle's contributions depend on C_bc, C_ac, g and |c| (only up to
-// C_bc + C_ac + 1), and most overlaps are 1 to 3: those go to 192 bins per
-// warp, which become weighted records when the walk of b's row ends. Rows
-// shorter than kHistMin queue every triangle. The enumeration is issue-bound
-// (87 % of the issue slots with one record per triangle), so instructions per
-// test are what counts. Graphs of up to kDenseSlots hyperedges index their
-// table by rank and need no hash.
-constexpr uint32_t kHistMin = 96, kHistMax = 1u << 16, kHistBins = 192;
+// with most triangles counted in a histogram instead of queued. For given
+// |a|, |b| and C_ab a triangle's contributions depend on C_bc, C_ac, g and |c|
+// (only up to C_bc + C_ac + 1), and most overlaps are small: those go to 288
+// bins per warp, which become weighted records when the warp has walked the
+// rows of all its b alike in |b| and C_ab (of 32 taken together). Fewer than
+// kHistMin tests queue every triangle. The enumeration is issue-bound (86 % of
+// the issue slots with a record per triangle, 31 ms on an 8K-hyperedge hub
+// graph), so instructions per test are what counts. Graphs of up to kDenseSlots
+// hyperedges index their table by rank and need no hash.
+constexpr uint32_t kHistMin = 96, kHistMax = 1u << 16, kHistBins = 288;
 constexpr unsigned kFastThreads = 512, kFastWarps = kFastThreads / kWarp, kFastCol = 4, kFastSlots = 4096;
 struct FastWarp {
   WarpCounts<kFastCol> counts;
@@ -1645,71 +1646,101 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_hh_fast(HHArgs A, uint32_t 
       const uint32_t osc = __ldg((at >> 31 ? A.mos : A.hos) + (at & 0x7fffffffu));
       add_triangle(W, cls, sa, hi >> 24, osc >> 8, (hi >> 16) & 0xffu, osc & 0xffu, hi & 0xffu, (hi >> 8) & 0xffu);
     };
-    for (uint64_t e = A.hoff[ra] + w; e < he; e += kFastWarps) {
-      const uint32_t rb = A.hnbr[e], osb = A.hos[e];
-      const Mask mab = (Mask)A.mask[ao + A.hpos[e]];
-      const Walk B = walk_of(A, ra, rb, e);
-      const uint32_t n = (uint32_t)(B.end - B.first);
-      const bool bins = n >= kHistMin && n < kHistMax;  // a bin's count fits a record's 16 bits
-      const uint32_t* hc = B.code + B.first;
-      const uint64_t part = ((uint64_t)osb << 48) | (B.code == A.hcode ? 0u : 0x80000000u);
-      const uint32_t bias = bins ? 0u : 4u;
-      // One round: the entries cur of the lanes, at hc + at. An entry past the
-      // row's end has a rank no table holds.
-      auto round = [&](uint32_t cur, uint32_t at) {
-        const uint32_t rc = cur >> 8, code = cur & 0xffu;
-        Mask v = 0;
-        if (kDense) {
-          v = val[min(rc - ra, n_ranks - ra)];
-        } else {
-          uint32_t bk = (rc * 2654435761u) >> shift;
-          int t;
-          for (;;) {
-            const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
-            t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
-            if (t >= 0 || k4.w == kEmpty) break;
-            bk = (bk + 1) & bmask;
+    // the warp takes every kFastWarps-th b, 32 at a time, a lane reading each
+    for (uint64_t e0 = A.hoff[ra] + w; e0 < he; e0 += kFastWarps * kWarp) {
+      const uint64_t e = e0 + (uint64_t)lane * kFastWarps;
+      uint32_t my_rb = 0, my_os = 0, my_first = 0, my_n = 0;
+      Mask my_mab = 0;
+      bool marked_row = false;
+      if (e < he) {
+        my_rb = A.hnbr[e];
+        my_os = A.hos[e];
+        my_mab = (Mask)A.mask[ao + A.hpos[e]];
+        const Walk B = walk_of(A, ra, my_rb, e);
+        my_first = (uint32_t)B.first;
+        my_n = (uint32_t)(B.end - B.first);
+        marked_row = B.code != A.hcode;
+      }
+      const unsigned in_marked = __ballot_sync(0xffffffffu, marked_row);
+      unsigned todo = __ballot_sync(0xffffffffu, my_n != 0);
+      while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const uint32_t osb = __shfl_sync(0xffffffffu, my_os, lead);
+        unsigned peers = todo & __ballot_sync(0xffffffffu, my_os == osb);
+        uint32_t total = (peers >> lane) & 1u ? min(my_n, kHistMax) : 0u;
+        for (int d = 16; d; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+        if (total >= kHistMax) {  // a bin's count has to fit a record's 16 bits
+          peers = 1u << lead;
+          total = __shfl_sync(0xffffffffu, my_n, lead);
+        }
+        todo &= ~peers;
+        const bool bins = total >= kHistMin && total < kHistMax;
+        const uint32_t bias = bins ? 0u : 4u;
+        for (unsigned left = peers; left; left &= left - 1) {
+          const int src = __ffs(left) - 1;
+          const uint32_t rb = __shfl_sync(0xffffffffu, my_rb, src), first = __shfl_sync(0xffffffffu, my_first, src),
+                         n = __shfl_sync(0xffffffffu, my_n, src);
+          const Mask mab = __shfl_sync(0xffffffffu, my_mab, src);
+          const bool sub = (in_marked >> src) & 1u;
+          const uint32_t* hc = (sub ? A.mcode : A.hcode) + first;
+          const uint64_t part = ((uint64_t)osb << 48) | (sub ? 0x80000000u : 0u);
+          // One round: the entries cur of the lanes, at hc + at. An entry past
+          // the row's end has a rank no table holds.
+          auto round = [&](uint32_t cur, uint32_t at) {
+            const uint32_t rc = cur >> 8, code = cur & 0xffu;
+            Mask v = 0;
+            if (kDense) {
+              v = val[min(rc - ra, n_ranks - ra)];
+            } else {
+              uint32_t bk = (rc * 2654435761u) >> shift;
+              int t;
+              for (;;) {
+                const uint4 k4 = reinterpret_cast<const uint4*>(keys)[bk];
+                t = k4.x == rc ? 0 : k4.y == rc ? 1 : k4.z == rc ? 2 : k4.w == rc ? 3 : -1;
+                if (t >= 0 || k4.w == kEmpty) break;
+                bk = (bk + 1) & bmask;
+              }
+              if (t >= 0) v = val[4 * bk + (uint32_t)t];
+            }
+            const uint32_t cac = bits(v), g = bits(v & mab);
+            const bool take = cac == 1 || (cac > 1 && rb > rc);  // three heavy pairs: once, b ranked highest
+            const bool slow = cac + ((code & 0x80u) >> 5) + bias > 3;
+            if (take && !slow) atomicAdd(&F->hist[g * 72 + cac * 24 + code - 24], 1u);
+            // the others wait as their entry's place and what is known of the
+            // triangle; |c| and C_bc are read when 32 have come together
+            queue_records(take && slow, part | ((uint64_t)(cac | (g << 8)) << 32) | (first + at), F->late, ln, late);
+          };
+          for (uint32_t c0 = 0; c0 < n; c0 += kHistMax) {
+            const uint32_t c1 = min(n, c0 + kHistMax);
+            // two rounds at a time, their successors' entries loaded before them
+            uint32_t at = c0 + lane;
+            uint32_t x = at < c1 ? __ldg(hc + at) : kEmpty, y = at + kWarp < c1 ? __ldg(hc + at + kWarp) : kEmpty;
+            for (uint32_t j0 = c0; j0 < c1; j0 += 2 * kWarp) {
+              const uint32_t to = at + 2 * kWarp;
+              const uint32_t xn = to < c1 ? __ldg(hc + to) : kEmpty,
+                             yn = to + kWarp < c1 ? __ldg(hc + to + kWarp) : kEmpty;
+              round(x, at);
+              if (j0 + kWarp < c1) round(y, at + kWarp);
+              at = to;
+              x = xn;
+              y = yn;
+            }
+            if (c1 < n) flush_counts(W, A.raw);
           }
-          if (t >= 0) v = val[4 * bk + (uint32_t)t];
         }
-        const uint32_t cac = bits(v), g = bits(v & mab);
-        const bool take = cac == 1 || (cac > 1 && rb > rc);  // three heavy pairs: once, b ranked highest
-        const bool slow = cac + ((code & 0x80u) >> 5) + bias > 3;
-        if (take && !slow) atomicAdd(&F->hist[g * 48 + cac * 16 + code - 16], 1u);
-        // the others wait as their entry's place and what is known of the
-        // triangle; |c| and C_bc are read when 32 have come together
-        queue_records(take && slow, part | ((uint64_t)(cac | (g << 8)) << 32) | ((uint32_t)B.first + at), F->late, ln,
-                      late);
-      };
-      for (uint32_t c0 = 0; c0 < n; c0 += kHistMax) {
-        const uint32_t c1 = min(n, c0 + kHistMax);
-        // two rounds at a time, their successors' entries loaded before them
-        uint32_t at = c0 + lane;
-        uint32_t x = at < c1 ? __ldg(hc + at) : kEmpty, y = at + kWarp < c1 ? __ldg(hc + at + kWarp) : kEmpty;
-        for (uint32_t j0 = c0; j0 < c1; j0 += 2 * kWarp) {
-          const uint32_t to = at + 2 * kWarp;
-          const uint32_t xn = to < c1 ? __ldg(hc + to) : kEmpty, yn = to + kWarp < c1 ? __ldg(hc + to + kWarp) : kEmpty;
-          round(x, at);
-          if (j0 + kWarp < c1) round(y, at + kWarp);
-          at = to;
-          x = xn;
-          y = yn;
+        if ((tests += min(total, kHistMax)) >= kFlushTests - 2 * kHistMax) {
+          flush_counts(W, A.raw);
+          tests = 0;
         }
-        if (c1 < n) flush_counts(W, A.raw);
-      }
-      if ((tests += min(n, kHistMax)) >= kFlushTests - 2 * kHistMax) {
-        flush_counts(W, A.raw);
-        tests = 0;
-      }
-      if (bins) {
+        if (!bins) continue;
         __syncwarp();
 #pragma unroll 1
         for (uint32_t k0 = 0; k0 < kHistBins; k0 += kWarp) {
-          const uint32_t k = k0 + lane;  // |c| (7 standing for 7 or more) + 8 (C_bc - 2) + 16 (C_ac - 1) + 48 g
-          const uint32_t c = F->hist[k], g = k / 48, m = k - 48 * g;
+          const uint32_t k = k0 + lane;  // |c| - 1 (7 for 8 or more) + 8 (C_bc - 2) + 24 (C_ac - 1) + 72 g
+          const uint32_t c = F->hist[k], g = k / 72, m = k - 72 * g, r = m % 24;
           if (c) F->hist[k] = 0;
-          queue_records(c != 0, pack6(osb >> 8, m & 7u, osb & 0xffu, 2 + ((m >> 3) & 1u), (m >> 4) + 1, g, c), F->q, qn,
-                        [&](uint64_t r) { add_record(W, cls, sa, r); });
+          queue_records(c != 0, pack6(osb >> 8, (r & 7u) + 1, osb & 0xffu, 2 + (r >> 3), m / 24 + 1, g, c), F->q, qn,
+                        [&](uint64_t x) { add_record(W, cls, sa, x); });
         }
       }
     }
