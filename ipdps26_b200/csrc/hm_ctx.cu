@@ -63,7 +63,16 @@ void trim_pool(hm_ctx* ctx, size_t keep) {
   cudaMemPoolTrimTo(ctx->pool, keep);
 }
 
-size_t pool_keep(const hm_ctx* ctx) { return std::min(kPoolKeep, ctx->budget / 32); }
+size_t pool_keep(const hm_ctx* ctx) {
+  // all of a small pool or nothing: part of a large one is seldom the part the
+  // next graph asks for, and mapping the rest anew took up to 60 ms
+  uint64_t held = 0;
+  if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return held <= std::min<uint64_t>(kPoolKeep, ctx->budget / 32) ? (size_t)held : 0;
+}
 
 }  // namespace hm
 

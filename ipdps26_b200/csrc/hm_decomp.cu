@@ -919,7 +919,8 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
       const uint32_t ra = A.hown[e], rb = A.hnbr[e], os = A.hos[e];
       const uint32_t a = A.slot[ra];
       const uint32_t za = A.esize[a], zb = os >> 8;
-      if (owns_pair(ra, za, rb, zb) && !A.spread[ra]) {
+      // (an unmarked owner spreads for its unmarked partners only)
+      if (owns_pair(ra, za, rb, zb) && !(A.spread[ra] && (!A.rmark || A.rmark[ra] || !A.rmark[rb]))) {
         const uint32_t b = A.slot[rb];
         un = A.rmark && !A.rmark[ra] && !A.rmark[rb];
         sa = za;
@@ -1068,10 +1069,8 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
   __shared__ uint32_t s_item;
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   constexpr unsigned kW = kSpreadThreads / kWarp;
-  // y of all hyperedges and, for an unmarked owner, of the marked ones
   const uint32_t vec = (A.n_nodes + 1) & ~1u;
-  uint2* y = A.y + (uint64_t)blockIdx.x * vec * (A.rmark ? 2 : 1);
-  uint2* ym = y + vec;
+  uint2* y = A.y + (uint64_t)blockIdx.x * vec;
   for (unsigned k = threadIdx.x; k < kRawClass; k += kSpreadThreads) cnt[k] = 0;
   for (;;) {
     __syncthreads();
@@ -1080,7 +1079,12 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
     if (s_item >= A.n_list) break;
     const uint32_t ra = A.list[s_item], a = A.slot[ra], sa = A.esize[a];
     const uint32_t* pa = A.vmem + A.voff[a];
-    const bool both = A.rmark && !A.rmark[ra];
+    // an unmarked owner's unmarked partners count marked third hyperedges only;
+    // its few marked ones are left to part_pairs
+    const bool un = A.rmark && !A.rmark[ra];
+    const uint2* fw = un ? A.fw_m : A.fw;
+    const uint32_t* ncat = un ? A.ncat_m : A.ncat;
+    const uint2* self = un ? A.self_m : A.self;
     // the block takes the rows of the members one after another (a node's
     // row can be hundreds of times another's)
     uint64_t cells = 0;
@@ -1091,14 +1095,9 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
       const uint32_t l = (uint32_t)(A.foff[v + 1] - o);
       for (uint32_t k = threadIdx.x; k < l; k += kSpreadThreads) {
         const uint32_t x = __ldg(A.fnbr + o + k);
-        const uint2 q = __ldg(A.fw + o + k);
+        const uint2 q = __ldg(fw + o + k);
         if (q.x) atomicAdd(&y[x].x, q.x);
         if (q.y) atomicAdd(&y[x].y, q.y);
-        if (both) {
-          const uint2 m = __ldg(A.fw_m + o + k);
-          if (m.x) atomicAdd(&ym[x].x, m.x);
-          if (m.y) atomicAdd(&ym[x].y, m.y);
-        }
       }
     }
     for (uint32_t i = 0; i < sa; ++i) cells += A.foff[pa[i] + 1] - A.foff[pa[i]];
@@ -1112,24 +1111,19 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
       const uint64_t e = e0 + (lane >> 3);
       uint32_t sb = 0, C = 0;
       uint64_t bo = 0;
-      bool un = false;
       if (e < he) {
         const uint32_t rb = A.hnbr[e], os = A.hos[e];
-        if (owns_pair(ra, sa, rb, os >> 8)) {
+        if (owns_pair(ra, sa, rb, os >> 8) && !(un && A.rmark[rb])) {
           sb = os >> 8;
           C = os & 0xffu;
           bo = A.voff[A.slot[rb]];
-          un = both && !A.rmark[rb];
         }
       }
-      const uint32_t* ncat = un ? A.ncat_m : A.ncat;
-      const uint2* self = un ? A.self_m : A.self;
       uint64_t t[5] = {0, 0, 0, 0, 0};  // q2, q3, r by category
       for (uint32_t j = lane & 7u; j < sb; j += 8) {
         const uint32_t v = __ldg(A.vmem + bo + j);
-        uint2 q = y[v];
+        const uint2 q = y[v];
         if (q.x != ~0u || q.y != ~0u) {
-          if (un) q = ym[v];
           t[0] += q.x;
           t[1] += q.y;
           continue;
@@ -1159,16 +1153,14 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
     }
     __syncthreads();
     if (A.n_nodes <= 4 * cells) {  // clear it all, two entries at a time (the vectors start at even entries)
-      for (uint32_t i = threadIdx.x; i < (both ? vec : vec / 2); i += kSpreadThreads)
+      for (uint32_t i = threadIdx.x; i < vec / 2; i += kSpreadThreads)
         reinterpret_cast<uint4*>(y)[i] = make_uint4(0, 0, 0, 0);
     } else {
       for (uint32_t i = w; i < sa; i += kW) {
         const uint32_t v = __ldg(pa + i);
         if (lane == 0) y[v] = make_uint2(0, 0);
         for (uint64_t k = A.foff[v] + lane; k < A.foff[v + 1]; k += kWarp) {
-          const uint32_t x = __ldg(A.fnbr + k);
-          y[x] = make_uint2(0, 0);
-          if (both) ym[x] = make_uint2(0, 0);
+          y[__ldg(A.fnbr + k)] = make_uint2(0, 0);
         }
       }
     }
@@ -2049,8 +2041,8 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
     // one node vector per block of k_spread_pairs, a sixteenth of the room at most
     const size_t vec = ((size_t)V + 1) & ~(size_t)1;
     P.y_blocks = (uint32_t)std::max<size_t>(
-        1, std::min<size_t>({(size_t)ctx->n_sms, (size_t)P.n_spread, room / 16 / (sizeof(uint2) * vec * (mark ? 2 : 1))}));
-    const size_t y_all = (size_t)P.y_blocks * vec * (mark ? 2 : 1);
+        1, std::min<size_t>({(size_t)ctx->n_sms, (size_t)P.n_spread, room / 16 / (sizeof(uint2) * vec)}));
+    const size_t y_all = (size_t)P.y_blocks * vec;
     HM_TRY(P.self.alloc(ctx, g->h2v_tail));
     if (mark) HM_TRY(P.self_m.alloc(ctx, g->h2v_tail));
     if (mark) HM_TRY(P.fw_m.alloc(ctx, 2 * pairs));

@@ -806,7 +806,8 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
     TouchArgs C = A;
     C.n_long = 0;
     C.short_ids = sids.p + n_large + n_mid;
-    C.slices = slices_for(n_short, sms * 4 * kWarps, 16);
+    // four slices per place: rows of up to 128 neighbours differ much in length
+    C.slices = slices_for(n_short, sms * 4 * kWarps * 4, 16);
     C.n = n_short * C.slices;
     C.queue = queues + 2;
     k_touch_warp<<<std::min<unsigned>(sms * 4, (C.n + kWarps - 1) / kWarps), kBlock, 0, st>>>(C);

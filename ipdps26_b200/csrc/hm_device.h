@@ -44,7 +44,8 @@ int dev_alloc(hm_ctx* ctx, void** p, size_t bytes);
 void dev_free(hm_ctx* ctx, void* p, size_t bytes);
 void trim_pool(hm_ctx* ctx, size_t keep = 0);  // returns the pool's cached free blocks past `keep` bytes to the device
 // What the pool keeps cached when a graph or server goes, so that the next one
-// of a context finds its memory mapped: at most kPoolKeep, a 32nd of the budget.
+// of a context finds its memory mapped: all it holds if that is at most
+// kPoolKeep and a 32nd of the budget, else nothing.
 constexpr size_t kPoolKeep = size_t(256) << 20;
 size_t pool_keep(const hm_ctx* ctx);
 
