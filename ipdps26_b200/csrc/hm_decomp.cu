@@ -384,11 +384,12 @@ __global__ void k_bucket_scatter(const uint8_t* code, uint32_t n, uint32_t* star
   }
 }
 
-// Launch shapes of the enumeration: 0 a warp searching a's row (few tests,
-// less than an eighth of the row, or a row no table holds), 1 and 2 the
+// Launch shapes of the enumeration: 0 a warp searching a's row (fewer tests
+// than kTableMin or an eighth of the row, or a row no table holds), 1 and 2 the
 // histogram kernel with 32-bit and 64-bit masks (up to 3072 entries ranked
 // above a), 3 the large tables (up to 12288, and centres of more than 64
 // members).
+constexpr uint64_t kTableMin = 64;
 constexpr uint32_t kHHSmall = 3072, kHHLarge = 12288;
 constexpr uint32_t kDenseSlots = 12288;  // up to this many hyperedges the tables are indexed by rank
 __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint8_t* esize,
@@ -406,7 +407,7 @@ __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t 
     if (work) {
       const uint32_t a = slot[r], l = len[a];
       unsigned shape = 0;
-      if (work * 8 >= l) {
+      if (work >= kTableMin && work * 8 >= l) {
         const bool narrow = esize[a] <= 32;
         uint32_t up = 0;
         if (!(narrow && n <= kDenseSlots)) {

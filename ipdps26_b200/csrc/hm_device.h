@@ -46,7 +46,7 @@ void trim_pool(hm_ctx* ctx, size_t keep = 0);  // returns the pool's cached free
 // What the pool keeps cached when a graph or server goes, so that the next one
 // of a context finds its memory mapped: all it holds if that is at most
 // kPoolKeep and a 32nd of the budget, else nothing.
-constexpr size_t kPoolKeep = size_t(256) << 20;
+constexpr size_t kPoolKeep = size_t(2) << 30;
 size_t pool_keep(const hm_ctx* ctx);
 
 // Owning device array; the context's budget is charged for its bytes.
