@@ -322,8 +322,10 @@ int hm_count_static30_async(hm_graph* g, uint64_t* d_out30, void* stream);
  * (MoCHy-master/main_exact.cpp:91-129): store read once
  * (4 nnz(H2V) + 8 nnz(H2H)), sum over id-ordered adjacent pairs of
  * 8 (d+(a) + d+(b)) with d+ the neighbours of larger id, and
- * 4 (|a| + |b|) per pair that closes a triangle. kernel_bytes is what this
- * engine's kernels read. Runs one extra diagnostic count (slow). */
+ * 4 (|a| + |b|) per pair that closes a triangle. kernel_bytes and probes are
+ * those of the enumeration of all triangles (what sharded counts run); a full
+ * count that takes the decomposition reads far less. Runs one extra diagnostic
+ * count (slow). */
 typedef struct hm_traffic_t {
   uint64_t store_bytes;
   uint64_t merge_bytes;
@@ -336,12 +338,15 @@ typedef struct hm_traffic_t {
 int hm_graph_traffic(hm_graph* g, hm_traffic_t* t);
 
 /* ---- launch schedules, and their autotuner --------------------------------
+ * They apply to the enumeration of triangles: sharded counts, vertex triads,
+ * small update batches, and graphs that the decomposition (light pairs in
+ * closed form) does not suit. The decomposition has no schedule.
  * Static count: the closed-triangle phase runs three persistent launch
  * shapes over one heaviest-first list of centres, split by the length d of
  * each centre's oriented row: d <= warp_row one warp per centre
  * (warp_row <= 128), d <= small_row one 256-thread block per centre with a
- * 4096-slot table (warp_row <= small_row <= 2048), longer rows blocks with an
- * 8192-slot table. Touched-triple count (the delta of every update batch):
+ * 4096-slot table (warp_row <= small_row <= 2048), longer rows 1024-thread blocks
+ * with a 16384-slot table. Touched-triple count (the delta of every update batch):
  * the same three shapes per marked hyperedge m by the length of its row:
  * <= touch_warp_row one warp (<= 128), <= touch_mid_row 4096-slot blocks
  * (touch_warp_row <= touch_mid_row <= 2048), longer rows 1024-thread blocks

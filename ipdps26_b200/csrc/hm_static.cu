@@ -7,6 +7,10 @@
 // one thread per hyperedge over closed triangles only and never sees open
 // triples; this file counts both.
 //
+// A full count of a graph with few heavy pairs goes to the decomposition
+// (hm_decomp.cu). Sharded counts, vertex triads, the traffic model and the
+// other graphs enumerate every triangle, here:
+//
 // Algorithm (all integer, exact):
 //   1. Open phase, one warp per centre a. Every unordered neighbour pair
 //      {b, c} of a is classified as if it were open: its class depends only on

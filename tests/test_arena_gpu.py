@@ -86,3 +86,36 @@ def test_tight_budget_trims_or_fails_cleanly(factor):
             assert err.status == HM_ERR_NOMEM, str(err)
         if factor >= 16.0:
             assert done == 6, str(err)
+
+
+def test_pooled_arena_moves_to_chunks_under_every_budget():
+    """A small store's arena starts in the context's pool and moves to mapped
+    chunks when it grows: in one piece while the budget holds both copies,
+    through host memory while it does not. Over budgets from the built store's
+    own bytes upwards a batch either fails with HM_ERR_NOMEM or leaves exactly
+    the store of an unlimited budget, and it succeeds from some budget on."""
+    from ipdps26_b200 import engine
+    from ipdps26_b200._lib import HM_ERR_NOMEM, HmError
+
+    rng = np.random.default_rng(13)
+    n_nodes = 64
+    off, mem = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(2500)])
+    io, im = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(2500)])
+
+    def run(c):
+        with engine.Graph(c, off, mem, n_nodes) as g:
+            used = c.memory()[0]
+            _, delta = g.apply_batch([], io, im)
+            return used, g.info().n_adjacent, g.count_static30().tolist(), delta.tolist()
+
+    with engine.Context(0) as free:
+        used, *want = run(free)
+    passed = []
+    for mb in range(0, 513, 16):
+        with engine.Context(0, mem_budget_bytes=int(used + (mb << 20))) as tight:
+            try:
+                passed.append(list(run(tight)[1:]) == want)
+            except HmError as e:
+                assert e.status == HM_ERR_NOMEM, str(e)
+                assert mb < 512, str(e)
+    assert passed and all(passed)

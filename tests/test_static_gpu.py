@@ -268,3 +268,27 @@ def test_oriented_rows_longer_than_the_table(ctx):
         every = g.count_touching30(np.arange(len(rows), dtype=np.uint32))
         assert full.tolist() == every.tolist()
         assert int(full.sum()) > 0
+
+
+# One bitmap of the slots per row: its last word holds 1 to 32 slots, it is
+# used up to 81,920 slots (sorted wedges beyond), a row of many wedges takes a
+# block instead of a warp, and shared positions past the 64th leave no mask bit.
+@pytest.mark.parametrize("n,n_nodes,kmax", [(1, 4, 3), (31, 20, 4), (32, 20, 4), (33, 20, 4), (63, 30, 4),
+                                            (64, 30, 70), (65, 30, 70), (150, 260, 255),
+                                            (81_919, 60_000, 4), (81_920, 60_000, 4), (81_921, 60_000, 4)])
+def test_h2h_rows_at_the_edges_of_the_bitmap(ctx, n, n_nodes, kmax):
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(n)
+    kmax = min(kmax, n_nodes)
+    rows = [sorted(set(rng.integers(0, n_nodes, size=int(rng.integers(1, kmax + 1))).tolist())) for _ in range(n)]
+    rows[-1] = list(range(kmax))  # the last slot's bit is set in many rows
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        holds = {}
+        for a, r in enumerate(rows):
+            for v in r:
+                holds.setdefault(v, []).append(a)
+        pairs = len({(a, b) for h in holds.values() for a in h for b in h if a < b})
+        assert g.info().n_adjacent == 2 * pairs
+        assert g.count_static30().tolist() == oracle.static30(off, mem, n_nodes).tolist()
