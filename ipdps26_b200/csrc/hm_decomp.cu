@@ -390,6 +390,10 @@ __global__ void k_bucket_scatter(const uint8_t* code, uint32_t n, uint32_t* star
 // above a), 3 the large tables (up to 12288, and centres of more than 64
 // members).
 constexpr uint64_t kTableMin = 64;
+// Up to this many heavy entries and tests (sum h^2) a graph is searched by entry,
+// one or two entries for each warp of the launch. With 17,000 entries (100K
+// hyperedges) the searches took 46 us of half the chip, the tables' launch 12 us.
+constexpr uint64_t kEntriesFew = 1 << 13, kEntryTests = 1 << 18;
 constexpr uint32_t kHHSmall = 3072, kHHLarge = 12288;
 constexpr uint32_t kDenseSlots = 12288;  // up to this many hyperedges the tables are indexed by rank
 __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t n, const uint8_t* esize,
@@ -595,6 +599,7 @@ struct NodeArgs {
   uint32_t n_work;
   unsigned int* queue;
   unsigned long long* raw;
+  uint32_t slices;  // part_nodes: item k is slice k % slices of node k / slices
 };
 
 __device__ __forceinline__ uint32_t node_hash(uint32_t key, uint32_t shift) { return (key * 2654435761u) >> shift; }
@@ -720,8 +725,9 @@ struct NodeWarp {
   uint32_t keys[kNodeWarpSlots];
   uint32_t filter[kWarp];
 };
-template <bool kTouch>
+template <bool kTouch, bool kSliced>
 __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
+  const uint32_t slices = kSliced ? A.slices : 1;
   const unsigned lane = lane_id();
   uint32_t* keys = S->keys;
   uint2* val = S->val;
@@ -730,10 +736,11 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
     uint32_t it = 0;
     if (lane == 0) it = atomicAdd(A.queue, 1u);
     it = __shfl_sync(0xffffffffu, it, 0);
-    if (it >= A.n_work) break;
-    const uint32_t u = A.work[it];
+    if (it / slices >= A.n_work) break;
+    const uint32_t u = A.work[it / slices], slice = it % slices;
     const uint64_t uo = A.poff[u];
     const uint32_t d = A.plen[u];
+    if (slice >= d) continue;
     uint32_t slots = 64, qn = 0;
     while (slots < 2 * d && slots < kNodeWarpSlots) slots <<= 1;
     const uint32_t shift = 32u - (31u - (uint32_t)__clz(slots)), mask = slots - 1;
@@ -747,8 +754,8 @@ __device__ void part_nodes(const NodeArgs& A, NodeWarp* S) {
     }
     __syncwarp();
     const uint32_t filter = S->filter[lane];
-    for (uint32_t i0 = 0; i0 < d; i0 += kWarp)
-      node_walk<kTouch, true>(A, keys, val, shift, mask, filter, uo, d, i0, 1, S->q, qn, F);
+    for (uint32_t i0 = slice; i0 < d; i0 += kWarp * slices)
+      node_walk<kTouch, true>(A, keys, val, shift, mask, filter, uo, d, i0, slices, S->q, qn, F);
     if (lane < qn) node_sum<kTouch>(S->q[lane], val, A, uo, F);  // the records name this node's table
     __syncwarp();
   }
@@ -850,6 +857,7 @@ struct PairArgs {
   uint2* y;               // per block of k_spread_pairs: n_nodes entries (rounded up to even), zero between items
   uint32_t n_nodes;
   uint32_t per_warp, wide;  // entries a warp takes at once; combinations from which it takes a pair as a whole
+  uint32_t slices;          // warps that share an entry (per_warp 1)
   unsigned int* queue;
   unsigned long long* raw;
 };
@@ -909,8 +917,9 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
   const unsigned lane = lane_id(), grp = lane >> 3, sub = lane & 7u;
   for (unsigned k = threadIdx.x; k < kRawClass; k += kBlock) cnt[k] = 0;
   __syncthreads();
-  for (uint64_t e0 = ((uint64_t)vb * kWarps + threadIdx.x / kWarp) * A.per_warp; e0 < A.nh;
-       e0 += (uint64_t)nb * kWarps * A.per_warp) {
+  const unsigned slice = threadIdx.x / kWarp % A.slices;
+  for (uint64_t e0 = ((uint64_t)vb * kWarps + threadIdx.x / kWarp) / A.slices * A.per_warp; e0 < A.nh;
+       e0 += (uint64_t)nb * kWarps / A.slices * A.per_warp) {
     const uint64_t e = e0 + grp;
     uint32_t sa = 0, sb = 0, C = 0;
     bool un = false;
@@ -967,14 +976,20 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
       todo &= todo - 1;
       const uint64_t k2 = q2, k3 = q3, s0 = r0, s1 = r1, s2 = r2;  // this lane's own pair, set aside
       q2 = q3 = r0 = r1 = r2 = 0;
-      run(lane, 32, __shfl_sync(0xffffffffu, sa, src), __shfl_sync(0xffffffffu, sb, src),
-          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pa, src)),
-          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pb, src)),
-          __shfl_sync(0xffffffffu, (unsigned long long)ma, src), __shfl_sync(0xffffffffu, (unsigned long long)mb, src),
-          __shfl_sync(0xffffffffu, (int)un, src) != 0);
+      const uint32_t na = __shfl_sync(0xffffffffu, sa, src), nb = __shfl_sync(0xffffffffu, sb, src);
+      const uint32_t* xa =
+          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pa, src));
+      const uint32_t* xb =
+          reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)pb, src));
+      const uint64_t sma = __shfl_sync(0xffffffffu, (unsigned long long)ma, src);
+      const uint64_t smb = __shfl_sync(0xffffffffu, (unsigned long long)mb, src);
+      const bool unmarked = __shfl_sync(0xffffffffu, (int)un, src) != 0;
+      if (A.slices == 1) run(lane, 32, na, nb, xa, xb, sma, smb, unmarked);  // a fixed step: 2 % of a 100K count
+      else run(slice * 32 + lane, A.slices * 32, na, nb, xa, xb, sma, smb, unmarked);
       __syncwarp();
       const uint64_t t2 = warp_sum(q2), t3 = warp_sum(q3), u0 = warp_sum(r0), u1 = warp_sum(r1), u2 = warp_sum(r2);
-      if ((int)lane == src) add_pair(cnt, sa, sb, C, t2, t3, u0, u1, u2, un);
+      // a further slice adds its sums alone, as an unmarked pair does
+      if ((int)lane == src) add_pair(cnt, sa, sb, C, t2, t3, u0, u1, u2, un || slice);
       q2 = k2;
       q3 = k3;
       r0 = s0;
@@ -1200,6 +1215,8 @@ struct HHArgs {
   const uint32_t* work;   // ranks of the centres
   uint32_t n_work;
   uint32_t slices;        // k_hh_large: item k is slice k % slices of centre k / slices
+  const uint32_t* hown;   // owner of every heavy entry
+  uint64_t entries;       // by entry: that many heavy entries, no work list (0: by centre)
   unsigned int* queue;
   unsigned long long* raw;
 };
@@ -1379,13 +1396,18 @@ __device__ __forceinline__ void fill_classes(int8_t* cls) {
   }
 }
 
-// One warp per centre with few tests: each c is searched in a's id-sorted row.
+// Searches: each c of b's heavy row past a is looked up in a's id-sorted row.
+// By centre (a warp takes all of a's heavy neighbours) for those with few
+// tests; by entry (a warp takes one heavy pair (a, b)) where the whole graph has
+// few, as then every search is in flight at once and no launch is needed for the
+// tables: with the counters in the last block, 1K hyperedges of 558 heavy
+// entries went from 75 to 72 us per count.
 constexpr unsigned kSearchCol = 4;
 struct SearchShared {
   WarpCounts<kSearchCol> wc[kWarps];
   int8_t cls[128];
 };
-__device__ void part_search(const HHArgs& A, SearchShared& S) {
+__device__ void part_search(unsigned vb, unsigned nb, const HHArgs& A, SearchShared& S) {
   const unsigned lane = lane_id();
   WarpCounts<kSearchCol>* W = &S.wc[threadIdx.x / kWarp];
   int8_t* cls = S.cls;
@@ -1393,17 +1415,30 @@ __device__ void part_search(const HHArgs& A, SearchShared& S) {
   clear_counts(W);
   __syncthreads();
   uint32_t tests = 0;
+  uint64_t it = (uint64_t)vb * kWarps + threadIdx.x / kWarp;  // by entry: every nb * kWarps-th
   for (;;) {
-    uint32_t it = 0;
-    if (lane == 0) it = atomicAdd(A.queue, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    if (it >= A.n_work) break;
-    const uint32_t ra = A.work[it], a = A.slot[ra];
+    uint64_t e, he;
+    uint32_t ra;
+    if (A.entries) {
+      if (it >= A.entries) break;
+      e = it;
+      he = it + 1;
+      ra = A.hown[e];
+      it += (uint64_t)nb * kWarps;
+    } else {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(A.queue, 1u);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= A.n_work) break;
+      ra = A.work[k];
+      e = A.hoff[ra];
+      he = A.hoff[ra + 1];
+    }
+    const uint32_t a = A.slot[ra];
     const uint64_t ao = A.off[a];
     const uint32_t al = A.len[a];
     const uint32_t sa = A.esize[a];
-    const uint64_t he = A.hoff[ra + 1];
-    for (uint64_t e = A.hoff[ra]; e < he; ++e) {
+    for (; e < he; ++e) {
       const uint32_t rb = A.hnbr[e], osb = A.hos[e];
       const uint64_t mab = A.mask[ao + A.hpos[e]];
       const Walk B = walk_of(A, ra, rb, e);
@@ -1755,25 +1790,75 @@ static_assert(kNodeSmall == 1024 / 4 * 3 && kNodeMid == 4096 / 4 * 3 && kNodeLar
 template <bool kTouch>
 __global__ void __launch_bounds__(kBlock, 6) k_node_tri_warp(NodeArgs A) {
   __shared__ NodeWarp S[kWarps];
-  part_nodes<kTouch>(A, &S[threadIdx.x / kWarp]);
+  part_nodes<kTouch, false>(A, &S[threadIdx.x / kWarp]);
+}
+
+// The counter block of the static count (hm_static.cu: 30 closed classes, 6
+// removals, 6 open-pair counts) from the raw sums, by one block: a thread per
+// sum adds it to the few counters it belongs to.
+struct FinishShared {
+  unsigned long long o[42];
+};
+__device__ void finish(FinishShared& S, const unsigned long long* raw, unsigned long long* out) {
+  unsigned long long* o = S.o;
+  const unsigned t = threadIdx.x;
+  auto sum = [&](unsigned k) { return __ldcg(raw + k); };  // written by other blocks' atomics, in L2
+  if (t < 42) o[t] = sum(t < 30 ? kRawClass + t : t < 36 ? kRawRem + t - 30 : kRawOpen + t - 36);
+  __syncthreads();
+  auto add = [&](unsigned k, unsigned long long n) { atomicAdd(&o[k], n); };
+  if (t < 4) {
+    const unsigned long long n = sum(kRawDist + t);
+    add(26 + t, n);
+    add(35, t * n);
+    add(34, (3 - t) * n);
+  } else if (t >= 32 && t < 42) {
+    const unsigned i = t - 32;  // the order of star_index
+    const unsigned x = i < 6 ? 0 : i < 9 ? 1 : 2, y = i < 6 ? (i < 3 ? 0 : i < 5 ? 1 : 2) : i < 8 ? 1 : 2;
+    const unsigned z = i < 6 ? (i < 3 ? i : i < 5 ? i - 2 : 2) : i < 8 ? i - 5 : 2;
+    const unsigned long long n = sum(kRawStar + i);
+    const unsigned ex = x > 0, ey = y > 0, ez = z > 0;
+    add(ex + ey + ez, n);
+    add(30 + (x == 2) + 2 * (ey + ez), n);
+    add(30 + (y == 2) + 2 * (ex + ez), n);
+    add(30 + (z == 2) + 2 * (ex + ey), n);
+  } else if (t >= 64 && t < 91) {
+    const unsigned i = t - 64, ua = i / 9, ub = i / 3 % 3, c = i % 3;
+    const unsigned long long n = sum(kRawPair + i);
+    const unsigned ea = ua > 0, eb = ub > 0, l = c > 0;
+    // regions: a's and b's own, the pair's, the common node, c's own if it has a second member
+    const int pat = (int)(ea | (eb << 1) | (l << 2) | (1u << 3) | (1u << 6));
+    add(static_class_of_pattern(pat), n);
+    add(30 + (ua > 1) + 2 * (eb + l), n);
+    add(30 + (ub > 1) + 2 * (ea + l), n);
+    add(30 + (c == 2) + 4, n);
+  }
+  __syncthreads();
+  if (t < 42) out[t] = o[t];
 }
 
 // The parts of a count that run in small blocks, side by side in one launch:
 // blocks [0, end[0]) search, [end[0], end[1]) sum the heavy pairs, then node
 // triangles of the short rows, open pairs, stars. At small sizes each part is
-// one wave of latency, so one launch takes as long as its slowest part.
+// one wave of latency, so one launch takes as long as its slowest part. It is
+// the count's last launch but for the counters, which its last block to end makes
+// from the sums where the grid is one wave (a launch of one block took 4 us of a
+// 1K-hyperedge count's 75); over several waves each block's wait for its own
+// sums to land cost more than that launch (7 us of 484 at 100K hyperedges).
 struct PartArgs {
   HHArgs search;
   PairArgs pairs;
   NodeArgs nodes;
   OpenArgs open;
   unsigned end[5];
+  unsigned int* ended;      // blocks that have added their sums (null: k_decomp_finish follows)
+  unsigned long long* out;  // 42 counters
 };
 union PartShared {
   SearchShared search;
   PairCounts pairs;
   NodeWarp nodes[kWarps];
   OpenHist open;
+  FinishShared finish;
 };
 template <bool kTouch>
 __global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ PartArgs A) {
@@ -1781,61 +1866,31 @@ __global__ void __launch_bounds__(kBlock, 4) k_parts(const __grid_constant__ Par
   PartShared& S = *reinterpret_cast<PartShared*>(mem);
   const unsigned b = blockIdx.x;
   if (b < A.end[0]) {
-    part_search(A.search, S.search);
+    part_search(b, A.end[0], A.search, S.search);
   } else if (b < A.end[1]) {
     part_pairs(b - A.end[0], A.end[1] - A.end[0], S.pairs, A.pairs);
   } else if (b < A.end[2]) {
-    part_nodes<kTouch>(A.nodes, &S.nodes[threadIdx.x / kWarp]);
+    part_nodes<kTouch, true>(A.nodes, &S.nodes[threadIdx.x / kWarp]);
   } else if (b < A.end[3]) {
     part_open(b - A.end[2], A.end[3] - A.end[2], S.open, A.open);
   } else {
     part_stars(b - A.end[3], A.end[4] - A.end[3], A.pairs.ncat, A.pairs.ncat_m, A.pairs.n_nodes, A.search.raw);
   }
+  if (!A.ended) return;
+  __shared__ bool last;
+  __threadfence();  // this thread's sums before the block's count
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(A.ended, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    finish(S.finish, A.search.raw, A.out);
+  }
 }
 
-// The counter block of the static count (hm_static.cu: 30 closed classes, 6
-// removals, 6 open-pair counts) from the raw sums.
 __global__ void k_decomp_finish(const unsigned long long* raw, unsigned long long* out) {
-  __shared__ unsigned long long s[kRawSize], o[42];
-  const unsigned t = threadIdx.x;
-  for (unsigned k = t; k < kRawSize; k += blockDim.x) s[k] = raw[k];
-  __syncthreads();
-  for (unsigned k = t; k < 42; k += blockDim.x)
-    o[k] = k < 30 ? s[kRawClass + k] : k < 36 ? s[kRawRem + k - 30] : s[kRawOpen + k - 36];
-  __syncthreads();
-  if (t == 0) {
-    for (unsigned k = 0; k < 4; ++k) {
-      const unsigned long long n = s[kRawDist + k];
-      o[26 + k] += n;
-      o[35] += k * n;
-      o[34] += (3 - k) * n;
-    }
-    unsigned i = 0;
-    for (unsigned x = 0; x < 3; ++x)
-      for (unsigned y = x; y < 3; ++y)
-        for (unsigned z = y; z < 3; ++z, ++i) {
-          const unsigned long long n = s[kRawStar + i];
-          const unsigned ex = x > 0, ey = y > 0, ez = z > 0;
-          o[ex + ey + ez] += n;
-          o[30 + (x == 2) + 2 * (ey + ez)] += n;
-          o[30 + (y == 2) + 2 * (ex + ez)] += n;
-          o[30 + (z == 2) + 2 * (ex + ey)] += n;
-        }
-    for (unsigned ua = 0; ua < 3; ++ua)
-      for (unsigned ub = 0; ub < 3; ++ub)
-        for (unsigned c = 0; c < 3; ++c) {
-          const unsigned long long n = s[kRawPair + (ua * 3 + ub) * 3 + c];
-          const unsigned ea = ua > 0, eb = ub > 0, l = c > 0;
-          // regions: a's and b's own, the pair's, the common node, c's own if it has a second member
-          const int pat = (int)(ea | (eb << 1) | (l << 2) | (1u << 3) | (1u << 6));
-          o[static_class_of_pattern(pat)] += n;
-          o[30 + (ua > 1) + 2 * (eb + l)] += n;
-          o[30 + (ub > 1) + 2 * (ea + l)] += n;
-          o[30 + (c == 2) + 4] += n;
-        }
-  }
-  __syncthreads();
-  for (unsigned k = t; k < 42; k += blockDim.x) out[k] = o[k];
+  __shared__ FinishShared S;
+  finish(S, raw, out);
 }
 
 unsigned bits_for(uint64_t n) {  // bits of the values 0 .. n - 1
@@ -1918,6 +1973,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
     return HM_OK;
   }
   P.nh = nh;
+  P.by_entry = nh <= kEntriesFew && h2 <= kEntryTests;
   HM_TRY(P.hnbr.alloc(ctx, nh));
   HM_TRY(P.hown.alloc(ctx, nh));
   HM_TRY(P.hos.alloc(ctx, nh));
@@ -2012,10 +2068,12 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   k_pair_plus_fill<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, P.tab_m.p, tslots, ndeg.p, P.noff.p,
                                                                ndeg.p + V, P.nnbr.p, P.nw.p, P.nw_m.p);
   HM_LAUNCH_CHECK();
-  k_hh_codes<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.slot.p, P.rank.p, E, g->esize.p, g->h2h_off.p,
+  if (!P.by_entry) {
+    k_hh_codes<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(P.slot.p, P.rank.p, E, g->esize.p, g->h2h_off.p,
                                                                    g->h2h_len.p, g->h2h_nbr.p, P.hoff.p, P.hnbr.p,
                                                                    P.hnext.p, P.rmark.p, P.moff.p, P.mnext.p, hcode.p, bk.p);
-  HM_LAUNCH_CHECK();
+    HM_LAUNCH_CHECK();
+  }
   k_spread_flags<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(
       P.slot.p, E, P.hoff.p, P.hnbr.p, P.hos.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, ndeg.p, P.spread.p, P.slist.p,
       bk.p + 2 * kBk);
@@ -2023,7 +2081,7 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   k_node_codes<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(P.noff.p, P.nlen.p, P.nnbr.p, V, ncode.p,
                                                                      bk.p + kBk);
   HM_LAUNCH_CHECK();
-  for (int l = 0; l < 2; ++l) {
+  for (int l = P.by_entry ? 1 : 0; l < 2; ++l) {
     uint32_t* b = bk.p + l * kBk;
     k_bucket_starts<<<1, kBuckets, 0, st>>>(b, b + kBuckets, b + 2 * kBuckets);
     HM_LAUNCH_CHECK();
@@ -2075,6 +2133,15 @@ int prepare_decomp(hm_graph* g) {
   return s;
 }
 
+// Warps that share an item of k_parts where there are few: a power of two, as
+// many as the chip holds and a block has at most. A warp alone took 19 us for the largest
+// heavy pair and 15 us for the longest node row of a 1K-hyperedge count.
+static uint32_t slices_of(uint64_t items, unsigned sms) {
+  uint32_t s = 1;
+  while (s < kWarps && items * s * 2 <= (uint64_t)sms * 8 * kWarps) s *= 2;
+  return s;
+}
+
 // One count: the raw sums cleared, the block-per-item launches, the small
 // parts side by side, and the counter block from the sums.
 template <bool kTouch>
@@ -2088,14 +2155,16 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   PartArgs A;
   A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hcode.p, g->h2h_off.p, g->h2h_len.p,
                     g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.rmark.p,
-                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, P.mcode.p, nullptr, 0, 1, nullptr, P.raw.p};
+                    P.moff.p, P.mnbr.p, P.mos.p, P.mpos.p, P.mnext.p, P.mcode.p, nullptr, 0, 1, P.hown.p,
+                    P.by_entry ? P.nh : 0, nullptr, P.raw.p};
   A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
                      g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
                      (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_m.p, P.fw_m.p, P.self_m.p, P.foff.p,
                      P.fnbr.p, P.fw.p, P.spread.p, P.slist.p, P.n_spread, P.self.p, P.y.p,
-                     V, P.nh < kPairFew ? 1u : 4u, P.nh < kPairFew ? 0u : kPairWide, queue + 8, P.raw.p};
+                     V, P.nh < kPairFew ? 1u : 4u, P.nh < kPairFew ? 0u : kPairWide,
+                     slices_of(P.nh, sms), queue + 8, P.raw.p};
   A.nodes = NodeArgs{P.noff.p, P.nlen.p, P.nnbr.p, P.nw.p, P.tab.p, (uint32_t)(P.tslots - 1), P.nw_m.p, P.tab_m.p,
-                     nullptr, 0, nullptr, P.raw.p};
+                     nullptr, 0, nullptr, P.raw.p, 1};
   A.open = OpenArgs{P.slot.p, E, g->h2v_off.p, g->h2v_mem.p, g->esize.p, g->h2h_len.p, P.ncat.p, P.ncat_m.p, P.hoff.p,
                     P.hnbr.p, P.hos.p, P.rmark.p, P.raw.p};
   auto hh_part = [&](int k) {
@@ -2157,15 +2226,20 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
     return (unsigned)std::min<uint64_t>(sms * most, (warps + kWarps - 1) / kWarps);
   };
   unsigned end = 0;
-  A.end[0] = end += blocks(n_search, 4);
-  A.end[1] = end += blocks((P.nh + A.pairs.per_warp - 1) / A.pairs.per_warp, 8);
-  A.end[2] = end += blocks(n_nodes, 8);
+  A.end[0] = end += blocks(P.by_entry ? P.nh : n_search, 4);
+  A.end[1] = end += blocks((P.nh * A.pairs.slices + A.pairs.per_warp - 1) / A.pairs.per_warp, 8);
+  A.nodes.slices = n_nodes ? slices_of(n_nodes, sms) : 1;
+  A.end[2] = end += blocks((uint64_t)n_nodes * A.nodes.slices, 8);
   A.end[3] = end += blocks(E, 8);
   A.end[4] = end += std::min<unsigned>(sms * 2, (V + kBlock - 1) / kBlock);
+  A.ended = end <= sms * 4 ? queue + 12 : nullptr;
+  A.out = counters;
   k_parts<kTouch><<<end, kBlock, 0, st>>>(A);
   HM_LAUNCH_CHECK();
-  k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, counters);
-  HM_LAUNCH_CHECK();
+  if (!A.ended) {
+    k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, counters);
+    HM_LAUNCH_CHECK();
+  }
   return HM_OK;
 }
 

@@ -213,6 +213,7 @@ struct Decomp {
   DArr<uint32_t> nlen, nnbr;
   DArr<uint2> nw;             // {W2, W3}
   DArr<uint32_t> hwork, nwork;  // centres and nodes by launch shape
+  bool by_entry = false;  // few heavy entries: searched one by one, no work list
   uint32_t hend[4] = {}, nend[4] = {};
   DArr<uint8_t> spread;         // per rank: its pairs go through a node vector
   DArr<uint32_t> slist;         // those ranks
@@ -242,6 +243,7 @@ struct Decomp {
     moff.release();
     mos.release();
     n_spread = y_blocks = 0;
+    by_entry = false;
     spread.release();
     self.release();
     y.release();

@@ -123,3 +123,31 @@ def test_touched_triples_by_decomposition(ctx, law, marked):
         dels, ins = gen.batch(p, 3, g.live_ids(), marked)
         _, delta = g.apply_batch(dels, ins.offsets, ins.members)
         assert (full.astype(np.int64) + delta).tolist() == g.count_static30().astype(np.int64).tolist()
+
+
+def _cliques(rng, sizes, n_free):
+    """Hyperedges in groups that share two nodes of their own (all pairs of a
+    group heavy), each with one of n_free common nodes (light pairs, and closed
+    triangles of all kinds)."""
+    rows, node = [], n_free
+    for k in sizes:
+        rows += [sorted([int(rng.integers(0, n_free)), node, node + 1]) for _ in range(k)]
+        node += 2
+    return rows, node
+
+
+# Searched pair by pair up to 2^13 heavy entries and a sum of squared heavy
+# degrees of 2^18, by centre beyond.
+@pytest.mark.parametrize("sizes", [[], [2], [9] * 113 + [2] * 28, [9] * 113 + [2] * 29,
+                                   [64] + [9] * 14 + [2] * 32, [64] + [9] * 14 + [2] * 33],
+                         ids=["none", "one-pair", "entries-2^13", "entries-past", "tests-2^18", "tests-past"])
+def test_few_heavy_pairs_searched_by_entry(ctx, sizes):
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(len(sizes))
+    rows, n_nodes = _cliques(rng, sizes + [1] * 200, 10)
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        want = oracle.static30(off, mem, n_nodes).tolist()
+        assert g.count_static30().tolist() == want
+        assert g.count_static30().tolist() == want  # replayed
