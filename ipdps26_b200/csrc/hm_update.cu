@@ -375,6 +375,37 @@ __global__ void k_arena_keys(const uint64_t* off, uint32_t n, uint64_t* key, uin
   }
 }
 
+// One warp copies a row's three arrays, four entries per lane in flight: one at
+// a time the loop waited out a load per 32 entries (2.7 ms per compaction of a
+// store of 50K rows, at a third of the copy bandwidth).
+__device__ __forceinline__ void copy_row(const uint32_t* nbr, const uint8_t* ovl, const uint64_t* mask, uint32_t* tnbr,
+                                         uint8_t* tovl, uint64_t* tmask, uint32_t l) {
+  constexpr unsigned kFlight = 4;
+  for (uint32_t k0 = lane_id(); k0 < l; k0 += kFlight * kWarp) {
+    uint32_t x[kFlight];
+    uint8_t o[kFlight];
+    uint64_t m[kFlight];
+#pragma unroll
+    for (unsigned t = 0; t < kFlight; ++t) {
+      const uint32_t k = k0 + t * kWarp;
+      if (k < l) {
+        x[t] = nbr[k];
+        o[t] = ovl[k];
+        m[t] = mask[k];
+      }
+    }
+#pragma unroll
+    for (unsigned t = 0; t < kFlight; ++t) {
+      const uint32_t k = k0 + t * kWarp;
+      if (k < l) {
+        tnbr[k] = x[t];
+        tovl[k] = o[t];
+        tmask[k] = m[t];
+      }
+    }
+  }
+}
+
 // phase 0: rows -> staging buffer (positions relative to base);
 // phase 1: staging -> final position, and the row offset is updated.
 __global__ void k_stage_rows(const uint32_t* slots, uint32_t n, uint64_t* off, const uint32_t* len,
@@ -383,21 +414,12 @@ __global__ void k_stage_rows(const uint32_t* slots, uint32_t n, uint64_t* off, c
   for (uint64_t i = global_warp(); i < n; i += n_warps()) {
     const uint32_t r = slots[i];
     const uint32_t l = len[r];
-    const uint64_t t = dst[i] - base;
+    const uint64_t d = dst[i], t = d - base;
     if (phase == 0) {
       const uint64_t s = off[r];
-      for (uint32_t k = lane_id(); k < l; k += kWarp) {
-        snbr[t + k] = nbr[s + k];
-        sovl[t + k] = ovl[s + k];
-        smask[t + k] = mask[s + k];
-      }
+      copy_row(nbr + s, ovl + s, mask + s, snbr + t, sovl + t, smask + t, l);
     } else {
-      const uint64_t d = dst[i];
-      for (uint32_t k = lane_id(); k < l; k += kWarp) {
-        nbr[d + k] = snbr[t + k];
-        ovl[d + k] = sovl[t + k];
-        mask[d + k] = smask[t + k];
-      }
+      copy_row(snbr + t, sovl + t, smask + t, nbr + d, ovl + d, mask + d, l);
       if (lane_id() == 0) off[r] = d;
     }
   }
