@@ -85,10 +85,12 @@ __device__ __forceinline__ uint32_t pair_index(uint32_t ua, uint32_t ub, uint32_
 // ---- preparation: ranks, heavy rows -------------------------------------------------
 
 // Per slot: degree (sort key), heavy neighbours; sums: [0] h^2, [1] d^2,
-// [2] node pairs of all hyperedges, [3] heavy entries.
+// [2] node pairs of all hyperedges, [3] heavy entries, [4] node pairs of the
+// marked hyperedges.
 __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint8_t* ovl, const uint8_t* esize,
-                              uint32_t n, uint32_t* heavy, uint32_t* ids, unsigned long long* sums) {
-  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0;
+                              const uint8_t* mark, uint32_t n, uint32_t* heavy, uint32_t* ids,
+                              unsigned long long* sums) {
+  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0;
   for (uint64_t a = global_warp(); a < n; a += n_warps()) {
     const uint64_t s = off[a];
     const uint32_t l = len[a];
@@ -102,6 +104,7 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
       h2 += (unsigned long long)c * c;
       d2 += (unsigned long long)l * l;
       np += z * (z - (z > 0)) / 2;
+      if (mark && mark[a]) mp += z * (z - (z > 0)) / 2;
       hs += c;
     }
   }
@@ -110,6 +113,7 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
     if (d2) atomicAdd(&sums[1], d2);
     if (np) atomicAdd(&sums[2], np);
     if (hs) atomicAdd(&sums[3], hs);
+    if (mp) atomicAdd(&sums[4], mp);
   }
 }
 
@@ -233,12 +237,12 @@ __device__ __forceinline__ uint2 pair_weight(const uint4* tab, uint32_t mask, ui
   }
 }
 
-// One warp per hyperedge, lanes over its node pairs.
+// One warp per hyperedge, lanes over its node pairs (with only: those marked there).
 __global__ void k_pair_insert(const uint64_t* off, const uint32_t* mem, const uint8_t* esize, const uint8_t* mark,
-                              uint32_t n, uint4* tab, uint2* wm, uint32_t mask) {
+                              const uint8_t* only, uint32_t n, uint4* tab, uint2* wm, uint32_t mask) {
   for (uint64_t e = global_warp(); e < n; e += n_warps()) {
     const uint32_t s = esize[e];
-    if (s < 2) continue;
+    if (s < 2 || (only && !only[e])) continue;
     const uint32_t* m = mem + off[e];
     const uint32_t np = s * (s - 1) / 2;
     for (uint32_t t = lane_id(); t < np; t += kWarp) {
@@ -844,7 +848,11 @@ struct PairArgs {
   // third ones only, from the marked hyperedges' sums
   const uint8_t* rmark;
   const uint32_t* ncat_m;
-  const uint2* tab_m;
+  // the marked hyperedges' node pairs in a table of their own: with a twelfth of
+  // 50K hyperedges marked it stays in L2 and most lookups end at an empty slot
+  // (heavy pairs and spread of four counts 50.0 -> 44.6 ms, building it 1.1 ms)
+  const uint4* tab_c;
+  uint32_t cmask;
   const uint2* fw_m;
   uint2* self_m;
   const uint64_t* foff;  // the node graph's rows, both directions (for spreading)
@@ -948,7 +956,8 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
     auto run = [&](uint32_t first, uint32_t step, uint32_t na, uint32_t nb, const uint32_t* xa, const uint32_t* xb,
                    uint64_t sma, uint64_t smb, bool unmarked) {
       const uint32_t* ncat = unmarked ? A.ncat_m : A.ncat;
-      const uint2* wm = unmarked ? A.tab_m : nullptr;
+      const uint4* tab = unmarked ? A.tab_c : A.tab;
+      const uint32_t tmask = unmarked ? A.cmask : A.tmask;
       const uint32_t all = na * nb;
       for (uint32_t t = first; t < all; t += step) {
         const uint32_t i = t / nb, j = t - i * nb;
@@ -963,7 +972,7 @@ __device__ void part_pairs(unsigned vb, unsigned nb, PairCounts& cnt, const Pair
         }
         const uint32_t w = __ldg(xb + j);
         if (j < 64 ? (smb >> j) & 1ull : in_list(xa, na, w)) continue;
-        const uint2 p = pair_weight(A.tab, A.tmask, v, w, wm);
+        const uint2 p = pair_weight(tab, tmask, v, w);
         q2 += p.x;
         q3 += p.y;
       }
@@ -1067,7 +1076,7 @@ __global__ void k_self_weights(PairArgs A, uint32_t n) {
         uint2 t = make_uint2(0, 0);
         for (uint32_t j = 0; j < s; ++j) {
           if (j == i) continue;
-          const uint2 p = pair_weight(A.tab, A.tmask, v, __ldg(A.vmem + o + j), k ? A.tab_m : nullptr);
+          const uint2 p = pair_weight(k ? A.tab_c : A.tab, k ? A.cmask : A.tmask, v, __ldg(A.vmem + o + j));
           t.x += p.x;
           t.y += p.y;
         }
@@ -1156,7 +1165,7 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_pairs(PairArgs A) {
           const uint32_t x = __ldg(A.vmem + bo + k);
           const uint2 u = y[x];
           if (u.x != ~0u || u.y != ~0u) continue;
-          const uint2 p = pair_weight(A.tab, A.tmask, v, x, un ? A.tab_m : nullptr);
+          const uint2 p = pair_weight(un ? A.tab_c : A.tab, un ? A.cmask : A.tmask, v, x);
           t[0] += p.x;
           t[1] += p.y;
         }
@@ -1937,13 +1946,13 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   HM_TRY(ids.alloc(ctx, E));
   HM_TRY(deg.alloc(ctx, E));
   HM_TRY(hcnt.alloc(ctx, E));
-  HM_TRY(sums.alloc(ctx, 4));
+  HM_TRY(sums.alloc(ctx, 5));
   HM_TRY(P.rank.alloc(ctx, E));
   HM_TRY(P.slot.alloc(ctx, E));
   HM_TRY(P.hoff.alloc(ctx, (size_t)E + 1));
-  HM_CUDA(cudaMemsetAsync(sums.p, 0, 4 * sizeof(unsigned long long), st));
+  HM_CUDA(cudaMemsetAsync(sums.p, 0, 5 * sizeof(unsigned long long), st));
   k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_ovl.p,
-                                                                      g->esize.p, E, heavy.p, ids.p, sums.p);
+                                                                      g->esize.p, mark, E, heavy.p, ids.p, sums.p);
   HM_LAUNCH_CHECK();
   const unsigned bits = bits_for(E);
   {
@@ -1958,13 +1967,15 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   k_rank_scatter<<<grid_for(E, kBlock), kBlock, 0, st>>>(P.slot.p, E, heavy.p, P.rank.p, hcnt.p);
   HM_LAUNCH_CHECK();
   HM_TRY(exclusive_scan(ctx, hcnt.p, P.hoff.p, E));
-  unsigned long long hs[4];
+  unsigned long long hs[5];
   HM_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
   const uint64_t h2 = hs[0], d2 = hs[1], pairs = hs[2], nh = hs[3];
   uint64_t tslots = 1024;
   while (tslots < 2 * pairs) tslots <<= 1;
-  const size_t need = tslots * (sizeof(uint4) + (mark ? sizeof(uint2) : 0)) + pairs * (mark ? 60 : 36) +
+  uint64_t cslots = 1024;  // the marked hyperedges' own table
+  while (cslots < 2 * hs[4]) cslots <<= 1;
+  const size_t need = tslots * (sizeof(uint4) + (mark ? sizeof(uint2) : 0)) + (mark ? cslots * sizeof(uint4) : 0) + pairs * (mark ? 60 : 36) +
                       nh * (22 + 24 + (mark ? 18 : 0));
   const size_t room = ctx->budget ? ctx->budget - std::min<size_t>(ctx->budget, ctx->used.load()) : SIZE_MAX;
   if (h2 > d2 / 4 || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
@@ -2028,6 +2039,9 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
     HM_TRY(P.tab_m.alloc(ctx, tslots));
     HM_TRY(P.nw_m.alloc(ctx, pairs));
     HM_CUDA(cudaMemsetAsync(P.tab_m.p, 0, sizeof(uint2) * tslots, st));
+    P.cslots = cslots;
+    HM_TRY(P.tab_c.alloc(ctx, cslots));
+    HM_CUDA(cudaMemsetAsync(P.tab_c.p, 0, sizeof(uint4) * cslots, st));
   }
   // node graph
   P.tslots = tslots;
@@ -2058,8 +2072,13 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   HM_LAUNCH_CHECK();
   const uint32_t tmask = (uint32_t)(tslots - 1);
   k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_mem.p, g->esize.p, mark,
-                                                                      E, P.tab.p, P.tab_m.p, tmask);
+                                                                      nullptr, E, P.tab.p, P.tab_m.p, tmask);
   HM_LAUNCH_CHECK();
+  if (mark) {
+    k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(
+        g->h2v_off.p, g->h2v_mem.p, g->esize.p, nullptr, mark, E, P.tab_c.p, nullptr, (uint32_t)(cslots - 1));
+    HM_LAUNCH_CHECK();
+  }
   k_pair_degrees<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p);
   HM_LAUNCH_CHECK();
   k_pair_plus_count<<<grid_for(tslots, kBlock), kBlock, 0, st>>>(P.tab.p, tslots, ndeg.p, P.nlen.p);
@@ -2159,7 +2178,8 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
                     P.by_entry ? P.nh : 0, nullptr, P.raw.p};
   A.pairs = PairArgs{P.hown.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hoff.p, P.nh, P.slot.p, g->h2h_off.p,
                      g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.ncat.p, P.tab.p,
-                     (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_m.p, P.fw_m.p, P.self_m.p, P.foff.p,
+                     (uint32_t)(P.tslots - 1), P.rmark.p, P.ncat_m.p, P.tab_c.p,
+                     (uint32_t)(P.cslots ? P.cslots - 1 : 0), P.fw_m.p, P.self_m.p, P.foff.p,
                      P.fnbr.p, P.fw.p, P.spread.p, P.slist.p, P.n_spread, P.self.p, P.y.p,
                      V, P.nh < kPairFew ? 1u : 4u, P.nh < kPairFew ? 0u : kPairWide,
                      slices_of(P.nh, sms), queue + 8, P.raw.p};

@@ -208,7 +208,7 @@ struct Decomp {
   uint64_t nh = 0;
   DArr<uint32_t> ncat;        // per node: hyperedges of one, two, more members
   DArr<uint4> tab;            // node pairs {x, y, W2, W3}
-  uint64_t tslots = 0;
+  uint64_t tslots = 0, cslots = 0;
   DArr<uint64_t> noff;        // oriented node rows
   DArr<uint32_t> nlen, nnbr;
   DArr<uint2> nw;             // {W2, W3}
@@ -228,13 +228,14 @@ struct Decomp {
   DArr<uint32_t> mnbr, mpos, mnext, mcode, ncat_m;
   DArr<uint16_t> mos;
   DArr<uint2> tab_m, nw_m, fw_m, self_m;
+  DArr<uint4> tab_c;  // node pairs of the marked hyperedges {x, y, W2, W3}
   DArr<unsigned long long> raw;
   CountCapture capture;
   ~Decomp() { capture.reset(); }
   void release() {
     capture.reset();
     decided = usable = false;
-    nh = tslots = 0;
+    nh = tslots = cslots = 0;
     for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist,
                     &mnbr, &mpos, &mnext, &mcode, &hcode, &ncat_m})
       a->release();
@@ -253,6 +254,7 @@ struct Decomp {
     hoff.release();
     hos.release();
     tab.release();
+    tab_c.release();
     noff.release();
     nw.release();
     raw.release();
