@@ -151,3 +151,22 @@ def test_few_heavy_pairs_searched_by_entry(ctx, sizes):
         want = oracle.static30(off, mem, n_nodes).tolist()
         assert g.count_static30().tolist() == want
         assert g.count_static30().tolist() == want  # replayed
+
+
+@pytest.mark.parametrize("groups", [20, 200])
+@pytest.mark.parametrize("marked", [1, 400, 1500])
+def test_touched_triples_of_few_heavy_pairs(ctx, groups, marked):
+    """Marked sets in graphs searched by entry, with several warps on a pair
+    (two hubs hold everything, so 400 marks or more go by the decomposition)."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(groups + marked)
+    rows, n_nodes = _cliques(rng, [4] * groups + [1] * (3000 - 4 * groups), 2)
+    off, mem = csr(rows)
+    ids = np.sort(rng.choice(3000, size=marked, replace=False)).astype(np.uint32)
+    rest_off, rest_mem = csr([r for k, r in enumerate(rows) if k not in set(ids.tolist())])
+    with engine.Graph(ctx, off, mem, n_nodes) as g, engine.Graph(ctx, rest_off, rest_mem, n_nodes) as rest:
+        got = g.count_touching30(ids)
+        assert got.tolist() == (g.count_static30() - rest.count_static30()).tolist()
+        g.set_touch_orientation(True)
+        assert got.tolist() == g.count_touching30(ids).tolist()
