@@ -738,9 +738,14 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     HM_CUDA(cudaMemsetAsync(total.p, 0, sizeof(unsigned long long), st));
     HM_CUDA(cudaMemsetAsync(g->h2h_ovl.p + base, 0, W, st));
     HM_CUDA(cudaMemsetAsync(g->h2h_mask.p + base, 0, sizeof(uint64_t) * W, st));
+    // The limit is the function's on the device, shared by every context: always
+    // the largest store's size, so that no thread lowers it between another
+    // context's call and its launch.
     auto run = [&](auto* kernel, unsigned groups, unsigned threads) -> int {
       const size_t smem = (size_t)groups * 2 * words * sizeof(uint32_t);
-      HM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      constexpr size_t kWordsMax = (kBitmapSlots + 31) / 32;
+      HM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(groups * 2 * kWordsMax * sizeof(uint32_t))));
       kernel<<<grid_for(n_rows, groups, (unsigned)ctx->n_sms * 16), threads, smem, st>>>(
           g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p, g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p, woff.p, d_rows, n_rows,
           words, base, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, total.p);
