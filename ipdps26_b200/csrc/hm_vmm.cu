@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <mutex>
-#include <new>
 
 #include "hm_device.h"
 
@@ -133,44 +132,27 @@ int GrowSpace::grow(hm_ctx* c, size_t bytes) {
   return HM_OK;
 }
 
-// From the pool (or nothing) to mapped chunks. Where the budget does not hold
-// both for a moment, the contents go through host memory: growth in chunks
-// needs no second copy, and a store it suits must still fit.
+// From the pool (or nothing) to mapped chunks. The old block is freed only once
+// the new one holds its contents, so a growth that fails leaves the space as it
+// was, at the same address. While both exist the budget is charged for the new
+// one alone: growth in chunks needs no second copy and a store it suits must
+// still fit, and the old block is kPooledMax at most.
 int GrowSpace::move_to_chunks(size_t bytes) {
   GrowSpace next;
   next.ctx = ctx;
   next.vmm = true;
+  uncharge(ctx, mapped);
   int s = next.grow_mapped(bytes);
   if (s == HM_OK && mapped) {
-    HM_CUDA(cudaMemcpyAsync(next.base, base, mapped, cudaMemcpyDeviceToDevice, ctx->stream));
-    dev_free(ctx, base, mapped);
-  } else if (s == HM_ERR_NOMEM && mapped) {
-    std::vector<char> host;
-    try {
-      host.resize(mapped);
-    } catch (const std::bad_alloc&) {
-      return s;
-    }
-    HM_CUDA(cudaMemcpyAsync(host.data(), base, mapped, cudaMemcpyDeviceToHost, ctx->stream));
-    HM_CUDA(cudaStreamSynchronize(ctx->stream));
-    dev_free(ctx, base, mapped);
-    base = nullptr;
-    s = next.grow_mapped(bytes);
-    if (s < 0) {  // back into the place just freed
-      void* q = nullptr;
-      const size_t was = mapped;
-      mapped = reserved = 0;
-      HM_TRY(dev_alloc(ctx, &q, was));
-      base = static_cast<char*>(q);
-      mapped = reserved = was;
-      HM_CUDA(cudaMemcpyAsync(base, host.data(), was, cudaMemcpyHostToDevice, ctx->stream));
-      HM_CUDA(cudaStreamSynchronize(ctx->stream));
-      return s;
-    }
-    HM_CUDA(cudaMemcpyAsync(next.base, host.data(), mapped, cudaMemcpyHostToDevice, ctx->stream));
-    HM_CUDA(cudaStreamSynchronize(ctx->stream));
+    const cudaError_t e = cudaMemcpyAsync(next.base, base, mapped, cudaMemcpyDeviceToDevice, ctx->stream);
+    if (e != cudaSuccess) s = set_error(HM_ERR_CUDA, "moving an arena to chunks: %s", cudaGetErrorString(e));
   }
-  if (s < 0) return s;
+  if (s < 0) {
+    next.release();
+    ctx->used.fetch_add(mapped);
+    return s;
+  }
+  if (mapped) cudaFreeAsync(base, ctx->stream);
   base = next.base;
   mapped = next.mapped;
   reserved = next.reserved;

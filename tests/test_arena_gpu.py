@@ -119,3 +119,43 @@ def test_pooled_arena_moves_to_chunks_under_every_budget():
                 assert e.status == HM_ERR_NOMEM, str(e)
                 assert mb < 512, str(e)
     assert passed and all(passed)
+
+
+def test_growth_of_a_pooled_arena_fails_whole():
+    """Every allocation of a batch that grows a pooled arena fails in turn. The
+    batch then ends in HM_ERR_NOMEM or, where the growth was optional, in the
+    store of an undisturbed one; the budget's account returns to nothing when
+    the graph goes, and the context's next graph is whole."""
+    from ipdps26_b200 import engine
+    from ipdps26_b200._lib import HM_ERR_NOMEM, HmError, lib
+
+    rng = np.random.default_rng(14)
+    n_nodes = 64
+    off, mem = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(2000)])
+    io, im = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(1500)])
+    dels = list(range(0, 400, 2))
+    with engine.Context(0) as c:
+
+        def run(n):
+            with engine.Graph(c, off, mem, n_nodes) as g:
+                lib.hm_debug_fail_allocations_after(n)
+                try:
+                    ids, delta = g.apply_batch(dels, io, im)
+                finally:
+                    lib.hm_debug_fail_allocations_after(-1)
+                return ids.tolist(), delta.tolist(), g.info().n_adjacent, g.count_static30().tolist()
+
+        want = run(-1)
+        failed, step = 0, 0
+        while step < 2000:
+            try:
+                got = run(step)
+                assert got == want, step
+                break  # no allocation left to fail
+            except HmError as e:
+                assert e.status == HM_ERR_NOMEM, f"{step}: {e}"
+                failed += 1
+            assert c.memory()[0] == 0, step
+            step += 1
+        assert failed > 20 and got == want
+        assert run(-1) == want
