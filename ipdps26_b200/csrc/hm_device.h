@@ -95,8 +95,8 @@ bool vmm_available();  // the driver's virtual memory management calls were foun
 // grows (CUDA virtual memory management). When the reservation is full a
 // larger one is reserved and the chunks already held are mapped into it, so
 // growth never copies data and never holds two copies at once. Each grow that
-// moves and each release synchronises the device (chunks are unmapped only
-// when no kernel can use them). A small first allocation comes from the
+// moves and each release waits for the context's stream (chunks are unmapped
+// only when no kernel can use them). A small first allocation comes from the
 // context's pool and moves to chunks when it grows; without VMM support all
 // growth is allocate-copy-free. Budget-charged like DArr.
 struct GrowSpace {

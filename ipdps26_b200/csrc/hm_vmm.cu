@@ -86,7 +86,11 @@ static int map_one(const Vmm& v, int device, CUdeviceptr va, size_t size, unsign
   return HM_OK;
 }
 
-// Unmaps chunks [i0, i1) of a reservation at va, one mapping at a time.
+// Unmaps chunks [i0, i1) of a reservation at va, one mapping at a time. The
+// caller has waited for the context's stream: every kernel that reads the
+// chunks runs on it, or was waited for by the call that launched it. (Waiting
+// for the device would end the captures other contexts have under way, and
+// fail itself while one is.)
 static void unmap_chunks(const Vmm& v, CUdeviceptr va, const std::vector<size_t>& sizes, size_t i0, size_t i1) {
   size_t at = 0;
   for (size_t i = 0; i < i0; ++i) at += sizes[i];
@@ -226,7 +230,7 @@ int GrowSpace::grow_mapped(size_t bytes) {
   }
   if (moved) {
     if (base) {
-      HM_CUDA(cudaDeviceSynchronize());
+      HM_CUDA(cudaStreamSynchronize(ctx->stream));
       unmap_chunks(v, (CUdeviceptr)base, sizes, 0, first);
       v.free((CUdeviceptr)base, reserved);
     }
@@ -248,7 +252,7 @@ void GrowSpace::shrink(size_t bytes) {
   }
   if (k == handles.size()) return;
   cudaSetDevice(ctx->device);
-  cudaDeviceSynchronize();
+  cudaStreamSynchronize(ctx->stream);
   unmap_chunks(v, (CUdeviceptr)base, sizes, k, handles.size());
   for (size_t i = k; i < handles.size(); ++i) v.release(handles[i]);
   uncharge(ctx, mapped - at);
@@ -264,7 +268,7 @@ void GrowSpace::release() {
   } else {
     const Vmm& v = vmm_api();
     cudaSetDevice(ctx->device);
-    cudaDeviceSynchronize();
+    cudaStreamSynchronize(ctx->stream);
     unmap_chunks(v, (CUdeviceptr)base, sizes, 0, handles.size());
     v.free((CUdeviceptr)base, reserved);
     for (auto h : handles) v.release(h);

@@ -51,3 +51,34 @@ def test_contexts_build_stores_of_different_sizes_at_once():
         return job
 
     _run([builds(1_000, 600) for _ in range(6)] + [builds(80_000, 150) for _ in range(3)])
+
+
+def test_contexts_count_and_update_at_once():
+    """Counts capture their launches while other contexts grow, release and
+    destroy stores; each context's results are those of a lone one."""
+    import numpy as np
+
+    from ipdps26_b200 import engine, gen
+
+    def rounds(n, seed, k, out):
+        def job():
+            p, h = _graph(n, seed)
+            dels, ins = gen.batch(p, 9, np.arange(n, dtype=np.uint32), 60)
+            with engine.Context(0) as c:
+                for _ in range(k):
+                    with engine.Graph.from_hypergraph(c, h) as g:
+                        full = g.count_static30().astype(np.int64)
+                        _, delta = g.apply_batch(dels, ins.offsets, ins.members)
+                        after = g.count_static30().astype(np.int64)
+                        assert (full + delta).tolist() == after.tolist()
+                        out.append((full.tolist(), after.tolist()))
+
+        return job
+
+    sizes = [(1_000, 150), (80_000, 60), (30_000, 100)]
+    got = [[] for _ in sizes]
+    _run([rounds(n, 20 + k, r, got[k]) for k, (n, r) in enumerate(sizes)])
+    for k, (n, r) in enumerate(sizes):
+        alone = []
+        rounds(n, 20 + k, 1, alone)()
+        assert len(got[k]) == r and all(x == alone[0] for x in got[k])
