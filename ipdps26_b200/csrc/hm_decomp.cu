@@ -2164,13 +2164,12 @@ static uint32_t slices_of(uint64_t items, unsigned sms) {
 // One count: the raw sums cleared, the block-per-item launches, the small
 // parts side by side, and the counter block from the sums.
 template <bool kTouch>
-static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
+static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters, Launches& L) {
   hm_ctx* ctx = g->ctx;
-  cudaStream_t st = ctx->stream;
   const unsigned sms = (unsigned)ctx->n_sms;
   const uint32_t E = g->n_slots, V = g->n_nodes;
   unsigned int* queue = reinterpret_cast<unsigned int*>(P.raw.p + kRawQueue);
-  HM_CUDA(cudaMemsetAsync(P.raw.p, 0, sizeof(unsigned long long) * kRawSize, st));
+  HM_TRY(L.zero(P.raw.p, kRawSize));
   PartArgs A;
   A.search = HHArgs{P.slot.p, P.rank.p, P.hoff.p, P.hnbr.p, P.hos.p, P.hpos.p, P.hnext.p, P.hcode.p, g->h2h_off.p, g->h2h_len.p,
                     g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, g->h2v_off.p, g->h2v_mem.p, g->esize.p, P.rmark.p,
@@ -2203,43 +2202,30 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   };
   if (const uint32_t n = hh_part(3)) {
     A.search.slices = std::min(16u, std::max(1u, 8 * sms / n));
-    k_hh_large<<<std::min(sms, n * A.search.slices), kHHThreads, kHHSmem, st>>>(A.search);
-    HM_LAUNCH_CHECK();
+    HM_TRY(L.run(k_hh_large, std::min(sms, n * A.search.slices), kHHThreads, kHHSmem, A.search));
   }
-  if (const uint32_t n = hh_part(2)) {
-    k_hh_fast<false, uint64_t><<<std::min(sms * 2, n), kFastThreads, fast_smem<uint64_t>(), st>>>(A.search, E);
-    HM_LAUNCH_CHECK();
-  }
+  if (const uint32_t n = hh_part(2))
+    HM_TRY(L.run(k_hh_fast<false, uint64_t>, std::min(sms * 2, n), kFastThreads, fast_smem<uint64_t>(), A.search, E));
   if (const uint32_t n = hh_part(1)) {
     if (E <= kDenseSlots)
-      k_hh_fast<true, uint32_t><<<std::min(sms * 2, n), kFastThreads, kDenseSmem, st>>>(A.search, E);
+      HM_TRY(L.run(k_hh_fast<true, uint32_t>, std::min(sms * 2, n), kFastThreads, kDenseSmem, A.search, E));
     else
-      k_hh_fast<false, uint32_t><<<std::min(sms * 2, n), kFastThreads, fast_smem<uint32_t>(), st>>>(A.search, E);
-    HM_LAUNCH_CHECK();
+      HM_TRY(L.run(k_hh_fast<false, uint32_t>, std::min(sms * 2, n), kFastThreads, fast_smem<uint32_t>(), A.search, E));
   }
   if (P.n_spread) {
-    k_self_weights<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(A.pairs, E);
-    HM_LAUNCH_CHECK();
-    k_spread_pairs<<<P.y_blocks, kSpreadThreads, 0, st>>>(A.pairs);
-    HM_LAUNCH_CHECK();
+    HM_TRY(L.run(k_self_weights, grid_for((uint64_t)E * 32, kBlock), kBlock, 0, A.pairs, E));
+    HM_TRY(L.run(k_spread_pairs, P.y_blocks, kSpreadThreads, 0, A.pairs));
   }
-  if (const uint32_t n = node_part(3)) {
-    k_node_tri<kTouch, 16384, 1024, 1><<<std::min(sms, n), 1024, node_smem(16384), st>>>(A.nodes);
-    HM_LAUNCH_CHECK();
-  }
-  if (const uint32_t n = node_part(2)) {
-    k_node_tri<kTouch, 4096, 512, 2><<<std::min(sms * 4, n), 512, node_smem(4096), st>>>(A.nodes);
-    HM_LAUNCH_CHECK();
-  }
-  if (const uint32_t n = node_part(1)) {
-    k_node_tri<kTouch, 1024, 256, 6><<<std::min(sms * 6, n), 256, node_smem(1024), st>>>(A.nodes);
-    HM_LAUNCH_CHECK();
-  }
+  if (const uint32_t n = node_part(3))
+    HM_TRY(L.run(k_node_tri<kTouch, 16384, 1024, 1>, std::min(sms, n), 1024, node_smem(16384), A.nodes));
+  if (const uint32_t n = node_part(2))
+    HM_TRY(L.run(k_node_tri<kTouch, 4096, 512, 2>, std::min(sms * 4, n), 512, node_smem(4096), A.nodes));
+  if (const uint32_t n = node_part(1))
+    HM_TRY(L.run(k_node_tri<kTouch, 1024, 256, 6>, std::min(sms * 6, n), 256, node_smem(1024), A.nodes));
   const uint32_t n_search = hh_part(0);
   uint32_t n_nodes = node_part(0);
   if (n_nodes > kNodesAlone) {
-    k_node_tri_warp<kTouch><<<std::min(sms * 12, (n_nodes + kWarps - 1) / kWarps), kBlock, 0, st>>>(A.nodes);
-    HM_LAUNCH_CHECK();
+    HM_TRY(L.run(k_node_tri_warp<kTouch>, std::min(sms * 12, (n_nodes + kWarps - 1) / kWarps), kBlock, 0, A.nodes));
     n_nodes = 0;
   }
   auto blocks = [&](uint64_t warps, unsigned most) {
@@ -2254,16 +2240,13 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters) {
   A.end[4] = end += std::min<unsigned>(sms * 2, (V + kBlock - 1) / kBlock);
   A.ended = end <= sms * 4 ? queue + 12 : nullptr;
   A.out = counters;
-  k_parts<kTouch><<<end, kBlock, 0, st>>>(A);
-  HM_LAUNCH_CHECK();
-  if (!A.ended) {
-    k_decomp_finish<<<1, 128, 0, st>>>(P.raw.p, counters);
-    HM_LAUNCH_CHECK();
-  }
+  HM_TRY(L.run(k_parts<kTouch>, end, kBlock, 0, A));
+  if (!A.ended)
+    HM_TRY(L.run(k_decomp_finish, 1, 128, 0, P.raw.p, counters));
   return HM_OK;
 }
 
-int launch_decomp(hm_graph* g) { return launch_parts<false>(g, g->decomp, g->counters.p); }
+int launch_decomp(hm_graph* g, Launches& L) { return launch_parts<false>(g, g->decomp, g->counters.p, L); }
 
 // The triples with a marked hyperedge, count(G) - count(G without them), by the
 // same forms: every sum over nodes, node pairs and heavy pairs minus the same
@@ -2279,7 +2262,8 @@ int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], 
   if (s >= 0) s = cnt.alloc(g->ctx, 42);
   if (s == HM_ERR_NOMEM || (s >= 0 && !P.usable)) return HM_OK;
   HM_TRY(s);
-  HM_TRY(launch_parts<true>(g, P, cnt.p));
+  Launches L{g->ctx->stream};
+  HM_TRY(launch_parts<true>(g, P, cnt.p, L));
   unsigned long long h[42];
   HM_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, g->ctx->stream));
   HM_CUDA(cudaStreamSynchronize(g->ctx->stream));

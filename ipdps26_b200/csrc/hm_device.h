@@ -9,6 +9,7 @@
 #include <functional>
 #include <cstdint>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "hm_internal.h"
@@ -174,12 +175,13 @@ struct TouchSchedule {
   uint32_t mid_row = 2048;
 };
 
-// Launch sequences of the static count captured as CUDA graphs (open phase,
-// closed phase), replayed while the arguments they were captured with hold.
+// Launch sequences of the static count kept as CUDA graphs (open phase, closed
+// phase), replayed while the arguments they were made with hold.
 struct CountCapture {
   static constexpr unsigned kKey = 27;
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   uint64_t key[kKey] = {};
+  uint32_t kernels = 0;  // of both
   bool valid = false;
   void reset() {
     for (auto& e : exec)
@@ -415,7 +417,8 @@ int prepare_static(hm_graph* g);       // for a full count, by whichever method 
 int prepare_enumeration(hm_graph* g);  // oriented rows and work list of the triangle enumeration
 // The count by decomposition (hm_decomp.cu), when g->decomp.usable.
 int prepare_decomp(hm_graph* g);
-int launch_decomp(hm_graph* g);
+struct Launches;
+int launch_decomp(hm_graph* g, Launches& L);
 int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done);
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags);
 int finish_static(hm_graph* g, uint64_t out30[30]);
@@ -500,6 +503,53 @@ struct StreamOrder {
 };
 
 #ifdef __CUDACC__
+// Kernels one after another: on a stream, or as the nodes of a CUDA graph. The
+// graph is put together node by node and not by capturing the stream, because
+// a wait for the whole device on any other thread of the program would end a
+// capture, and fail there.
+struct Launches {
+  cudaStream_t st;
+  cudaGraph_t graph = nullptr;
+  cudaGraphNode_t last = nullptr;
+  uint32_t kernels = 0;
+  template <class... P, class... A>
+  int run(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, A&&... args) {
+    std::tuple<P...> values(static_cast<A&&>(args)...);
+    void* ptrs[sizeof...(P)];
+    std::apply([&](auto&... v) { unsigned i = 0; ((ptrs[i++] = (void*)&v), ...); }, values);
+    ++kernels;
+    if (!graph) {
+      HM_CUDA(cudaLaunchKernel((const void*)kernel, dim3(grid), dim3(block), ptrs, smem, st));
+      return HM_OK;
+    }
+    cudaKernelNodeParams n = {};
+    n.func = (void*)kernel;
+    n.gridDim = dim3(grid);
+    n.blockDim = dim3(block);
+    n.sharedMemBytes = (unsigned)smem;
+    n.kernelParams = ptrs;
+    cudaGraphNode_t node = nullptr;
+    HM_CUDA(cudaGraphAddKernelNode(&node, graph, &last, last ? 1 : 0, &n));
+    last = node;
+    return HM_OK;
+  }
+  int zero(void* p, size_t words) {  // words of 8 bytes
+    if (!graph) {
+      HM_CUDA(cudaMemsetAsync(p, 0, 8 * words, st));
+      return HM_OK;
+    }
+    cudaMemsetParams m = {};
+    m.dst = p;
+    m.elementSize = 4;
+    m.width = 2 * words;
+    m.height = 1;
+    cudaGraphNode_t node = nullptr;
+    HM_CUDA(cudaGraphAddMemsetNode(&node, graph, &last, last ? 1 : 0, &m));
+    last = node;
+    return HM_OK;
+  }
+};
+
 // The orientation of the oriented rows: b is "above" a when (deg b, b) >
 // (deg a, a), deg the H2H degree; every triangle is found once, from its
 // lowest-ranked corner, and hub rows stay short.

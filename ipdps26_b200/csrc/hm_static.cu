@@ -841,8 +841,7 @@ int prepare_static(hm_graph* g) {
 // (4096-slot tables, 4 blocks per SM), then the short rows, one warp each.
 // queues holds three zeroed counters, one per launch.
 template <bool kTriads = false>
-static int launch_closed(hm_ctx* ctx, ClosedArgs base, const uint32_t bounds[4], unsigned int* queues) {
-  cudaStream_t st = ctx->stream;
+static int launch_closed(hm_ctx* ctx, Launches& L, ClosedArgs base, const uint32_t bounds[4], unsigned int* queues) {
   for (int part = 0; part < 3; ++part) {
     const uint32_t n = bounds[part + 1] - bounds[part];
     if (n <= base.shard) continue;
@@ -853,50 +852,51 @@ static int launch_closed(hm_ctx* ctx, ClosedArgs base, const uint32_t bounds[4],
     const uint32_t items = (n - base.shard + base.n_shards - 1) / base.n_shards;
     if (part == 0) {
       const unsigned grid = std::min<unsigned>((unsigned)ctx->n_sms, items);
-      k_closed<kBigSlots, 1, kTriads, kBigThreads><<<grid, kBigThreads, closed_smem_bytes(kBigSlots), st>>>(A);
+      HM_TRY(L.run(k_closed<kBigSlots, 1, kTriads, kBigThreads>, grid, kBigThreads, closed_smem_bytes(kBigSlots), A));
     } else if (part == 1) {
       const unsigned grid = std::min<unsigned>((unsigned)ctx->n_sms * 4, items);
-      k_closed<kSmallSlots, 4, kTriads><<<grid, kClosedBlock, closed_smem_bytes(kSmallSlots), st>>>(A);
+      HM_TRY(L.run(k_closed<kSmallSlots, 4, kTriads>, grid, kClosedBlock, closed_smem_bytes(kSmallSlots), A));
     } else {
       const unsigned grid = std::min<unsigned>((unsigned)ctx->n_sms * 4, (items + kClosedWarps - 1) / kClosedWarps);
-      k_closed_warp<kTriads><<<grid, kClosedBlock, 0, st>>>(A);
+      HM_TRY(L.run(k_closed_warp<kTriads>, grid, kClosedBlock, 0, A));
     }
-    HM_LAUNCH_CHECK();
   }
   return HM_OK;
 }
+template <bool kTriads = false>
+static int launch_closed(hm_ctx* ctx, const ClosedArgs& base, const uint32_t bounds[4], unsigned int* queues) {
+  Launches L{ctx->stream};
+  return launch_closed<kTriads>(ctx, L, base, bounds, queues);
+}
 
-// Captures the launches body() makes on stream st as an executable graph.
+// The launches body makes, as an executable graph.
 template <class F>
-static int capture_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
-  HM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  const int s = body();
-  cudaGraph_t graph = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(st, &graph);
-  if (s < 0 || e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    if (s < 0) return s;
-    return set_error(HM_ERR_CUDA, "stream capture of the static count: %s", cudaGetErrorString(e));
+static int make_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec, uint32_t* kernels) {
+  Launches L{st};
+  HM_CUDA(cudaGraphCreate(&L.graph, 0));
+  int s = body(L);
+  if (s >= 0) {
+    const cudaError_t e = cudaGraphInstantiate(exec, L.graph, 0);
+    if (e != cudaSuccess) {
+      *exec = nullptr;
+      s = set_error(HM_ERR_CUDA, "graph instantiation of the static count: %s", cudaGetErrorString(e));
+    }
   }
-  const cudaError_t ei = cudaGraphInstantiate(exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (ei != cudaSuccess) {
-    *exec = nullptr;
-    return set_error(HM_ERR_CUDA, "graph instantiation of the static count: %s", cudaGetErrorString(ei));
-  }
-  return HM_OK;
+  cudaGraphDestroy(L.graph);
+  *kernels += L.kernels;
+  return s;
 }
 
-// Replays the two phases' captures, capturing them first when the key has
-// changed.
+// Replays the two phases' graphs, making them first when the key has changed.
 template <class F0, class F1>
-static int run_captured(hm_graph* g, CountCapture& C, const uint64_t key[CountCapture::kKey], F0&& open_phase,
-                        bool any_open, F1&& closed_phase, bool any_closed) {
+static int run_graphs(hm_graph* g, CountCapture& C, const uint64_t key[CountCapture::kKey], F0&& open_phase,
+                      bool any_open, F1&& closed_phase, bool any_closed) {
   cudaStream_t st = g->ctx->stream;
   if (!C.valid || std::memcmp(C.key, key, sizeof(C.key)) != 0) {
     C.reset();
-    if (any_open) HM_TRY(capture_graph(st, open_phase, &C.exec[0]));
-    if (any_closed) HM_TRY(capture_graph(st, closed_phase, &C.exec[1]));
+    C.kernels = 0;
+    if (any_open) HM_TRY(make_graph(st, open_phase, &C.exec[0], &C.kernels));
+    if (any_closed) HM_TRY(make_graph(st, closed_phase, &C.exec[1], &C.kernels));
     std::memcpy(C.key, key, sizeof(C.key));
     C.valid = true;
   }
@@ -911,8 +911,8 @@ static int run_captured(hm_graph* g, CountCapture& C, const uint64_t key[CountCa
 // Launches both phases for one shard of the centres; the counters land in
 // g->counters ([0,30) closed classes, [30,36) open-pair removals, [36,42)
 // open-pair counts, [42..44] work queues). edge_flags is for diagnostics.
-// Each phase is captured once as a CUDA graph and replayed while everything
-// its launches were captured with (store and work-list arrays, the split,
+// Each phase is made into a CUDA graph once and replayed while everything
+// its launches were made with (store and work-list arrays, the split,
 // the shard) is unchanged; the diagnostic form launches directly.
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags) {
   hm_ctx* ctx = g->ctx;
@@ -922,8 +922,8 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
         (uint64_t)g->h2h_mask.p, (uint64_t)g->h2v_off.p, (uint64_t)g->h2v_mem.p, (uint64_t)g->esize.p,
         (uint64_t)g->counters.p};
     // one graph: its parts run side by side, so the open pairs have no time of their own
-    auto count = [&]() { return launch_decomp(g); };
-    return run_captured(g, g->decomp.capture, key, count, false, count, true);
+    auto count = [&](Launches& L) { return launch_decomp(g, L); };
+    return run_graphs(g, g->decomp.capture, key, count, false, count, true);
   }
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots;
@@ -934,24 +934,22 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
                   shard,         n_shards,      nullptr,       dev,          edge_flags,
                   nullptr,       nullptr};
   with_groups(g, args);
-  auto open_phase = [&]() -> int {
-    HM_CUDA(cudaMemsetAsync(dev, 0, sizeof(unsigned long long) * 48, st));
-    if (E) {
-      k_open_pairs<<<(unsigned)ctx->n_sms * 8, kOpenBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
-                                                                   g->h2h_ovl.p, g->esize.p, nullptr, E, shard,
-                                                                   n_shards, nullptr, nullptr, dev + 36);
-      HM_LAUNCH_CHECK();
-    }
+  auto open_phase = [&](Launches& L) -> int {
+    HM_TRY(L.zero(dev, 48));
+    if (E)
+      HM_TRY(L.run(k_open_pairs, (unsigned)ctx->n_sms * 8, kOpenBlock, 0, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
+                   g->h2h_ovl.p, g->esize.p, nullptr, E, shard, n_shards, nullptr, nullptr, dev + 36));
     return HM_OK;
   };
-  auto closed_phase = [&]() -> int {
-    return launch_closed(ctx, args, bounds, reinterpret_cast<unsigned int*>(dev + 42));
+  auto closed_phase = [&](Launches& L) -> int {
+    return launch_closed(ctx, L, args, bounds, reinterpret_cast<unsigned int*>(dev + 42));
   };
   if (edge_flags) {
+    Launches L{st};
     HM_CUDA(cudaEventRecord(g->ev[0], st));
-    HM_TRY(open_phase());
+    HM_TRY(open_phase(L));
     HM_CUDA(cudaEventRecord(g->ev[1], st));
-    HM_TRY(closed_phase());
+    HM_TRY(closed_phase(L));
     HM_CUDA(cudaEventRecord(g->ev[2], st));
     return HM_OK;
   }
@@ -965,7 +963,7 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
       (uint64_t)args.wopos,    (uint64_t)g->h2h_mask.p,  0};
   bool any_closed = false;
   for (int part = 0; part < 3; ++part) any_closed = any_closed || bounds[part + 1] - bounds[part] > shard;
-  return run_captured(g, g->capture, key, open_phase, true, closed_phase, any_closed);
+  return run_graphs(g, g->capture, key, open_phase, true, closed_phase, any_closed);
 }
 
 namespace {
@@ -984,9 +982,9 @@ __global__ void k_finish30(const unsigned long long* c, uint64_t* out30) {
 int count_static30_async(hm_graph* g, uint64_t* d_out30, cudaStream_t user) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
-  // The first count of a graph captures its launches as CUDA graphs on the
-  // context stream and may wait on it; neither works inside a capture that
-  // the event below would pull the context stream into.
+  // The first count of a graph allocates and may wait on the context stream;
+  // neither works inside a capture that the event below would pull the context
+  // stream into.
   for (cudaStream_t s : {user, st}) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     const cudaError_t e = cudaStreamIsCapturing(s, &cs);

@@ -82,3 +82,34 @@ def test_contexts_count_and_update_at_once():
         alone = []
         rounds(n, 20 + k, 1, alone)()
         assert len(got[k]) == r and all(x == alone[0] for x in got[k])
+
+
+def test_counts_while_the_program_waits_for_the_device():
+    """A first count makes its graphs without capturing a stream, so a wait for
+    the whole device on another thread neither fails nor disturbs it."""
+    import torch
+
+    from ipdps26_b200 import engine
+
+    done = threading.Event()
+
+    def waits():
+        while not done.is_set():
+            torch.cuda.synchronize()
+
+    def counts():
+        try:
+            _, h = _graph(3_000, 31)
+            with engine.Context(0) as c:
+                want = None
+                for _ in range(60):
+                    with engine.Graph.from_hypergraph(c, h) as g:
+                        for on in (True, False):  # either method
+                            g.set_static_groups(on)
+                            got = [g.count_static30().tolist() for _ in range(2)]
+                            want = want or got[0]
+                            assert got == [want, want]
+        finally:
+            done.set()
+
+    _run([counts, waits])
