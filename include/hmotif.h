@@ -150,6 +150,27 @@ int hm_debug_touch_orientation(hm_graph* g, int by_id);
  * oriented rows grouped by the member each neighbour shares with the row owner;
  * 0 visits every oriented entry. Counts are the same every way; tests run them. */
 int hm_debug_static_groups(hm_graph* g, int on);
+/* Which ways the last counts of graph g took (diagnostics; fields of counts not
+ * made yet are 0). The shapes are the launch shapes of the enumeration of
+ * triangles with two or three heavy pairs: centres searched, by 32-bit and by
+ * 64-bit tables, by large tables. */
+typedef struct hm_routes {
+  uint64_t arena_entries;     /* H2H arena: live entries, */
+  uint64_t arena_tail;        /* entries up to its tail, */
+  uint64_t arena_capacity;    /* entries it holds */
+  uint32_t static_decomposed; /* last full static count: 1 by decomposition, 0 by enumeration */
+  uint32_t static_by_entry;   /* heavy pairs searched one by one, no shapes */
+  uint32_t static_centres[4];
+  uint32_t static_spread;     /* owners whose pairs go through a node vector */
+  uint32_t static_kernels;    /* kernels launched by each such count */
+  uint32_t touch_decomposed;  /* last touched-triple count, as above */
+  uint32_t touch_by_entry;
+  uint32_t touch_centres[4];
+  uint32_t touch_spread;
+  uint32_t temporal_pairs;    /* last synchronous temporal count: events counted by pairs of window events, */
+  uint32_t temporal_sets;     /* by pairs of node-sets */
+} hm_routes;
+int hm_debug_routes(hm_graph* g, hm_routes* out);
 
 /* ---- the device store ------------------------------------------------- */
 /* Builds H2V (hyperedge -> sorted members), V2H (node -> sorted hyperedges)

@@ -372,6 +372,16 @@ extern "C" int hm_debug_static_groups(hm_graph* g, int on) {
   return HM_OK;
 }
 
+extern "C" int hm_debug_routes(hm_graph* g, hm_routes* out) {
+  if (!g || !out) return hm::set_error(HM_ERR_INVALID, "hm_debug_routes: NULL argument");
+  CtxLock lock(g->ctx);
+  *out = g->routes;
+  out->arena_entries = g->h2h_nnz;
+  out->arena_tail = g->h2h_tail;
+  out->arena_capacity = g->h2h_cap;
+  return HM_OK;
+}
+
 extern "C" int hm_debug_touch_orientation(hm_graph* g, int by_id) {
   if (!g) return hm::set_error(HM_ERR_INVALID, "hm_debug_touch_orientation: NULL graph");
   g->touch_by_id = by_id != 0;

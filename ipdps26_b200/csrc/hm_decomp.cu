@@ -2246,6 +2246,12 @@ static int launch_parts(hm_graph* g, Decomp& P, unsigned long long* counters, La
   return HM_OK;
 }
 
+void routes_of(const Decomp& P, uint32_t* by_entry, uint32_t centres[4], uint32_t* spread) {
+  *by_entry = P.by_entry;
+  for (int k = 0; k < 4; ++k) centres[k] = P.hend[k] - (k ? P.hend[k - 1] : 0);
+  *spread = P.n_spread;
+}
+
 int launch_decomp(hm_graph* g, Launches& L) { return launch_parts<false>(g, g->decomp, g->counters.p, L); }
 
 // The triples with a marked hyperedge, count(G) - count(G without them), by the
@@ -2269,6 +2275,7 @@ int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], 
   HM_CUDA(cudaStreamSynchronize(g->ctx->stream));
   for (int k = 0; k < 30; ++k) out30[k] = h[k];
   for (int k = 0; k < 6; ++k) out30[20 + k] += h[36 + k] - h[30 + k];
+  routes_of(P, &g->routes.touch_by_entry, g->routes.touch_centres, &g->routes.touch_spread);
   *done = true;
   return HM_OK;
 }

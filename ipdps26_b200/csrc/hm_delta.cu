@@ -685,8 +685,11 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   if (may_decomp && cost > std::max<uint64_t>(kDecompMin, kDecompEntries * g->h2h_nnz)) {
     bool done = false;
     HM_TRY(count_touching_decomp(g, mark.p, out, &done));
+    g->routes.touch_decomposed = done;
     if (done) return HM_OK;
   }
+  g->routes.touch_decomposed = g->routes.touch_by_entry = g->routes.touch_spread = 0;
+  for (auto& c : g->routes.touch_centres) c = 0;
   const uint32_t n_long = hcls[0], n_large = hcls[1], n_mid = hcls[2];
   HM_TRY(centres.alloc(ctx, nc));
   k_list_flagged<<<grid_for(E, kBlock), kBlock, 0, st>>>(flag.p, pos.p, E, centres.p);

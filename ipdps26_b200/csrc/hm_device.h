@@ -371,6 +371,7 @@ struct hm_graph {
   hm::DArr<uint32_t> t_rank;    // position -> rank of its time among the distinct times
 
   hm::PhaseTimes times;
+  hm_routes routes{};
 
   ~hm_graph() {
     capture.reset();
@@ -419,6 +420,7 @@ int prepare_enumeration(hm_graph* g);  // oriented rows and work list of the tri
 int prepare_decomp(hm_graph* g);
 struct Launches;
 int launch_decomp(hm_graph* g, Launches& L);
+void routes_of(const Decomp& P, uint32_t* by_entry, uint32_t centres[4], uint32_t* spread);
 int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done);
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags);
 int finish_static(hm_graph* g, uint64_t out30[30]);

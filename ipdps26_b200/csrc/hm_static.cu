@@ -923,7 +923,11 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
         (uint64_t)g->counters.p};
     // one graph: its parts run side by side, so the open pairs have no time of their own
     auto count = [&](Launches& L) { return launch_decomp(g, L); };
-    return run_graphs(g, g->decomp.capture, key, count, false, count, true);
+    HM_TRY(run_graphs(g, g->decomp.capture, key, count, false, count, true));
+    routes_of(g->decomp, &g->routes.static_by_entry, g->routes.static_centres, &g->routes.static_spread);
+    g->routes.static_decomposed = 1;
+    g->routes.static_kernels = g->decomp.capture.kernels;
+    return HM_OK;
   }
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots;
@@ -963,7 +967,11 @@ int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_
       (uint64_t)args.wopos,    (uint64_t)g->h2h_mask.p,  0};
   bool any_closed = false;
   for (int part = 0; part < 3; ++part) any_closed = any_closed || bounds[part + 1] - bounds[part] > shard;
-  return run_graphs(g, g->capture, key, open_phase, true, closed_phase, any_closed);
+  HM_TRY(run_graphs(g, g->capture, key, open_phase, true, closed_phase, any_closed));
+  g->routes.static_decomposed = g->routes.static_by_entry = g->routes.static_spread = 0;
+  for (auto& c : g->routes.static_centres) c = 0;
+  g->routes.static_kernels = g->capture.kernels;
+  return HM_OK;
 }
 
 namespace {

@@ -1114,7 +1114,7 @@ int count_temporal96(hm_graph* g, int64_t delta, uint64_t out96[96]) {
   HM_CUDA(cudaEventCreate(&e0));
   HM_CUDA(cudaEventCreate(&e1));
   const int rc = launch_temporal(g, delta, lo, acc, e0, e1);
-  unsigned long long h[103];  // up to the projection sizes
+  unsigned long long h[kAccSize];
   cudaError_t ce = rc < 0 ? cudaSuccess : cudaMemcpyAsync(h, acc.p, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (rc >= 0 && ce == cudaSuccess) ce = cudaStreamSynchronize(st);
   float ms = 0;
@@ -1129,6 +1129,9 @@ int count_temporal96(hm_graph* g, int64_t delta, uint64_t out96[96]) {
   g->times.t_nbrs = h[98];
   g->times.t_closed_pairs = h[99];
   g->times.t_open_pairs = h[100];
+  const uint32_t* shapes = reinterpret_cast<const uint32_t*>(h + 107);
+  g->routes.temporal_pairs = shapes[0] + shapes[1] + shapes[2];
+  g->routes.temporal_sets = shapes[3];
   if (h[97])
     return set_error(HM_ERR_LIMIT, "temporal count: an event has more than %u neighbours inside its window",
                      kMaxNbrs);

@@ -57,6 +57,27 @@ class Timings(C.Structure):
     ]
 
 
+class Routes(C.Structure):
+    """Which ways the last counts of a graph took (hm_routes)."""
+
+    _fields_ = [
+        ("arena_entries", C.c_uint64),
+        ("arena_tail", C.c_uint64),
+        ("arena_capacity", C.c_uint64),
+        ("static_decomposed", C.c_uint32),
+        ("static_by_entry", C.c_uint32),
+        ("static_centres", C.c_uint32 * 4),
+        ("static_spread", C.c_uint32),
+        ("static_kernels", C.c_uint32),
+        ("touch_decomposed", C.c_uint32),
+        ("touch_by_entry", C.c_uint32),
+        ("touch_centres", C.c_uint32 * 4),
+        ("touch_spread", C.c_uint32),
+        ("temporal_pairs", C.c_uint32),
+        ("temporal_sets", C.c_uint32),
+    ]
+
+
 class TemporalTraffic(C.Structure):
     _fields_ = [
         ("events", C.c_uint64),
@@ -185,6 +206,7 @@ _lib.bind(
         "hm_graph_unfill": (C.c_int, [vp, u32p, C.c_uint32, u32p, u64p, i64p]),
         "hm_debug_touch_orientation": (C.c_int, [vp, C.c_int]),
         "hm_debug_static_groups": (C.c_int, [vp, C.c_int]),
+        "hm_debug_routes": (C.c_int, [vp, C.POINTER(Routes)]),
         "hm_count_vertex_triads": (C.c_int, [vp, u64p]),
         "hm_graph_set_schedule": (C.c_int, [vp, C.POINTER(Schedule)]),
         "hm_graph_get_schedule": (C.c_int, [vp, C.POINTER(Schedule)]),
@@ -441,6 +463,11 @@ class Graph:
         """Walk of the static count: grouped rows with the shared-member group
         counted in bulk (default), or every oriented entry (same counts)."""
         check(lib.hm_debug_static_groups(self._h, int(on)), "hm_debug_static_groups")
+
+    def routes(self) -> Routes:
+        r = Routes()
+        check(lib.hm_debug_routes(self._h, C.byref(r)), "hm_debug_routes")
+        return r
 
     def set_touch_orientation(self, by_id: bool) -> None:
         """Walk order of the touched-triple counts (same counts either way)."""

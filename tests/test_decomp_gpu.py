@@ -170,3 +170,110 @@ def test_touched_triples_of_few_heavy_pairs(ctx, groups, marked):
         assert got.tolist() == (g.count_static30() - rest.count_static30()).tolist()
         g.set_touch_orientation(True)
         assert got.tolist() == g.count_touching30(ids).tolist()
+
+
+def _core(rng, n, n_nodes, sizes, hubs, n_hubs, light, pad):
+    """A heavy core (n hyperedges, each with `hubs` members out of n_hubs shared
+    nodes) in a graph whose pairs are mostly light: `light` hyperedges meet in
+    one node, which a third of the core holds too, so that the core goes by the
+    decomposition; `pad` hyperedges apart from all others take slots only."""
+    hub, rows = n_nodes, []
+    for k in range(n):
+        s = int(rng.choice(sizes))
+        r = set(rng.choice(n_hubs, size=min(hubs, s, n_hubs), replace=False).tolist())
+        if k % 3 == 0 and len(r) < s:
+            r.add(hub)
+        while len(r) < s:
+            r.add(int(rng.integers(0, n_nodes)))
+        rows.append(sorted(r))
+    rows += [[hub, hub + 1 + i] for i in range(light)]
+    free = hub + 1 + light
+    rows += [[free + 2 * i, free + 2 * i + 1] for i in range(pad)]
+    return rows, free + 2 * pad
+
+
+# name: sizes, hub members, hubs, core hyperedges, nodes, light hyperedges, launch shapes that have to run
+CORES = {
+    "masks-31-32-33": ([2, 3, 31, 32, 33], 2, 12, 260, 220, 500, (1, 2)),
+    "masks-63-64-65": ([2, 4, 63, 64, 65], 2, 20, 220, 400, 500, (1, 2, 3)),
+    "centres-above-64": ([4, 40, 66, 90, 130, 255], 3, 30, 160, 900, 500, (1, 2, 3)),
+    "overlaps-past-3": ([6, 7, 8, 9, 10], 5, 9, 300, 60, 700, (1,)),
+    "rows-around-96": ([3, 4], 2, 8, 800, 4000, 900, (0, 1)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CORES))
+@pytest.mark.parametrize("pad", [0, 12_300], ids=["by-rank", "hashed"])
+@pytest.mark.parametrize("seed", range(2))
+def test_heavy_core_runs_its_kernels(ctx, name, pad, seed):
+    """The edges of the table kernels, on graphs the decomposition takes: the
+    launch shapes named above are the ones that ran."""
+    from ipdps26_b200 import engine
+
+    *law, shapes = CORES[name]
+    sizes, hubs, n_hubs, n, n_nodes, light = law
+    rows, n_all = _core(np.random.default_rng(50 + seed), n, n_nodes, sizes, hubs, n_hubs, light, pad)
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, n_all) as g:
+        got = g.count_static30()
+        r = g.routes()
+        assert r.static_decomposed and not r.static_by_entry
+        assert all(r.static_centres[k] for k in shapes), list(r.static_centres)
+        assert r.static_spread or name != "centres-above-64"
+        assert got.tolist() == oracle.static30(off, mem, n_all).tolist()
+        g.set_static_groups(False)
+        assert got.tolist() == g.count_static30().tolist()
+        assert not g.routes().static_decomposed
+
+
+@pytest.mark.parametrize("seed", range(2))
+def test_large_centres_searched_by_entry(ctx, seed):
+    """Few heavy pairs, most of centres above 64 members: the triple overlap of
+    each by merging the three lists."""
+    from ipdps26_b200 import engine
+
+    rows, n_all = _core(np.random.default_rng(70 + seed), 40, 900, [65, 66, 101, 180, 255], 3, 20, 300, 0)
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, n_all) as g:
+        got = g.count_static30()
+        assert g.routes().static_decomposed and g.routes().static_by_entry
+        assert got.tolist() == oracle.static30(off, mem, n_all).tolist()
+
+
+@pytest.mark.parametrize("name", sorted(CORES))
+@pytest.mark.parametrize("pad", [0, 12_300], ids=["by-rank", "hashed"])
+def test_touched_triples_of_a_heavy_core(ctx, name, pad):
+    """The same kernels with marks: half of the core and most light hyperedges
+    are marked, and the count is the full one minus that of the rest."""
+    from ipdps26_b200 import engine
+
+    sizes, hubs, n_hubs, n, n_nodes, _, shapes = CORES[name]
+    rng = np.random.default_rng(90)
+    rows, n_all = _core(rng, n, n_nodes, sizes, hubs, n_hubs, 700, pad)
+    ids = np.sort(np.concatenate([rng.choice(n, size=n // 2, replace=False), np.arange(n, n + 650)])).astype(np.uint32)
+    off, mem = csr(rows)
+    rest_off, rest_mem = csr([r for k, r in enumerate(rows) if k not in set(ids.tolist())])
+    with engine.Graph(ctx, off, mem, n_all) as g:
+        got = g.count_touching30(ids)
+        r = g.routes()
+        assert r.touch_decomposed and not r.touch_by_entry
+        assert all(r.touch_centres[k] for k in shapes if k), list(r.touch_centres)
+        want = oracle.static30(off, mem, n_all) - oracle.static30(rest_off, rest_mem, n_all)
+        assert got.tolist() == want.tolist()
+        g.set_touch_orientation(True)
+        assert got.tolist() == g.count_touching30(ids).tolist()
+        assert not g.routes().touch_decomposed
+
+
+def test_rows_past_the_largest_table(ctx):
+    """Hub rows of more than 12,288 higher-ranked neighbours (searched), of more
+    than 3,072 (large tables), and shorter ones, against the enumeration."""
+    from ipdps26_b200 import engine, gen
+
+    n = 16_000
+    with engine.Graph.from_hypergraph(ctx, gen.static(gen.config1(seed=4, n_nodes=n // 2, n_edges=n))) as g:
+        got = g.count_static30()
+        r = g.routes()
+        assert r.static_decomposed and r.static_centres[0] and r.static_centres[1] and r.static_centres[3]
+        g.set_static_groups(False)
+        assert got.tolist() == g.count_static30().tolist()
