@@ -368,6 +368,7 @@ struct hm_graph {
   hm::DArr<uint64_t> t_exact;   // position -> bits of the event's top nodes
   hm::DArr<uint64_t> t_other;   // position -> hash word of its other members
   hm::DArr<uint32_t> t_size;    // position -> members
+  hm::DArr<uint32_t> t_degree;  // position -> occurrences of its members in all events
   hm::DArr<uint32_t> t_rank;    // position -> rank of its time among the distinct times
 
   hm::PhaseTimes times;

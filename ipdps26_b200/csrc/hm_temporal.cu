@@ -17,8 +17,8 @@
 // of the events containing it; static id -> positions of its occurrences.
 //
 // Windows of up to 2048 events go to k_temporal_pairs, which looks at every pair
-// of the window's events (see there). The others go to k_temporal, one block per
-// event a (position p), over the window [lo, p):
+// of the window's events (see there), but for the longest in streams that
+// by_sets tells. The others go to k_temporal, one block per event a (position p), over the window [lo, p):
 //   1. neighbours b of a: walk the window occurrences of a's nodes, keep the
 //      first occurrence of each static id, and accumulate the overlap C_ab and
 //      the positions of a's members it contains (mask) in a shared hash;
@@ -38,6 +38,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "hm_classes.h"
@@ -154,7 +155,8 @@ __global__ void k_gather_len(const uint32_t* order, uint32_t n, const uint32_t* 
 
 // Launch shapes of the count, by the events in the window: 0 a warp per event,
 // 1 and 2 a block per event (all three in k_temporal_pairs), 3 k_temporal. An
-// event of no members or more than kPairMembers always goes to k_temporal.
+// event of no members or more than kPairMembers always goes to k_temporal, and
+// shape 2 does in streams that by_sets tells.
 constexpr uint32_t kPairCap0 = 64, kPairCap1 = 512, kPairCap2 = 2048;
 // Streams of fewer events than the GPU holds warps give all but the smallest
 // windows a block: the time is then that of the few events one place takes in
@@ -162,18 +164,102 @@ constexpr uint32_t kPairCap0 = 64, kPairCap1 = 512, kPairCap2 = 2048;
 constexpr uint32_t kFewEvents = 6000, kFewCap0 = 8;
 constexpr uint32_t kPairMembers = 32;
 
+// The longest windows (shape 2) are not always cheaper by pairs of events:
+// k_temporal walks its event's nodes and takes a node-set once however often it
+// occurs, which wins where few of the window's events share a member with a, or
+// few node-sets take turns. With s the window's occurrences of a's nodes, f the
+// share of them that are a node-set's first, and s' the same as s for a
+// neighbour, about n = s w / (s + w) of the w events share a member with a, and
+// an event takes, in ns of a full GPU,
+//   pairs  w / 25 + n^2 / 400 + n (w - n) / 850
+//   sets   16 + s / 10 + f n s' / 25.
+// Both kernels were timed on 50 streams of 5 to 5,000 node-sets at windows of
+// 100 to 2,000 events; past 512 the sums agree with the faster one on all of
+// them. 10,000 events, windows of 2,000, ms by sets / by pairs: 5 node-sets in
+// turn 4.3 / 26.7, 100: 11.0 / 29.8, 400: 40.4 / 28.8; 300 sets over rare nodes
+// 0.16 / 0.86. Windows of 400 differ less (20,000 events: 0.26 / 0.28 over rare
+// nodes, 6.6 / 2.7 with common ones) and stay by pairs. The whole stream goes one
+// way: split by event, each kernel's last events (0.9 ms each by pairs) are waited
+// for in turn. Finding out costs 30,000 events of 8.9 ms less than 1 %.
+struct SetsArgs {
+  const uint32_t* sp;      // position -> static id
+  const uint32_t* prev;    // position -> previous position of the same
+  const uint32_t* degree;  // position -> occurrences of its nodes in the whole stream
+  const uint32_t* order;
+  const uint64_t* hoff;
+  const uint32_t* hmem;
+  const uint64_t* voff;    // node -> positions
+  const uint32_t* vlen;
+  const uint32_t* vpos;
+  float* cost;             // ns by pairs, by sets
+};
+
+__device__ __forceinline__ bool by_sets(const float* cost) { return cost[1] < cost[0]; }
+
+// The number of values below x in the sorted list v[0..n).
+__device__ __forceinline__ uint32_t count_below(const uint32_t* v, uint32_t n, uint32_t x) {
+  uint32_t l = 0, h = n;
+  while (l < h) {
+    const uint32_t m = (l + h) >> 1;
+    if (v[m] < x) l = m + 1;
+    else h = m;
+  }
+  return l;
+}
+
+// Whole warp: both costs of event p, added `times` over. Two lanes per member,
+// for the ends of its range, then for four places of it each.
+__device__ void add_costs(const SetsArgs& S, uint32_t p, uint32_t lo, uint32_t size, uint32_t n_events, float times) {
+  const unsigned lane = lane_id();
+  const uint32_t w = p - lo, sa = S.sp[p];
+  const uint32_t* m = S.hmem + S.hoff[S.order[p]];
+  float d = (float)S.degree[lo + (uint32_t)((2 * lane + 1) * (uint64_t)w / 64)];
+  float s = 0, firsts = 0;
+  for (uint32_t i = lane / 2; i < ((size + 15) & ~15u); i += 16) {
+    uint32_t end = 0;
+    const uint32_t* v = S.vpos;
+    if (i < size) {
+      v += S.voff[m[i]];
+      end = count_below(v, S.vlen[m[i]], lane & 1u ? p : lo);
+    }
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, end, 1);
+    const uint32_t a = min(end, other), l = max(end, other) - a;
+    if (!l) continue;
+    s += 0.5f * (float)l;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t q = v[a + (uint32_t)((2 * (4 * (lane & 1u) + k) + 1) * (uint64_t)l / 16)], pr = S.prev[q];
+      if (S.sp[q] != sa && (pr == kNone || pr < lo)) firsts += 0.125f * (float)l;
+    }
+  }
+  __syncwarp();
+  for (int k = 16; k; k >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, k);
+    firsts += __shfl_xor_sync(0xffffffffu, firsts, k);
+    d += __shfl_xor_sync(0xffffffffu, d, k);
+  }
+  if (lane == 0) {
+    const float fw = (float)w, n = s * fw / (s + fw), f = s > 0 ? firsts / s : 0.0f;
+    const float walk = fmaxf(s, d / 32.0f * (fw / (float)n_events));
+    atomicAdd(&S.cost[0], times * (fw / 25.0f + n * n / 400.0f + n * (fw - n) / 850.0f));
+    atomicAdd(&S.cost[1], times * (16.0f + s / 10.0f + f * n * walk / 25.0f));
+  }
+}
+
 // Window start of every position, and the positions of each shape (list k at
 // lists + k n, its length in counts[k]); an empty window has nothing to count.
-// cap0: windows up to it take a warp.
+// cap0: windows up to it take a warp. One event of shape 2 of each 32 events
+// stands for theirs in the costs.
 __global__ void k_window_lo(const int64_t* t, const uint32_t* size, uint32_t n, int64_t delta, uint32_t cap0,
-                            uint32_t* lo, uint32_t* lists, unsigned int* counts) {
+                            SetsArgs S, uint32_t* lo, uint32_t* lists, unsigned int* counts) {
   for (uint64_t p0 = gtid() & ~31ull; p0 < n; p0 += gstride()) {
     const uint64_t p = p0 + lane_id();
     int shape = -1;
+    uint32_t l = 0;
     if (p < n) {
       const int64_t tp = t[p];
       // first q with t[q] + delta >= t[p]
-      uint32_t l = 0, h = (uint32_t)p;
+      uint32_t h = (uint32_t)p;
       while (l < h) {
         const uint32_t mid = (l + h) >> 1;
         if (t[mid] + delta < tp) l = mid + 1;
@@ -183,6 +269,12 @@ __global__ void k_window_lo(const int64_t* t, const uint32_t* size, uint32_t n, 
       const uint32_t w = (uint32_t)p - l;
       if (w)
         shape = size[p] - 1u >= kPairMembers || w > kPairCap2 ? 3 : w > kPairCap1 ? 2 : w > cap0 ? 1 : 0;
+    }
+    const unsigned big = __ballot_sync(0xffffffffu, shape == 2);
+    if (big) {
+      const int src = (int)__fns(big, 0, 1 + (int)((p0 >> 5) % (unsigned)__popc(big)));
+      const uint32_t q = (uint32_t)p0 + (uint32_t)src;
+      add_costs(S, q, __shfl_sync(0xffffffffu, l, src), size[q], n, (float)__popc(big));
     }
     for (int k = 0; k < 4; ++k) {
       const unsigned m = __ballot_sync(0xffffffffu, shape == k);
@@ -204,20 +296,23 @@ __global__ void k_set_top(const uint32_t* node, uint32_t n, uint8_t* top) {
 __device__ __forceinline__ uint64_t other_bit(uint32_t v) { return 1ull << ((v * 2654435761u) >> 26); }
 
 __global__ void k_signatures(const uint32_t* order, uint32_t n, const uint64_t* off, const uint32_t* len,
-                             const uint32_t* mem, const uint8_t* top, uint64_t* exact, uint64_t* other,
-                             uint32_t* size) {
+                             const uint32_t* mem, const uint8_t* top, const uint32_t* vlen, uint64_t* exact,
+                             uint64_t* other, uint32_t* size, uint32_t* degree) {
   for (uint64_t p = gtid(); p < n; p += gstride()) {
     const uint32_t e = order[p], l = len[e];
     const uint32_t* m = mem + off[e];
     uint64_t x = 0, o = 0;
+    uint32_t d = 0;
     for (uint32_t i = 0; i < l; ++i) {
       const uint32_t v = m[i], t = top[v];
+      d += vlen[v];
       if (t < 64) x |= 1ull << t;
       else o |= other_bit(v);
     }
     exact[p] = x;
     other[p] = o;
     size[p] = l;
+    degree[p] = d;
   }
 }
 
@@ -256,8 +351,12 @@ struct TArgs {
   // each event in its window, [1] adjacent pairs among them, [2] pairs
   // (b, c) with c adjacent to a neighbour b but not to the event
   unsigned long long* stats;
-  const uint32_t* list;      // the first launch's events
+  const uint32_t* list;      // the first launch's events: shape 3,
   const unsigned int* n_list;
+  const uint32_t* list2;     // and shape 2 where by_sets(cost),
+  const unsigned int* n_list2;
+  const float* cost;
+  unsigned int* n_pairs2;    // which leaves the pair kernel that many of it
   unsigned int* queue2;      // the deferred launch's queue
   unsigned int* n_deferred;  // events set aside by the first launch
   uint32_t* deferred;
@@ -329,7 +428,7 @@ constexpr size_t temporal_smem() {
 }
 
 // Block per event; kS hash slots hold up to kM window neighbours. The first
-// launch (kFirst) takes the events of shape 3 and sets aside those with more
+// launch (kFirst) takes the events of its lists and sets aside those with more
 // neighbours in a deferred list; the second takes that list with a larger
 // table, and reports an event that overflows it too.
 template <uint32_t kS, uint32_t kM, bool kFirst>
@@ -350,6 +449,12 @@ __global__ void __launch_bounds__(kBlock) k_temporal(TArgs A) {
   __shared__ int8_t tab[128];
   __shared__ uint32_t sam[256];
   __shared__ uint32_t s_item, s_nla;
+  const uint32_t n_list = kFirst ? *A.n_list : *A.n_deferred;
+  const uint32_t n_list2 = kFirst ? *A.n_list2 : 0;
+  const bool sets = kFirst && by_sets(A.cost);
+  if (kFirst && blockIdx.x == 0 && threadIdx.x == 0) *A.n_pairs2 = sets ? 0 : n_list2;
+  const uint32_t n_items = n_list + (sets ? n_list2 : 0);
+  if (!n_items) return;
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   unsigned long long n_nbrs = 0, n_closed = 0, n_open_b = 0;  // this thread's share of A.stats
   for (unsigned k = threadIdx.x; k < kWarps * 96; k += blockDim.x) (&wcnt[0][0])[k] = 0;
@@ -368,8 +473,8 @@ __global__ void __launch_bounds__(kBlock) k_temporal(TArgs A) {
     }
     __syncthreads();
     const uint32_t item = s_item;
-    if (item >= (kFirst ? *A.n_list : *A.n_deferred)) break;
-    const uint32_t p = kFirst ? A.list[item] : A.deferred[item];
+    if (item >= n_items) break;
+    const uint32_t p = !kFirst ? A.deferred[item] : item < n_list ? A.list[item] : A.list2[item - n_list];
     const uint32_t lo = A.lo[p];
     const uint32_t ea = A.order[p];
     const uint32_t sa = A.sp[p];
@@ -987,8 +1092,10 @@ static int build_temporal_index(hm_graph* g) {
   HM_TRY(g->t_other.alloc(ctx, n));
   HM_TRY(g->t_size.alloc(ctx, n));
   HM_TRY(g->t_rank.alloc(ctx, n));
+  HM_TRY(g->t_degree.alloc(ctx, n));
   k_signatures<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_order.p, n, g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p,
-                                                        g->t_top.p, g->t_exact.p, g->t_other.p, g->t_size.p);
+                                                        g->t_top.p, g->t_vlen.p, g->t_exact.p, g->t_other.p,
+                                                        g->t_size.p, g->t_degree.p);
   HM_LAUNCH_CHECK();
   k_time_steps<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, n, plen.p);
   HM_LAUNCH_CHECK();
@@ -1010,12 +1117,13 @@ __global__ void k_temporal_finish(const unsigned long long* acc, uint64_t* out96
 }  // namespace
 
 // Queues the window starts and the counting kernels on the context stream:
-// acc receives the 96 counts, [96] unused, [97] the overflow flag, [98..100]
-// the window-projection sizes, [101] the deferred launch's queue, [102] the
-// number of deferred events, [103..106] queues and [107..110] lengths of the
-// four shapes' lists; lo holds the window starts, the lists and the deferred
-// events. Events e0/e1 bracket the kernels.
-constexpr size_t kAccSize = 111;
+// acc receives the 96 counts, [96] the costs by pairs and by sets, [97] the
+// overflow flag, [98..100] the window-projection sizes, [101] the deferred
+// launch's queue, [102] the number of deferred events, [103..106] queues and
+// [107..108] lengths of the four shapes' lists, [109] shape 2's for the pair
+// kernel; lo holds the window starts, the
+// lists and the deferred events. Events e0/e1 bracket the kernels.
+constexpr size_t kAccSize = 110;
 template <uint32_t kGroupWarps, uint32_t kCap, unsigned kThreads, unsigned kMinBlocks>
 static int launch_pairs(hm_ctx* ctx, const PairArgs& A, uint32_t n) {
   constexpr size_t smem = pair_smem<kGroupWarps, kCap, kThreads>();
@@ -1042,20 +1150,13 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
   uint32_t* lists = lo.p + n;
   auto u32 = [&](size_t k) { return reinterpret_cast<unsigned int*>(acc.p + k); };
   unsigned int* counts = u32(107);  // four consecutive counts
+  unsigned int* n_pairs2 = u32(109);
+  float* cost = reinterpret_cast<float*>(acc.p + 96);
+  const SetsArgs sets{g->t_static.p, g->t_prev.p, g->t_degree.p, g->t_order.p, g->h2v_off.p,
+                      g->h2v_mem.p,  g->t_voff.p, g->t_vlen.p,   g->t_vpos.p,  cost};
   k_window_lo<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, g->t_size.p, n, delta,
-                                                      n < kFewEvents ? kFewCap0 : kPairCap0, lo.p, lists, counts);
+                                                      n < kFewEvents ? kFewCap0 : kPairCap0, sets, lo.p, lists, counts);
   HM_LAUNCH_CHECK();
-  PairArgs P{nullptr, nullptr, nullptr, lo.p, g->t_static.p, g->t_prev.p, g->t_rank.p, g->t_exact.p, g->t_other.p,
-             g->t_size.p, g->t_order.p, g->h2v_off.p, g->h2v_mem.p, g->t_top.p, acc.p, acc.p + 98};
-  auto shape = [&](int k) {
-    P.list = lists + (size_t)k * n;
-    P.n_list = counts + k;
-    P.queue = u32(103 + k);
-    return P;
-  };
-  HM_TRY((launch_pairs<16, kPairCap2, 512, 2>(ctx, shape(2), n)));
-  HM_TRY((launch_pairs<8, kPairCap1, 256, 5>(ctx, shape(1), n)));
-  HM_TRY((launch_pairs<1, kPairCap0, 256, 5>(ctx, shape(0), n)));
   TArgs A{n,
           g->t_order.p,
           g->t_static.p,
@@ -1077,6 +1178,10 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
           acc.p + 98,
           lists + 3 * (size_t)n,
           counts + 3,
+          lists + 2 * (size_t)n,
+          counts + 2,
+          cost,
+          n_pairs2,
           u32(101),
           u32(102),
           lo.p + 5 * (size_t)n};
@@ -1086,11 +1191,23 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
                                (int)kSmemSmall));
   HM_CUDA(cudaFuncSetAttribute(k_temporal<kSlotsLarge, kNbrsLarge, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kSmemLarge));
+  // before the pair kernels: it tells them whether shape 2 is left to them
   k_temporal<kSlotsSmall, kNbrsSmall, true>
       <<<std::min<unsigned>((unsigned)ctx->n_sms * 4, n), kBlock, kSmemSmall, st>>>(A);
   HM_LAUNCH_CHECK();
   k_temporal<kSlotsLarge, kNbrsLarge, false><<<(unsigned)ctx->n_sms, kBlock, kSmemLarge, st>>>(A);
   HM_LAUNCH_CHECK();
+  PairArgs P{nullptr, nullptr, nullptr, lo.p, g->t_static.p, g->t_prev.p, g->t_rank.p, g->t_exact.p, g->t_other.p,
+             g->t_size.p, g->t_order.p, g->h2v_off.p, g->h2v_mem.p, g->t_top.p, acc.p, acc.p + 98};
+  auto shape = [&](int k) {
+    P.list = lists + (size_t)k * n;
+    P.n_list = k == 2 ? n_pairs2 : counts + k;
+    P.queue = u32(103 + k);
+    return P;
+  };
+  HM_TRY((launch_pairs<16, kPairCap2, 512, 2>(ctx, shape(2), n)));
+  HM_TRY((launch_pairs<8, kPairCap1, 256, 5>(ctx, shape(1), n)));
+  HM_TRY((launch_pairs<1, kPairCap0, 256, 5>(ctx, shape(0), n)));
   if (e1) HM_CUDA(cudaEventRecord(e1, st));
   return HM_OK;
 }
@@ -1130,8 +1247,10 @@ int count_temporal96(hm_graph* g, int64_t delta, uint64_t out96[96]) {
   g->times.t_closed_pairs = h[99];
   g->times.t_open_pairs = h[100];
   const uint32_t* shapes = reinterpret_cast<const uint32_t*>(h + 107);
-  g->routes.temporal_pairs = shapes[0] + shapes[1] + shapes[2];
-  g->routes.temporal_sets = shapes[3];
+  float cost[2];
+  std::memcpy(cost, h + 96, sizeof(cost));
+  g->routes.temporal_sets = shapes[3] + (cost[1] < cost[0] ? shapes[2] : 0);
+  g->routes.temporal_pairs = shapes[0] + shapes[1] + shapes[2] + shapes[3] - g->routes.temporal_sets;
   if (h[97])
     return set_error(HM_ERR_LIMIT, "temporal count: an event has more than %u neighbours inside its window",
                      kMaxNbrs);

@@ -183,3 +183,28 @@ def test_temporal_at_the_window_shapes_edges(ctx, window, ties):
         assert g.count_temporal(window).tolist() == want.tolist()
         t = g.temporal_traffic()
         assert t.events == len(rows) and t.window_neighbours > 0
+
+
+@pytest.mark.parametrize("law", ["common", "turns", "rare"])
+@pytest.mark.parametrize("window", [511, 512, 513, 700, 2047, 2048])
+def test_temporal_by_pairs_or_by_node_sets(ctx, window, law):
+    """Streams with windows past 512 events: distinct node-sets over common nodes
+    are counted by pairs of events, few node-sets in turn and node-sets over
+    rare nodes by the walk of node-sets. Against the oracle."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(window)
+    n, n_nodes = window + 40, {"common": 100, "turns": 40, "rare": 5 * window}[law]
+    distinct = 12 if law == "turns" else n
+    rows = [rng.choice(n_nodes, size=int(rng.integers(2, 5)), replace=False).tolist() for _ in range(distinct)]
+    off, mem = csr([rows[i % distinct] for i in range(n)])
+    times = np.arange(n, dtype=np.int64)
+    with engine.Graph(ctx, off, mem, n_nodes, times) as g:
+        got = g.count_temporal(window)
+        r = g.routes()
+    assert r.temporal_pairs + r.temporal_sets == n - 1
+    if law == "common" or window <= 512:
+        assert r.temporal_sets == 0
+    elif window >= 700:  # at 513 both take about as long
+        assert r.temporal_sets == n - 1 - 512
+    assert got.tolist() == oracle.temporal96(off, mem, times, window).tolist()
