@@ -158,6 +158,7 @@ typedef struct hm_routes {
   uint64_t arena_entries;     /* H2H arena: live entries, */
   uint64_t arena_tail;        /* entries up to its tail, */
   uint64_t arena_capacity;    /* entries it holds */
+  uint32_t rows_bitmap;       /* last rows built: 1 by bitmaps, 0 by sorting */
   uint32_t static_decomposed; /* last full static count: 1 by decomposition, 0 by enumeration */
   uint32_t static_by_entry;   /* heavy pairs searched one by one, no shapes */
   uint32_t static_centres[4];

@@ -671,7 +671,17 @@ int build_v2h(hm_graph* g) {
   return HM_OK;
 }
 
-constexpr uint32_t kBitmapSlots = 81920;  // 20 KB of bitmap and prefix counts per group
+// Rows go by bitmaps in stores of up to kBitmapSlots slots: a block of four
+// groups of a warp then takes at most 113 KB of shared memory, and two are on an
+// SM. Builds of the served graphs' law, sort / bitmaps: 20K slots 0.57 / 0.42 ms,
+// 80K 3.2 / 2.7, 110K 4.7 / 4.2, 160K (one block) 8.4 / 13.5. A row's bitmap is
+// cleared and summed whole, so rows of few wedges over many slots are faster
+// sorted, unless there are so few of them that the sort's launches tell: stores
+// pooled of small graphs (27 neighbours a row), 20K slots 0.46 / 0.41 ms, 40K
+// 0.56 / 0.64, 80K 0.76 / 1.98, but 3,800 rows inserted into the last 0.97 / 0.97
+// and 400 0.77 / 0.74.
+constexpr uint32_t kBitmapSlots = 113 << 10;
+constexpr uint64_t kBitmapFew = 1 << 24;  // words of all rows' bitmaps
 constexpr unsigned kBitmapWarps = 4;      // groups of a warp each per block
 constexpr uint64_t kBitmapLong = 1024;    // wedges per row on average from which a row takes a block
 
@@ -730,8 +740,10 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     HM_LAUNCH_CHECK();
     return HM_OK;
   }
-  if (g->n_slots <= kBitmapSlots) {
-    const uint32_t words = (g->n_slots + 31) / 32;
+  const uint32_t words = (g->n_slots + 31) / 32;
+  const uint64_t all_words = (uint64_t)n_rows * words;
+  g->routes.rows_bitmap = g->n_slots <= kBitmapSlots && (all_words <= kBitmapFew || all_words / 32 <= W);
+  if (g->routes.rows_bitmap) {
     const bool by_block = W / n_rows >= kBitmapLong;
     DArr<unsigned long long> total;
     HM_TRY(total.alloc(ctx, 1));

@@ -64,6 +64,7 @@ class Routes(C.Structure):
         ("arena_entries", C.c_uint64),
         ("arena_tail", C.c_uint64),
         ("arena_capacity", C.c_uint64),
+        ("rows_bitmap", C.c_uint32),
         ("static_decomposed", C.c_uint32),
         ("static_by_entry", C.c_uint32),
         ("static_centres", C.c_uint32 * 4),

@@ -121,6 +121,41 @@ def test_pooled_arena_moves_to_chunks_under_every_budget():
     assert passed and all(passed)
 
 
+def test_rows_by_bitmaps_or_sorted(ctx):
+    """The two ways adjacency rows are built: on both sides of the slot limit the
+    same store, and a store of many short rows sorted, short batches into it by
+    bitmaps, against the oracle."""
+    from ipdps26_b200 import engine, gen
+    from oracle import oracle
+
+    n = 113 << 10
+    h = gen.static(gen.params(3, n // 2, n, 2, 25, 2.5, 1.2, 1000.0))
+    with engine.Graph(ctx, h.offsets, h.members, h.n_nodes + 1) as g:
+        assert g.routes().rows_bitmap
+        want = g.info().n_adjacent, g.count_static30().tolist()
+    off, mem = np.append(h.offsets, h.offsets[-1] + 1).astype(np.uint64), np.append(h.members, h.n_nodes).astype(np.uint32)
+    with engine.Graph(ctx, off, mem, h.n_nodes + 1) as g:  # one more hyperedge, apart from the others
+        assert not g.routes().rows_bitmap
+        assert (g.info().n_adjacent, g.count_static30().tolist()) == want
+
+    rng = np.random.default_rng(15)
+    rows = [sorted(6 * (k // 5) + rng.choice(6, size=3, replace=False)) for k in range(40_000)]
+    n_nodes = 6 * 8_000
+    off, mem = csr(rows)
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        assert not g.routes().rows_bitmap
+        before = g.count_static30()
+        assert before.tolist() == oracle.static30(off, mem, n_nodes).tolist()
+        new = rows[100:400]
+        io, im = csr(new)
+        _, delta = g.apply_batch(list(range(50)), io, im)
+        assert g.routes().rows_bitmap
+        off, mem = csr(rows[50:] + new)
+        want = oracle.static30(off, mem, n_nodes)
+        assert g.count_static30().tolist() == want.tolist()
+        assert (before.astype(np.int64) + delta).tolist() == want.astype(np.int64).tolist()
+
+
 def test_growth_of_a_pooled_arena_fails_whole():
     """Every allocation of a batch that grows a pooled arena fails in turn. The
     batch then ends in HM_ERR_NOMEM or, where the growth was optional, in the
