@@ -388,7 +388,7 @@ int build_h2v(hm_graph* g, const uint64_t* h_off, const uint32_t* h_mem, uint32_
 int build_v2h(hm_graph* g);
 int build_h2h_rows(hm_graph* g);
 int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
-                 const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written, uint64_t* end);
+                 const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written);
 int build_plus(hm_graph* g);
 int build_plus_groups(hm_graph* g);
 void release_plus_groups(hm_graph* g);

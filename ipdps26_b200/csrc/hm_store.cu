@@ -241,15 +241,17 @@ __global__ void k_chunk_emit(const int* beg, const int* end, const uint32_t* key
 // and adds each wedge's overlap and position bit at its neighbour's place. One
 // launch instead of expand, segmented sort, count, scan, starts and emit (15
 // launches, the sort of rows of a thousand wedges alone 0.12 ms; build and
-// count of a 20K-hyperedge graph 1.20 ms with them). Rows are written at their
-// wedge offsets, ovl and mask zeroed before.
+// count of a 20K-hyperedge graph 1.20 ms with them). A row knows its length
+// before it writes and takes the next free place (*total), so that the rows leave
+// no holes; ovl and mask are zeroed before.
 template <unsigned kGroupWarps>
 __global__ void k_rows_bitmap(const uint64_t* h_off, const uint32_t* h_len, const uint32_t* h_mem,
                               const uint64_t* v_off, const uint32_t* v_len, const uint32_t* v_edge,
-                              const uint64_t* woff, const uint32_t* rows, uint32_t n, uint32_t words, uint64_t base,
-                              uint64_t* row_off, uint32_t* row_len, uint32_t* nbr, uint8_t* ovl, uint64_t* mask,
+                              const uint32_t* rows, uint32_t n, uint32_t words, uint64_t base, uint64_t* row_off,
+                              uint32_t* row_len, uint32_t* nbr, uint8_t* ovl, uint64_t* mask,
                               unsigned long long* total) {
   extern __shared__ uint32_t bm[];
+  __shared__ uint64_t s_dst;  // of a block's row
   const unsigned w = threadIdx.x / kWarp, lane = lane_id();
   const unsigned gw = kGroupWarps == 1 ? 0 : w, gt = kGroupWarps == 1 ? lane : threadIdx.x;
   const unsigned groups = blockDim.x / kWarp / kGroupWarps, group = kGroupWarps == 1 ? w : 0;
@@ -262,7 +264,6 @@ __global__ void k_rows_bitmap(const uint64_t* h_off, const uint32_t* h_len, cons
   };
   for (uint64_t i = (uint64_t)blockIdx.x * groups + group; i < n; i += (uint64_t)gridDim.x * groups) {
     const uint32_t r = row_at(rows, i);
-    const uint64_t dst = base + woff[i];
     const uint64_t s = h_off[r];
     const uint32_t l = h_len[r];
     for (uint32_t k = gt; k < words; k += kThreads) bits[k] = 0;
@@ -293,12 +294,15 @@ __global__ void k_rows_bitmap(const uint64_t* h_off, const uint32_t* h_len, cons
         if (k < words) pre[k] = len + x - c;
         len += __shfl_sync(0xffffffffu, x, 31);
       }
+    uint64_t dst = 0;
     if (gt == 0) {
+      dst = base + (len ? atomicAdd(total, (unsigned long long)len) : 0ull);
       row_off[r] = dst;
       row_len[r] = len;
-      if (len) atomicAdd(total, (unsigned long long)len);
+      if (kGroupWarps > 1) s_dst = dst;
     }
     sync();
+    dst = kGroupWarps > 1 ? s_dst : __shfl_sync(0xffffffffu, dst, 0);
     for (uint32_t k = gt; k < words; k += kThreads) {
       uint64_t q = dst + pre[k];
       for (uint32_t m = bits[k]; m; m &= m - 1) nbr[q++] = (k << 5) | (uint32_t)(__ffs(m) - 1);
@@ -688,13 +692,13 @@ constexpr uint64_t kBitmapLong = 1024;    // wedges per row on average from whic
 // H2H rows of the listed slots (all slots when d_rows is null): by bitmaps, or
 // in chunks of the wedge stream: expand, segmented sort, run-length.
 // reserve(W) is called once with an upper bound on the entries and returns the
-// arena position where the rows are written; *written receives the entries
-// emitted and *end how far past that position they reach.
+// arena position where the rows are written, one after another; *written
+// receives the entries emitted.
 int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
-                 const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written, uint64_t* end_out) {
+                 const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
-  *written = *end_out = 0;
+  *written = 0;
   if (g->n_slots >= (1u << 24))
     return set_error(HM_ERR_LIMIT, "H2H: %u hyperedge slots exceed the 2^24 limit of the packed sort key", g->n_slots);
   DArr<uint64_t> wedges, woff;
@@ -759,7 +763,7 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
       HM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(groups * 2 * kWordsMax * sizeof(uint32_t))));
       kernel<<<grid_for(n_rows, groups, (unsigned)ctx->n_sms * 16), threads, smem, st>>>(
-          g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p, g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p, woff.p, d_rows, n_rows,
+          g->h2v_off.p, g->h2v_len.p, g->h2v_mem.p, g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p, d_rows, n_rows,
           words, base, g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, g->h2h_mask.p, total.p);
       HM_LAUNCH_CHECK();
       return HM_OK;
@@ -768,7 +772,6 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     else HM_TRY(run(k_rows_bitmap<1>, kBitmapWarps, kBitmapWarps * kWarp));
     HM_CUDA(cudaMemcpyAsync(written, total.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     HM_CUDA(cudaStreamSynchronize(st));
-    *end_out = W;
     return HM_OK;
   }
   uint64_t chunk_cap = std::min<uint64_t>(W, kChunkCap);
@@ -828,7 +831,7 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
     out += chunk_total;
     r0 = r1;
   }
-  *written = *end_out = out;
+  *written = out;
   return HM_OK;
 }
 
@@ -847,9 +850,9 @@ int build_h2h_rows(hm_graph* g) {
     *base = 0;
     return HM_OK;
   };
-  uint64_t written = 0, end = 0;
-  HM_TRY(h2h_rows_for(g, nullptr, E, reserve, &written, &end));
-  g->h2h_tail = end;
+  uint64_t written = 0;
+  HM_TRY(h2h_rows_for(g, nullptr, E, reserve, &written));
+  g->h2h_tail = written;
   g->h2h_nnz = written;
   return HM_OK;
 }

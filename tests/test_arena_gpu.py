@@ -194,3 +194,18 @@ def test_growth_of_a_pooled_arena_fails_whole():
             step += 1
         assert failed > 20 and got == want
         assert run(-1) == want
+
+
+@pytest.mark.parametrize("members", [3, 12])
+def test_built_rows_leave_no_holes(ctx, members):
+    """Bitmap rows lie one after another, so what the wedge bound reserves past
+    them is free for a first batch (of rows taken by warps, and by blocks)."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(16)
+    n, n_nodes = 1200, 40  # most pairs share members: far more wedges than entries
+    off, mem = csr([sorted(rng.choice(n_nodes, size=members, replace=False).tolist()) for _ in range(n)])
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        r = g.routes()
+        assert r.rows_bitmap and r.arena_tail == r.arena_entries == g.info().n_adjacent
+        assert r.arena_capacity > r.arena_tail
