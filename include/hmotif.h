@@ -148,7 +148,8 @@ int hm_debug_touch_orientation(hm_graph* g, int by_id);
  * of pairs sharing one member in closed form and enumerates only those with two
  * or three pairs sharing more, where that is the cheaper way, else walks
  * oriented rows grouped by the member each neighbour shares with the row owner;
- * 0 visits every oriented entry. Counts are the same every way; tests run them. */
+ * 0 visits every oriented entry; 2 takes the closed forms whatever they cost, for
+ * touched-triple counts too. Counts are the same every way; tests run them. */
 int hm_debug_static_groups(hm_graph* g, int on);
 /* Which ways the last counts of graph g took (diagnostics; fields of counts not
  * made yet are 0). The shapes are the launch shapes of the enumeration of

@@ -367,8 +367,9 @@ extern "C" int hm_graph_temporal_traffic(const hm_graph* g, hm_temporal_traffic_
 extern "C" int hm_debug_static_groups(hm_graph* g, int on) {
   if (!g) return hm::set_error(HM_ERR_INVALID, "hm_debug_static_groups: NULL graph");
   CtxLock lock(g->ctx);
+  if (!on || (on == 2) != g->force_decomp) hm::release_plus_groups(g);
   g->use_groups = on != 0;
-  if (!g->use_groups) hm::release_plus_groups(g);
+  g->force_decomp = on == 2;
   return HM_OK;
 }
 

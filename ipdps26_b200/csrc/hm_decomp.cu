@@ -86,11 +86,13 @@ __device__ __forceinline__ uint32_t pair_index(uint32_t ua, uint32_t ub, uint32_
 
 // Per slot: degree (sort key), heavy neighbours; sums: [0] h^2, [1] d^2,
 // [2] node pairs of all hyperedges, [3] heavy entries, [4] node pairs of the
-// marked hyperedges.
+// marked hyperedges, [5] node triples of all hyperedges, [6] d^3 / n of those of
+// more than 64 members.
+constexpr unsigned kSums = 7;
 __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint8_t* ovl, const uint8_t* esize,
                               const uint8_t* mark, uint32_t n, uint32_t* heavy, uint32_t* ids,
                               unsigned long long* sums) {
-  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0;
+  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0, t3 = 0, d3 = 0;
   for (uint64_t a = global_warp(); a < n; a += n_warps()) {
     const uint64_t s = off[a];
     const uint32_t l = len[a];
@@ -105,6 +107,8 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
       d2 += (unsigned long long)l * l;
       np += z * (z - (z > 0)) / 2;
       if (mark && mark[a]) mp += z * (z - (z > 0)) / 2;
+      if (z >= 3) t3 += z * (z - 1) * (z - 2) / 6;
+      if (z > 64) d3 += (unsigned long long)l * l / n * l;
       hs += c;
     }
   }
@@ -114,6 +118,8 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
     if (np) atomicAdd(&sums[2], np);
     if (hs) atomicAdd(&sums[3], hs);
     if (mp) atomicAdd(&sums[4], mp);
+    if (t3) atomicAdd(&sums[5], t3);
+    if (d3) atomicAdd(&sums[6], d3);
   }
 }
 
@@ -190,16 +196,24 @@ __global__ void k_heavy_rows(const uint64_t* key, const uint32_t* pos, uint64_t 
 // ---- preparation: node graph --------------------------------------------------------
 
 // Hyperedges of each node by size category (3 per node); with marks, the
-// marked ones alone into ncat_m too.
+// marked ones alone into ncat_m too. classes: per kClass-th of an octave of the
+// nodes' other members (hyperedge by hyperedge), the sums of about D and D^2, D
+// the distinct ones among `even` nodes.
+constexpr unsigned kClass = 4, kClasses = 33 * kClass;
 __global__ void k_node_cats(const uint64_t* voff, const uint32_t* vlen, const uint32_t* vedge, const uint8_t* esize,
-                            const uint8_t* mark, uint32_t n_nodes, uint32_t* ncat, uint32_t* ncat_m) {
+                            const uint8_t* mark, uint32_t n_nodes, float even, uint32_t* ncat, uint32_t* ncat_m, float* classes) {
+  __shared__ float cls[2 * kClasses];
+  for (unsigned k = threadIdx.x; k < 2 * kClasses; k += blockDim.x) cls[k] = 0;
+  __syncthreads();
   for (uint64_t v = global_warp(); v < n_nodes; v += n_warps()) {
     const uint64_t s = voff[v];
     const uint32_t l = vlen[v];
     uint32_t c[6] = {0, 0, 0, 0, 0, 0};
+    uint32_t others = 0;  // at most 254 of at most 2^24 hyperedges
     for (uint32_t i = lane_id(); i < l; i += kWarp) {
       const uint32_t e = vedge[s + i], z = esize[e];
       const bool m = mark && mark[e];
+      others += z - 1;
       c[0] += z == 1;
       c[1] += z == 2;
       c[2] += z >= 3;
@@ -213,7 +227,33 @@ __global__ void k_node_cats(const uint64_t* voff, const uint32_t* vlen, const ui
       if (lane_id() == 0 && k < 3) ncat[3 * v + k] = c[k];
       if (lane_id() == 0 && k >= 3 && mark) ncat_m[3 * v + k - 3] = c[k];
     }
+    for (int d = 16; d; d >>= 1) others += __shfl_xor_sync(0xffffffffu, others, d);
+    if (lane_id() == 0 && others) {
+      const float x = (float)others, distinct = even * (1.0f - expf(-x / even));
+      const unsigned k = (unsigned)(log2f(x) * kClass);
+      atomicAdd(&cls[2 * k], distinct);
+      atomicAdd(&cls[2 * k + 1], distinct * distinct);
+    }
   }
+  __syncthreads();
+  for (unsigned k = threadIdx.x; k < 2 * kClasses; k += blockDim.x)
+    if (cls[k] != 0) atomicAdd(&classes[k], cls[k]);
+}
+
+// About the entries walked for the node triangles: a node of D neighbours, a share
+// s of all neighbourhoods that of nodes of higher degree, is a neighbour in (1 - s)
+// D rows and has s D entries in its own. Within 4 % of the walk on 19 graphs of
+// even degrees, a fifth to a half of it on those with hubs.
+double node_walk(const float* classes) {
+  double total = 0, above = 0, walk = 0;
+  for (unsigned k = 0; k < kClasses; ++k) total += classes[2 * k];
+  for (unsigned k = kClasses; k-- > 0;) {
+    const double own = classes[2 * k], s = total > 0 ? (above + own / 2) / total : 0;
+    // within a class the shares run through own / total
+    walk += (double)classes[2 * k + 1] * (s * (1 - s) - (total > 0 ? own * own / (total * total) / 12 : 0));
+    above += own;
+  }
+  return walk;
 }
 
 // Node-pair table: open addressing over 16-byte entries {x, y, W2, W3},
@@ -440,7 +480,8 @@ __global__ void k_hh_codes(const uint32_t* slot, const uint32_t* rank, uint32_t 
 // 4096-slot tables, 3 the largest table, or the global pair table past it.
 constexpr uint32_t kNodeWarpRow = 128, kNodeWarpWork = 2048, kNodeSmall = 768, kNodeMid = 3072, kNodeLarge = 12288;
 __global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const uint32_t* nbr, uint32_t n,
-                             uint8_t* code, uint32_t* hist) {
+                             uint8_t* code, uint32_t* hist, unsigned long long* total) {
+  unsigned long long all = 0;  // entries the node triangles walk
   for (uint64_t u = global_warp(); u < n; u += n_warps()) {
     const uint32_t d = plen[u];
     uint8_t c = 255;
@@ -448,6 +489,7 @@ __global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const u
       uint64_t work = 0;
       for (uint32_t i = lane_id(); i < d; i += kWarp) work += plen[nbr[poff[u] + i]];
       work = warp_sum(work);
+      all += work;
       if (work)
         c = bucket_code(d <= kNodeWarpRow && work <= kNodeWarpWork ? 0u : d <= kNodeSmall ? 1u : d <= kNodeMid ? 2u : 3u,
                         work);
@@ -457,6 +499,7 @@ __global__ void k_node_codes(const uint64_t* poff, const uint32_t* plen, const u
       if (c != 255) atomicAdd(&hist[c], 1u);
     }
   }
+  if (lane_id() == 0 && all) atomicAdd(total, all);
 }
 
 // ---- counting: nodes, open pairs ------------------------------------------------------
@@ -1931,9 +1974,23 @@ static int decomp_attrs() {
 // Whether the decomposition is the cheaper count, and its structures if so.
 // It enumerates sum h^2 / 2 tests; the oriented rows hold about a quarter of
 // sum d^2 / 2 entries to probe (measured 0.24 to 0.30 on the named laws), and
-// a test costs about as much as a probe, so the line is sum h^2 = sum d^2 / 4.
-// With mark (per slot) the structures of a touched-triple count.
-static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
+// a test costs about as much as a probe, so it needs sum h^2 <= sum d^2 / 4. Then
+// the node graph has to be worth it: W entries walked for its triangles and P
+// node pairs, against what the other count does besides probing. In units of
+// 1.2 ns / 1000 of a full GPU, with nnz = sum d and B = sum d^3 / n over the
+// hyperedges of more than 64 members (their triangles are merged, not masked):
+//   static   4 h^2 + 8 W + 50 P            against   d^2 + 200 nnz + 300 B
+//   touched  h^2 min(1, 3 m / n) + 8 W + 250 P                5/2 c
+// (m marked of n, c the entries of their walk; P costs it a table that a static
+// count keeps). Of 27 graphs and 81 marked sets timed both ways the sums name the
+// faster one but for those within a third of each other. Decomposed / enumerated,
+// ms: 8K hub hyperedges 13.7 / 146, 100K of 4 to 8 members over 200K nodes 0.31 /
+// 0.56, 20K of 20 to 40 over 20K nodes 25.4 / 18.6, 20K of 60 to 100 over 2M nodes
+// 23.5 / 1.2 (and 54 / 0.7 to prepare). Before the table is built W is taken from
+// node_walk, or 3/2 of the hyperedges' own node triples (the least measured).
+// With mark (per slot) the structures of a touched-triple count of `marked`
+// hyperedges and walk cost `cost`.
+static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t marked = 0, uint64_t cost = 0) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
   const uint32_t E = g->n_slots, V = g->n_nodes;
@@ -1946,11 +2003,20 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   HM_TRY(ids.alloc(ctx, E));
   HM_TRY(deg.alloc(ctx, E));
   HM_TRY(hcnt.alloc(ctx, E));
-  HM_TRY(sums.alloc(ctx, 5));
+  HM_TRY(sums.alloc(ctx, kSums + kClasses));  // and the nodes' classes
   HM_TRY(P.rank.alloc(ctx, E));
   HM_TRY(P.slot.alloc(ctx, E));
   HM_TRY(P.hoff.alloc(ctx, (size_t)E + 1));
-  HM_CUDA(cudaMemsetAsync(sums.p, 0, 5 * sizeof(unsigned long long), st));
+  HM_TRY(P.ncat.alloc(ctx, 3 * (size_t)V));
+  if (mark) HM_TRY(P.ncat_m.alloc(ctx, 3 * (size_t)V));
+  HM_CUDA(cudaMemsetAsync(sums.p, 0, (kSums + kClasses) * sizeof(unsigned long long), st));
+  // as many nodes of one degree would give the adjacency there is
+  const double mem = (double)g->h2v_nnz;
+  const float even = (float)std::max(1.0, std::min((double)V, mem * mem / ((double)g->h2h_nnz + mem + 1.0)));
+  k_node_cats<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p,
+                                                                    g->esize.p, mark, V, even, P.ncat.p, P.ncat_m.p,
+                                                                    reinterpret_cast<float*>(sums.p + kSums));
+  HM_LAUNCH_CHECK();
   k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_ovl.p,
                                                                       g->esize.p, mark, E, heavy.p, ids.p, sums.p);
   HM_LAUNCH_CHECK();
@@ -1967,9 +2033,11 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   k_rank_scatter<<<grid_for(E, kBlock), kBlock, 0, st>>>(P.slot.p, E, heavy.p, P.rank.p, hcnt.p);
   HM_LAUNCH_CHECK();
   HM_TRY(exclusive_scan(ctx, hcnt.p, P.hoff.p, E));
-  unsigned long long hs[5];
+  unsigned long long hs[kSums + kClasses];
   HM_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
+  float hc[2 * kClasses];
+  std::memcpy(hc, hs + kSums, sizeof(hc));
   const uint64_t h2 = hs[0], d2 = hs[1], pairs = hs[2], nh = hs[3];
   uint64_t tslots = 1024;
   while (tslots < 2 * pairs) tslots <<= 1;
@@ -1978,7 +2046,14 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   const size_t need = tslots * (sizeof(uint4) + (mark ? sizeof(uint2) : 0)) + (mark ? cslots * sizeof(uint4) : 0) + pairs * (mark ? 60 : 36) +
                       nh * (22 + 24 + (mark ? 18 : 0));
   const size_t room = ctx->budget ? ctx->budget - std::min<size_t>(ctx->budget, ctx->used.load()) : SIZE_MAX;
-  if (h2 > d2 / 4 || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
+  auto worth = [&](double walk) {
+    if (g->force_decomp) return true;
+    if (h2 > d2 / 4) return false;
+    const double own = mark ? (double)h2 * std::min(1.0, 3.0 * marked / E) : 4.0 * (double)h2;
+    const double other = mark ? 2.5 * (double)cost : (double)d2 + 200.0 * (double)g->h2h_nnz + 300.0 * (double)hs[6];
+    return own + 8.0 * walk + (mark ? 250.0 : 50.0) * (double)pairs <= other;
+  };
+  if (!worth(std::max(1.5 * (double)hs[5], node_walk(hc))) || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
     P.release();
     P.decided = true;
     return HM_OK;
@@ -2035,7 +2110,6 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
       k_marked_next<<<grid_for(nh, kBlock), kBlock, 0, st>>>(P.hown.p, P.hnbr.p, nh, P.moff.p, P.mnbr.p, P.mnext.p);
       HM_LAUNCH_CHECK();
     }
-    HM_TRY(P.ncat_m.alloc(ctx, 3 * (size_t)V));
     HM_TRY(P.tab_m.alloc(ctx, tslots));
     HM_TRY(P.nw_m.alloc(ctx, pairs));
     HM_CUDA(cudaMemsetAsync(P.tab_m.p, 0, sizeof(uint2) * tslots, st));
@@ -2045,7 +2119,6 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   }
   // node graph
   P.tslots = tslots;
-  HM_TRY(P.ncat.alloc(ctx, 3 * (size_t)V));
   HM_TRY(P.tab.alloc(ctx, tslots));
   HM_TRY(P.noff.alloc(ctx, (size_t)V + 1));
   HM_TRY(P.nlen.alloc(ctx, V));
@@ -2060,16 +2133,15 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
   DArr<uint8_t> hcode, ncode;
   constexpr uint32_t kBk = 2 * kBuckets + 4;
   HM_TRY(ndeg.alloc(ctx, 2 * (size_t)V));
-  HM_TRY(bk.alloc(ctx, 2 * kBk + 1));  // and the number of spreading owners
+  // and the number of spreading owners, nothing, the node triangles' walk (8 bytes)
+  constexpr uint32_t kBkAll = 2 * kBk + 4;
+  HM_TRY(bk.alloc(ctx, kBkAll));
   HM_TRY(hcode.alloc(ctx, E));
   HM_TRY(ncode.alloc(ctx, V));
   HM_CUDA(cudaMemsetAsync(P.tab.p, 0, sizeof(uint4) * tslots, st));
   HM_CUDA(cudaMemsetAsync(P.nlen.p, 0, sizeof(uint32_t) * V, st));
   HM_CUDA(cudaMemsetAsync(ndeg.p, 0, sizeof(uint32_t) * 2 * V, st));
-  HM_CUDA(cudaMemsetAsync(bk.p, 0, sizeof(uint32_t) * (2 * kBk + 1), st));
-  k_node_cats<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(g->v2h_off.p, g->v2h_len.p, g->v2h_edge.p,
-                                                                    g->esize.p, mark, V, P.ncat.p, P.ncat_m.p);
-  HM_LAUNCH_CHECK();
+  HM_CUDA(cudaMemsetAsync(bk.p, 0, sizeof(uint32_t) * kBkAll, st));
   const uint32_t tmask = (uint32_t)(tslots - 1);
   k_pair_insert<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2v_off.p, g->h2v_mem.p, g->esize.p, mark,
                                                                       nullptr, E, P.tab.p, P.tab_m.p, tmask);
@@ -2098,7 +2170,8 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
       bk.p + 2 * kBk);
   HM_LAUNCH_CHECK();
   k_node_codes<<<grid_for((uint64_t)V * 32, kBlock), kBlock, 0, st>>>(P.noff.p, P.nlen.p, P.nnbr.p, V, ncode.p,
-                                                                     bk.p + kBk);
+                                                                     bk.p + kBk,
+                                                                     reinterpret_cast<unsigned long long*>(bk.p + 2 * kBk + 2));
   HM_LAUNCH_CHECK();
   for (int l = P.by_entry ? 1 : 0; l < 2; ++l) {
     uint32_t* b = bk.p + l * kBk;
@@ -2109,9 +2182,16 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark) {
                                                             l ? P.nwork.p : P.hwork.p);
     HM_LAUNCH_CHECK();
   }
-  uint32_t ends[2 * kBk + 1];
+  uint32_t ends[kBkAll];
   HM_CUDA(cudaMemcpyAsync(ends, bk.p, sizeof(ends), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
+  unsigned long long walk = 0;
+  std::memcpy(&walk, ends + 2 * kBk + 2, sizeof(walk));
+  if (!worth((double)walk)) {
+    P.release();
+    P.decided = true;
+    return HM_OK;
+  }
   std::memcpy(P.hend, ends + 2 * kBuckets, sizeof(P.hend));
   std::memcpy(P.nend, ends + kBk + 2 * kBuckets, sizeof(P.nend));
   P.n_spread = ends[2 * kBk];
@@ -2260,11 +2340,12 @@ int launch_decomp(hm_graph* g, Launches& L) { return launch_parts<false>(g, g->d
 // pair is unmarked), and only the triangles with two or three heavy pairs that
 // hold a mark enumerated. *done = false (and nothing counted) where the graph
 // does not suit the decomposition or the device has no room for it.
-int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done) {
+int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint32_t marked, uint64_t cost, uint64_t out30[30],
+                          bool* done) {
   *done = false;
   Decomp P;
   DArr<unsigned long long> cnt;
-  int s = build_decomp(g, P, mark);
+  int s = build_decomp(g, P, mark, marked, cost);
   if (s >= 0) s = cnt.alloc(g->ctx, 42);
   if (s == HM_ERR_NOMEM || (s >= 0 && !P.usable)) return HM_OK;
   HM_TRY(s);

@@ -614,6 +614,11 @@ __global__ void k_count_classes(const uint64_t* key, uint32_t n, unsigned int* c
 
 }  // namespace
 
+// From how many entries of k_touch_cost, and how many per adjacency entry, a
+// touched count may go by the decomposition (whose own rule is at build_decomp),
+// ms walked / decomposed: 10K wide hyperedges, 50 marked (10 per entry) 1.8 / 5.3,
+// 200 (48) 5.9 / 6.1, 1,000 (227) 32.6 / 8.5; 50K of them, 200 (18) 15.5 / 20.4, 1,000
+// (82) 39 / 22.7; 4K hub hyperedges, 50 (28) 2.04 / 2.06, 200 (107) 9.4 / 2.4.
 constexpr uint64_t kDecompMin = 1ull << 28, kDecompEntries = 32;
 
 int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const TouchRows& rows, uint64_t* out) {
@@ -665,10 +670,6 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   }
   k_count_classes<<<grid_for(n, kBlock), kBlock, 0, st>>>(skeys.p, n, classes_d);
   HM_LAUNCH_CHECK();
-  // Whether the decomposition is the cheaper count: the walk goes through about
-  // 1e11 of k_touch_cost's entries per second, the decomposition's preparation
-  // and closed forms take what about kDecompEntries of them per adjacency
-  // entry take.
   const bool may_decomp = !rows.gos && !by_id;
   uint64_t cost = 0;
   if (may_decomp) {
@@ -682,9 +683,9 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   HM_CUDA(cudaMemcpyAsync(&nc, pos.p + E, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaMemcpyAsync(hcls, classes_d, sizeof(hcls), cudaMemcpyDeviceToHost, st));
   HM_CUDA(cudaStreamSynchronize(st));
-  if (may_decomp && cost > std::max<uint64_t>(kDecompMin, kDecompEntries * g->h2h_nnz)) {
+  if (may_decomp && (g->force_decomp || cost > std::max<uint64_t>(kDecompMin, kDecompEntries * g->h2h_nnz))) {
     bool done = false;
-    HM_TRY(count_touching_decomp(g, mark.p, out, &done));
+    HM_TRY(count_touching_decomp(g, mark.p, n, cost, out, &done));
     g->routes.touch_decomposed = done;
     if (done) return HM_OK;
   }

@@ -330,6 +330,7 @@ struct hm_graph {
   // in b (0xff when they share several, or when it is past 63 in either).
   bool grp_valid = false;
   bool use_groups = true;  // hm_debug_static_groups: off walks every entry (same counts)
+  bool force_decomp = false;  // and 2 decomposes whatever it costs
   hm::DArr<uint32_t> grp_nbr;
   hm::DArr<uint16_t> grp_os;
   hm::DArr<uint64_t> grp_base;   // per slot: its group table's first entry
@@ -422,7 +423,8 @@ int prepare_decomp(hm_graph* g);
 struct Launches;
 int launch_decomp(hm_graph* g, Launches& L);
 void routes_of(const Decomp& P, uint32_t* by_entry, uint32_t centres[4], uint32_t* spread);
-int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint64_t out30[30], bool* done);
+int count_touching_decomp(hm_graph* g, const uint8_t* mark, uint32_t marked, uint64_t cost, uint64_t out30[30],
+                          bool* done);
 int launch_static(hm_graph* g, uint32_t shard, uint32_t n_shards, uint8_t* edge_flags);
 int finish_static(hm_graph* g, uint64_t out30[30]);
 int count_static30(hm_graph* g, uint32_t shard, uint32_t n_shards, uint64_t out30[30]);

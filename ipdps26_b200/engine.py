@@ -460,9 +460,10 @@ class Graph:
         check(lib.hm_graph_autotune(self._h, int(sample_stride), C.byref(r)), "hm_graph_autotune")
         return r
 
-    def set_static_groups(self, on: bool) -> None:
+    def set_static_groups(self, on: bool | int) -> None:
         """Walk of the static count: grouped rows with the shared-member group
-        counted in bulk (default), or every oriented entry (same counts)."""
+        counted in bulk (default), or every oriented entry, or (2) by closed
+        forms whatever they cost (same counts)."""
         check(lib.hm_debug_static_groups(self._h, int(on)), "hm_debug_static_groups")
 
     def routes(self) -> Routes:

@@ -206,8 +206,8 @@ CORES = {
 @pytest.mark.parametrize("pad", [0, 12_300], ids=["by-rank", "hashed"])
 @pytest.mark.parametrize("seed", range(2))
 def test_heavy_core_runs_its_kernels(ctx, name, pad, seed):
-    """The edges of the table kernels, on graphs the decomposition takes: the
-    launch shapes named above are the ones that ran."""
+    """The edges of the table kernels: the launch shapes named above are the ones
+    that ran."""
     from ipdps26_b200 import engine
 
     *law, shapes = CORES[name]
@@ -215,6 +215,7 @@ def test_heavy_core_runs_its_kernels(ctx, name, pad, seed):
     rows, n_all = _core(np.random.default_rng(50 + seed), n, n_nodes, sizes, hubs, n_hubs, light, pad)
     off, mem = csr(rows)
     with engine.Graph(ctx, off, mem, n_all) as g:
+        g.set_static_groups(2)  # whatever its node graph costs
         got = g.count_static30()
         r = g.routes()
         assert r.static_decomposed and not r.static_by_entry
@@ -235,6 +236,7 @@ def test_large_centres_searched_by_entry(ctx, seed):
     rows, n_all = _core(np.random.default_rng(70 + seed), 40, 900, [65, 66, 101, 180, 255], 3, 20, 300, 0)
     off, mem = csr(rows)
     with engine.Graph(ctx, off, mem, n_all) as g:
+        g.set_static_groups(2)
         got = g.count_static30()
         assert g.routes().static_decomposed and g.routes().static_by_entry
         assert got.tolist() == oracle.static30(off, mem, n_all).tolist()
@@ -254,6 +256,7 @@ def test_touched_triples_of_a_heavy_core(ctx, name, pad):
     off, mem = csr(rows)
     rest_off, rest_mem = csr([r for k, r in enumerate(rows) if k not in set(ids.tolist())])
     with engine.Graph(ctx, off, mem, n_all) as g:
+        g.set_static_groups(2)
         got = g.count_touching30(ids)
         r = g.routes()
         assert r.touch_decomposed and not r.touch_by_entry
@@ -277,3 +280,46 @@ def test_rows_past_the_largest_table(ctx):
         assert r.static_decomposed and r.static_centres[0] and r.static_centres[1] and r.static_centres[3]
         g.set_static_groups(False)
         assert got.tolist() == g.count_static30().tolist()
+
+
+def _uniform(n, lo, hi, n_nodes):
+    rng = np.random.default_rng(n + hi)
+    z = rng.integers(lo, hi + 1, n)
+    off = np.concatenate([[0], np.cumsum(z)]).astype(np.uint64)
+    return off, rng.integers(0, n_nodes, int(off[-1])).astype(np.uint32), n_nodes
+
+
+@pytest.mark.parametrize("law,static,touched", [
+    ((20_000, 60, 100, 2_000_000), False, False),  # large hyperedges, seldom adjacent: refused before the table
+    ((20_000, 20, 40, 20_000), False, False),      # refused by the node graph's own size
+    ((3_000, 30, 60, 3_000), False, False),
+    ((20_000, 8, 16, 10_000), True, True),
+    ((30_000, 3, 6, 3_000), True, True),
+    ((20_000, 2, 4, 1_000_000), False, False),
+    ("hub", True, True),
+], ids=str)
+def test_closed_forms_where_their_node_graph_is_worth_it(ctx, law, static, touched):
+    """The dispatch weighs the node graph's walk against the enumeration, and for
+    touched triples against the walk of the marked rows (half of the graph
+    marked); both ways give the same counts."""
+    from ipdps26_b200 import engine, gen
+
+    if law == "hub":
+        h = gen.static(gen.config1(seed=2, n_nodes=2_000, n_edges=4_000))
+        off, mem, n_nodes = h.offsets, h.members, h.n_nodes
+    else:
+        off, mem, n_nodes = _uniform(*law)
+    n = len(off) - 1
+    ids = np.arange(0, n, 2, dtype=np.uint32)
+    with engine.Graph(ctx, off, mem, n_nodes) as g:
+        got = g.count_static30(), g.count_touching30(ids)
+        r = g.routes()
+        assert (bool(r.static_decomposed), bool(r.touch_decomposed)) == (static, touched)
+        g.set_static_groups(0 if static else 2)
+        if static or law[1] < 40:  # the closed forms of the largest take tens of milliseconds and 3 GB
+            assert g.count_static30().tolist() == got[0].tolist()
+        g.set_static_groups(2)
+        g.set_touch_orientation(touched)
+        if touched or law[1] < 40:
+            assert g.count_touching30(ids).tolist() == got[1].tolist()
+            assert bool(g.routes().touch_decomposed) != touched
