@@ -2053,11 +2053,13 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t ma
     const double other = mark ? 2.5 * (double)cost : (double)d2 + 200.0 * (double)g->h2h_nnz + 300.0 * (double)hs[6];
     return own + 8.0 * walk + (mark ? 250.0 : 50.0) * (double)pairs <= other;
   };
-  if (!worth(std::max(1.5 * (double)hs[5], node_walk(hc))) || nh >= (1ull << 31) || tslots > (1ull << 31) || need > room / 2) {
+  P.need = need;
+  if (!worth(std::max(1.5 * (double)hs[5], node_walk(hc))) || nh >= (1ull << 31) || tslots > (1ull << 31)) {
     P.release();
     P.decided = true;
     return HM_OK;
   }
+  if (need > room / 2) return set_error(HM_ERR_NOMEM, "decomposition: %zu bytes of %zu", need, room);
   P.nh = nh;
   P.by_entry = nh <= kEntriesFew && h2 <= kEntryTests;
   HM_TRY(P.hnbr.alloc(ctx, nh));
@@ -2222,13 +2224,22 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t ma
 }
 
 int prepare_decomp(hm_graph* g) {
-  if (g->decomp.decided) return HM_OK;
-  const int s = build_decomp(g, g->decomp, nullptr);
-  if (s < 0) g->decomp.release();
+  hm_ctx* ctx = g->ctx;
+  Decomp& P = g->decomp;
+  auto others = [&] { return ctx->used.load() - std::min(ctx->used.load(), plus_bytes(g)); };
+  auto room = [&] { return ctx->budget - std::min(ctx->budget, ctx->used.load()); };
+  if (P.decided && !(P.need && others() < P.others && P.need <= room() / 2)) return HM_OK;
+  const int s = build_decomp(g, P, nullptr);
+  const size_t need = P.need;
+  if (s < 0) P.release();
   if (s == HM_ERR_NOMEM) {  // no room for it: the enumeration of all triangles needs less
-    g->decomp.decided = true;
+    P.decided = true;
+    P.need = std::max<size_t>(need, 1);
+    P.others = others();
     return HM_OK;
   }
+  P.need = 0;
+  if (P.usable) release_groups(g);  // a full count walks them no more
   return s;
 }
 

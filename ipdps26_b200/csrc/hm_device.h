@@ -200,6 +200,8 @@ struct CountCapture {
 struct Decomp {
   bool decided = false;  // whether the graph suits it has been looked at
   bool usable = false;   // it does, and everything below is built
+  size_t need = 0;       // bytes it was refused for (0: not for room), and what the rest of the
+  size_t others = 0;     // context held then; looked at again once that is less
   DArr<uint32_t> rank, slot;  // slot -> rank, rank -> slot
   DArr<uint64_t> hoff;        // rank -> its heavy entries
   DArr<uint32_t> hnbr, hown;  // neighbour's rank, owner's rank
@@ -237,6 +239,7 @@ struct Decomp {
   void release() {
     capture.reset();
     decided = usable = false;
+    need = others = 0;
     nh = tslots = cslots = 0;
     for (auto* a : {&rank, &slot, &hnbr, &hown, &hpos, &hnext, &ncat, &nlen, &nnbr, &hwork, &nwork, &slist,
                     &mnbr, &mpos, &mnext, &mcode, &hcode, &ncat_m})
@@ -392,7 +395,9 @@ int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
                  const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written);
 int build_plus(hm_graph* g);
 int build_plus_groups(hm_graph* g);
+void release_groups(hm_graph* g);
 void release_plus_groups(hm_graph* g);
+size_t plus_bytes(const hm_graph* g);  // of the oriented rows and their grouped copy
 void release_plus(hm_graph* g);
 // Oriented rows of a subset of slots (indexed by slot; only listed slots valid).
 struct PlusRows {

@@ -804,8 +804,7 @@ static int prepare_counters(hm_graph* g) {
   return HM_OK;
 }
 
-// Everything the enumeration kernels need that only changes with the graph.
-int prepare_enumeration(hm_graph* g) {
+static int prepare_enumeration_once(hm_graph* g) {
   if (!g->plus_valid) {
     HM_TRY(build_plus(g));
     g->work_valid = false;
@@ -814,12 +813,25 @@ int prepare_enumeration(hm_graph* g) {
     // the grouped rows are a shortcut: without room for them the count walks
     // the oriented rows in full
     const int s = build_plus_groups(g);
-    if (s == HM_ERR_NOMEM) release_plus_groups(g);
-    else HM_TRY(s);
+    if (s == HM_ERR_NOMEM) {
+      release_groups(g);
+      if (g->decomp.usable) return s;
+    } else {
+      HM_TRY(s);
+    }
   }
   if (!g->work_valid && g->n_slots) HM_TRY(closed_worklist(g));
   HM_TRY(prepare_counters(g));
   return prepare_static_attrs();
+}
+
+// Everything the enumeration kernels need that only changes with the graph. A
+// decomposition kept from a full count makes room where it is needed.
+int prepare_enumeration(hm_graph* g) {
+  const int s = prepare_enumeration_once(g);
+  if (s != HM_ERR_NOMEM || !g->decomp.usable) return s;
+  g->decomp.release();
+  return prepare_enumeration_once(g);
 }
 
 // A full count of the graph goes by decomposition where that is the cheaper

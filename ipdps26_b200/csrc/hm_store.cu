@@ -523,12 +523,21 @@ void release_plus(hm_graph* g) {
 // The static count's own structures: the grouped rows and the decomposition.
 void release_plus_groups(hm_graph* g) {
   g->decomp.release();
+  release_groups(g);
+}
+
+void release_groups(hm_graph* g) {
   g->grp_nbr.release();
   g->grp_os.release();
   g->grp_base.release();
   g->grp_tab.release();
   g->grp_opos.release();
   g->grp_valid = false;
+}
+
+size_t plus_bytes(const hm_graph* g) {
+  return g->long_off.bytes() + g->long_mask.bytes() + g->plus_nbr.bytes() + g->plus_os.bytes() + g->grp_nbr.bytes() +
+         g->grp_os.bytes() + g->grp_base.bytes() + g->grp_tab.bytes() + g->grp_opos.bytes();
 }
 
 struct WidenU64 {

@@ -323,3 +323,82 @@ def test_closed_forms_where_their_node_graph_is_worth_it(ctx, law, static, touch
         if touched or law[1] < 40:
             assert g.count_touching30(ids).tolist() == got[1].tolist()
             assert bool(g.routes().touch_decomposed) != touched
+
+
+def test_refused_for_room_is_looked_at_again():
+    """A count without room for the closed forms (7 MB of tables, which may take
+    half of the room) enumerates, and takes them once the context has the room; a
+    batch or a rebuild is not needed."""
+    from ipdps26_b200 import engine, gen
+
+    h, other = (gen.static(gen.params(s, 4_000, 8_000, 2, 25, 2.5, 1.2, 1000.0)) for s in (6, 7))
+    with engine.Context(0) as c:
+        with engine.Graph.from_hypergraph(c, h), engine.Graph.from_hypergraph(c, other):
+            used = c.memory()[0]
+    with engine.Context(0, mem_budget_bytes=used + (11 << 20)) as c:
+        b = engine.Graph.from_hypergraph(c, other)
+        with engine.Graph.from_hypergraph(c, h) as g:
+            want = g.count_static30().tolist()
+            assert not g.routes().static_decomposed
+            assert g.count_static30().tolist() == want
+            assert not g.routes().static_decomposed
+            b.close()
+            assert g.count_static30().tolist() == want
+            assert g.routes().static_decomposed
+
+
+def test_closed_forms_take_the_grouped_rows_place(ctx):
+    """After tuning (which walks the grouped rows) a full count by closed forms
+    gives the grouped rows' memory back."""
+    from ipdps26_b200 import engine, gen
+
+    h = gen.static(gen.config1(seed=8, n_nodes=2_000, n_edges=4_000))
+    used = lambda: ctx.memory()[0]
+    with engine.Graph.from_hypergraph(ctx, h) as g:
+        base = used()
+        g.count_static30()
+        closed = used() - base
+    with engine.Graph.from_hypergraph(ctx, h) as g:
+        base = used()
+        g.autotune()
+        tuned = used() - base
+        g.count_static30()
+        assert g.routes().static_decomposed
+        both = used() - base
+        oriented = 7 * g.info().n_oriented  # bytes of the grouped rows per oriented entry
+        assert both <= tuned + closed - oriented
+        g.count_static30_shard(0, 2)  # walks them again, and keeps the closed forms
+        assert used() - base >= both + oriented
+        g.count_static30()
+        assert used() - base >= both + oriented
+
+
+def test_sharded_counts_have_the_room_they_had():
+    """Budgets that hold a store and its oriented rows: sharded counts succeed
+    after a full count wherever they do before one."""
+    from ipdps26_b200 import engine, gen
+    from ipdps26_b200._lib import HM_ERR_NOMEM, HmError
+
+    h = gen.static(gen.config1(seed=9, n_nodes=3_000, n_edges=6_000))
+
+    def run(budget, full):
+        with engine.Context(0, mem_budget_bytes=budget) as c:
+            try:
+                with engine.Graph.from_hypergraph(c, h) as g:
+                    if full:
+                        g.count_static30()
+                    return (g.count_static30_shard(0, 2) + g.count_static30_shard(1, 2)).tolist()
+            except HmError as e:
+                assert e.status == HM_ERR_NOMEM, str(e)
+                return None
+
+    with engine.Context(0) as c:
+        with engine.Graph.from_hypergraph(c, h) as g:
+            store, want = c.memory()[0], g.count_static30().tolist()
+    seen = 0
+    for mb in range(0, 400, 10):
+        first, after = run(store + (mb << 20), False), run(store + (mb << 20), True)
+        assert first in (None, want) and after in (None, want)
+        assert first is None or after is not None, mb
+        seen += first is not None
+    assert seen
