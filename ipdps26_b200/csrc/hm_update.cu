@@ -569,9 +569,11 @@ static int compact_h2h(hm_graph* g, uint64_t extra) {
   // request (later batches compact more often).
   // A small store keeps four times its live size free, up to kSmallSlack
   // entries (64 MB): its batches each rewrite most rows, and a compaction costs
-  // it as much as the patching itself.
+  // it as much as the patching itself. Only while the context holds less than an
+  // eighth of its budget: many such stores in a context leave room for more.
   constexpr uint64_t kSmallSlack = (64ull << 20) / 13;
-  uint64_t slack = std::max(live / 2, std::min(4 * live, kSmallSlack));
+  const bool roomy = !ctx->budget || ctx->used.load() < ctx->budget / 8;
+  uint64_t slack = std::max(live / 2, roomy ? std::min(4 * live, kSmallSlack) : 0);
   if (ctx->budget) slack = std::min<uint64_t>(slack, ctx->budget / 10 / 13);
   if (live + std::max<uint64_t>(extra, slack) <= g->h2h_cap) return HM_OK;
   const uint64_t lean = live + extra + (live + extra) / 32 + 1024;

@@ -209,3 +209,29 @@ def test_built_rows_leave_no_holes(ctx, members):
         r = g.routes()
         assert r.rows_bitmap and r.arena_tail == r.arena_entries == g.info().n_adjacent
         assert r.arena_capacity > r.arena_tail
+
+
+def test_small_arenas_stay_lean_in_a_full_context():
+    """A small store's arena keeps several times its rows free while the context
+    has plenty of room, and half of them once it does not, so that a context
+    holds as many updated stores as fit by their rows."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(17)
+    n_nodes = 64
+    off, mem = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(1500)])
+    io, im = csr([sorted(rng.choice(n_nodes, size=4, replace=False).tolist()) for _ in range(500)])
+    granules = 3 * (2 << 20) / 13  # of the three arrays
+    graphs, free = [], []
+    with engine.Context(0, mem_budget_bytes=800 << 20) as c:
+        for _ in range(14):
+            g = engine.Graph(c, off, mem, n_nodes)
+            g.apply_batch([], io, im)
+            graphs.append(g)
+            r = g.routes()
+            free.append((r.arena_capacity - 1.5 * r.arena_entries, c.memory()[0] > 150 << 20))
+        assert free[0][0] > r.arena_entries and not free[0][1]
+        lean = [f for f, full in free if full]
+        assert len(lean) > 4 and max(lean) <= granules, free
+        for g in graphs:
+            g.close()
