@@ -171,6 +171,7 @@ typedef struct hm_routes {
   uint32_t touch_spread;
   uint32_t temporal_pairs;    /* last synchronous temporal count: events counted by pairs of window events, */
   uint32_t temporal_sets;     /* by pairs of node-sets */
+  uint32_t temporal_top;      /* the node in most events, first to get a signature bit */
 } hm_routes;
 int hm_debug_routes(hm_graph* g, hm_routes* out);
 

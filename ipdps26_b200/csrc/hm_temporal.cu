@@ -1078,15 +1078,18 @@ static int build_temporal_index(hm_graph* g) {
   if (V) {
     k_iota<<<grid_for(V, kBlock), kBlock, 0, st>>>(vid.p, V);
     HM_LAUNCH_CHECK();
+    int lb = 1;  // a node may be in all n events
+    while (lb < 32 && (1ull << lb) <= n) ++lb;
     size_t tb = 0;
     HM_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, g->t_vlen.p, vlen_s.p, vid.p, vid_s.p, (int64_t)V, 0,
-                                                      eb, st));
+                                                      lb, st));
     DArr<uint8_t> tmp;
     HM_TRY(tmp.alloc(ctx, tb));
     HM_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.p, tb, g->t_vlen.p, vlen_s.p, vid.p, vid_s.p, (int64_t)V, 0,
-                                                      eb, st));
+                                                      lb, st));
     k_set_top<<<1, 64, 0, st>>>(vid_s.p, std::min<uint32_t>(V, 64), g->t_top.p);
     HM_LAUNCH_CHECK();
+    HM_CUDA(cudaMemcpyAsync(&g->routes.temporal_top, vid_s.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   }
   HM_TRY(g->t_exact.alloc(ctx, n));
   HM_TRY(g->t_other.alloc(ctx, n));

@@ -76,6 +76,7 @@ class Routes(C.Structure):
         ("touch_spread", C.c_uint32),
         ("temporal_pairs", C.c_uint32),
         ("temporal_sets", C.c_uint32),
+        ("temporal_top", C.c_uint32),
     ]
 
 

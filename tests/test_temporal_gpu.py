@@ -208,3 +208,18 @@ def test_temporal_by_pairs_or_by_node_sets(ctx, window, law):
     elif window >= 700:  # at 513 both take about as long
         assert r.temporal_sets == n - 1 - 512
     assert got.tolist() == oracle.temporal96(off, mem, times, window).tolist()
+
+
+@pytest.mark.parametrize("n", [255, 256, 257])
+def test_node_in_every_event_has_a_signature_bit(ctx, n):
+    """The sort that picks the 64 nodes in most events compares counts up to the
+    number of events itself."""
+    from ipdps26_b200 import engine
+
+    rng = np.random.default_rng(n)
+    rows = [[7] + rng.choice(np.arange(8, 200), size=2, replace=False).tolist() for _ in range(n)]
+    off, mem = csr(rows)
+    times = np.arange(n, dtype=np.int64)
+    with engine.Graph(ctx, off, mem, 200, times) as g:
+        assert g.count_temporal(20).tolist() == oracle.temporal96(off, mem, times, 20).tolist()
+        assert g.routes().temporal_top == 7
