@@ -270,12 +270,6 @@ __global__ void k_window_lo(const int64_t* t, const uint32_t* size, uint32_t n, 
       if (w)
         shape = size[p] - 1u >= kPairMembers || w > kPairCap2 ? 3 : w > kPairCap1 ? 2 : w > cap0 ? 1 : 0;
     }
-    const unsigned big = __ballot_sync(0xffffffffu, shape == 2);
-    if (big) {
-      const int src = (int)__fns(big, 0, 1 + (int)((p0 >> 5) % (unsigned)__popc(big)));
-      const uint32_t q = (uint32_t)p0 + (uint32_t)src;
-      add_costs(S, q, __shfl_sync(0xffffffffu, l, src), size[q], n, (float)__popc(big));
-    }
     for (int k = 0; k < 4; ++k) {
       const unsigned m = __ballot_sync(0xffffffffu, shape == k);
       if (!m) continue;
@@ -283,6 +277,13 @@ __global__ void k_window_lo(const int64_t* t, const uint32_t* size, uint32_t n, 
       if (lane_id() == 0) base = atomicAdd(&counts[k], (unsigned)__popc(m));
       base = __shfl_sync(0xffffffffu, base, 0);
       if (shape == k) lists[(uint64_t)k * n + base + __popc(m & ((1u << lane_id()) - 1u))] = (uint32_t)p;
+    }
+    // after the lists: they stay in about the order of the events
+    const unsigned big = __ballot_sync(0xffffffffu, shape == 2);
+    if (big) {
+      const int src = (int)__fns(big, 0, 1 + (int)((p0 >> 5) % (unsigned)__popc(big)));
+      const uint32_t q = (uint32_t)p0 + (uint32_t)src;
+      add_costs(S, q, __shfl_sync(0xffffffffu, l, src), size[q], n, (float)__popc(big));
     }
   }
 }
