@@ -670,7 +670,9 @@ int count_touching_rows(hm_graph* g, const uint32_t* d_ids, uint32_t n, const To
   }
   k_count_classes<<<grid_for(n, kBlock), kBlock, 0, st>>>(skeys.p, n, classes_d);
   HM_LAUNCH_CHECK();
-  const bool may_decomp = !rows.gos && !by_id;
+  // (the cost is at most every entry's row, and no row is longer than the graph)
+  const bool may_decomp =
+      !rows.gos && !by_id && (g->force_decomp || (double)g->h2h_nnz * g->n_live > (double)kDecompMin);
   uint64_t cost = 0;
   if (may_decomp) {
     k_touch_cost<<<grid_for((uint64_t)n * 32, kBlock), kBlock, 0, st>>>(d_ids, n, g->h2h_off.p, g->h2h_len.p,
