@@ -380,6 +380,12 @@ extern "C" int hm_debug_routes(hm_graph* g, hm_routes* out) {
   out->arena_entries = g->h2h_nnz;
   out->arena_tail = g->h2h_tail;
   out->arena_capacity = g->h2h_cap;
+  if (g->t_ready && g->n_nodes) {
+    std::vector<uint8_t> top(g->n_nodes);
+    HM_CUDA(cudaMemcpyAsync(top.data(), g->t_top.p, top.size(), cudaMemcpyDeviceToHost, g->ctx->stream));
+    HM_CUDA(cudaStreamSynchronize(g->ctx->stream));
+    out->temporal_top = (uint32_t)(std::find(top.begin(), top.end(), 0) - top.begin());
+  }
   return HM_OK;
 }
 

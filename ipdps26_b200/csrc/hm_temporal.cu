@@ -158,10 +158,11 @@ __global__ void k_gather_len(const uint32_t* order, uint32_t n, const uint32_t* 
 // event of no members or more than kPairMembers always goes to k_temporal, and
 // shape 2 does in streams that by_sets tells.
 constexpr uint32_t kPairCap0 = 64, kPairCap1 = 512, kPairCap2 = 2048;
-// Streams of fewer events than the GPU holds warps give all but the smallest
-// windows a block: the time is then that of the few events one place takes in
-// turn (2,000 events, windows of about 50: 46 us by warps).
-constexpr uint32_t kFewEvents = 6000, kFewCap0 = 8;
+// Streams of fewer events than the GPU holds warps (of the shape 0 launch) give all
+// but the smallest windows a block: the time is then that of the few events one
+// place takes in turn (2,000 events, windows of about 50: 46 us by warps).
+constexpr unsigned kPairBlock0 = 256, kPairBlocks0 = 5;
+constexpr uint32_t kFewCap0 = 8;
 constexpr uint32_t kPairMembers = 32;
 
 // The longest windows (shape 2) are not always cheaper by pairs of events:
@@ -1090,7 +1091,6 @@ static int build_temporal_index(hm_graph* g) {
                                                       lb, st));
     k_set_top<<<1, 64, 0, st>>>(vid_s.p, std::min<uint32_t>(V, 64), g->t_top.p);
     HM_LAUNCH_CHECK();
-    HM_CUDA(cudaMemcpyAsync(&g->routes.temporal_top, vid_s.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   }
   HM_TRY(g->t_exact.alloc(ctx, n));
   HM_TRY(g->t_other.alloc(ctx, n));
@@ -1158,8 +1158,9 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
   float* cost = reinterpret_cast<float*>(acc.p + 96);
   const SetsArgs sets{g->t_static.p, g->t_prev.p, g->t_degree.p, g->t_order.p, g->h2v_off.p,
                       g->h2v_mem.p,  g->t_voff.p, g->t_vlen.p,   g->t_vpos.p,  cost};
+  const uint32_t places = (uint32_t)ctx->n_sms * kPairBlocks0 * (kPairBlock0 / kWarp);
   k_window_lo<<<grid_for(n, kBlock), kBlock, 0, st>>>(g->t_time.p, g->t_size.p, n, delta,
-                                                      n < kFewEvents ? kFewCap0 : kPairCap0, sets, lo.p, lists, counts);
+                                                      n < places ? kFewCap0 : kPairCap0, sets, lo.p, lists, counts);
   HM_LAUNCH_CHECK();
   TArgs A{n,
           g->t_order.p,
@@ -1211,7 +1212,7 @@ static int launch_temporal(hm_graph* g, int64_t delta, DArr<uint32_t>& lo, DArr<
   };
   HM_TRY((launch_pairs<16, kPairCap2, 512, 2>(ctx, shape(2), n)));
   HM_TRY((launch_pairs<8, kPairCap1, 256, 5>(ctx, shape(1), n)));
-  HM_TRY((launch_pairs<1, kPairCap0, 256, 5>(ctx, shape(0), n)));
+  HM_TRY((launch_pairs<1, kPairCap0, kPairBlock0, kPairBlocks0>(ctx, shape(0), n)));
   if (e1) HM_CUDA(cudaEventRecord(e1, st));
   return HM_OK;
 }
