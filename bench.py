@@ -510,10 +510,15 @@ def engine_arm(args, rank, world, local_rank):
     g = engine.Graph.from_hypergraph(ctx, h)
     stream = torch.cuda.ExternalStream(engine.lib.hm_ctx_stream(ctx.handle))
 
-    # the launch schedule, picked by the autotuner on rank 0 before any timing;
-    # every rank must split the work list the same way for the shards to add up
+    # a full count by closed forms has no launch schedule; otherwise the autotuner
+    # picks it on rank 0 before any timing (every rank must split the work list the
+    # same way for the shards to add up)
     tune = None
-    if not args.no_tune:
+    closed_forms = False
+    if world == 1:
+        g.count_static30()
+        closed_forms = bool(g.routes().static_decomposed)
+    if not args.no_tune and not closed_forms:
         if rank == 0:
             tune = g.autotune(args.tune_stride).as_dict()
         if world > 1:
@@ -544,6 +549,7 @@ def engine_arm(args, rank, world, local_rank):
         e1.record(stream)
         torch.cuda.synchronize()
         closed_tri = int(g.timings().closed_triangles)
+        launches = int(g.routes().static_kernels) * args.steps
         wall = time.perf_counter() - t0
         if world > 1:
             dist.barrier()
@@ -571,26 +577,26 @@ def engine_arm(args, rank, world, local_rank):
                     Path(args.write_traffic).write_text(json.dumps(tr, indent=1))
             # one step = the count kernels; per-launch duration from CUDA events
             t_launch = (statistics.mean(closed_ms) + statistics.mean(open_ms)) / 1000.0
-            achieved = tr["b_static"] / t_launch / 1e9
             traffic = None
             tp = ROOT / "profiles" / "static_count_dram.json"
             if tp.exists():
                 tj = json.loads(tp.read_text())
                 if tj.get("key") == traffic_key(args):
                     traffic = tj.get("dram_bytes_per_step")
-            roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                    "traffic": traffic, "peak_kind": peak_kind,
-                    "traffic_gbs": traffic / t_launch / 1e9 if traffic else None,
-                    "algorithmic_bytes": tr["b_static"], "kernel_model_bytes": tr["kernel_bytes"],
-                    "kernel_model_gbs": tr["kernel_bytes"] / t_launch / 1e9,
+            # the closed forms move what ncu measured; the enumeration what its model says
+            moved = traffic if closed_forms else tr["kernel_bytes"]
+            achieved = moved / t_launch / 1e9 if moved else None
+            roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                    "frac": achieved / hbm if achieved else None, "traffic": traffic, "peak_kind": peak_kind,
+                    "reference_algorithm_bytes": tr["b_static"], "enumeration_model_bytes": tr["kernel_bytes"],
                     "kernel": "the decomposed count's launches (k_hh_large, k_hh_fast, k_self_weights, "
                               "k_spread_pairs, k_node_tri, k_node_tri_warp, k_parts, k_decomp_finish), replayed as "
-                              "one captured CUDA graph: one static count",
-                    "basis": "achieved = algorithmic_bytes (the reference algorithm's merge bytes per count) "
-                             "/ count time; light pairs are counted in closed form and only triangles with two "
-                             "or more heavy pairs visited, so the count moves `traffic` bytes (ncu) and frac "
-                             "passes 1; kernel_model_bytes models the enumeration of all triangles "
-                             "(sharded counts)",
+                              "one CUDA graph: one static count" if closed_forms else
+                              "k_open_pairs and the closed-phase launches, replayed as two CUDA graphs",
+                    "basis": "achieved = DRAM bytes of one count (ncu, `traffic`) / count time; the count is "
+                             "issue-bound integer work, and the bytes of the reference's algorithm "
+                             "(reference_algorithm_bytes) are not moved by it" if closed_forms else
+                             "achieved = bytes of the enumeration's model / count time",
                     "closed_ms": statistics.mean(closed_ms), "open_ms": statistics.mean(open_ms)}
         e2e = None
         if not args.no_e2e:
@@ -603,7 +609,8 @@ def engine_arm(args, rank, world, local_rank):
                 torch.cuda.synchronize()
                 t0 = time.perf_counter()
                 with engine.Graph(ctx, off, mem, h.n_nodes) as g2:
-                    g2.set_schedule(*g.schedule)  # the tuned schedule of this workload
+                    if tune:
+                        g2.set_schedule(*g.schedule)  # the tuned schedule of this workload
                     c26 = g2.count_static()
                 times.append(time.perf_counter() - t0)
             e2e = {"value": int(c26.sum()) / statistics.mean(times), "unit": UNIT,
@@ -617,6 +624,8 @@ def engine_arm(args, rank, world, local_rank):
         mem_gb["before_updates"] = ctx.memory()[0] / 1e9
         print(f"[bench] device memory in use: {mem_gb}", file=sys.stderr, flush=True)
         updates = None
+        if args.update_batches > 0 and not args.no_tune and tune is None:
+            tune = g.autotune(args.tune_stride).as_dict()  # for the batches' touched-triple counts
         if args.update_batches > 0:
             updates = update_section(args, g, p, counts)
         g_sched = g.schedule
@@ -631,10 +640,11 @@ def engine_arm(args, rank, world, local_rank):
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1000 * dev_s / args.steps, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "int64", "data": "synthetic",
-            # per step: the ten kernels of the decomposed count (profiles/static_count_dram.json lists
-            # them); a shard runs k_open_pairs and the three closed-phase launch shapes
-            "config": {**config_of(args, world), "schedule": list(g_sched)},
-            "gpu_launches": (10 if world == 1 else 4) * args.steps,
+            # by closed forms the count has no schedule; the touched-triple counts of the batches do
+            "config": {**config_of(args, world), "count": "closed forms" if closed_forms else "enumeration",
+                       "schedule": None if closed_forms else list(g_sched)},
+            "gpu_launches": launches,  # of this rank, per step as the last count made them
+            "touch_schedule": list(g_sched)[2:],
             "autotune": tune,
             "triples_per_step": triples, "closed_triangles_per_step": closed_tri,
             "closed_triangles_per_s": closed_tri * args.steps / dev_s,
