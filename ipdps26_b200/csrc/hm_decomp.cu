@@ -1646,7 +1646,7 @@ __global__ void __launch_bounds__(kHHThreads, 1) k_hh_large(HHArgs A) {
 // bins per warp, which become weighted records when the warp has walked the
 // rows of all its b alike in |b| and C_ab (of 32 taken together). Fewer than
 // kHistMin tests queue every triangle. The enumeration is issue-bound (86 % of
-// the issue slots with a record per triangle, 31 ms on an 8K-hyperedge hub
+// the issue slots with a record per triangle, 31 ms on a 60K-hyperedge wide
 // graph), so instructions per test are what counts. Graphs of up to kDenseSlots
 // hyperedges index their table by rank and need no hash.
 constexpr uint32_t kHistMin = 96, kHistMax = 1u << 16, kHistBins = 288;

@@ -161,7 +161,7 @@ struct PhaseTimes {
 // Which launch shape of the closed phase takes a centre, by the length d of
 // its oriented row: d <= warp_row one warp each (warp_row <= 128, the warp
 // kernel's 256-slot tables), d <= small_row blocks with 4096-slot tables,
-// longer rows blocks with 8192-slot tables. Counts never depend on it.
+// longer rows 1024-thread blocks with 16384-slot tables. Counts never depend on it.
 struct ClosedSchedule {
   uint32_t warp_row = 128;
   uint32_t small_row = 2048;

@@ -701,12 +701,14 @@ constexpr uint64_t kBitmapLong = 1024;    // wedges per row on average from whic
 // H2H rows of the listed slots (all slots when d_rows is null): by bitmaps, or
 // in chunks of the wedge stream: expand, segmented sort, run-length.
 // reserve(W) is called once with an upper bound on the entries and returns the
-// arena position where the rows are written, one after another; *written
-// receives the entries emitted.
+// arena position where the rows are written, one after another; *written (if
+// not null) receives the entries emitted.
 int h2h_rows_for(hm_graph* g, const uint32_t* d_rows, uint32_t n_rows,
                  const std::function<int(uint64_t, uint64_t*)>& reserve, uint64_t* written) {
   hm_ctx* ctx = g->ctx;
   cudaStream_t st = ctx->stream;
+  uint64_t none = 0;
+  if (!written) written = &none;
   *written = 0;
   if (g->n_slots >= (1u << 24))
     return set_error(HM_ERR_LIMIT, "H2H: %u hyperedge slots exceed the 2^24 limit of the packed sort key", g->n_slots);

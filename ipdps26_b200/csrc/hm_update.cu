@@ -863,10 +863,9 @@ int apply_batch_hooks(hm_graph* g, const uint32_t* h_dels, uint32_t n_del, const
     HM_LAUNCH_CHECK();
     // a deleted id that was reused is rebuilt, not skipped-as-dead: both skip
   }
-  uint64_t written = 0;
   if (n_ins) {
     auto reserve = [&](uint64_t W, uint64_t* base) { return reserve_h2h(g, W, base); };
-    HM_TRY(h2h_rows_for(g, ids.p, n_ins, reserve, &written));
+    HM_TRY(h2h_rows_for(g, ids.p, n_ins, reserve, nullptr));
   }
 
   trace.mark("h2h_inserted_rows");
