@@ -34,6 +34,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -87,31 +88,42 @@ __device__ __forceinline__ uint32_t pair_index(uint32_t ua, uint32_t ub, uint32_
 // Per slot: degree (sort key), heavy neighbours; sums: [0] h^2, [1] d^2,
 // [2] node pairs of all hyperedges, [3] heavy entries, [4] node pairs of the
 // marked hyperedges, [5] node triples of all hyperedges, [6] d^3 / n of those of
-// more than 64 members.
-constexpr unsigned kSums = 7;
-__global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint8_t* ovl, const uint8_t* esize,
-                              const uint8_t* mark, uint32_t n, uint32_t* heavy, uint32_t* ids,
+// more than 64 members, [7] how many those are; largest: [8] |a| |b| of a heavy
+// pair, [9] members.
+constexpr unsigned kSums = 10;
+__global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint32_t* nbr, const uint8_t* ovl,
+                              const uint8_t* esize, const uint8_t* mark, uint32_t n, uint32_t* heavy, uint32_t* ids,
                               unsigned long long* sums) {
-  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0, t3 = 0, d3 = 0;
+  unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0, t3 = 0, d3 = 0, big = 0;
+  uint32_t pair = 0, most = 0;
   for (uint64_t a = global_warp(); a < n; a += n_warps()) {
     const uint64_t s = off[a];
     const uint32_t l = len[a];
+    const unsigned long long z = esize[a];
     uint32_t c = 0;
-    for (uint32_t i = lane_id(); i < l; i += kWarp) c += ovl[s + i] >= 2;
+    for (uint32_t i = lane_id(); i < l; i += kWarp)
+      if (ovl[s + i] >= 2) {
+        ++c;
+        pair = max(pair, (uint32_t)z * esize[nbr[s + i]]);
+      }
     for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
     if (lane_id() == 0) {
       heavy[a] = c;
       ids[a] = (uint32_t)a;
-      const unsigned long long z = esize[a];
+      most = max(most, (uint32_t)z);
       h2 += (unsigned long long)c * c;
       d2 += (unsigned long long)l * l;
       np += z * (z - (z > 0)) / 2;
       if (mark && mark[a]) mp += z * (z - (z > 0)) / 2;
       if (z >= 3) t3 += z * (z - 1) * (z - 2) / 6;
-      if (z > 64) d3 += (unsigned long long)l * l / n * l;
+      if (z > 64) {
+        d3 += (unsigned long long)l * l / n * l;
+        ++big;
+      }
       hs += c;
     }
   }
+  for (int d = 16; d; d >>= 1) pair = max(pair, __shfl_xor_sync(0xffffffffu, pair, d));
   if (lane_id() == 0) {
     if (h2) atomicAdd(&sums[0], h2);
     if (d2) atomicAdd(&sums[1], d2);
@@ -120,6 +132,9 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
     if (mp) atomicAdd(&sums[4], mp);
     if (t3) atomicAdd(&sums[5], t3);
     if (d3) atomicAdd(&sums[6], d3);
+    if (big) atomicAdd(&sums[7], big);
+    if (pair) atomicMax(&sums[8], (unsigned long long)pair);
+    if (most) atomicMax(&sums[9], (unsigned long long)most);
   }
 }
 
@@ -1975,19 +1990,26 @@ static int decomp_attrs() {
 // It enumerates sum h^2 / 2 tests; the oriented rows hold about a quarter of
 // sum d^2 / 2 entries to probe (measured 0.24 to 0.30 on the named laws), and
 // a test costs about as much as a probe, so it needs sum h^2 <= sum d^2 / 4. Then
-// the node graph has to be worth it: W entries walked for its triangles and P
-// node pairs, against what the other count does besides probing. In units of
-// 1.2 ns / 1000 of a full GPU, with nnz = sum d and B = sum d^3 / n over the
-// hyperedges of more than 64 members (their triangles are merged, not masked):
-//   static   4 h^2 + 8 W + 50 P            against   d^2 + 200 nnz + 300 B
-//   touched  h^2 min(1, 3 m / n) + 8 W + 250 P                5/2 c
-// (m marked of n, c the entries of their walk; P costs it a table that a static
-// count keeps). Of 27 graphs and 81 marked sets timed both ways the sums name the
-// faster one but for those within a third of each other. Decomposed / enumerated,
-// ms: 8K hub hyperedges 13.7 / 146, 100K of 4 to 8 members over 200K nodes 0.31 /
-// 0.56, 20K of 20 to 40 over 20K nodes 25.4 / 18.6, 20K of 60 to 100 over 2M nodes
-// 23.5 / 1.2 (and 54 / 0.7 to prepare). Before the table is built W is taken from
-// node_walk, or 3/2 of the hyperedges' own node triples (the least measured).
+// the node graph has to be worth it: W entries walked for its triangles, P node
+// pairs, and the latency of the largest items, which a few warps sum while the rest
+// of the GPU is done: Z members at most, X = |a| |b| of a heavy pair at most, a share
+// L of the GPU's warps with a heavy pair. With nnz = sum d and B = sum d^3 / n over
+// the hyperedges of more than 64 members times their share of all (their triangles
+// are merged, not masked), in ns beside 60 us each:
+//   decomposed  0.0014 h^2 + 0.008 W + 0.06 P + 3.7 Z^2 + 16 X L
+//   enumerated  0.0011 d^2 + 12.6 sqrt(d^2) + 0.048 nnz + 0.3 B
+// and for the touched triples of m of n hyperedges, whose walk goes through c entries
+// (and whose tables are built for one count)
+//   decomposed  0.0014 h^2 min(1, 3 m / n) + 0.01 W + 0.3 P + 3.7 Z^2 + 16 X L
+//   walked      0.003 c.
+// Fitted on 300 graphs timed both ways, of 100 to 50K hyperedges of all laws and
+// sizes: the way the sums name takes 1.4 % more than the better one on average, at
+// most 1.8 times as long. Decomposed / enumerated, ms: 8K hub hyperedges 13.7 /
+// 146, 100K of 4 to 8 members over 200K nodes 0.31 / 0.56, 3,458 hyperedges, a few of
+// them of up to 120 members, 0.66 / 0.10, 20K of 20 to 40 over 20K nodes 25.4 / 18.6,
+// 20K of 60 to 100 over 2M nodes 23.5 / 1.2 (and 54 / 0.7 to prepare). Before the
+// table is built W is taken from node_walk, or 3/2 of the hyperedges' own node
+// triples (the least measured).
 // With mark (per slot) the structures of a touched-triple count of `marked`
 // hyperedges and walk cost `cost`.
 static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t marked = 0, uint64_t cost = 0) {
@@ -2017,8 +2039,8 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t ma
                                                                     g->esize.p, mark, V, even, P.ncat.p, P.ncat_m.p,
                                                                     reinterpret_cast<float*>(sums.p + kSums));
   HM_LAUNCH_CHECK();
-  k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_ovl.p,
-                                                                      g->esize.p, mark, E, heavy.p, ids.p, sums.p);
+  k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
+                                                                      g->h2h_ovl.p, g->esize.p, mark, E, heavy.p, ids.p, sums.p);
   HM_LAUNCH_CHECK();
   const unsigned bits = bits_for(E);
   {
@@ -2049,9 +2071,14 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t ma
   auto worth = [&](double walk) {
     if (g->force_decomp) return true;
     if (h2 > d2 / 4) return false;
-    const double own = mark ? (double)h2 * std::min(1.0, 3.0 * marked / E) : 4.0 * (double)h2;
-    const double other = mark ? 2.5 * (double)cost : (double)d2 + 200.0 * (double)g->h2h_nnz + 300.0 * (double)hs[6];
-    return own + 8.0 * walk + (mark ? 250.0 : 50.0) * (double)pairs <= other;
+    const double lone = std::min(1.0, (double)nh / (ctx->n_sms * 8.0 * kWarps));
+    const double largest = 3.7 * (double)hs[9] * (double)hs[9] + 16.0 * (double)hs[8] * lone;
+    if (mark)
+      return 0.0014 * (double)h2 * std::min(1.0, 3.0 * marked / E) + 0.01 * walk + 0.3 * (double)pairs + largest <=
+             0.003 * (double)cost;
+    return 0.0014 * (double)h2 + 0.008 * walk + 0.06 * (double)pairs + largest <=
+           0.0011 * (double)d2 + 12.6 * std::sqrt((double)d2) + 0.048 * (double)g->h2h_nnz +
+               0.3 * (double)hs[6] * (double)hs[7] / E;
   };
   P.need = need;
   if (!worth(std::max(1.5 * (double)hs[5], node_walk(hc))) || nh >= (1ull << 31) || tslots > (1ull << 31)) {
