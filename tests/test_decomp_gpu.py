@@ -297,6 +297,7 @@ def _uniform(n, lo, hi, n_nodes):
     ((30_000, 3, 6, 3_000), True, True),
     ((20_000, 2, 4, 1_000_000), False, False),
     ("hub", True, True),
+    ("large", False, False),                       # a hyperedge of 120 members, alone on a warp for most of the count
 ], ids=str)
 def test_closed_forms_where_their_node_graph_is_worth_it(ctx, law, static, touched):
     """The dispatch weighs the node graph's walk against the enumeration, and for
@@ -307,6 +308,9 @@ def test_closed_forms_where_their_node_graph_is_worth_it(ctx, law, static, touch
     if law == "hub":
         h = gen.static(gen.config1(seed=2, n_nodes=2_000, n_edges=4_000))
         off, mem, n_nodes = h.offsets, h.members, h.n_nodes
+    elif law == "large":
+        h = gen.static(gen.params(50_140, 6_214, 3_458, 1, 200, 2.543, 0.988, 50.0, dedupe=True))
+        off, mem, n_nodes = h.offsets, h.members, h.n_nodes
     else:
         off, mem, n_nodes = _uniform(*law)
     n = len(off) - 1
@@ -316,11 +320,11 @@ def test_closed_forms_where_their_node_graph_is_worth_it(ctx, law, static, touch
         r = g.routes()
         assert (bool(r.static_decomposed), bool(r.touch_decomposed)) == (static, touched)
         g.set_static_groups(0 if static else 2)
-        if static or law[1] < 40:  # the closed forms of the largest take tens of milliseconds and 3 GB
+        if static or law == "large" or law[1] < 40:  # the closed forms of the largest take tens of milliseconds and 3 GB
             assert g.count_static30().tolist() == got[0].tolist()
         g.set_static_groups(2)
         g.set_touch_orientation(touched)
-        if touched or law[1] < 40:
+        if touched or law == "large" or law[1] < 40:
             assert g.count_touching30(ids).tolist() == got[1].tolist()
             assert bool(g.routes().touch_decomposed) != touched
 
