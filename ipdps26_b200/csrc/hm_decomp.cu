@@ -89,11 +89,17 @@ __device__ __forceinline__ uint32_t pair_index(uint32_t ua, uint32_t ub, uint32_
 // [2] node pairs of all hyperedges, [3] heavy entries, [4] node pairs of the
 // marked hyperedges, [5] node triples of all hyperedges, [6] d^3 / n of those of
 // more than 64 members, [7] how many those are; largest: [8] |a| |b| of a heavy
-// pair, [9] members.
+// pair, [9] members. A pair's larger hyperedge looks for [8], and only where it can
+// be above large_pair: rows of nbr that are not needed are not read (50K wide-law
+// hyperedges, batches of 4K: 2 % of the time). All blocks add to the same words, so a
+// block adds its warps' sums up first.
 constexpr unsigned kSums = 10;
 __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const uint32_t* nbr, const uint8_t* ovl,
-                              const uint8_t* esize, const uint8_t* mark, uint32_t n, uint32_t* heavy, uint32_t* ids,
-                              unsigned long long* sums) {
+                              const uint8_t* esize, const uint8_t* mark, uint32_t n, uint32_t large_pair,
+                              uint32_t* heavy, uint32_t* ids, unsigned long long* sums) {
+  __shared__ unsigned long long all[kSums];
+  if (threadIdx.x < kSums) all[threadIdx.x] = 0;
+  __syncthreads();
   unsigned long long h2 = 0, d2 = 0, np = 0, hs = 0, mp = 0, t3 = 0, d3 = 0, big = 0;
   uint32_t pair = 0, most = 0;
   for (uint64_t a = global_warp(); a < n; a += n_warps()) {
@@ -101,11 +107,15 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
     const uint32_t l = len[a];
     const unsigned long long z = esize[a];
     uint32_t c = 0;
-    for (uint32_t i = lane_id(); i < l; i += kWarp)
-      if (ovl[s + i] >= 2) {
-        ++c;
-        pair = max(pair, (uint32_t)z * esize[nbr[s + i]]);
-      }
+    if (z * z > max(large_pair, pair) && z * z > *(volatile unsigned long long*)&sums[8]) {
+      for (uint32_t i = lane_id(); i < l; i += kWarp)
+        if (ovl[s + i] >= 2) {
+          ++c;
+          pair = max(pair, (uint32_t)z * esize[nbr[s + i]]);
+        }
+    } else {
+      for (uint32_t i = lane_id(); i < l; i += kWarp) c += ovl[s + i] >= 2;
+    }
     for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
     if (lane_id() == 0) {
       heavy[a] = c;
@@ -125,16 +135,21 @@ __global__ void k_heavy_count(const uint64_t* off, const uint32_t* len, const ui
   }
   for (int d = 16; d; d >>= 1) pair = max(pair, __shfl_xor_sync(0xffffffffu, pair, d));
   if (lane_id() == 0) {
-    if (h2) atomicAdd(&sums[0], h2);
-    if (d2) atomicAdd(&sums[1], d2);
-    if (np) atomicAdd(&sums[2], np);
-    if (hs) atomicAdd(&sums[3], hs);
-    if (mp) atomicAdd(&sums[4], mp);
-    if (t3) atomicAdd(&sums[5], t3);
-    if (d3) atomicAdd(&sums[6], d3);
-    if (big) atomicAdd(&sums[7], big);
-    if (pair) atomicMax(&sums[8], (unsigned long long)pair);
-    if (most) atomicMax(&sums[9], (unsigned long long)most);
+    if (h2) atomicAdd(&all[0], h2);
+    if (d2) atomicAdd(&all[1], d2);
+    if (np) atomicAdd(&all[2], np);
+    if (hs) atomicAdd(&all[3], hs);
+    if (mp) atomicAdd(&all[4], mp);
+    if (t3) atomicAdd(&all[5], t3);
+    if (d3) atomicAdd(&all[6], d3);
+    if (big) atomicAdd(&all[7], big);
+    if (pair) atomicMax(&all[8], (unsigned long long)pair);
+    if (most) atomicMax(&all[9], (unsigned long long)most);
+  }
+  __syncthreads();
+  if (threadIdx.x < kSums && all[threadIdx.x]) {
+    if (threadIdx.x < 8) atomicAdd(&sums[threadIdx.x], all[threadIdx.x]);
+    else atomicMax(&sums[threadIdx.x], all[threadIdx.x]);
   }
 }
 
@@ -2039,8 +2054,12 @@ static int build_decomp(hm_graph* g, Decomp& P, const uint8_t* mark, uint32_t ma
                                                                     g->esize.p, mark, V, even, P.ncat.p, P.ncat_m.p,
                                                                     reinterpret_cast<float*>(sums.p + kSums));
   HM_LAUNCH_CHECK();
-  k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p,
-                                                                      g->h2h_ovl.p, g->esize.p, mark, E, heavy.p, ids.p, sums.p);
+  // a heavy pair's 16 ns |a| |b| below 9 us, or a hundredth of the other way's least
+  // time (sum d^2 >= nnz^2 / n), cannot decide
+  const double least = mark ? 0.003 * (double)cost : 0.0011 * (double)g->h2h_nnz * (double)g->h2h_nnz / E;
+  const uint32_t large_pair = (uint32_t)std::min(65025.0, std::max(576.0, 0.01 * least / 16));
+  k_heavy_count<<<grid_for((uint64_t)E * 32, kBlock), kBlock, 0, st>>>(
+      g->h2h_off.p, g->h2h_len.p, g->h2h_nbr.p, g->h2h_ovl.p, g->esize.p, mark, E, large_pair, heavy.p, ids.p, sums.p);
   HM_LAUNCH_CHECK();
   const unsigned bits = bits_for(E);
   {
